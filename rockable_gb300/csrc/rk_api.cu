@@ -862,7 +862,7 @@ void rk_destroy(rk_ctx* x) {
   free_entrybuf(c.eb[0]);
   free_entrybuf(c.eb[1]);
   NLWork& w = c.w;
-  dfree(w.pairs); dfree(w.hp); dfree(w.hp_tmp); dfree(w.hp_mask); dfree(w.cand); dfree(w.cand_tmp);
+  dfree(w.pairs); dfree(w.hp); dfree(w.hp_tmp); dfree(w.hp_mask); dfree(w.cand); dfree(w.cand_tmp); dfree(w.cand_unsure);
   dfree(w.flag); dfree(w.stale); dfree(w.stale_src); dfree(w.fkey); dfree(w.fsrc); dfree(w.jkeys); dfree(w.jtmp);
   dfree(w.tmp); dfree(w.counter); dfree(w.gkeys); dfree(w.gtmp); dfree(w.gover); dfree(w.gis_over); dfree(w.gmark);
   if (w.gstat) cudaFree(w.gstat);
@@ -907,6 +907,7 @@ int rk_upload_shapes(rk_ctx* x, const rk_shapes* sh) {
   c.shape_nv.assign(ns, 0);
   c.shape_ne.assign(ns, 0);
   c.shape_nf.assign(ns, 0);
+  c.max_nv = c.max_ne = c.max_nf = 0;
   for (int k = 0; k < ns; k++) {
     int v = sh->vert_ofs[k + 1] - sh->vert_ofs[k];
     int e = sh->edge_ofs[k + 1] - sh->edge_ofs[k];
@@ -916,6 +917,9 @@ int rk_upload_shapes(rk_ctx* x, const rk_shapes* sh) {
     c.shape_nv[k] = v;
     c.shape_ne[k] = e;
     c.shape_nf[k] = f;
+    c.max_nv = std::max(c.max_nv, v);
+    c.max_ne = std::max(c.max_ne, e);
+    c.max_nf = std::max(c.max_nf, f);
   }
   c.shape_vmax.assign(ns, 0.0);
   for (int k = 0; k < ns; k++)

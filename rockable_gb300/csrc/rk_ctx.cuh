@@ -32,6 +32,7 @@ struct NLWork {
   uint32_t* hp_mask = nullptr;   // kMaskWords * hp_cap
   uint64_t* cand = nullptr;      // cand_cap new entry keys
   uint64_t* cand_tmp = nullptr;  // cand_cap (sort)
+  uint32_t* cand_unsure = nullptr;  // cand_cap: positions of the keys the float classification left undecided
   int64_t cand_hint = 0;         // candidates found by the previous rebuild
   int64_t* flag = nullptr;       // old_cap + 1
   uint64_t* stale = nullptr;     // old_cap
@@ -122,6 +123,7 @@ struct Ctx {
   std::vector<int> shape_nv;  // vertices per shape
   std::vector<double> shape_radius;
   std::vector<int> shape_ne, shape_nf;
+  int max_nv = 0, max_ne = 0, max_nf = 0;  // largest counts of one shape
   std::vector<double> shape_vmax;      // largest vertex distance from the shape centre
   std::vector<int> body_shape;
   std::vector<double> body_hom;

@@ -15,9 +15,9 @@
 //
 // Pipeline (all on the context stream, a few host reads of counts):
 //   body_obb -> pairs (all-pairs AABB filter or uniform grid, then the FP64
-//   SAT) -> half-pairs (both directions, radix-sorted) -> candidates (one
-//   warp per half-pair: cull mask, NEAR keys appended) -> key sort -> old-entry
-//   classification and order-preserving compaction -> merge by key ->
+//   SAT) -> half-pairs (both directions, radix-sorted) -> cull mask ->
+//   candidates (one warp per half-pair: NEAR keys appended) -> FP64 predicate
+//   of the undecided ones -> key sort -> old-entry classification and order-preserving compaction -> merge by key ->
 //   history carry -> i-side offsets and j-side list.
 #include <algorithm>
 #include <cstdio>
@@ -800,22 +800,25 @@ __device__ __forceinline__ int classify_vf(const Scene& s, const float4* sp, int
   return classify_vf_tri(p, gpt(sp[fv[0]]), gpt(sp[fv[1]]), gpt(sp[fv[2]]), alim, mag);
 }
 
-// the float class decides unless it is 0
-#define RK_DECIDE(cls, exact) ([&] { const int c_ = (cls); return c_ > 0 || (c_ == 0 && (exact)); }())
-
 // Candidate sub-contacts of the half-pairs: one warp per half-pair (owner b
-// -> partner p).  The lanes first compute, in parallel, the owner vertices
-// that pass the OBB cull (FP64 SAT of the vertex cube against p's box
-// enlarged by dVerlet; this mask also tells the old-entry pass which
-// candidates were tested) and the sub-elements of each body that a
-// conservative float bounding-sphere test leaves within reach of the other
-// body; those index lists go to shared memory.  The lanes then sweep the
-// products of the lists 32 candidates at a time: float sphere prefilter,
-// then the FP64 NEAR predicate, and the survivors are appended with one
-// atomic per warp and ballot.  Appending leaves the keys unordered; they are
-// sorted afterwards.  The float tests only skip candidates that cannot be
-// NEAR, so the NEAR set is exactly the one of testing every candidate.
+// -> partner p).  The lanes first narrow both bodies down to the
+// sub-elements that can be near the other one (a separating slab between the
+// two cores, the other body's box and bounding sphere; index lists in shared
+// memory; k_cull_mask gave the owner vertices that pass Rockable's OBB cull),
+// then sweep the products of the lists 32 candidates at a time: float sphere
+// prefilter, then the float classification of the NEAR predicate, and what
+// it accepts or leaves undecided is appended with one atomic per warp and
+// ballot; k_near_exact runs the FP64 predicate on the undecided ones.
+// Appending leaves the half-pairs unordered; the keys are sorted afterwards.
+// The float tests only skip candidates that cannot be NEAR, so the NEAR set
+// is exactly the one of testing every candidate.
+// Measured on the packed column of 50 000 grains (1.6 M entries): 7.92 ms
+// with the vertex cull and the FP64 predicates inlined and no slab, 6.8 ms
+// with the slab, 3.14 ms split (plus 0.60 ms k_cull_mask, 0.065 ms
+// k_near_exact); bound by the instruction stream (1.8 G warp instructions).
 constexpr int kCandWarps = 4;  // warps per block
+// counters of a candidate pass, after the number of keys: undecided candidates, those the FP64 predicate rejected
+constexpr int kCandUnsure = 2, kCandRejected = 3;
 
 // Root-versus-leaf test of the two-level pruning: true when a sub-element
 // sphere (centre, radius in .w) lies farther than `reach` from the other
@@ -853,10 +856,95 @@ __device__ __noinline__ bool cull_fp64(const double* obb, double dmax, const dou
   return obb_intersect(op, sub);
 }
 
+// One warp's lists in dynamic shared memory, sized by the shapes' largest
+// vertex, edge and face counts (fixed 1024-entry lists held the kernel to 4
+// blocks per SM): the vertices' coordinates along the pair's separating
+// direction, owner / partner vertices, owner edges, partner edges and faces.
 struct CandLists {
-  uint16_t bv[64], pv[64];                   // owner / partner vertices
-  uint16_t be[kMaxSub], pe[kMaxSub], pf[kMaxSub];  // owner edges, partner edges and faces
+  float *bproj, *pproj;
+  uint16_t *bv, *pv, *be, *pe, *pf;
 };
+__host__ __device__ inline size_t cand_list_bytes(int mv, int me, int mf) {
+  return (size_t)((2 * mv * 4 + 2 * (2 * mv + 2 * me + mf) + 15) / 16 * 16);
+}
+__device__ __forceinline__ CandLists cand_lists(char* p, int mv, int me) {
+  CandLists L;
+  L.bproj = reinterpret_cast<float*>(p);
+  L.pproj = L.bproj + mv;
+  L.bv = reinterpret_cast<uint16_t*>(L.pproj + mv);
+  L.pv = L.bv + mv;
+  L.be = L.pv + mv;
+  L.pe = L.be + me;
+  L.pf = L.pe + me;
+  return L;
+}
+
+// Slab between two bodies' cores along one direction: the owner's vertices
+// all lie below bmax, the partner's above pmin (coordinates along the unit
+// direction, relative to the partner's centre; also left per vertex in L).
+struct Slab {
+  float bmax, pmin;
+};
+
+__device__ __forceinline__ unsigned int slab_ord(float f) {
+  const unsigned int u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// A direction that separates the vertices of b and p about as far as their
+// hulls are apart, by Gilbert's algorithm on the hulls' difference, the whole
+// warp on one pair: each step takes the two hulls' extreme vertices along the
+// current difference v (a lane per vertex, warp-wide integer min / max
+// reductions of ordered float bits) and moves v to the point of the segment
+// towards their difference that is nearest the origin.  Any direction gives
+// a valid slab; a few steps make it tight enough for the pruning, and the
+// search stops once the gap exceeds `enough` (no sub-element can be near).
+__device__ __forceinline__ Slab pair_slab(const float4* sb, int nvb, const float4* sp, int nvp, G3 cb, G3 cp,
+                                          float enough, float tol, int lane, const CandLists& L) {
+  const unsigned full = 0xffffffffu;
+  const int b0 = min(lane, nvb - 1), b1 = min(lane + 32, nvb - 1), p0 = min(lane, nvp - 1), p1 = min(lane + 32, nvp - 1);
+  const G3 xb0 = gsub(gpt(sb[b0]), cp), xp0 = gsub(gpt(sp[p0]), cp);
+  G3 xb1 = xb0, xp1 = xp0;
+  if (nvb > 32) xb1 = gsub(gpt(sb[b1]), cp);
+  if (nvp > 32) xp1 = gsub(gpt(sp[p1]), cp);
+  G3 v = gsub(cp, cb), dir = {0.f, 0.f, 0.f};
+  float best = -3.0e38f;
+  Slab S = {3.0e38f, -3.0e38f};
+  for (int it = 0; it < 12; it++) {
+    const float v2 = gdot(v, v);
+    if (!(v2 > 1e-20f)) break;
+    const float inv = rsqrtf(v2);
+    const G3 d = {v.x * inv, v.y * inv, v.z * inv};
+    const float tb0 = gdot(xb0, d), tb1 = gdot(xb1, d), tp0 = gdot(xp0, d), tp1 = gdot(xp1, d);
+    const bool ub = tb1 > tb0, up = tp1 < tp0;
+    const unsigned ob = slab_ord(ub ? tb1 : tb0), op = slab_ord(up ? tp1 : tp0);
+    const unsigned mb = __reduce_max_sync(full, ob), mp = __reduce_min_sync(full, op);
+    const int lb = __ffs(__ballot_sync(full, ob == mb)) - 1, lp = __ffs(__ballot_sync(full, op == mp)) - 1;
+    const float bmax = __shfl_sync(full, ub ? tb1 : tb0, lb), pmin = __shfl_sync(full, up ? tp1 : tp0, lp);
+    if (pmin - bmax > best) {
+      best = pmin - bmax;
+      S.bmax = bmax;
+      S.pmin = pmin;
+      dir = d;
+    }
+    const float len = v2 * inv;
+    if (best > enough || len - best < tol) break;
+    const G3 eb = ub ? xb1 : xb0, ep = up ? xp1 : xp0;
+    const G3 w = {__shfl_sync(full, ep.x, lp) - __shfl_sync(full, eb.x, lb),
+                  __shfl_sync(full, ep.y, lp) - __shfl_sync(full, eb.y, lb),
+                  __shfl_sync(full, ep.z, lp) - __shfl_sync(full, eb.z, lb)};
+    const G3 vw = gsub(v, w);
+    const float l2 = gdot(vw, vw);
+    if (!(l2 > 1e-20f)) break;
+    v = gmad(v, -clamp01(gdot(v, vw) / l2), vw);
+  }
+  if (lane < nvb) L.bproj[lane] = gdot(xb0, dir);
+  if (lane + 32 < nvb) L.bproj[lane + 32] = gdot(xb1, dir);
+  if (lane < nvp) L.pproj[lane] = gdot(xp0, dir);
+  if (lane + 32 < nvp) L.pproj[lane + 32] = gdot(xp1, dir);
+  __syncwarp();
+  return S;
+}
 
 // Indices k < n with pred(k), in increasing order, written by the warp.
 template <class Pred>
@@ -873,152 +961,157 @@ __device__ __forceinline__ int warp_list(uint16_t* list, int n, int lane, Pred p
   return cnt;
 }
 
-__device__ __forceinline__ void warp_emit(bool ok, uint64_t key, int lane, uint64_t* out, int64_t cap,
-                                          unsigned long long* counter) {
+// Which owner vertices of a half-pair (b -> p) pass Rockable's OBB cull
+// (Rockable.cpp:1385-1391: the vertex cube against the partner's OBB enlarged
+// by dVerlet); the mask also tells the old-entry pass which candidates were
+// tested.  16 lanes per half-pair, a lane per vertex.
+// Float pre-test of the fifteen axes of the separating-axis test (the
+// partner box's axes, the cube's -- the world axes -- and their cross
+// products): separated along one by more than the rounding margin -> the
+// FP64 test is false as well; the vertex inside the box shrunk by the margin,
+// or an overlap by more than the margin along all fifteen -> the FP64 test is
+// true as well; only the cases in between run the FP64 test, so the mask is
+// the FP64 test's.  With the distance-only tests (GEOM) a conservative float
+// test does (a vertex out of reach of the partner's bounding sphere), since
+// an untested candidate only keeps its old entry.
+template <bool GEOM>
+__global__ void __launch_bounds__(128) k_cull_mask(Scene s, const uint64_t* hp, int64_t nhp, uint32_t* mask) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t h = t >> 4;
+  const int l = (int)(t & 15), shift = threadIdx.x & 16;
+  const bool live = h < nhp;
+  const uint64_t key = live ? hp[h] : 0ull;
+  const int b = (int)(key >> 21), p = (int)(key & ((1u << 21) - 1));
+  const int sh = s.shape[b];
+  const int nvb = live ? s.vert_ofs[sh + 1] - s.vert_ofs[sh] : 0;
+  const float4* sbv = s.sph + s.sph_ofs[b];
+  const float dmax = d2f(s.dVerlet), fr = d2f(s.rad[b] + s.dVerlet);
+  const float* of = s.bobbf + 15 * (int64_t)p;
+  const float4 cpp = make_float4(d2f(s.pos[3 * (int64_t)p]), d2f(s.pos[3 * (int64_t)p + 1]),
+                                 d2f(s.pos[3 * (int64_t)p + 2]), s.bnd[p]);
+  const float reach = d2f(s.rad[b] + s.rad[p] + s.dVerlet);
+  const float fe[3][3] = {{of[3], of[4], of[5]}, {of[6], of[7], of[8]}, {of[9], of[10], of[11]}};
+  const float fext[3] = {of[12] + dmax, of[13] + dmax, of[14] + dmax};
+  const float mag = fmaxf(fmaxf(fabsf(of[0]), fabsf(of[1])), fabsf(of[2])) + fext[0] + fext[1] + fext[2] + fr;
+  uint32_t m[2] = {0u, 0u};
+  int rounds = (nvb + 15) >> 4;
+  rounds = max(rounds, __shfl_xor_sync(0xffffffffu, rounds, 16));
+  for (int it = 0; it < rounds; it++) {
+    const int v = 16 * it + l;
+    bool hit = false;
+    if (v < nvb) {
+      const float4 pv = sbv[v];
+      if (GEOM) {
+        const float dx = pv.x - cpp.x, dy = pv.y - cpp.y, dz = pv.z - cpp.z;
+        const float mg = fmaxf(fmaxf(fmaxf(fabsf(cpp.x), fabsf(cpp.y)), fabsf(cpp.z)) + cpp.w,
+                               fmaxf(fmaxf(fabsf(pv.x), fabsf(pv.y)), fabsf(pv.z)));
+        float lim = reach + cpp.w;
+        lim = lim + 1e-4f * lim + 1e-6f * mg + 2e-6f;
+        hit = dx * dx + dy * dy + dz * dz <= lim * lim;
+      } else {
+        const float dw[3] = {pv.x - of[0], pv.y - of[1], pv.z - of[2]};
+        bool out = false, in = true, clear = true;
+        float tb[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {  // the box's axes
+          tb[i] = dw[0] * fe[i][0] + dw[1] * fe[i][1] + dw[2] * fe[i][2];
+          const float tt = fabsf(tb[i]);
+          const float lim = fext[i] + fr * (fabsf(fe[i][0]) + fabsf(fe[i][1]) + fabsf(fe[i][2]));
+          const float mm = 1e-6f * (mag + tt) + 1e-9f;
+          out = out || tt > lim + mm;
+          in = in && tt < fext[i] - mm;
+          clear = clear && tt < lim - mm;
+        }
+        if (!out && !in) {
+          const float mm = 1e-6f * mag + 1e-9f, mc = 4e-6f * mag + 1e-9f;
+#pragma unroll
+          for (int j = 0; j < 3; j++) {  // the world axes
+            const float tt = fabsf(dw[j]);
+            const float lim = fext[0] * fabsf(fe[0][j]) + fext[1] * fabsf(fe[1][j]) + fext[2] * fabsf(fe[2][j]) + fr;
+            out = out || tt > lim + mm;
+            clear = clear && tt < lim - mm;
+          }
+#pragma unroll
+          for (int i = 0; i < 3; i++) {  // box axis i x world axis j
+            const int i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+              const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
+              const float tt = fabsf(tb[i2] * fe[i1][j] - tb[i1] * fe[i2][j]);
+              const float lim = fext[i1] * fabsf(fe[i2][j]) + fext[i2] * fabsf(fe[i1][j]) +
+                                fr * (fabsf(fe[i][j2]) + fabsf(fe[i][j1]));
+              out = out || tt > lim + mc;
+              clear = clear && tt < lim - mc;
+            }
+          }
+        }
+        if (out) hit = false;
+        else if (in || clear) hit = true;
+        else hit = cull_fp64(s.bobb + 15 * (int64_t)p, s.dVerlet, s.gv + 3 * s.gv_ofs[b], v, s.rad[b] + s.dVerlet);
+      }
+    }
+    const uint32_t bits = (__ballot_sync(0xffffffffu, hit) >> shift) & 0xffffu;
+    if (it < 2) m[0] |= bits << (16 * (it & 1));
+    else m[1] |= bits << (16 * (it & 1));
+  }
+  if (live && l == 0) {
+    mask[kMaskWords * h] = m[0];
+    mask[kMaskWords * h + 1] = m[1];
+  }
+}
+
+// Appends the keys of the lanes with ok; those the float classification left
+// undecided (unsure) are also listed by their position, for k_near_exact.
+__device__ __forceinline__ void warp_emit(bool ok, bool unsure, uint64_t key, int lane, uint64_t* out, uint32_t* unc,
+                                          int64_t cap, unsigned long long* counter) {
   const unsigned bal = __ballot_sync(0xffffffffu, ok);
   if (!bal) return;
   unsigned long long base = 0;
   if (lane == 0) base = atomicAdd(counter, (unsigned long long)__popc(bal));
   base = __shfl_sync(0xffffffffu, base, 0);
-  if (ok) {
-    const unsigned long long at = base + __popc(bal & ((1u << lane) - 1u));
-    if ((int64_t)at < cap) out[at] = key;
+  const unsigned lt = (1u << lane) - 1u;
+  const unsigned long long at = base + __popc(bal & lt);
+  if (ok && (int64_t)at < cap) out[at] = key;
+  const unsigned un = __ballot_sync(0xffffffffu, ok && unsure);
+  if (!un) return;
+  if (lane == 0) base = atomicAdd(counter + kCandUnsure, (unsigned long long)__popc(un));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (ok && unsure) {
+    const unsigned long long u = base + __popc(un & lt);
+    if ((int64_t)u < cap) unc[u] = (uint32_t)at;
   }
 }
 
-// The FP64 variant asks for 4 blocks per SM (128 registers, a few spills to
-// L1) instead of 3 at 166 registers: it is latency-bound.
+// Float only: the FP64 predicates of the undecided candidates run in
+// k_near_exact.  Inlined here they made the kernel's code too large for the
+// instruction caches (more than half of its stall cycles were instruction
+// fetches) and held it to 128 registers.
 template <bool GEOM>
-__global__ void __launch_bounds__(32 * kCandWarps, GEOM ? 1 : 4)
-k_candidates(Scene s, const uint64_t* hp, int64_t nhp, uint32_t* mask, uint64_t* out, int64_t cap,
-             unsigned long long* counter) {
-  __shared__ CandLists lists[kCandWarps];
+__global__ void __launch_bounds__(32 * kCandWarps)
+k_candidates(Scene s, const uint64_t* hp, int64_t nhp, const uint32_t* mask, int mv, int me, int mf, uint64_t* out,
+             uint32_t* unc, int64_t cap, unsigned long long* counter) {
+  extern __shared__ __align__(16) char list_mem[];
   const int lane = threadIdx.x & 31;
-  CandLists& L = lists[threadIdx.x >> 5];
+  const CandLists L = cand_lists(list_mem + (threadIdx.x >> 5) * cand_list_bytes(mv, me, mf), mv, me);
   const int64_t stride = (int64_t)gridDim.x * kCandWarps;
   for (int64_t h = (int64_t)blockIdx.x * kCandWarps + (threadIdx.x >> 5); h < nhp; h += stride) {
     __syncwarp();  // the previous half-pair's lists have been read
     const uint64_t key = hp[h];
     const int b = (int)(key >> 21), p = (int)(key & ((1u << 21) - 1));
-    PairView P;
-    P.gb = s.gv + 3 * s.gv_ofs[b];
-    P.gp = s.gv + 3 * s.gv_ofs[p];
-    P.sb = s.shape[b];
-    P.sp = s.shape[p];
-    P.Rb = s.rad[b];
-    P.Rp = s.rad[p];
-    P.dmax = s.dVerlet;
-    const int nvb = s.vert_ofs[P.sb + 1] - s.vert_ofs[P.sb];
-    const int nvp = s.vert_ofs[P.sp + 1] - s.vert_ofs[P.sp];
-    const int neb = s.edge_ofs[P.sb + 1] - s.edge_ofs[P.sb];
-    const int nep = s.edge_ofs[P.sp + 1] - s.edge_ofs[P.sp];
-    const int nfp = s.face_ofs[P.sp + 1] - s.face_ofs[P.sp];
-    // owner-vertex cull (Rockable.cpp:1385-1391): the vertex cube against
-    // the partner's OBB enlarged by dVerlet.  With the distance-only tests a
-    // conservative float test does (a vertex out of reach of the partner's
-    // bounding sphere), since an untested candidate only keeps its old entry.
-    uint32_t m0, m1;
-    if (GEOM) {
-      const float4* sbv = s.sph + s.sph_ofs[b];
-      const float4 cpp = make_float4(d2f(s.pos[3 * p]), d2f(s.pos[3 * p + 1]), d2f(s.pos[3 * p + 2]), s.bnd[p]);
-      const float reach = d2f(P.Rb + P.Rp + P.dmax);
-      bool hit0 = false, hit1 = false;
-      for (int half = 0; half < 2; half++) {
-        const int v = lane + 32 * half;
-        if (v < nvb) {
-          const float4 a = sbv[v];
-          const float dx = a.x - cpp.x, dy = a.y - cpp.y, dz = a.z - cpp.z;
-          const float mg = fmaxf(fmaxf(fmaxf(fabsf(cpp.x), fabsf(cpp.y)), fabsf(cpp.z)) + cpp.w,
-                                 fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)));
-          float lim = reach + cpp.w;
-          lim = lim + 1e-4f * lim + 1e-6f * mg + 2e-6f;
-          const bool hit = dx * dx + dy * dy + dz * dz <= lim * lim;
-          if (half == 0) hit0 = hit;
-          else hit1 = hit;
-        }
-      }
-      m0 = __ballot_sync(0xffffffffu, hit0);
-      m1 = __ballot_sync(0xffffffffu, hit1);
-    } else {
-      Obb op = load_obb(s.bobb + 15 * p);
-      enlarge(op, P.dmax);
-      const double r = P.Rb + P.dmax;
-      // Float pre-test of the fifteen axes of the separating-axis test (the
-      // partner box's axes, the cube's -- the world axes -- and their
-      // cross products): separated along one by more than the rounding
-      // margin -> the FP64 test is false as well; the vertex inside the box
-      // shrunk by the margin, or an overlap by more than the margin along
-      // all fifteen -> the FP64 test is true as well; only the cases in
-      // between run the FP64 test, so the mask is unchanged.
-      const float fcx = d2f(op.c.x), fcy = d2f(op.c.y), fcz = d2f(op.c.z);
-      const float fe[3][3] = {{d2f(op.e0.x), d2f(op.e0.y), d2f(op.e0.z)},
-                              {d2f(op.e1.x), d2f(op.e1.y), d2f(op.e1.z)},
-                              {d2f(op.e2.x), d2f(op.e2.y), d2f(op.e2.z)}};
-      const float fext[3] = {d2f(op.ext.x), d2f(op.ext.y), d2f(op.ext.z)};
-      const float fr = d2f(r);
-      const float4* sbv = s.sph + s.sph_ofs[b];
-      const float mag = fmaxf(fmaxf(fabsf(fcx), fabsf(fcy)), fabsf(fcz)) + fext[0] + fext[1] + fext[2] + fr;
-      bool hit0 = false, hit1 = false;
-      for (int half = 0; half < 2; half++) {
-        const int v = lane + 32 * half;
-        if (v < nvb) {
-          const float4 pv = sbv[v];
-          const float dw[3] = {pv.x - fcx, pv.y - fcy, pv.z - fcz};
-          bool out = false, in = true, clear = true;
-          float tb[3];
-          for (int i = 0; i < 3; i++) {  // the box's axes
-            tb[i] = dw[0] * fe[i][0] + dw[1] * fe[i][1] + dw[2] * fe[i][2];
-            const float t = fabsf(tb[i]);
-            const float lim = fext[i] + fr * (fabsf(fe[i][0]) + fabsf(fe[i][1]) + fabsf(fe[i][2]));
-            const float m = 1e-6f * (mag + t) + 1e-9f;
-            out = out || t > lim + m;
-            in = in && t < fext[i] - m;
-            clear = clear && t < lim - m;
-          }
-          if (!out && !in) {
-            const float m = 1e-6f * mag + 1e-9f, mc = 4e-6f * mag + 1e-9f;
-            for (int j = 0; j < 3; j++) {  // the world axes
-              const float t = fabsf(dw[j]);
-              const float lim = fext[0] * fabsf(fe[0][j]) + fext[1] * fabsf(fe[1][j]) + fext[2] * fabsf(fe[2][j]) + fr;
-              out = out || t > lim + m;
-              clear = clear && t < lim - m;
-            }
-            for (int i = 0; i < 3; i++) {  // box axis i x world axis j
-              const int i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
-              for (int j = 0; j < 3; j++) {
-                const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
-                const float t = fabsf(tb[i2] * fe[i1][j] - tb[i1] * fe[i2][j]);
-                const float lim = fext[i1] * fabsf(fe[i2][j]) + fext[i2] * fabsf(fe[i1][j]) +
-                                  fr * (fabsf(fe[i][j2]) + fabsf(fe[i][j1]));
-                out = out || t > lim + mc;
-                clear = clear && t < lim - mc;
-              }
-            }
-          }
-          bool hit;
-          if (out) {
-            hit = false;
-          } else if (in || clear) {
-            hit = true;
-          } else {
-            hit = cull_fp64(s.bobb + 15 * p, P.dmax, P.gb, v, r);
-          }
-          if (half == 0) hit0 = hit;
-          else hit1 = hit;
-        }
-      }
-      m0 = __ballot_sync(0xffffffffu, hit0);
-      m1 = __ballot_sync(0xffffffffu, hit1);
-    }
-    if (lane == 0) {
-      mask[kMaskWords * h] = m0;
-      mask[kMaskWords * h + 1] = m1;
-    }
+    const int shb = s.shape[b], shp = s.shape[p];
+    const double Rb = s.rad[b], Rp = s.rad[p], dmax = s.dVerlet;
+    const int nvb = s.vert_ofs[shb + 1] - s.vert_ofs[shb];
+    const int nvp = s.vert_ofs[shp + 1] - s.vert_ofs[shp];
+    const int ob0 = s.edge_ofs[shb], op0 = s.edge_ofs[shp];
+    const int neb = s.edge_ofs[shb + 1] - ob0;
+    const int nep = s.edge_ofs[shp + 1] - op0;
+    const int nfp = s.face_ofs[shp + 1] - s.face_ofs[shp];
+    const uint32_t m0 = mask[kMaskWords * h], m1 = mask[kMaskWords * h + 1];
     // conservative float filter: a candidate whose bounding spheres are
     // farther apart than the NEAR distance allows cannot be NEAR
     const float4* sb = s.sph + s.sph_ofs[b];
     const float4* sp = s.sph + s.sph_ofs[p];
-    const float sum = d2f(P.Rb + P.Rp + P.dmax);
+    const float sum = d2f(Rb + Rp + dmax);
     const float4 cb = make_float4(d2f(s.pos[3 * b]), d2f(s.pos[3 * b + 1]), d2f(s.pos[3 * b + 2]), s.bnd[b]);
     const float4 cp = make_float4(d2f(s.pos[3 * p]), d2f(s.pos[3 * p + 1]), d2f(s.pos[3 * p + 2]), s.bnd[p]);
     // margin for the float rounding of coordinates of magnitude up to `mag`
@@ -1032,11 +1125,11 @@ k_candidates(Scene s, const uint64_t* hp, int64_t nhp, uint32_t* mask, uint64_t*
       lim = lim + 1e-4f * lim + slack;
       return dx * dx + dy * dy + dz * dz > lim * lim;
     };
-    const float ve_ext = d2f(1.0 + 2.0 * P.dmax);
+    const float ve_ext = d2f(1.0 + 2.0 * dmax);
     const float glim = sum + 1e-4f * sum + slack;
     const float glim2 = glim * glim;
     const float alim = sum - (1e-4f * sum + slack);  // float acceptance: the NEAR distance shrunk by the margin
-    const float dmaxf = d2f(P.dmax);
+    const float dmaxf = d2f(dmax);
     const bool lower = b < p;  // vertex-vertex and edge-edge pairs are tested in the i < j direction only
     // Two-level pruning (the role of Rockable's per-shape OBB trees,
     // Rockable.cpp:1440-1541, Shape.cpp:628-670): a sub-element stays in
@@ -1050,29 +1143,47 @@ k_candidates(Scene s, const uint64_t* hp, int64_t nhp, uint32_t* mask, uint64_t*
     // beyond their ends (the vertex-edge projection test), so its reach
     // grows by that much (an edge is at most the partner's diameter long)
     const float vreach = sum + 2.f * dmaxf * cp.w;
+    // First the slab between the two cores along a separating direction: an
+    // element beyond the NEAR distance from the other core's side of it is
+    // farther than that from all of the other body's elements.  Two hulls in
+    // touch keep the few elements within dVerlet of the plane between them
+    // (the boxes and spheres, kept as second tests, leave most of the facing
+    // half), and a pair whose gap exceeds the NEAR distance keeps none.
+    const float slim = vreach + 1e-4f * vreach + slack;
+    const Slab S = pair_slab(sb, nvb, sp, nvp, gpt(cb), gpt(cp), slim, 0.05f * sum, lane, L);
+    if (S.pmin - S.bmax > slim) continue;
+    const float blow = S.pmin - slim, phigh = S.bmax + slim;
     const int nbv = warp_list(L.bv, nvb, lane, [&](int v) {
-      return (((v < 32 ? m0 : m1) >> (v & 31)) & 1u) != 0u && !box_far(bxp, sb[v], vreach, slack);
+      return (((v < 32 ? m0 : m1) >> (v & 31)) & 1u) != 0u && L.bproj[v] >= blow && !box_far(bxp, sb[v], vreach, slack);
     });
     const int npv = lower ? warp_list(L.pv, nvp, lane, [&](int w) {
-      return !far(sp[w], cb, cb.w) && !box_far(bxb, sp[w], sum, slack);
+      return L.pproj[w] <= phigh && !far(sp[w], cb, cb.w) && !box_far(bxb, sp[w], sum, slack);
     }) : 0;
     const int npe = warp_list(L.pe, nep, lane, [&](int e) {
+      const int* ev = s.edges + 2 * (op0 + e);
+      if (fminf(L.pproj[ev[0]], L.pproj[ev[1]]) > phigh) return false;
       const float4 se = sp[nvp + e];
       const float4 sx = make_float4(se.x, se.y, se.z, ve_ext * se.w);  // the vertex-edge test's extended edge
       return !far(se, cb, cb.w + sx.w) && !box_far(bxb, sx, sum, slack);
     });
     const int npf = warp_list(L.pf, nfp, lane, [&](int f) {
+      const int fo = s.face_ofs[shp] + f;
+      float low = 3.0e38f;
+      for (int q = s.face_vofs[fo]; q < s.face_vofs[fo + 1]; q++) low = fminf(low, L.pproj[s.face_verts[q]]);
+      if (low > phigh) return false;
       const float4 sf = sp[nvp + nep + f];
       return !far(sf, cb, cb.w + sf.w) && !box_far(bxb, sf, sum, slack);
     });
     const int nbe = lower ? warp_list(L.be, neb, lane, [&](int e) {
+      const int* ev = s.edges + 2 * (ob0 + e);
+      if (fmaxf(L.bproj[ev[0]], L.bproj[ev[1]]) < blow) return false;
       const float4 se = sb[nvb + e];
       return !far(se, cp, cp.w + se.w) && !box_far(bxp, se, sum, slack);
     }) : 0;
     // vertex-vertex
     for (int base = 0, tot = nbv * npv; base < tot; base += 32) {
       const int c = base + lane;
-      bool ok = false;
+      bool ok = false, unsure = false;
       int v = 0, w = 0;
       if (c < tot) {
         v = L.bv[c / npv];
@@ -1081,55 +1192,62 @@ k_candidates(Scene s, const uint64_t* hp, int64_t nhp, uint32_t* mask, uint64_t*
           const G3 d = gsub(gpt(sb[v]), gpt(sp[w]));
           ok = gdot(d, d) <= glim2;
         } else {
-          ok = !far(sb[v], sp[w], 0.f) && (accept_vv(gpt(sb[v]), gpt(sp[w]), alim) || near_vv(P, v, w));
+          ok = !far(sb[v], sp[w], 0.f);
+          unsure = !accept_vv(gpt(sb[v]), gpt(sp[w]), alim);
         }
       }
-      warp_emit(ok, entry_key((uint32_t)b, (uint32_t)p, 0u, (uint32_t)v, (uint32_t)w), lane, out, cap, counter);
+      warp_emit(ok, unsure, entry_key((uint32_t)b, (uint32_t)p, 0u, (uint32_t)v, (uint32_t)w), lane, out, unc, cap, counter);
     }
     // vertex-edge
     for (int base = 0, tot = nbv * npe; base < tot; base += 32) {
       const int c = base + lane;
-      bool ok = false;
+      bool ok = false, unsure = false;
       int v = 0, e = 0;
       if (c < tot) {
         v = L.bv[c / npe];
         e = L.pe[c % npe];
         const float4 se = sp[nvp + e];
         if (GEOM) {
-          const int eo = s.edge_ofs[P.sp] + e;
+          const int eo = s.edge_ofs[shp] + e;
           ok = !far(sb[v], se, se.w) &&
                pt_seg_d2(gpt(sb[v]), gpt(sp[s.edges[2 * eo]]), gpt(sp[s.edges[2 * eo + 1]])) <= glim2;
         } else {
           // exact rejection first: Rockable's vertex-edge test accepts a
           // projection slightly off the edge, never a line distance above it
-          const int eo = s.edge_ofs[P.sp] + e;
+          const int eo = s.edge_ofs[shp] + e;
           const G3 pv = gpt(sb[v]), e0 = gpt(sp[s.edges[2 * eo]]), e1 = gpt(sp[s.edges[2 * eo + 1]]);
-          ok = !far(sb[v], se, ve_ext * se.w) && pt_line_d2(pv, e0, e1) <= glim2 &&
-               RK_DECIDE(classify_ve(pv, e0, e1, alim, dmaxf, mag), near_ve(s, P, v, e));
+          if (!far(sb[v], se, ve_ext * se.w) && pt_line_d2(pv, e0, e1) <= glim2) {
+            const int c_ = classify_ve(pv, e0, e1, alim, dmaxf, mag);
+            ok = c_ >= 0;
+            unsure = c_ == 0;
+          }
         }
       }
-      warp_emit(ok, entry_key((uint32_t)b, (uint32_t)p, 1u, (uint32_t)v, (uint32_t)e), lane, out, cap, counter);
+      warp_emit(ok, unsure, entry_key((uint32_t)b, (uint32_t)p, 1u, (uint32_t)v, (uint32_t)e), lane, out, unc, cap, counter);
     }
     // vertex-face
     for (int base = 0, tot = nbv * npf; base < tot; base += 32) {
       const int c = base + lane;
-      bool ok = false;
+      bool ok = false, unsure = false;
       int v = 0, f = 0;
       if (c < tot) {
         v = L.bv[c / npf];
         f = L.pf[c % npf];
         const float4 sf = sp[nvp + nep + f];
-        if (GEOM) ok = !far(sb[v], sf, sf.w) && pt_poly_d2(s, sp, P.sp, f, gpt(sb[v])) <= glim2;
-        else  // exact rejection first: NEAR needs the polygon within reach
-          ok = !far(sb[v], sf, sf.w) && pt_poly_d2(s, sp, P.sp, f, gpt(sb[v])) <= glim2 &&
-               RK_DECIDE(classify_vf(s, sp, P.sp, f, gpt(sb[v]), alim, mag), near_vf(s, P, v, f));
+        if (GEOM) ok = !far(sb[v], sf, sf.w) && pt_poly_d2(s, sp, shp, f, gpt(sb[v])) <= glim2;
+        else if (!far(sb[v], sf, sf.w) && pt_poly_d2(s, sp, shp, f, gpt(sb[v])) <= glim2) {
+          // (exact rejection first: NEAR needs the polygon within reach)
+          const int c_ = classify_vf(s, sp, shp, f, gpt(sb[v]), alim, mag);
+          ok = c_ >= 0;
+          unsure = c_ == 0;
+        }
       }
-      warp_emit(ok, entry_key((uint32_t)b, (uint32_t)p, 2u, (uint32_t)v, (uint32_t)f), lane, out, cap, counter);
+      warp_emit(ok, unsure, entry_key((uint32_t)b, (uint32_t)p, 2u, (uint32_t)v, (uint32_t)f), lane, out, unc, cap, counter);
     }
     // edge-edge
     for (int base = 0, tot = nbe * npe; base < tot; base += 32) {
       const int c = base + lane;
-      bool ok = false;
+      bool ok = false, unsure = false;
       int e1 = 0, e2 = 0;
       if (c < tot) {
         e1 = L.be[c / npe];
@@ -1138,7 +1256,7 @@ k_candidates(Scene s, const uint64_t* hp, int64_t nhp, uint32_t* mask, uint64_t*
         if (GEOM) {
           // nearly parallel edges (ill-conditioned closest points) within
           // sphere reach are kept: an extra entry is harmless, a missing one not
-          const int ob = s.edge_ofs[P.sb] + e1, op = s.edge_ofs[P.sp] + e2;
+          const int ob = s.edge_ofs[shb] + e1, op = s.edge_ofs[shp] + e2;
           const G3 a0 = gpt(sb[s.edges[2 * ob]]), a1 = gpt(sb[s.edges[2 * ob + 1]]);
           const G3 b0 = gpt(sp[s.edges[2 * op]]), b1 = gpt(sp[s.edges[2 * op + 1]]);
           const G3 d1 = gsub(a1, a0), d2 = gsub(b1, b0), nx = gcross(d1, d2);
@@ -1146,16 +1264,50 @@ k_candidates(Scene s, const uint64_t* hp, int64_t nhp, uint32_t* mask, uint64_t*
           ok = !far(s1, s2, s1.w + s2.w) && (parallel || seg_seg_d2(a0, a1, b0, b1) <= glim2);
         } else {
           // exact rejection first: NEAR needs the edges' lines within reach
-          const int ob = s.edge_ofs[P.sb] + e1, op = s.edge_ofs[P.sp] + e2;
+          const int ob = s.edge_ofs[shb] + e1, op = s.edge_ofs[shp] + e2;
           const G3 a0 = gpt(sb[s.edges[2 * ob]]), a1 = gpt(sb[s.edges[2 * ob + 1]]);
           const G3 b0 = gpt(sp[s.edges[2 * op]]), b1 = gpt(sp[s.edges[2 * op + 1]]);
-          ok = !far(s1, s2, s1.w + s2.w) && !lines_far(a0, a1, b0, b1, glim2) &&
-               RK_DECIDE(classify_ee(a0, a1, b0, b1, alim, mag), near_ee(s, P, e1, e2));
+          if (!far(s1, s2, s1.w + s2.w) && !lines_far(a0, a1, b0, b1, glim2)) {
+            const int c_ = classify_ee(a0, a1, b0, b1, alim, mag);
+            ok = c_ >= 0;
+            unsure = c_ == 0;
+          }
         }
       }
-      warp_emit(ok, entry_key((uint32_t)b, (uint32_t)p, 3u, (uint32_t)e1, (uint32_t)e2), lane, out, cap, counter);
+      warp_emit(ok, unsure, entry_key((uint32_t)b, (uint32_t)p, 3u, (uint32_t)e1, (uint32_t)e2), lane, out, unc, cap, counter);
     }
   }
+}
+
+// The undecided candidates' FP64 NEAR predicate (Particle.cpp:88-209), one
+// thread each: a key that is not NEAR becomes all ones, which the stable
+// sort puts behind every valid key (owner and partner cannot both be the
+// largest index), so that the order the sort relies on is kept.
+__global__ void k_near_exact(Scene s, const uint32_t* unc, int64_t n, uint64_t* keys, unsigned long long* counter) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  bool gone = false;
+  if (k < n) {
+    const uint64_t x = keys[unc[k]];
+    const int b = (int)(x >> 43), p = (int)((x >> 22) & ((1u << 21) - 1));
+    const int t = (int)((x >> 20) & 3u), is = (int)((x >> 10) & 1023u), js = (int)(x & 1023u);
+    PairView P;
+    P.gb = s.gv + 3 * s.gv_ofs[b];
+    P.gp = s.gv + 3 * s.gv_ofs[p];
+    P.sb = s.shape[b];
+    P.sp = s.shape[p];
+    P.Rb = s.rad[b];
+    P.Rp = s.rad[p];
+    P.dmax = s.dVerlet;
+    bool near;
+    if (t == 0) near = near_vv(P, is, js);
+    else if (t == 1) near = near_ve(s, P, is, js);
+    else if (t == 2) near = near_vf(s, P, is, js);
+    else near = near_ee(s, P, is, js);
+    gone = !near;
+    if (gone) keys[unc[k]] = ~0ull;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, gone);
+  if ((threadIdx.x & 31) == 0 && m) atomicAdd(counter + kCandRejected, (unsigned long long)__popc(m));
 }
 
 
@@ -1503,35 +1655,49 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
     c.kernels += 13;
   }
   // ---- candidates: appended by one warp per half-pair, then sorted by key
-  int64_t ncand = 0;
+  int64_t ncand = 0, nunsure = 0;
   if (nhp > 0) {
     const int64_t want = std::max<int64_t>(w.cand_hint, 4 * nhp) + 1024;
     if (w.cand_cap < want) {
       int64_t nc = want + want / 4;
-      if ((rc = grow(c, w.cand, w.cand_cap, nc)) || (rc = grow(c, w.cand_tmp, w.cand_cap, nc))) return rc;
+      if ((rc = grow(c, w.cand, w.cand_cap, nc)) || (rc = grow(c, w.cand_tmp, w.cand_cap, nc)) ||
+          (rc = grow(c, w.cand_unsure, w.cand_cap, nc)))
+        return rc;
       w.cand_cap = nc;
     }
+    if (s.near_geometric) k_cull_mask<true><<<nblk(16 * nhp, 128), 128, 0, st>>>(s, w.hp, nhp, w.hp_mask);
+    else k_cull_mask<false><<<nblk(16 * nhp, 128), 128, 0, st>>>(s, w.hp, nhp, w.hp_mask);
+    c.kernels++;
+    const size_t smem = kCandWarps * cand_list_bytes(c.max_nv, c.max_ne, c.max_nf);
     const unsigned grid = (unsigned)std::min<int64_t>((nhp + kCandWarps - 1) / kCandWarps, 152 * 16);
     for (int attempt = 0; attempt < 4; attempt++) {
-      RKCHK(cudaMemsetAsync(w.counter + 3, 0, 8, st));
+      RKCHK(cudaMemsetAsync(w.counter + 3, 0, 32, st));
       if (s.near_geometric)
-        k_candidates<true><<<grid, 32 * kCandWarps, 0, st>>>(s, w.hp, nhp, w.hp_mask, w.cand, w.cand_cap, w.counter + 3);
+        k_candidates<true><<<grid, 32 * kCandWarps, smem, st>>>(s, w.hp, nhp, w.hp_mask, c.max_nv, c.max_ne, c.max_nf,
+                                                                w.cand, w.cand_unsure, w.cand_cap, w.counter + 3);
       else
-        k_candidates<false><<<grid, 32 * kCandWarps, 0, st>>>(s, w.hp, nhp, w.hp_mask, w.cand, w.cand_cap,
-                                                              w.counter + 3);
+        k_candidates<false><<<grid, 32 * kCandWarps, smem, st>>>(s, w.hp, nhp, w.hp_mask, c.max_nv, c.max_ne, c.max_nf,
+                                                                 w.cand, w.cand_unsure, w.cand_cap, w.counter + 3);
       c.kernels++;
-      unsigned long long cnt = 0;
-      RKCHK(cudaMemcpyAsync(&cnt, w.counter + 3, 8, cudaMemcpyDeviceToHost, st));
+      unsigned long long cnt[kCandUnsure + 1] = {};
+      RKCHK(cudaMemcpyAsync(cnt, w.counter + 3, sizeof cnt, cudaMemcpyDeviceToHost, st));
       RKCHK(cudaStreamSynchronize(st));
-      ncand = (int64_t)cnt;
+      ncand = (int64_t)cnt[0];
+      nunsure = (int64_t)cnt[kCandUnsure];
       if (ncand <= w.cand_cap) break;
       int64_t nc = ncand + ncand / 4 + 1024;
-      if ((rc = grow(c, w.cand, w.cand_cap, nc)) || (rc = grow(c, w.cand_tmp, w.cand_cap, nc))) return rc;
+      if ((rc = grow(c, w.cand, w.cand_cap, nc)) || (rc = grow(c, w.cand_tmp, w.cand_cap, nc)) ||
+          (rc = grow(c, w.cand_unsure, w.cand_cap, nc)))
+        return rc;
       w.cand_cap = nc;
       ncand = -1;
     }
     if (ncand < 0) { c.err = "candidate buffer kept overflowing"; return RK_ERR_CAPACITY; }
     w.cand_hint = ncand + ncand / 8;
+    if (nunsure > 0) {
+      k_near_exact<<<nblk(nunsure, 128), 128, 0, st>>>(s, w.cand_unsure, nunsure, w.cand, w.counter + 3);
+      c.kernels++;
+    }
     if (ncand > 1) {
       if ((rc = ensure_tmp(c, (int64_t)sort_temp_bytes(ncand)))) return rc;
       // A stable sort by (owner, partner) alone orders the keys completely:
@@ -1561,6 +1727,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
     c.kernels += 3;
     nstale = read_i64(c, w.flag + no);
   }
+  if (nunsure > 0) ncand -= read_i64(c, (const int64_t*)(w.counter + 3 + kCandRejected));  // sorted to the end
   // compact (flags copied to stale_src: use a separate pass into stale / cand_src)
   if (w.fin_cap < nstale + ncand + 1) {
     int64_t nc = nstale + ncand + (nstale + ncand) / 2 + 1024;
