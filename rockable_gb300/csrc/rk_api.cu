@@ -70,6 +70,11 @@ void bind_entries(Ctx& c) {
   s.gn = b.gn; s.gpos = b.gpos; s.gvel = b.gvel;
 }
 
+// the near set is made anew by the next step that uses it
+cudaError_t near_set_stale(Ctx& c) {
+  return cudaMemsetAsync(c.s.flags + FLAG_NEAR_STALE, 1, 1, c.stream);
+}
+
 static void free_entrybuf(EntryBuf& b) {
   dfree(b.ei); dfree(b.ej); dfree(b.etsub); dfree(b.ekey); dfree(b.dn); dfree(b.fn); dfree(b.ft); dfree(b.mom);
   dfree(b.damp); dfree(b.bond); dfree(b.gn); dfree(b.gpos); dfree(b.gvel);
@@ -97,7 +102,8 @@ int ensure_entry_capacity(Ctx& c, int which, int64_t n) {
     Scene& s = c.s;
     if ((rc = dalloc(c, s.act, cap)) || (rc = dalloc(c, s.cf, 3 * cap)) || (rc = dalloc(c, s.cmi, 3 * cap)) ||
         (rc = dalloc(c, s.cmj, 3 * cap)) || (rc = dalloc(c, s.jlist, cap)) || (rc = dalloc(c, s.nperm, cap)) ||
-        (rc = dalloc(c, s.egv, cap)) || (rc = dalloc(c, s.slow, cap)))
+        (rc = dalloc(c, s.egv, cap)) || (rc = dalloc(c, s.slow, cap)) || (rc = dalloc(c, s.nflag, cap)) ||
+        (rc = dalloc(c, s.nrec, 2 * cap)) || (rc = dalloc(c, s.srec, 2 * cap)) || (rc = dalloc(c, s.glist, 2 * cap)))
       return rc;
     c.contrib_cap = cap;
   }
@@ -235,6 +241,12 @@ static void settle_before_update(Ctx& c) {
 // does), so it can act from the first windows and departs from that method
 // only as far as its training carries it.
 static const int kMinWindows = 2;
+// Time of the candidates-to-index part of a rebuild on a list small enough
+// that its launches and read-backs are all of it.
+static const double kRebuildFixedMs = 0.6;
+// Longest window the cost model proposes: its displacement rate is a
+// prediction for the next window, and the network learns once per window.
+static const int64_t kMaxWindow = 320;
 
 static double to_f(unsigned int bits) {
   float f;
@@ -378,34 +390,32 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
   // faster than the skin (more sub-element pairs come within reach): the
   // non-active entries are scaled by (skin ratio)^alpha, alpha learnt from
   // the rebuilds that changed the skin (1.6, the power measured on hull-grain
-  // piles, to start).  The step time is measured over the last window,
-  // with the narrow phase (timed by events, proportional to the list) apart;
-  // the last full rebuild is timed in two parts, the broad phase (70 %
-  // fixed) and the candidates-to-index part (proportional to the list); the
-  // partial refreshes of the window are counted and timed.  The interval is
-  // the number of steps the predicted displacement rate takes to use half
-  // the skin (with a margin), which is also when the guard would force it.
+  // piles, to start).  A step itself does not depend on the list's size (it
+  // runs on the near set); the last full rebuild is timed in two parts, the
+  // broad phase (70 % fixed) and the candidates-to-index part, proportional
+  // to the list beyond the latency of its launches and read-backs
+  // (kRebuildFixedMs); the partial refreshes of the window are counted and
+  // timed.  The interval is the number of steps the predicted displacement
+  // rate takes to use half the skin (with a margin), which is also when the
+  // guard would force it.
   const double margin = 1.3, alpha = k.alpha;
   const double skin_before = k.skin;
   const double C = (double)std::max<int64_t>(1, ne0), A = std::min(active, C);
   // partial refreshes of the window: their rate grows as the skin shrinks
-  // (the fast bodies use it up sooner); their time is part of the window's
-  // step time and is taken out of it
+  // (the fast bodies use it up sooner)
   const double P = (double)k.partial_in_window / (double)std::max<int64_t>(1, k.since);
   const double Rp = k.partial_ms;
-  const double T = std::max(0.0, (k.step_ms > 0 ? k.step_ms : 0.2) - P * Rp);
-  const double Tn = k.narrow_cnt > 0 ? std::min(T, k.narrow_acc / (double)k.narrow_cnt) : 0.4 * T;
   const double Rbp = k.rebuild_bp_ms > 0 ? k.rebuild_bp_ms : 2.0;
   const double Rvar = k.rebuild_var_ms > 0 ? k.rebuild_var_ms : 2.0;
+  const double Rfix = std::min(Rvar, kRebuildFixedMs);
   double best = 1e300, best_s = k.skin;
   int64_t best_k = k.interval;
   for (int m = -4; m <= 4; m++) {
     double sk = std::min(k.cfg.skin_max, std::max(k.cfg.skin_min, k.skin * std::pow(2.0, 0.25 * m)));
     double kk = std::floor(0.5 * sk / std::max(u * margin * (1.0 + churn), 1e-30));
-    int64_t ki = (int64_t)std::max<double>(k.cfg.interval_min, std::min<double>(k.cfg.interval_max, kk));
+    int64_t ki = (int64_t)std::max<double>(k.cfg.interval_min, std::min<double>((double)std::min<int64_t>(k.cfg.interval_max, std::max<int64_t>(kMaxWindow, k.cfg.interval_min)), kk));
     double ratio = (A + (C - A) * std::pow(sk / std::max(k.skin, 1e-30), alpha)) / C;
-    double J = (T - Tn) + Tn * ratio + (Rbp * (0.7 + 0.3 * ratio) + Rvar * ratio) / (double)ki +
-               P * (k.skin / sk) * Rp;
+    double J = (Rbp * (0.7 + 0.3 * ratio) + Rfix + (Rvar - Rfix) * ratio) / (double)ki + P * (k.skin / sk) * Rp;
     if (J < best) { best = J; best_s = sk; best_k = ki; }
   }
   k.skin = best_s;
@@ -461,8 +471,6 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
   CK(cudaMemsetAsync(s.flags + FLAG_NEED_UPDATE, 0, sizeof(unsigned long long), c.stream));
   k.since = 0;
   k.partial_since_global = 0;
-  k.narrow_acc = 0.0;
-  k.narrow_cnt = 0;
   k.partial_in_window = 0;
   CK(cudaEventRecord(k.ea, c.stream));
   return 0;
@@ -475,18 +483,17 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
 // rebuild swaps the entry buffers, a parameter call changes scalars), then
 // replayed.  Same kernels, same arguments, same order as the launch-by-launch
 // path, so the results are identical.
-static int step_launches(Ctx& c, bool time_narrow = true) {
+static int step_launches(Ctx& c, bool near) {
   Scene& s = c.s;
   int n = 0;
   n += launch_controls_pre(s, c.stream);
   n += launch_drift(s, c.stream);
-  n += launch_glob_vertices(s, c.stream);
-  // the skin's cost model wants the narrow-phase time
-  const bool timed = time_narrow && c.skin.on && c.skin.nev[0];
-  if (timed) cudaEventRecord(c.skin.nev[0], c.stream);
-  n += c.form == RK_FORM_MIXED ? launch_narrow_force_mixed(s, c.stream) : launch_narrow_force(s, c.stream);
-  if (timed) cudaEventRecord(c.skin.nev[1], c.stream);
-  n += launch_gather_heavy(s, c.stream) + launch_gather_accel(s, 1, c.stream);
+  if (near) n += launch_near_update(s, c.stream);
+  else n += launch_glob_vertices(s, c.stream);
+  if (near) n += launch_narrow_near(s, c.stream);
+  else n += c.form == RK_FORM_MIXED ? launch_narrow_force_mixed(s, c.stream) : launch_narrow_force(s, c.stream);
+  if (near) n += launch_gather_near(s, c.stream);
+  else n += launch_gather_heavy(s, c.stream) + launch_gather_accel(s, 1, c.stream);
   n += launch_breakage(s, c.stream);
   return n;
 }
@@ -564,31 +571,30 @@ static int graph_install(Ctx& c, cudaGraph_t g, cudaGraphExec_t* ex, const char*
   return RK_OK;
 }
 
-static int step_graph(Ctx& c) {
+static int step_graph(Ctx& c, bool near) {
   Scene& s = c.s;
-  const bool stale = !c.gexec || c.gform != c.form || std::memcmp(&c.gscene, &s, sizeof(Scene)) != 0;
+  const int v = near ? 1 : 0;
+  const bool stale = !c.gexec[v] || c.gform[v] != c.form || std::memcmp(&c.gscene[v], &s, sizeof(Scene)) != 0;
   if (stale) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(s.flags + FLAG_NACTIVE, 0, sizeof(unsigned long long), c.stream);
-    int n = step_launches(c);
+    int n = step_launches(c, near);
     cudaError_t e = cudaStreamEndCapture(c.stream, &g);
     if (e != cudaSuccess) {
       if (g) cudaGraphDestroy(g);
       c.err = std::string("step graph capture: ") + cudaGetErrorString(e);
       return RK_ERR_CUDA;
     }
-    const int rc = graph_install(c, g, &c.gexec, "step graph");
+    const int rc = graph_install(c, g, &c.gexec[v], "step graph");
     if (rc) return rc;
-    std::memcpy(&c.gscene, &s, sizeof(Scene));  // byte copy: the comparison above is bytewise
-    c.gform = c.form;
-    c.glaunched = n;
+    std::memcpy(&c.gscene[v], &s, sizeof(Scene));  // byte copy: the comparison above is bytewise
+    c.gform[v] = c.form;
+    c.glaunched[v] = n;
     c.graph_captures++;
   }
-  CK(cudaGraphLaunch(c.gexec, c.stream));
-  c.skin.narrow_timed = c.skin.on && c.skin.nev[0];
+  CK(cudaGraphLaunch(c.gexec[v], c.stream));
   c.graph_replays++;
-  c.kernels += c.glaunched;
+  c.kernels += c.glaunched[v];
   return RK_OK;
 }
 
@@ -599,12 +605,21 @@ static int step_graph(Ctx& c) {
 // batch that fits, so that no step is skipped for want of work.
 constexpr int kSkinBatch = 16;
 
+// Whether a step runs on the near set (rk_near.cu): another step of the call
+// follows, and the contact geometry is not being recorded for every entry.
+static bool near_step(const Ctx& c, bool more_follow) {
+  return more_follow && c.s.ne > 0 && c.s.egv_ok && !c.s.record_geom;
+}
+
 // The graph of a batch of 2^lg steps, opened by k_skin_begin; each step's
-// resultant kernel closes it (skin_batch_step_end); the narrow phase of the
-// first step is timed for the skin's cost model.  Captured with s.sk_ctl set,
+// resultant kernel closes it (skin_batch_step_end).  Captured with s.sk_ctl set,
 // like the launches it holds.
-static int batch_graph(Ctx& c, int lg) {
+// `near` (the batches that another step follows) is part of the key: a batch
+// of one step exists in both variants, at 0 and at 5.
+static int batch_graph(Ctx& c, int lg, bool near) {
   Scene& s = c.s;
+  const int steps = 1 << lg;
+  if (!near) lg = 5;
   const bool stale =
       !c.bexec[lg] || c.bform[lg] != c.form || std::memcmp(&c.bscene[lg], &s, sizeof(Scene)) != 0;
   if (stale) {
@@ -612,7 +627,7 @@ static int batch_graph(Ctx& c, int lg) {
     CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
     int n = 0;
     n += launch_skin_begin(s, c.stream);
-    for (int q = 0; q < (1 << lg); q++) n += step_launches(c, q == 0);
+    for (int q = 0; q < steps; q++) n += step_launches(c, near);
     const cudaError_t e = cudaStreamEndCapture(c.stream, &g);
     if (e != cudaSuccess) {
       if (g) cudaGraphDestroy(g);
@@ -641,8 +656,10 @@ static int skin_partial(Ctx& c, int64_t nflag);
 static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   Skin& k = c.skin;
   Scene& s = c.s;
+  // the call's last step is a batch of its own: it computes the whole list
+  const bool near = near_step(c, left > 1);
   int lg = 0;
-  while (lg < 4 && (int64_t)2 << lg <= left) lg++;
+  while (near && lg < 4 && (int64_t)2 << lg <= left - 1) lg++;
   const int64_t want = (int64_t)1 << lg;
   unsigned int* in = k.h_ctl;
   unsigned int* out = k.h_ctl + 16;
@@ -658,7 +675,14 @@ static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   in[7] = 0u;
   CK(cudaMemcpyAsync(k.d_ctl, in, 8 * sizeof(unsigned int), cudaMemcpyHostToDevice, c.stream));
   s.sk_ctl = k.d_ctl;
-  int rc = batch_graph(c, lg);
+  int rc = RK_OK;
+  if (c.use_graphs) {
+    rc = batch_graph(c, lg, near);
+  } else {
+    int n = launch_skin_begin(s, c.stream);
+    for (int64_t q = 0; q < want; q++) n += step_launches(c, near);
+    c.kernels += n;
+  }
   s.sk_ctl = nullptr;
   if (rc) return rc;
   CK(cudaMemcpyAsync(out, k.d_ctl, 16 * sizeof(unsigned int), cudaMemcpyDeviceToHost, c.stream));
@@ -678,16 +702,6 @@ static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   c.more_steps_follow = ex < left;
   c.forces_stale = s.nheavy_lazy > 0;
   k.since = out[2];
-  if (k.nev[0]) {  // the first step of the batch ran its narrow phase between these events
-    float nms = 0.f;
-    if (cudaEventElapsedTime(&nms, k.nev[0], k.nev[1]) == cudaSuccess) {
-      k.narrow_acc += nms;
-      k.narrow_cnt++;
-    } else {
-      cudaGetLastError();
-    }
-  }
-  k.narrow_timed = false;
   k.have_pred = false;
   const unsigned int* hg = out + 8;
   const double dmax = to_f(hg[0]), vmax = to_f(hg[1]), gmax = to_f(hg[2]);
@@ -753,25 +767,12 @@ int skin_after_step(Ctx& c) {
     CK(cudaEventSynchronize(k.gev[slot ^ 1]));
     const double pcrit = to_f(k.partial_since_global > 0 ? hp[7] : hp[6]);
     const bool due = pcrit >= 0.5 * k.skin * 0.98 || k.since >= k.interval;
-    if (!due) {
-      k.narrow_timed = false;  // this step's events may still be running
-      return 0;
-    }
+    if (!due) return 0;
   }
   // this step's guard: the exact values of this state
   CK(cudaEventSynchronize(k.gev[slot]));
   int rc;
   if (!pipe && (rc = read_flags(c))) return rc;
-  if (k.narrow_timed) {
-    float nms = 0.f;
-    if (cudaEventElapsedTime(&nms, k.nev[0], k.nev[1]) == cudaSuccess) {
-      k.narrow_acc += nms;
-      k.narrow_cnt++;
-    } else {
-      cudaGetLastError();  // not timed this step: the model falls back to its default share
-    }
-    k.narrow_timed = false;
-  }
   k.have_pred = pipe;  // holds until a refresh moves the snapshots
   const double dmax = to_f(hg[0]), vmax = to_f(hg[1]), gmax = to_f(hg[2]);
   const int64_t nflag = (int64_t)hg[3];
@@ -841,7 +842,8 @@ void rk_destroy(rk_ctx* x) {
   Ctx& c = x->c;
   cudaSetDevice(c.device);
   if (c.stream) cudaStreamSynchronize(c.stream);
-  if (c.gexec) cudaGraphExecDestroy(c.gexec);
+  for (cudaGraphExec_t e : c.gexec)
+    if (e) cudaGraphExecDestroy(e);
   for (cudaGraphExec_t e : c.bexec)
     if (e) cudaGraphExecDestroy(e);
   for (int k = 0; k < 8; k++)
@@ -853,7 +855,9 @@ void rk_destroy(rk_ctx* x) {
   dfree(s.hom); dfree(s.mass); dfree(s.inertia); dfree(s.rad); dfree(s.inv_mi); dfree(s.shape); dfree(s.group); dfree(s.cluster);
   dfree(s.gv_ofs); dfree(s.gv_body); dfree(s.lv); dfree(s.gv); dfree(s.gvr); dfree(s.posf); dfree(s.rotm); dfree(s.gsum); dfree(s.uv64); dfree(s.uvf); dfree(s.bobb); dfree(s.bobbf); dfree(s.baabb); dfree(s.dpos); dfree(s.dq);
   dfree(s.table); dfree(s.controls);
-  dfree(s.act); dfree(s.cf); dfree(s.cmi); dfree(s.cmj); dfree(s.iofs); dfree(s.jofs); dfree(s.jsplit); dfree(s.jlist); dfree(s.nperm); dfree(s.egv); dfree(s.slow);
+  dfree(s.act); dfree(s.cf); dfree(s.cmi); dfree(s.cmj); dfree(s.iofs); dfree(s.jofs); dfree(s.jsplit); dfree(s.jlist); dfree(s.nperm); dfree(s.egv);
+  dfree(s.nflag); dfree(s.nrec); dfree(s.srec); dfree(s.slow); dfree(s.glist); dfree(s.gcnt); dfree(s.npos); dfree(s.nq); dfree(s.nallow);
+  dfree(s.qf); dfree(s.rate); dfree(s.swing); dfree(s.big);
   dfree(s.heavy); dfree(s.is_heavy); dfree(s.sph); dfree(s.sph_ofs); dfree(s.sph_body); dfree(s.heavy_lazy); dfree(s.bnd);
   dfree(s.needres); dfree(s.scene_of); dfree(s.bf_surf);
   dfree(c.name_chars); dfree(c.name_ofs);
@@ -882,7 +886,7 @@ void rk_destroy(rk_ctx* x) {
     if (k.h_ctl) cudaFreeHost(k.h_ctl);
     if (k.bev) cudaEventDestroy(k.bev);
     if (k.ea) cudaEventDestroy(k.ea);
-    for (cudaEvent_t e : {k.nev[0], k.nev[1], k.pa, k.pb, k.gev[0], k.gev[1]})
+    for (cudaEvent_t e : {k.pa, k.pb, k.gev[0], k.gev[1]})
       if (e) cudaEventDestroy(e);
     if (k.eb) cudaEventDestroy(k.eb);
   }
@@ -970,6 +974,7 @@ int rk_upload_shapes(rk_ctx* x, const rk_shapes* sh) {
     }
     c.kernels += launch_body_verts(c.s, c.stream);
     CK(cudaGetLastError());
+    CK(near_set_stale(c));
   }
   return RK_OK;
 }
@@ -1036,9 +1041,13 @@ int rk_upload_bodies(rk_ctx* x, const rk_bodies* b) {
       (rc = dupload(c, s.sph_ofs, sph_ofs.data(), n + 1)) || (rc = dalloc(c, s.sph, sph_ofs[n])) ||
       (rc = dupload(c, s.sph_body, sph_body.data(), std::max<int64_t>(sph_ofs[n], 1))) ||
       (rc = dupload(c, s.is_heavy, (const uint8_t*)nullptr, n)) || (rc = dalloc(c, s.heavy, n)) ||
-      (rc = dalloc(c, s.heavy_lazy, n)) || (rc = dalloc(c, s.bnd, n)) || (rc = dalloc(c, s.needres, n)))
+      (rc = dalloc(c, s.heavy_lazy, n)) || (rc = dalloc(c, s.bnd, n)) || (rc = dalloc(c, s.needres, n)) ||
+      (rc = dalloc(c, s.gcnt, n)) || (rc = dalloc(c, s.npos, 3 * n)) || (rc = dalloc(c, s.nq, 4 * n)) ||
+      (rc = dalloc(c, s.nallow, n)) || (rc = dalloc(c, s.qf, n)) || (rc = dalloc(c, s.rate, n)) ||
+      (rc = dalloc(c, s.swing, n)) || (rc = dalloc(c, s.big, n)))
     return rc;
   s.nlv = 0;
+  s.nbig = 0;
   s.nheavy = 0;
   s.nheavy_lazy = 0;
   dfree(s.scene_of);
@@ -1421,12 +1430,12 @@ int rk_set_skin(rk_ctx* x, const rk_skin_config* cfg) {
   for (double& r : k.rates) r = 0.0;
   s.dVerlet = k.skin;
   s.DVerlet = cfg->dverlet_ratio * k.skin;
-  for (cudaEvent_t* e : {&k.nev[0], &k.nev[1], &k.pa, &k.pb, &k.gev[0], &k.gev[1]})
+  for (cudaEvent_t* e : {&k.pa, &k.pb, &k.gev[0], &k.gev[1]})
     if (!*e) CK(cudaEventCreate(e));
   k.gslot = 0;
   k.have_pred = false;
-  k.narrow_acc = k.partial_ms = 0.0;
-  k.narrow_cnt = k.partial_in_window = 0;
+  k.partial_ms = 0.0;
+  k.partial_in_window = 0;
   k.on = true;
   skin_bind(c, true);
   s.near_geometric = cfg->exact_contacts ? 1 : 0;
@@ -1495,8 +1504,10 @@ int rk_set_autotune(rk_ctx* x, int rounds) {
 
 int rk_get_block_sizes(const rk_ctx* x, int32_t* tpb) {
   if (!x || !tpb) return RK_ERR_ARG;
+  const Scene& s = x->c.s;
   const int def[4] = {128, 128, 256, 128};
-  for (int k = 0; k < 4; k++) tpb[k] = x->c.s.tpb[k] > 0 ? x->c.s.tpb[k] : def[k];
+  const int64_t items[4] = {s.ne, s.n, s.nvert, s.n};
+  for (int k = 0; k < 4; k++) tpb[k] = s.tpb[k] > 0 ? s.tpb[k] : items[k] < kSmallLaunch * 32 ? 32 : def[k];
   return RK_OK;
 }
 
@@ -1547,6 +1558,7 @@ int rk_accelerations(rk_ctx* x) {
   if ((rc = ready(c))) return rc;
   Scene& s = c.s;
   CK(cudaMemsetAsync(s.flags + FLAG_NACTIVE, 0, sizeof(unsigned long long), c.stream));
+  CK(near_set_stale(c));  // contacts are computed at positions that no drift has checked
   launch_glob_vertices(s, c.stream, true);
   if (c.form == RK_FORM_MIXED) launch_narrow_force_mixed(s, c.stream);
   else launch_narrow_force(s, c.stream);
@@ -1599,7 +1611,7 @@ int rk_step(rk_ctx* x, int64_t nsteps, rk_step_report* rep) {
   for (int64_t it = 0; it < nsteps; it++) {
     const bool tuning = c.tune_left > 0 && !c.profiling;
     const bool graphed = c.use_graphs && !c.profiling && !tuning;
-    if (graphed && c.skin.on && c.skin.d_ctl && guard_pipelined(c)) {
+    if (!c.profiling && !tuning && c.skin.on && c.skin.d_ctl && guard_pipelined(c)) {
       // the skin's decisions taken on the device, a batch of steps per round trip
       int64_t ex = 0;
       if ((rc = skin_batch(c, nsteps - it, &ex))) return rc;
@@ -1609,10 +1621,9 @@ int rk_step(rk_ctx* x, int64_t nsteps, rk_step_report* rep) {
     c.t += s.dt;
     c.interVerletC += s.dt;
     c.more_steps_follow = it + 1 < nsteps;
+    const bool near = !tuning && near_step(c, c.more_steps_follow);
     if (graphed) {
-      if ((rc = step_graph(c))) return rc;
-    } else {
-      CK(cudaMemsetAsync(s.flags + FLAG_NACTIVE, 0, sizeof(unsigned long long), c.stream));
+      if ((rc = step_graph(c, near))) return rc;
     }
     int ph = 0;
     auto mark = [&](int phase, bool end) {
@@ -1635,14 +1646,13 @@ int rk_step(rk_ctx* x, int64_t nsteps, rk_step_report* rep) {
     } else if (!graphed) {
       mark(0, false); phase(0, launch_controls_pre(s, c.stream));
       mark(1, false); phase(1, launch_drift(s, c.stream));
-      mark(2, false); phase(2, launch_glob_vertices(s, c.stream));
+      mark(2, false); phase(2, near ? launch_near_update(s, c.stream) : launch_glob_vertices(s, c.stream));
       mark(3, false);
-      const bool ntimed = c.skin.on && c.skin.nev[0];
-      if (ntimed) cudaEventRecord(c.skin.nev[0], c.stream);
-      phase(3, c.form == RK_FORM_MIXED ? launch_narrow_force_mixed(s, c.stream) : launch_narrow_force(s, c.stream));
-      if (ntimed) cudaEventRecord(c.skin.nev[1], c.stream);
-      c.skin.narrow_timed = ntimed;
-      mark(4, false); phase(4, launch_gather_heavy(s, c.stream) + launch_gather_accel(s, 1, c.stream));
+      phase(3, near ? launch_narrow_near(s, c.stream)
+                    : c.form == RK_FORM_MIXED ? launch_narrow_force_mixed(s, c.stream) : launch_narrow_force(s, c.stream));
+      mark(4, false);
+      phase(4, near ? launch_gather_near(s, c.stream)
+                    : launch_gather_heavy(s, c.stream) + launch_gather_accel(s, 1, c.stream));
       mark(5, false); phase(5, launch_breakage(s, c.stream));
     }
     c.forces_stale = s.nheavy_lazy > 0;

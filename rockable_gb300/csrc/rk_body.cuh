@@ -10,6 +10,7 @@
 #define RK_BODY_HELPERS
 #include "rk_engine.cuh"
 #include "rk_guard.cuh"
+#include "rk_near.cuh"
 
 namespace rk {
 
@@ -146,8 +147,8 @@ __device__ __forceinline__ void body_resultant(const Scene& s, int64_t b, V3& F,
   }
 }
 
+__device__ __forceinline__ void finish_body(const Scene& s, int64_t b, V3 F, V3 M, int apply_kick);
 __device__ __forceinline__ void gather_body(const Scene& s, int64_t b, int apply_kick) {
-  const bool driven = b < s.n_driven;
   if (s.is_heavy[b] == 2) {
     // a driven body whose resultant feeds no state (no force / moment
     // control): summed on demand by k_gather_heavy when downloaded
@@ -157,6 +158,12 @@ __device__ __forceinline__ void gather_body(const Scene& s, int64_t b, int apply
   }
   V3 F, M;
   body_resultant(s, b, F, M);
+  finish_body(s, b, F, M, apply_kick);
+}
+
+// Newton-Euler and the second half-kick of body b from its resultant.
+__device__ __forceinline__ void finish_body(const Scene& s, int64_t b, V3 F, V3 M, int apply_kick) {
+  const bool driven = b < s.n_driven;
   const double fm = 1.0 - s.num_damp, fp = 1.0 + s.num_damp;
   const V3 vel = ld3(s.vel, b), vrot = ld3(s.vrot, b);
   const double mass = s.mass[b];
@@ -250,10 +257,7 @@ namespace RK_BODY_NS {
 
 #ifndef RK_BODY_GLOB_ONLY
 // ----------------------------------------------------------------- K1 ----
-__global__ void k_drift(Scene s) {
-  if (step_halted(s)) return;
-  int64_t i = s.n_driven + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= s.n) return;
+__device__ __forceinline__ void drift_body(const Scene& s, int64_t i) {
   V3 p = ld3(s.pos, i), v = ld3(s.vel, i), a = ld3(s.acc, i);
   V3 w = ld3(s.vrot, i), al = ld3(s.arot, i);
   Q4 q = ldq(s.Q, i);
@@ -280,6 +284,14 @@ __global__ void k_drift(Scene s) {
   st3(s.vel, i, v);
   stq(s.Q, i, q);
   st3(s.vrot, i, w);
+}
+// the free bodies' drift; every body's part of the near set's check
+__global__ void k_drift(Scene s) {
+  if (step_halted(s)) return;
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= s.n) return;
+  if (i >= s.n_driven) drift_body(s, i);
+  near_track(s, i);
 }
 
 #endif  // RK_BODY_GLOB_ONLY
@@ -319,6 +331,125 @@ __global__ void k_gather_accel(Scene s, int apply_kick) {
   if (b < s.n) gather_body(s, b, apply_kick);
   // the learned skin's guard on the state this step leaves (all lanes)
   if (s.sk_out && apply_kick) skin_guard_body(s, b);
+  if (s.sk_ctl) skin_batch_step_end(s);
+}
+
+// The same on the near set: a body's few near entries (glist, in the serial
+// order) instead of its whole list.  The first nbig blocks take a big body
+// each (walls under force control: thousands of entries): the block loads the
+// contributions of 128 positions at a time, packs the active ones in shared
+// memory, and six lanes add the six components in the serial order while the
+// next positions are on their way -- a chain of one addition per contact, with
+// its operands at hand, instead of one that also broadcasts them by shuffles.
+// Bodies whose resultant the step does not use (driven, no force or moment
+// control) have no state to update.
+// kGatherNear threads per block.
+template <int kGatherNear>
+__global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
+  if (step_halted(s)) return;
+  __shared__ double sh[2][kGatherNear][6];
+  __shared__ int wcnt[2][kGatherNear / 32];
+  int64_t guard = s.n;
+  if ((int)blockIdx.x < s.nbig) {
+    const int64_t b = s.big[blockIdx.x];
+    const int* list = s.glist + s.iofs[b] + s.jofs[b];
+    const int L = s.gcnt[b], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    V3 F, M;
+    init_resultant(s, b, F, M);
+    const double start[6] = {F.x, F.y, F.z, M.x, M.y, M.z};
+    double acc = 0.0;
+#pragma unroll
+    for (int d = 0; d < 6; d++)
+      if (lane == d) acc = start[d];
+    double c[6];
+    bool on = false;
+    auto fetch = [&](int p) {
+      on = false;
+      if (p >= L) return;
+      const int x = list[p];
+      const int64_t e = x & kGlistEntry;
+      on = s.act[e] != 0;
+      if (!on) return;
+      const bool jside = x < 0;
+      const V3 f = ld3(s.cf, e), m = jside ? ld3(s.cmj, e) : ld3(s.cmi, e);
+      c[0] = jside ? -f.x : f.x; c[1] = jside ? -f.y : f.y; c[2] = jside ? -f.z : f.z;
+      c[3] = m.x; c[4] = m.y; c[5] = m.z;
+    };
+    fetch(threadIdx.x);
+    int buf = 0;
+    for (int p0 = 0; p0 < L; p0 += kGatherNear, buf ^= 1) {
+      const unsigned bal = __ballot_sync(0xffffffffu, on);
+      if (lane == 0) wcnt[buf][warp] = __popc(bal);
+      __syncthreads();  // (also: the sums of the buffer before this one are done)
+      int at = __popc(bal & ((1u << lane) - 1u)), all = 0;
+      for (int w = 0; w < kGatherNear / 32; w++) {
+        if (w < warp) at += wcnt[buf][w];
+        all += wcnt[buf][w];
+      }
+      if (on)
+#pragma unroll
+        for (int d = 0; d < 6; d++) sh[buf][at][d] = c[d];
+      __syncthreads();
+      fetch(p0 + kGatherNear + threadIdx.x);
+      if (warp == 0 && lane < 6) {
+        int k = 0;
+        for (; k + 8 <= all; k += 8) {
+          double v[8];
+#pragma unroll
+          for (int u = 0; u < 8; u++) v[u] = sh[buf][k + u][lane];
+#pragma unroll
+          for (int u = 0; u < 8; u++) acc = acc + v[u];
+        }
+        for (; k < all; k++) acc = acc + sh[buf][k][lane];
+      }
+    }
+    if (warp == 0) {
+      const double r0 = __shfl_sync(0xffffffffu, acc, 0), r1 = __shfl_sync(0xffffffffu, acc, 1);
+      const double r2 = __shfl_sync(0xffffffffu, acc, 2), r3 = __shfl_sync(0xffffffffu, acc, 3);
+      const double r4 = __shfl_sync(0xffffffffu, acc, 4), r5 = __shfl_sync(0xffffffffu, acc, 5);
+      if (lane == 0) {
+        finish_body(s, b, v3(r0, r1, r2), v3(r3, r4, r5), 1);
+        guard = b;
+      }
+    }
+  } else {
+    const int64_t b = ((int64_t)blockIdx.x - s.nbig) * kGatherNear + threadIdx.x;
+    if (b < s.n) {
+      const int64_t base = s.iofs[b] + s.jofs[b];
+      const bool used = s.needres[b] != 0;
+      const bool big = used && s.iofs[b + 1] + s.jofs[b + 1] - base > kNearBig;
+      if (!big) guard = b;
+      if (used && !big) {
+        const int L = s.gcnt[b];
+        const int* list = s.glist + base;
+        V3 F, M;
+        init_resultant(s, b, F, M);
+        for (int p0 = 0; p0 < L; p0 += 4) {  // four positions loaded together, added in order
+          int x[4];
+          bool a[4];
+          V3 f[4], m[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) x[u] = p0 + u < L ? list[p0 + u] : 0;
+#pragma unroll
+          for (int u = 0; u < 4; u++) a[u] = p0 + u < L && s.act[x[u] & kGlistEntry];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int64_t e = x[u] & kGlistEntry;
+            f[u] = a[u] ? ld3(s.cf, e) : v3(0, 0, 0);
+            m[u] = a[u] ? ld3(x[u] < 0 ? s.cmj : s.cmi, e) : v3(0, 0, 0);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            if (!a[u]) continue;
+            F = x[u] < 0 ? F - f[u] : F + f[u];
+            M = M + m[u];
+          }
+        }
+        finish_body(s, b, F, M, 1);
+      }
+    }
+  }
+  if (s.sk_out) skin_guard_body(s, guard);
   if (s.sk_ctl) skin_batch_step_end(s);
 }
 

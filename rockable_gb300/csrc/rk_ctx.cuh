@@ -73,12 +73,10 @@ struct Skin {
   unsigned int* h_ctl = nullptr;
   cudaEvent_t bev = nullptr;
   int64_t partial = 0, partial_bodies = 0, partial_since_global = 0, since_global = 0;
-  // measured in the current window: narrow-phase time per step (events
-  // around its launch, in the step graph too) and partial-refresh cost
-  double narrow_acc = 0.0, partial_ms = 0.0;
-  int64_t narrow_cnt = 0, partial_in_window = 0;
-  cudaEvent_t nev[2] = {nullptr, nullptr}, pa = nullptr, pb = nullptr;
-  bool narrow_timed = false;
+  // partial refreshes of the current window, and their measured cost
+  double partial_ms = 0.0;
+  int64_t partial_in_window = 0;
+  cudaEvent_t pa = nullptr, pb = nullptr;
   // double-buffered guard read-back (8 words per slot) and its events
   cudaEvent_t gev[2] = {nullptr, nullptr};
   int gslot = 0;
@@ -174,16 +172,18 @@ struct Ctx {
   cudaEvent_t tev[8] = {};
   // CUDA graph of one step's launches (re-captured when the scene changes)
   int use_graphs = 0;
-  cudaGraphExec_t gexec = nullptr;
-  Scene gscene{};       // the scene the graph was captured with
-  int gform = -1;
-  int glaunched = 0;    // kernels per replay
+  // [0]: a step on the whole list, [1]: on the near set
+  cudaGraphExec_t gexec[2] = {nullptr, nullptr};
+  Scene gscene[2]{};             // the scene the graph was captured with
+  int gform[2] = {-1, -1};
+  int glaunched[2] = {0, 0};     // kernels per replay
   int64_t graph_captures = 0, graph_replays = 0;
-  // the graphs of batches of 1, 2, 4, 8, 16 skin steps (same rules as the step graph)
-  cudaGraphExec_t bexec[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-  Scene bscene[5]{};
-  int bform[5] = {-1, -1, -1, -1, -1};
-  int blaunched[5] = {0, 0, 0, 0, 0};
+  // the graphs of batches of 1, 2, 4, 8, 16 skin steps on the near set, and of
+  // one step on the whole list (same rules as the step graph)
+  cudaGraphExec_t bexec[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  Scene bscene[6]{};
+  int bform[6] = {-1, -1, -1, -1, -1, -1};
+  int blaunched[6] = {0, 0, 0, 0, 0, 0};
 };
 
 // Neighbour-list update; with `only` (device flags per body), only the pairs
@@ -192,5 +192,6 @@ int rebuild_nl(Ctx& c, const uint8_t* only = nullptr);
 int heavy_list(Ctx& c);
 int ensure_entry_capacity(Ctx& c, int which, int64_t n);
 void bind_entries(Ctx& c);
+cudaError_t near_set_stale(Ctx& c);
 
 }  // namespace rk

@@ -32,6 +32,12 @@ constexpr int kMaxBody = 1 << 21;   // body index limit of the sort key
 constexpr int kMaskWords = 2;       // vertex cull mask words per half-pair (<= 64 vertices)
 constexpr int kHeavy = 64;          // entries above which a body's resultant is summed by a block
 constexpr int kHeavyWarp = 1024;    // mixed form: up to this many, by its warp inside the resultant kernel
+constexpr int kGlistLane = 28, kGlistEntry = (1 << 27) - 1;  // fields of a glist word (entry indices have 27 bits)
+// Per-entry and per-body kernels over fewer items than this (one warp per SM) run in blocks of one
+// warp by default: a warp-wide FP64 instruction holds an SM's FP64 pipe for about 20 cycles, so a
+// small launch is faster spread over all SMs than packed into blocks of four warps.
+constexpr int64_t kSmallLaunch = 152 * 4;  // warps
+constexpr int kNearBig = 1024;      // near steps: bodies with more entries than this are handled by a block each
 
 __host__ __device__ __forceinline__ uint64_t entry_key(uint32_t i, uint32_t j, uint32_t t, uint32_t isub,
                                                        uint32_t jsub) {
@@ -135,13 +141,29 @@ struct Scene {
   int64_t* jsplit;  // n: first j-side slot of body b whose entry follows b's own block
   int* jlist;     // ne
   int* nperm;     // ne: entries grouped by sub-contact type (the narrow phase's thread order)
-  int* slow;      // ne: the mixed narrow phase's entries for the full path, in the regions of
-                  // nperm's type runs (type t from flags[FLAG_TOFS + t])
   // ne: global vertex indices of each entry's sub-elements (k_entry_gv, after every list change):
   // vertex-vertex (a, b), vertex-edge (a, p1, p2), vertex-triangle (a, A, B, C; w = -1 for
   // faces of more than 3 vertices), edge-edge (pi1, pi2, pj1, pj2)
   int4* egv;
   int egv_ok;     // egv holds the current list (global vertex indices fit in an int)
+  // near set (rk_near.cu): the entries that can be active before some body has moved more than its
+  // allowance; all others are skipped by the steps that another step of the same call follows
+  uint8_t* nflag;   // ne: 1 for the entries of the near set
+  int4* nrec;       // 2 ne: the near set, in the regions of nperm's type runs: (entry, i, j, etsub), egv
+  int4* srec;       // 2 ne: the same for the entries that the step's narrow phase computes (FP64 form)
+  int* slow;        // ne: those entries in the mixed form, in the regions of nperm's type runs (type t
+                    // from flags[FLAG_TOFS + t])
+  int* glist;       // 2 ne: per body (from iofs[b] + jofs[b]) the near entries of its resultant in the
+                    // serial order (mixed form: own block, j side): bit 31 set for the j side, at
+                    // kGlistLane its position in the block or j side modulo kGatherLanes, the entry below
+  int* gcnt;        // n: how many
+  double *npos, *nq;  // 3n, 4n: positions and orientations when the set was made
+  float* nallow;    // n: motion allowed since (largest displacement of a point of the body)
+  float4* qf;       // n: orientation rounded to FP32, written with the drift
+  float* rate;      // n: bound of the speed of a point of the body, written with the drift
+  float* swing;     // n: largest distance of a vertex from the body centre, rounded up
+  int* big;         // bodies of more than kNearBig entries whose resultant the step uses
+  int nbig;
   int* heavy;     // bodies whose entry count exceeds kHeavy (summed by a block each)
   int nheavy;
   int* heavy_lazy;    // heavy driven bodies whose resultant feeds no state (summed on demand)
@@ -181,13 +203,16 @@ struct Scene {
   unsigned long long* flags;  // [0] need_update, [1] n_active, [2] n_broken_step, [3] guard max pos2 bits,
                               // [4] guard max rot bits, [5] guard reset pending, [6] error code,
                               // [7] 1 + index of a body with non-finite state, [8..11] entries of
-                              // each type in `slow` (zero between steps), [12] arrival ticket of
+                              // each type in `srec` or `slow` (zero between steps), [12] arrival ticket of
                               // the full-path kernel's blocks, [13..17] first nperm position of
-                              // each type (and ne)
+                              // each type (and ne), [18] the near set is out of date, [19..22] its
+                              // entries of each type, [23..26] the same while it is being made
+                              // (zero between), [27] arrival ticket of its last kernel
 };
 
 enum { FLAG_NEED_UPDATE = 0, FLAG_NACTIVE = 1, FLAG_NBROKEN = 2, FLAG_GPOS = 3, FLAG_GROT = 4, FLAG_GRESET = 5,
-       FLAG_ERROR = 6, FLAG_NONFINITE = 7, FLAG_NSLOW = 8, FLAG_SLOW_TICKET = 12, FLAG_TOFS = 13, FLAG_COUNT = 18 };
+       FLAG_ERROR = 6, FLAG_NONFINITE = 7, FLAG_NSLOW = 8, FLAG_SLOW_TICKET = 12, FLAG_TOFS = 13, FLAG_NEAR_STALE = 18, FLAG_NNEAR = 19, FLAG_NNEW = 23,
+       FLAG_NEAR_TICKET = 27, FLAG_COUNT = 28 };
 
 // step kernels (rk_step.cu)
 int launch_controls_pre(const Scene& s, cudaStream_t st);
@@ -197,6 +222,11 @@ int launch_drift(const Scene& s, cudaStream_t st);
 int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all = false, const uint8_t* mark = nullptr);
 int launch_narrow_force(const Scene& s, cudaStream_t st);
 int launch_narrow_force_mixed(const Scene& s, cudaStream_t st);
+// the same over the near set (steps that another step of the call follows), after launch_near_update,
+// which lists what the narrow phase has to compute
+int launch_near_update(const Scene& s, cudaStream_t st);
+int launch_narrow_near(const Scene& s, cudaStream_t st);
+int launch_gather_near(const Scene& s, cudaStream_t st);
 int launch_gather_accel(const Scene& s, int apply_kick, cudaStream_t st);
 int launch_gather_heavy(const Scene& s, cudaStream_t st);
 int launch_gather_heavy_lazy(const Scene& s, cudaStream_t st);
@@ -211,12 +241,14 @@ __device__ __forceinline__ bool step_halted(const Scene& s) { return s.sk_ctl !=
 
 int launch_fused_glob(const Scene& s, unsigned blocks, int threads, int only_listed, const uint8_t* mark,
                       cudaStream_t st);
-// with_drift: the step's launch, which makes the free bodies' drift first (the mixed form
-// has no separate drift launch: launch_drift returns 0 for it)
-int launch_body_frames(const Scene& s, unsigned blocks, int threads, int with_drift, cudaStream_t st);
+// in_step: the matrices are the step's (launch_drift_frames)
+int launch_body_frames(const Scene& s, unsigned blocks, int threads, int in_step, cudaStream_t st);
+int launch_drift_frames(const Scene& s, unsigned blocks, int threads, cudaStream_t st);
 int launch_body_verts(const Scene& s, cudaStream_t st);
 int launch_fused_gather(const Scene& s, unsigned blocks, int threads, int apply_kick, cudaStream_t st);
 int launch_fused_heavy(const Scene& s, const int* list, int count, cudaStream_t st);
+int launch_narrow_near_mixed(const Scene& s, cudaStream_t st);
+int launch_fused_gather_near(const Scene& s, unsigned blocks, int threads, cudaStream_t st);
 int launch_skin_begin(const Scene& s, cudaStream_t st);
 cudaError_t fused_attributes(int which, cudaFuncAttributes* a);
 cudaError_t narrow_mixed_attributes(cudaFuncAttributes* a);

@@ -127,11 +127,6 @@ __device__ __forceinline__ void drift_body(const Scene& s, int64_t i) {
   st3(s.vrot, i, addinc(w, dt_2 * lf));
   stq(s.Q, i, q4(fma(c, qd.s, qd.s), fma(c, qd.v.x, qd.v.x), fma(c, qd.v.y, qd.v.y), fma(c, qd.v.z, qd.v.z)));
 }
-__global__ void k_drift(Scene s) {
-  if (step_halted(s)) return;
-  const int64_t i = s.n_driven + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < s.n) drift_body(s, i);
-}
 
 // Resultants, Newton-Euler and the second half-kick (Rockable.cpp:3837-3866,
 // 2084-2117 in the FP64 form); driven bodies take the generic FP64 path.
@@ -244,40 +239,103 @@ __global__ void k_gather_accel(Scene s, int apply_kick) {
   if (s.sk_ctl) skin_batch_step_end(s);
 }
 
-// The mixed form's per-step body frames, in place of the FP64 world vertices:
-// one thread per body computes the FP64 rotation matrix of its quaternion
-// (the matrix of qrot, Particle.cpp:55-65 places the vertices with it) for
-// the narrow phase's FP64 path, which places only the vertices of the
-// entries it computes, and its FP32 copy; then the block's threads write the
-// FP32 offsets (world vertex - centre, the FP32 test's coordinates) of all
-// the block's bodies' vertices, coalesced, from the FP32 matrix.  The FP64
-// work per body is one matrix instead of one rotation per vertex.
-// With DRIFT (the step's launch), each free body's thread first makes its
-// drift (the first half of the velocity-Verlet step, above), so that the
-// frames read the state the drift just wrote: one launch and one pass over
-// the bodies instead of two.
-template <bool DRIFT>
+// k_gather_sums on the near set: the same lanes add the same contributions in
+// the same order (an entry left out of the set is inactive), found through
+// the body's short list (glist, the own block first): each word names the
+// lane, so that a step gives the same bits on the near set and on the whole
+// list.
+__global__ void k_gather_sums_near(Scene s) {
+  if (step_halted(s)) return;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t b = t / kGatherLanes;
+  const int l = (int)(t % kGatherLanes);
+  const bool group_sum = b < s.n && b >= s.n_driven && (s.is_heavy[b] == 0 || s.is_heavy[b] == 3);
+  float a[6] = {0, 0, 0, 0, 0, 0};
+  if (group_sum) {
+    const int* list = s.glist + s.iofs[b] + s.jofs[b];
+    const int L = s.gcnt[b];
+    for (int p0 = 0; p0 < L; p0 += 4) {
+      int x[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) x[u] = p0 + u < L ? list[p0 + u] : -1;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (p0 + u >= L || ((x[u] >> kGlistLane) & (kGatherLanes - 1)) != l) continue;
+        const int e = x[u] & kGlistEntry;
+        if (!s.act[e]) continue;
+        const V3 f = ld3(s.cf, e), m = ld3(x[u] < 0 ? s.cmj : s.cmi, e);
+        if (x[u] < 0) {
+          a[0] -= d2f(f.x); a[1] -= d2f(f.y); a[2] -= d2f(f.z);
+        } else {
+          a[0] += d2f(f.x); a[1] += d2f(f.y); a[2] += d2f(f.z);
+        }
+        a[3] += d2f(m.x); a[4] += d2f(m.y); a[5] += d2f(m.z);
+      }
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < 6; d++)
+    for (int o = kGatherLanes / 2; o > 0; o >>= 1) a[d] += __shfl_xor_sync(0xffffffffu, a[d], o);
+  if (group_sum && l == 0)
+#pragma unroll
+    for (int d = 0; d < 6; d++) s.gsum[6 * b + d] = a[d];
+}
+
+// The FP64 rotation matrix of body b's quaternion, to rotm.
+__device__ __forceinline__ void frame64(const Scene& s, int64_t b, double* R) {
+  const Q4 q = ldq(s.Q, b);
+  const double xx = q.v.x * q.v.x, yy = q.v.y * q.v.y, zz = q.v.z * q.v.z;
+  const double xy = q.v.x * q.v.y, xz = q.v.x * q.v.z, yz = q.v.y * q.v.z;
+  const double sx = q.s * q.v.x, sy = q.s * q.v.y, sz = q.s * q.v.z;
+  const double r[9] = {1.0 - 2.0 * (yy + zz), 2.0 * (xy - sz),       2.0 * (xz + sy),
+                       2.0 * (xy + sz),       1.0 - 2.0 * (xx + zz), 2.0 * (yz - sx),
+                       2.0 * (xz - sy),       2.0 * (yz + sx),       1.0 - 2.0 * (xx + yy)};
+#pragma unroll
+  for (int d = 0; d < 9; d++) {
+    R[d] = r[d];
+    s.rotm[9 * b + d] = r[d];
+  }
+}
+
+// The step's drift (the first half of the velocity-Verlet step, above) and
+// FP64 frames: one thread per body makes the drift of a free body and
+// computes the rotation matrix of the quaternion (the matrix of qrot,
+// Particle.cpp:55-65 places the vertices with it), from which the narrow
+// phase's FP64 path places the few vertices it needs; and every body's part
+// of the near set's check.
+__global__ void k_drift_frames(Scene s) {
+  if (step_halted(s)) return;
+  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (b >= s.n) return;
+  if (b >= s.n_driven) drift_body(s, b);
+  double R[9];
+  frame64(s, b, R);
+  near_track(s, b);
+}
+
+// What a step on the whole list and a list update need besides: the FP32
+// vertex offsets (world vertex - centre, the FP32 test's coordinates) of every
+// body, written coalesced by the block from FP32 copies of its bodies'
+// rotation matrices, and the centres rounded to FP32.  STEP: the matrices are
+// those of the step (rotm); otherwise they are computed here.
+template <bool STEP>
 __global__ void k_body_frames(Scene s) {
   if (step_halted(s)) return;
   extern __shared__ float fr[];  // [blockDim.x][10]: the FP32 matrix (and a pad)
   const int64_t b0 = blockIdx.x * (int64_t)blockDim.x;
   const int64_t b = b0 + threadIdx.x;
   if (b < s.n) {
-    if (DRIFT && b >= s.n_driven) drift_body(s, b);
-    const Q4 q = ldq(s.Q, b);
-    const double xx = q.v.x * q.v.x, yy = q.v.y * q.v.y, zz = q.v.z * q.v.z;
-    const double xy = q.v.x * q.v.y, xz = q.v.x * q.v.z, yz = q.v.y * q.v.z;
-    const double sx = q.s * q.v.x, sy = q.s * q.v.y, sz = q.s * q.v.z;
-    const double R[9] = {1.0 - 2.0 * (yy + zz), 2.0 * (xy - sz),       2.0 * (xz + sy),
-                         2.0 * (xy + sz),       1.0 - 2.0 * (xx + zz), 2.0 * (yz - sx),
-                         2.0 * (xz - sy),       2.0 * (yz + sx),       1.0 - 2.0 * (xx + yy)};
-    double* out = s.rotm + 9 * b;
+    float* f = fr + 10 * threadIdx.x;
+    double R[9];
+    if (STEP) {
 #pragma unroll
-    for (int d = 0; d < 9; d++) {
-      out[d] = R[d];
-      fr[10 * threadIdx.x + d] = d2f(R[d]);
+      for (int d = 0; d < 9; d++) R[d] = s.rotm[9 * b + d];
+    } else {
+      frame64(s, b, R);
     }
-    fr[10 * threadIdx.x + 9] = 0.f;
+#pragma unroll
+    for (int d = 0; d < 9; d++) f[d] = d2f(R[d]);
+    f[9] = 0.f;
     const V3 p = ld3(s.pos, b);
     s.posf[b] = make_float4(d2f(p.x), d2f(p.y), d2f(p.z), d2f(s.rad[b]));
   }
@@ -340,8 +398,8 @@ __global__ void __launch_bounds__(kHeavyThreads) k_gather_heavy(Scene s, const i
 
 }  // namespace mx
 
-int launch_body_frames(const Scene& s, unsigned blocks, int threads, int with_drift, cudaStream_t st) {
-  if (with_drift) mx::k_body_frames<true><<<blocks, threads, 10 * sizeof(float) * threads, st>>>(s);
+int launch_body_frames(const Scene& s, unsigned blocks, int threads, int in_step, cudaStream_t st) {
+  if (in_step) mx::k_body_frames<true><<<blocks, threads, 10 * sizeof(float) * threads, st>>>(s);
   else mx::k_body_frames<false><<<blocks, threads, 10 * sizeof(float) * threads, st>>>(s);
   return 1;
 }
@@ -355,6 +413,16 @@ int launch_fused_gather(const Scene& s, unsigned blocks, int threads, int apply_
   mx::k_gather_accel<<<blocks, threads, 0, st>>>(s, apply_kick);
   return 2;
 }
+int launch_drift_frames(const Scene& s, unsigned blocks, int threads, cudaStream_t st) {
+  mx::k_drift_frames<<<blocks, threads, 0, st>>>(s);
+  return 1;
+}
+int launch_fused_gather_near(const Scene& s, unsigned blocks, int threads, cudaStream_t st) {
+  int k = launch_gather_heavy(s, st);
+  mx::k_gather_sums_near<<<(unsigned)((s.n * kGatherLanes + 127) / 128), 128, 0, st>>>(s);
+  mx::k_gather_accel<<<blocks, threads, 0, st>>>(s, 1);
+  return k + 2;
+}
 int launch_fused_heavy(const Scene& s, const int* list, int count, cudaStream_t st) {
   mx::k_gather_heavy<<<count, mx::kHeavyThreads, 0, st>>>(s, list);
   return 1;
@@ -362,7 +430,7 @@ int launch_fused_heavy(const Scene& s, const int* list, int count, cudaStream_t 
 cudaError_t fused_attributes(int which, cudaFuncAttributes* a) {
   if (which == 1) return cudaFuncGetAttributes(a, mx::k_gather_accel);
   if (which == 2) return cudaFuncGetAttributes(a, mx::k_body_frames<true>);
-  return cudaFuncGetAttributes(a, mx::k_drift);
+  return cudaFuncGetAttributes(a, mx::k_drift_frames);
 }
 
 }  // namespace rk

@@ -23,6 +23,7 @@
 #include "../../include/rk_gpu.h"
 #include "rk_bits.cuh"
 #include "rk_engine.cuh"
+#include "rk_near.cuh"
 
 namespace rk {
 
@@ -80,7 +81,8 @@ __device__ __forceinline__ float amax(F3 a) { return fmaxf(fabsf(a.x), fmaxf(fab
 // vertices relative to body j's centre (the FP32 offsets gvr, plus the
 // difference of the two centres rounded to FP32, posf), the same projection
 // parameters as the FP64 path, and the separation's length.
-//   kApart    the overlap estimate dnf errs by a few ulps of the coordinates
+//   kApart    the projection or the closest points lie inside their ranges by
+//             more than their rounding error, and the overlap estimate dnf errs by a few ulps of the coordinates
 //             (relative ones, and the centres' absolute ones: `cmag`), so an
 //             estimate above a margin of 2e-6 m plus 2e-6 of the relative
 //             coordinates' magnitude plus 4e-7 of the centres' proves dn > 0:
@@ -124,11 +126,9 @@ __device__ __forceinline__ int apart_f32(const Scene& s, int type, int i, int j,
     const float E2 = dotf(E, E);
     const float r = dotf(w, E) / E2;
     mag = fmaxf(amax(a), fmaxf(amax(p1), amax(p2)));
-    if (r <= 0.f || r >= 1.f) {
-      // r's error: that of w and E (a few ulps of the coordinates) over |E|
-      const float tol = 1e-5f + 4e-7f * (mag + cmag) * rsqrtf(E2) * (1.f + fabsf(r));
-      return (r < -tol || r > 1.f + tol) ? kOutside : 0;
-    }
+    // r's error: that of w and E (a few ulps of the coordinates) over |E|
+    const float tol = 1e-5f + 4e-7f * (mag + cmag) * rsqrtf(E2) * (1.f + fabsf(r));
+    if (!(r > tol && r < 1.f - tol)) return (r < -tol || r > 1.f + tol) ? kOutside : 0;
     d = w - r * E;
   } else if (type == 2) {
     if (!(pre && G.w >= 0)) return 0;  // polygons other than triangles: the FP64 path
@@ -154,22 +154,26 @@ __device__ __forceinline__ int apart_f32(const Scene& s, int type, int i, int j,
     edge(bA, cA);
     edge(cA, z);
     mag = fmaxf(amax(a), fmaxf(amax(A), fmaxf(amax(B), amax(C))));
-    if (!odd) {
+    {
       // the projection clearly outside the triangle: farther than the
       // rounding of the coordinates beyond one of its edges (in the plane,
-      // on the side away from the third vertex)
+      // on the side away from the third vertex); clearly inside: farther than
+      // that from all three
       const float tol = 1e-9f + 1e-6f * (mag + cmag);
       const F3 Pv = P, cA2 = cA;
       const float o = dotf(crossf(bA, cA2), nn);  // the triangle's winding about nn
       if (!(fabsf(o) > 0.f)) return 0;
       const F3 ed[3] = {bA, cA2 - bA, -cA2};
       const F3 st[3] = {f3(0, 0, 0), bA, cA2};
+      bool in = odd != 0;
       for (int q = 0; q < 3; q++) {
         const F3 e = ed[q];
         const float side = dotf(crossf(e, Pv - st[q]), nn) * rsqrtf(dotf(e, e));
-        if ((o > 0.f ? -side : side) > tol) return kOutside;
+        const float beyond = o > 0.f ? -side : side;
+        if (!odd && beyond > tol) return kOutside;
+        in = in && beyond < -tol;
       }
-      return 0;
+      if (!in) return 0;
     }
     *dnf = dist - rsum;
     return *dnf > 2e-6f + 2e-6f * mag + 4e-7f * cmag ? kApart : 0;
@@ -190,14 +194,13 @@ __device__ __forceinline__ int apart_f32(const Scene& s, int type, int i, int j,
     const float a = dotf(Ei, w), b = dotf(Ej, w);
     const float ss = (ee * b - a * dd) * f, tt = (c * b - ee * a) * f;
     mag = fmaxf(fmaxf(amax(pi1), amax(pi2)), fmaxf(amax(pj1), amax(pj2)));
-    if (ss <= 0.f || ss >= 1.f || tt <= 0.f || tt >= 1.f) {
-      // well-conditioned pairs only (the sine of the edges' angle above
-      // 0.1): the parameters' error is then a few ulps of the coordinates
-      // over the shorter edge, amplified by at most 100 by the solve
-      if (!(f * c * dd < 100.f)) return 0;
-      const float tol = 1e-5f + 4e-5f * (mag + cmag) * rsqrtf(fminf(c, dd)) * (1.f + fabsf(ss) + fabsf(tt));
+    // well-conditioned pairs only (the sine of the edges' angle above
+    // 0.1): the parameters' error is then a few ulps of the coordinates
+    // over the shorter edge, amplified by at most 100 by the solve
+    if (!(f * c * dd < 100.f)) return 0;
+    const float tol = 1e-5f + 4e-5f * (mag + cmag) * rsqrtf(fminf(c, dd)) * (1.f + fabsf(ss) + fabsf(tt));
+    if (!(ss > tol && ss < 1.f - tol && tt > tol && tt < 1.f - tol))
       return (ss < -tol || ss > 1.f + tol || tt < -tol || tt > 1.f + tol) ? kOutside : 0;
-    }
     d = (w + ss * Ei) - tt * Ej;
   }
   *dnf = sqrtf(dotf(d, d)) - rsum;
@@ -559,8 +562,9 @@ __global__ void k_narrow_mixed_quick(Scene s) {
   }
 }
 
-// Pass 2: the full path over the four lists, one after the other, by whole
-// warps (grid-stride); the last block to finish empties the lists for the
+// Pass 2: the full path over the four lists (also the narrow phase of a step
+// on the near set: k_near_entries fills the same lists then, and both give
+// the same bits), one after the other, by whole warps (grid-stride); the last block to finish empties the lists for the
 // next step.  At least 5 blocks per SM: 96 registers, no spills, 20 warps
 // per SM instead of 16 (latency-bound otherwise).
 constexpr int kSlowThreads = 128;
@@ -573,8 +577,8 @@ __global__ void __launch_bounds__(kSlowThreads, 5) k_narrow_mixed_full(Scene s) 
     total += cnt[t];
   }
   const int lane = threadIdx.x & 31;
-  const int64_t nwarps = ((int64_t)gridDim.x * kSlowThreads) >> 5;
-  for (int64_t base = ((blockIdx.x * (int64_t)kSlowThreads + threadIdx.x) >> 5) * 32; base < total;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t base = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; base < total;
        base += nwarps * 32) {
     const int64_t q = base + lane;
     bool active = false;
@@ -603,14 +607,20 @@ __global__ void __launch_bounds__(kSlowThreads, 5) k_narrow_mixed_full(Scene s) 
   }
 }
 
+int launch_narrow_near_mixed(const Scene& s, cudaStream_t st) {
+  // small counts on blocks of one warp, spread over all SMs: a warp-wide FP64
+  // instruction holds an SM's FP64 pipe for about 20 cycles
+  const int t = s.ne < kSmallLaunch * 32 * 32 ? 32 : kSlowThreads;  // (a few percent of the entries are listed)
+  const int64_t blocks = std::min<int64_t>((s.ne + t - 1) / t, 152 * 640 / t);
+  k_narrow_mixed_full<<<(unsigned)std::max<int64_t>(blocks, 1), t, 0, st>>>(s);
+  return 1;
+}
+
 int launch_narrow_force_mixed(const Scene& s, cudaStream_t st) {
   if (s.ne <= 0) return 0;
   const int t = s.tpb[0] > 0 ? s.tpb[0] : 128;
   k_narrow_mixed_quick<<<(unsigned)((s.ne + t - 1) / t), t, 0, st>>>(s);
-  // enough warps for every entry to have a lane, up to 16 blocks per SM
-  const int64_t blocks = std::min<int64_t>((s.ne + kSlowThreads - 1) / kSlowThreads, 152 * 16);
-  k_narrow_mixed_full<<<(unsigned)blocks, kSlowThreads, 0, st>>>(s);
-  return 2;
+  return 1 + launch_narrow_near_mixed(s, st);
 }
 cudaError_t narrow_mixed_attributes(cudaFuncAttributes* a) { return cudaFuncGetAttributes(a, k_narrow_mixed_quick); }
 

@@ -190,6 +190,7 @@ __global__ void k_heavy(Scene s, unsigned long long* count) {
     }
     s.jsplit[b] = lo;
   }
+  if (c > kNearBig && s.needres[b]) s.big[atomicAdd(&count[2], 1ull)] = (int)b;
   bool h = c > kHeavy;
   uint8_t kind = 0;
   if (h && s.needres[b] && s.fast_body && c <= kHeavyWarp) {
@@ -1845,7 +1846,8 @@ int heavy_list(Ctx& c) {
     c.kernels++;
     s.egv_ok = 1;
   }
-  // counter slots 1, 2: heavy bodies, deferred heavy bodies; 4: listed vertices
+  RKCHK(near_set_stale(c));
+  // counter slots 1, 2: heavy bodies, deferred heavy bodies; 3: big bodies; 4: listed vertices
   RKCHK(cudaMemsetAsync(c.w.counter + 1, 0, 32, c.stream));
   k_heavy<<<nblk(s.n, 256), 256, 0, c.stream>>>(s, c.w.counter + 1);
   c.kernels++;
@@ -1854,6 +1856,7 @@ int heavy_list(Ctx& c) {
   RKCHK(cudaStreamSynchronize(c.stream));
   s.nheavy = (int)nh[0];
   s.nheavy_lazy = (int)nh[1];
+  s.nbig = (int)nh[2];
   s.nlv = (int64_t)nh[3];
   return 0;
 }

@@ -11,9 +11,17 @@
 //                                   Euler, second half-kick      3806-3868, 2131-2155
 //   bond_break / iface_break        postponed bond rupture       Rockable.cpp:3350-3413
 //
+// A step that another step of the same call follows runs on the near set
+// (rk_near.cu) instead of the whole list: drift, near_entries and near_bodies
+// (what the set's entries and bodies need), narrow_near, gather_near,
+// breakage; the same bits.  Per step of the packed column of 50 000 grains
+// (1.6 M entries): 60 + 736 + 114 us (vertices, narrow phase, resultants) on
+// the whole list, 18 + 85 + 34 us on the near set.
+//
 // Bit parity: compiled with --fmad=false; the resultant of every body is
 // summed in the reference's serial order (entries in key order), so the FP64
 // form reproduces the CPU path bit for bit.
+#include <algorithm>
 #include <cstdio>
 
 #include "../../include/rk_gpu.h"
@@ -214,6 +222,197 @@ __device__ __forceinline__ void law_sticked(const Scene& s, const LawIn& L, doub
 // ----------------------------------------------------------------- K2 ----
 __device__ __forceinline__ V3 gvx(const double* g, int k) { return v3(g[3 * k], g[3 * k + 1], g[3 * k + 2]); }
 
+// Entry e of the neighbour list (bodies, packed type and sub-elements; NEAR:
+// its global vertex indices): update, law, contributions; returns whether it
+// is active.
+template <bool NEAR>
+__device__ __forceinline__ bool narrow_entry(const Scene& s, int64_t e, int i, int j, uint32_t ts, int4 G) {
+  const int type = tsub_type(ts), isub = tsub_isub(ts), jsub = tsub_jsub(ts);
+  const double dn_old = s.dn[e];
+  const int bond = s.bond[e];
+  // vertices: from the step's world-vertex table, or (NEAR, a few entries)
+  // placed here by the same operations, found through the entry's index
+  // table; other polygons than triangles go through the shape tables
+  const double* gi = NEAR ? nullptr : s.gv + 3 * s.gv_ofs[i];
+  const double* gj = NEAR ? nullptr : s.gv + 3 * s.gv_ofs[j];
+  const V3 xi = ld3(s.pos, i), xj = ld3(s.pos, j);
+  Q4 qi, qj;
+  if (NEAR) {
+    qi = ldq(s.Q, i);
+    qj = ldq(s.Q, j);
+  }
+  auto pi_ = [&](int k) { return xi + qrot(qi, ld3(s.uv64, k)); };
+  auto pj_ = [&](int k) { return xj + qrot(qj, ld3(s.uv64, k)); };
+  const double Ri = s.rad[i], Rj = s.rad[j];
+  V3 n = v3(0, 0, 0), cpos = v3(0, 0, 0);
+  double dn = 0.0;
+  bool ok = true;
+  if (type == 0) {  // vertex-vertex
+    const V3 a = NEAR ? pi_(G.x) : gvx(gi, isub), b = NEAR ? pj_(G.y) : gvx(gj, jsub);
+    n = a - b;
+    dn = normalize(n) - (Ri + Rj);
+    cpos = a - n * (Ri + 0.5 * dn);
+  } else if (type == 1) {  // vertex-edge
+    V3 p1, p2, a;
+    if (NEAR) {
+      a = pi_(G.x);
+      p1 = pj_(G.y);
+      p2 = pj_(G.z);
+    } else {
+      const int eo = s.edge_ofs[s.shape[j]] + jsub;
+      p1 = gvx(gj, s.edges[2 * eo]);
+      p2 = gvx(gj, s.edges[2 * eo + 1]);
+      a = gvx(gi, isub);
+    }
+    V3 E = p2 - p1, v = a - p1;
+    double r = dot(v, E) / dot(E, E);
+    if (r <= 0.0 || r >= 1.0) {
+      ok = false;
+    } else {
+      n = a - (p1 + r * E);
+      dn = normalize(n) - (Ri + Rj);
+      cpos = a - n * (Ri + 0.5 * dn);
+    }
+  } else if (type == 2) {  // vertex-face
+    const bool tri = NEAR && G.w >= 0;
+    int nbv = 3, o = 0;
+    const int* fv = nullptr;
+    if (!tri) {
+      const int fo = s.face_ofs[s.shape[j]] + jsub;
+      fv = s.face_verts + s.face_vofs[fo];
+      nbv = s.face_vofs[fo + 1] - s.face_vofs[fo];
+      if (NEAR) o = (int)s.gv_ofs[j];
+    }
+    const V3 A = NEAR ? pj_(tri ? G.y : o + fv[0]) : gvx(gj, fv[0]);
+    const V3 B = NEAR ? pj_(tri ? G.z : o + fv[1]) : gvx(gj, fv[1]);
+    const V3 C = NEAR ? pj_(tri ? G.w : o + fv[nbv - 1]) : gvx(gj, fv[nbv - 1]);
+    const V3 a = NEAR ? pi_(G.x) : gvx(gi, isub);
+    V3 v = a - A;
+    V3 v1 = B - A;
+    normalize(v1);
+    V3 v2 = C - A;
+    n = cross(v1, v2);
+    normalize(n);
+    double dist = dot(v, n);
+    if (dist < 0.0) { n = -n; dist = -dist; }
+    V3 P = a - dist * n;
+    int odd = 0;
+    v2 = cross(n, v1);
+    double ori1 = dot(P, v1), ori2 = dot(P, v2);
+    // (each vertex's coordinates in the plane serve its two sides)
+    double pa1 = dot(A, v1), pa2 = dot(A, v2);
+    const double a1 = pa1, a2 = pa2;
+    for (int iva = 0; iva < nbv; ++iva) {
+      const int ivb = iva + 1;
+      double pb1 = a1, pb2 = a2;
+      if (ivb < nbv) {
+        const V3 pb = ivb == 1 ? B : ivb == nbv - 1 ? C : NEAR ? pj_(o + fv[ivb]) : gvx(gj, fv[ivb]);
+        pb1 = dot(pb, v1);
+        pb2 = dot(pb, v2);
+      }
+      if ((pa2 < ori2 && pb2 >= ori2) || (pb2 < ori2 && pa2 >= ori2)) {
+        if (pa1 + (ori2 - pa2) / (pb2 - pa2) * (pb1 - pa1) < ori1) odd = 1 - odd;
+      }
+      pa1 = pb1;
+      pa2 = pb2;
+    }
+    if (odd) {
+      dn = dist - (Ri + Rj);
+      cpos = a - n * (Ri + 0.5 * dn);
+    } else {
+      ok = false;
+    }
+  } else {  // edge-edge
+    V3 pi1, pi2, pj1, pj2;
+    if (NEAR) {
+      pi1 = pi_(G.x);
+      pi2 = pi_(G.y);
+      pj1 = pj_(G.z);
+      pj2 = pj_(G.w);
+    } else {
+      const int eoi = s.edge_ofs[s.shape[i]] + isub, eoj = s.edge_ofs[s.shape[j]] + jsub;
+      pi1 = gvx(gi, s.edges[2 * eoi]);
+      pi2 = gvx(gi, s.edges[2 * eoi + 1]);
+      pj1 = gvx(gj, s.edges[2 * eoj]);
+      pj2 = gvx(gj, s.edges[2 * eoj + 1]);
+    }
+    V3 Ei = pi2 - pi1, Ej = pj2 - pj1, v = pi1 - pj1;
+    double c = dot(Ei, Ei), d = dot(Ej, Ej), ee = dot(Ei, Ej);
+    double f = (c * d) - (ee * ee);
+    if (fabs(f) > 1.0e-12) {
+      f = 1.0 / f;
+      double a = dot(Ei, v), b = dot(Ej, v);
+      double ss = (ee * b - a * d) * f;
+      double tt = (c * b - ee * a) * f;
+      if (ss <= 0.0 || ss >= 1.0 || tt <= 0.0 || tt >= 1.0) {
+        ok = false;
+      } else {
+        n = (pi1 + ss * Ei) - (pj1 + tt * Ej);
+        dn = normalize(n) - (Ri + Rj);
+        cpos = pi1 + ss * Ei - n * (Ri + 0.5 * dn);
+      }
+    } else {
+      ok = false;
+    }
+  }
+  const V3 wi = ld3(s.vrot, i), wj = ld3(s.vrot, j);
+  V3 cvel;
+  double fn;
+  V3 ft, mom;
+  if (ok) {
+    const V3 vi = ld3(s.vel, i), vj = ld3(s.vel, j);
+    cvel = (vj - cross(cpos - xj, wj)) - (vi - cross(cpos - xi, wi));
+    fn = s.fn[e];
+    ft = ld3(s.ft, e);
+    mom = ld3(s.mom, e);
+    if (s.record_geom || bond >= 0) {
+      st3(s.gn, e, n);
+      st3(s.gpos, e, cpos);
+      st3(s.gvel, e, cvel);
+    }
+  } else {  // Interaction::deactivate (Interaction.cpp:123-128)
+    dn = 0.0;
+    fn = 0.0;
+    ft = v3(0, 0, 0);
+    mom = v3(0, 0, 0);
+    if (bond >= 0) {  // a bonded entry stays active with its previous geometry
+      n = ld3(s.gn, e);
+      cpos = ld3(s.gpos, e);
+      cvel = ld3(s.gvel, e);
+    } else {
+      cvel = v3(0, 0, 0);
+    }
+  }
+  const bool active = (dn < 0.0 || bond >= 0);
+  if (active) {
+    LawIn L;
+    L.dn = dn; L.dn_old = ok ? dn_old : 0.0; L.damp = s.damp[e];
+    L.n = n; L.vel = cvel; L.cpos = cpos;
+    L.wi = wi; L.wj = wj; L.xi = xi; L.xj = xj;
+    L.i_driven = i < s.n_driven;
+    L.gi = s.group[i]; L.gj = s.group[j];
+    L.ci = s.cluster[i]; L.cj = s.cluster[j];
+    L.bond = bond;
+    if (s.law == RK_LAW_AVALANCHE) law_avalanche(s, L, fn, ft, mom);
+    else if (s.law == RK_LAW_STICKEDLINKS) law_sticked(s, L, fn, ft, mom);
+    else law_default(s, L, fn, ft, mom);
+    // Rockable::incrementResultants (Rockable.cpp:2752-2789)
+    V3 f = fn * n + ft;
+    V3 Ci = (cpos - xi), Cj = (cpos - xj);
+    st3(s.cf, e, f);
+    st3(s.cmi, e, cross(Ci, f) + mom);
+    st3(s.cmj, e, cross(Cj, -f) - mom);
+  }
+  s.dn[e] = dn;
+  if (active || !ok) {
+    s.fn[e] = fn;
+    st3(s.ft, e, ft);
+    st3(s.mom, e, mom);
+  }
+  s.act[e] = active ? 1 : 0;
+  return active;
+}
+
 __global__ void k_narrow_force(Scene s) {
   if (step_halted(s)) return;
   // threads follow the entries grouped by sub-contact type (fewer divergent
@@ -222,153 +421,16 @@ __global__ void k_narrow_force(Scene s) {
   bool active = false;
   if (k < s.ne) {
     const int64_t e = s.nperm[k];
-    const int i = s.ei[e], j = s.ej[e];
-    const uint32_t ts = s.etsub[e];
-    const int type = tsub_type(ts), isub = tsub_isub(ts), jsub = tsub_jsub(ts);
-    const double dn_old = s.dn[e];
-    const int bond = s.bond[e];
-    const double* gi = s.gv + 3 * s.gv_ofs[i];
-    const double* gj = s.gv + 3 * s.gv_ofs[j];
-    const double Ri = s.rad[i], Rj = s.rad[j];
-    V3 n = v3(0, 0, 0), cpos = v3(0, 0, 0);
-    double dn = 0.0;
-    bool ok = true;
-    if (type == 0) {  // vertex-vertex
-      V3 a = gvx(gi, isub), b = gvx(gj, jsub);
-      n = a - b;
-      dn = normalize(n) - (Ri + Rj);
-      cpos = a - n * (Ri + 0.5 * dn);
-    } else if (type == 1) {  // vertex-edge
-      const int sj = s.shape[j];
-      const int eo = s.edge_ofs[sj] + jsub;
-      V3 p1 = gvx(gj, s.edges[2 * eo]), p2 = gvx(gj, s.edges[2 * eo + 1]);
-      V3 a = gvx(gi, isub);
-      V3 E = p2 - p1, v = a - p1;
-      double r = dot(v, E) / dot(E, E);
-      if (r <= 0.0 || r >= 1.0) {
-        ok = false;
-      } else {
-        n = a - (p1 + r * E);
-        dn = normalize(n) - (Ri + Rj);
-        cpos = a - n * (Ri + 0.5 * dn);
-      }
-    } else if (type == 2) {  // vertex-face
-      const int sj = s.shape[j];
-      const int fo = s.face_ofs[sj] + jsub;
-      const int v0 = s.face_vofs[fo], nbv = s.face_vofs[fo + 1] - v0;
-      const int* fv = s.face_verts + v0;
-      V3 A = gvx(gj, fv[0]), B = gvx(gj, fv[1]), C = gvx(gj, fv[nbv - 1]);
-      V3 a = gvx(gi, isub);
-      V3 v = a - A;
-      V3 v1 = B - A;
-      normalize(v1);
-      V3 v2 = C - A;
-      n = cross(v1, v2);
-      normalize(n);
-      double dist = dot(v, n);
-      if (dist < 0.0) { n = -n; dist = -dist; }
-      V3 P = a - dist * n;
-      int odd = 0;
-      v2 = cross(n, v1);
-      double ori1 = dot(P, v1), ori2 = dot(P, v2);
-      for (int iva = 0; iva < nbv; ++iva) {
-        int ivb = iva + 1;
-        if (ivb == nbv) ivb = 0;
-        V3 pa = gvx(gj, fv[iva]), pb = gvx(gj, fv[ivb]);
-        double pa1 = dot(pa, v1), pb1 = dot(pb, v1), pa2 = dot(pa, v2), pb2 = dot(pb, v2);
-        if ((pa2 < ori2 && pb2 >= ori2) || (pb2 < ori2 && pa2 >= ori2)) {
-          if (pa1 + (ori2 - pa2) / (pb2 - pa2) * (pb1 - pa1) < ori1) odd = 1 - odd;
-        }
-      }
-      if (odd) {
-        dn = dist - (Ri + Rj);
-        cpos = a - n * (Ri + 0.5 * dn);
-      } else {
-        ok = false;
-      }
-    } else {  // edge-edge
-      const int si = s.shape[i], sj = s.shape[j];
-      const int eoi = s.edge_ofs[si] + isub, eoj = s.edge_ofs[sj] + jsub;
-      V3 pi1 = gvx(gi, s.edges[2 * eoi]), pi2 = gvx(gi, s.edges[2 * eoi + 1]);
-      V3 pj1 = gvx(gj, s.edges[2 * eoj]), pj2 = gvx(gj, s.edges[2 * eoj + 1]);
-      V3 Ei = pi2 - pi1, Ej = pj2 - pj1, v = pi1 - pj1;
-      double c = dot(Ei, Ei), d = dot(Ej, Ej), ee = dot(Ei, Ej);
-      double f = (c * d) - (ee * ee);
-      if (fabs(f) > 1.0e-12) {
-        f = 1.0 / f;
-        double a = dot(Ei, v), b = dot(Ej, v);
-        double ss = (ee * b - a * d) * f;
-        double tt = (c * b - ee * a) * f;
-        if (ss <= 0.0 || ss >= 1.0 || tt <= 0.0 || tt >= 1.0) {
-          ok = false;
-        } else {
-          n = (pi1 + ss * Ei) - (pj1 + tt * Ej);
-          dn = normalize(n) - (Ri + Rj);
-          cpos = pi1 + ss * Ei - n * (Ri + 0.5 * dn);
-        }
-      } else {
-        ok = false;
-      }
-    }
-    const V3 xi = ld3(s.pos, i), xj = ld3(s.pos, j);
-    const V3 wi = ld3(s.vrot, i), wj = ld3(s.vrot, j);
-    V3 cvel;
-    double fn;
-    V3 ft, mom;
-    if (ok) {
-      const V3 vi = ld3(s.vel, i), vj = ld3(s.vel, j);
-      cvel = (vj - cross(cpos - xj, wj)) - (vi - cross(cpos - xi, wi));
-      fn = s.fn[e];
-      ft = ld3(s.ft, e);
-      mom = ld3(s.mom, e);
-      if (s.record_geom || bond >= 0) {
-        st3(s.gn, e, n);
-        st3(s.gpos, e, cpos);
-        st3(s.gvel, e, cvel);
-      }
-    } else {  // Interaction::deactivate (Interaction.cpp:123-128)
-      dn = 0.0;
-      fn = 0.0;
-      ft = v3(0, 0, 0);
-      mom = v3(0, 0, 0);
-      if (bond >= 0) {  // a bonded entry stays active with its previous geometry
-        n = ld3(s.gn, e);
-        cpos = ld3(s.gpos, e);
-        cvel = ld3(s.gvel, e);
-      } else {
-        cvel = v3(0, 0, 0);
-      }
-    }
-    active = (dn < 0.0 || bond >= 0);
-    if (active) {
-      LawIn L;
-      L.dn = dn; L.dn_old = ok ? dn_old : 0.0; L.damp = s.damp[e];
-      L.n = n; L.vel = cvel; L.cpos = cpos;
-      L.wi = wi; L.wj = wj; L.xi = xi; L.xj = xj;
-      L.i_driven = i < s.n_driven;
-      L.gi = s.group[i]; L.gj = s.group[j];
-      L.ci = s.cluster[i]; L.cj = s.cluster[j];
-      L.bond = bond;
-      if (s.law == RK_LAW_AVALANCHE) law_avalanche(s, L, fn, ft, mom);
-      else if (s.law == RK_LAW_STICKEDLINKS) law_sticked(s, L, fn, ft, mom);
-      else law_default(s, L, fn, ft, mom);
-      // Rockable::incrementResultants (Rockable.cpp:2752-2789)
-      V3 f = fn * n + ft;
-      V3 Ci = (cpos - xi), Cj = (cpos - xj);
-      st3(s.cf, e, f);
-      st3(s.cmi, e, cross(Ci, f) + mom);
-      st3(s.cmj, e, cross(Cj, -f) - mom);
-    }
-    s.dn[e] = dn;
-    if (active || !ok) {
-      s.fn[e] = fn;
-      st3(s.ft, e, ft);
-      st3(s.mom, e, mom);
-    }
-    s.act[e] = active ? 1 : 0;
+    active = narrow_entry<false>(s, e, s.ei[e], s.ej[e], s.etsub[e], make_int4(0, 0, 0, 0));
   }
   unsigned m = __ballot_sync(0xffffffffu, active);
   if ((threadIdx.x & 31) == 0 && m) atomicAdd(&s.flags[FLAG_NACTIVE], (unsigned long long)__popc(m));
+}
+
+constexpr int kNarrowNear = 128;
+__global__ void __launch_bounds__(kNarrowNear) k_narrow_near(Scene s) {
+  if (step_halted(s)) return;
+  near_narrow(s, [&](int4 R, int4 G) { return narrow_entry<true>(s, R.x, R.y, R.z, (uint32_t)R.w, G); });
 }
 
 // ----------------------------------------------------------------- K3 ----
@@ -541,7 +603,9 @@ int launch_controls_pre(const Scene& s, cudaStream_t st) {
   k_controls_pre<<<1, 32, 0, st>>>(s);
   return 1;
 }
-static inline int tpb_or(const Scene& s, int k, int d) { return s.tpb[k] > 0 ? s.tpb[k] : d; }
+static inline int tpb_or(const Scene& s, int k, int d, int64_t items) {
+  return s.tpb[k] > 0 ? s.tpb[k] : items < kSmallLaunch * 32 ? 32 : d;
+}
 
 // The per-body kernels come in two builds (rk_body.cuh): exact (this file,
 // no contraction) and fused (rk_fast.cu), the latter for the mixed form.
@@ -557,27 +621,29 @@ __global__ void k_body_verts(Scene s) {
   const double u[3] = {h * sv[0], h * sv[1], h * sv[2]};
   for (int d = 0; d < 3; d++) s.uv64[3 * k + d] = u[d];
   s.uvf[k] = make_float4((float)u[0], (float)u[1], (float)u[2], 0.f);
+  const float r = __double2float_ru(sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2])) * (1.f + 1e-6f);
+  atomicMax(reinterpret_cast<unsigned int*>(s.swing) + b, __float_as_uint(r));  // non-negative: ordered as their bits
 }
 int launch_body_verts(const Scene& s, cudaStream_t st) {
   if (s.nvert <= 0) return 0;
+  cudaMemsetAsync(s.swing, 0, (size_t)s.n * sizeof(float), st);
   k_body_verts<<<nblk(s.nvert, 256), 256, 0, st>>>(s);
   return 1;
 }
 
 int launch_drift(const Scene& s, cudaStream_t st) {
-  int64_t nf = s.n - s.n_driven;
-  if (nf <= 0) return 0;
-  const int t = tpb_or(s, 3, 128);
-  if (s.fast_body) return 0;  // made by the step's body-frame launch (launch_glob_vertices)
-  exact::k_drift<<<nblk(nf, t), t, 0, st>>>(s);
+  if (s.n <= 0) return 0;
+  const int t = tpb_or(s, 3, 128, s.n);
+  if (s.fast_body) return launch_drift_frames(s, nblk(s.n, t), t, st);
+  exact::k_drift<<<nblk(s.n, t), t, 0, st>>>(s);
   return 1;
 }
 int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all, const uint8_t* mark) {
   const int64_t nv = all || s.fast_body ? s.nvert : s.nlv;
   if (nv <= 0) return 0;
-  const int t = tpb_or(s, 2, 256);
+  const int t = tpb_or(s, 2, 256, nv);
   if (s.fast_body) {
-    // the mixed form's step needs only the FP32 offsets and the FP64 frames;
+    // the mixed form's step needs only the FP32 offsets (and the drift's frames);
     // a list update needs the FP64 world vertices as well
     int k = launch_body_frames(s, nblk(s.n, t), t, all ? 0 : 1, st);
     if (all) k += launch_fused_glob(s, nblk(nv, t), t, 0, mark, st);
@@ -588,15 +654,28 @@ int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all, const uint8_
 }
 int launch_narrow_force(const Scene& s, cudaStream_t st) {
   if (s.ne <= 0) return 0;
-  const int t = tpb_or(s, 0, 128);
+  const int t = tpb_or(s, 0, 128, s.ne);
   k_narrow_force<<<nblk(s.ne, t), t, 0, st>>>(s);
+  return 1;
+}
+int launch_narrow_near(const Scene& s, cudaStream_t st) {
+  if (s.fast_body) return launch_narrow_near_mixed(s, st);
+  const int t = s.ne < kSmallLaunch * 32 * 32 ? 32 : kNarrowNear;  // (a few percent of the entries are listed)
+  const int64_t blocks = std::min<int64_t>((s.ne + t - 1) / t, 152 * 4 * kNarrowNear / t);  // one resident wave
+  k_narrow_near<<<(unsigned)std::max<int64_t>(blocks, 1), t, 0, st>>>(s);
+  return 1;
+}
+int launch_gather_near(const Scene& s, cudaStream_t st) {
+  const bool small = s.n < kSmallLaunch * 32;
+  const int t = small ? 32 : 128;
+  if (s.fast_body) return launch_fused_gather_near(s, nblk(s.n, t), t, st);
+  if (small) exact::k_gather_near<32><<<(unsigned)s.nbig + nblk(s.n, 32), 32, 0, st>>>(s);
+  else exact::k_gather_near<128><<<(unsigned)s.nbig + nblk(s.n, 128), 128, 0, st>>>(s);
   return 1;
 }
 int launch_gather_accel(const Scene& s, int apply_kick, cudaStream_t st) {
   if (s.n <= 0) return 0;
-  // (a batched skin step zeroes it in k_skin_begin)
-  if (s.sk_out && apply_kick && !s.sk_ctl) cudaMemsetAsync(s.sk_out, 0, 8 * sizeof(unsigned int), st);
-  const int t = tpb_or(s, 1, 128);
+  const int t = tpb_or(s, 1, 128, s.n);
   if (s.fast_body) return launch_fused_gather(s, nblk(s.n, t), t, apply_kick, st);  // one body per thread
   exact::k_gather_accel<<<nblk(s.n, t), t, 0, st>>>(s, apply_kick);
   return 1;
