@@ -147,7 +147,8 @@ __device__ __forceinline__ void body_resultant(const Scene& s, int64_t b, V3& F,
   }
 }
 
-__device__ __forceinline__ void finish_body(const Scene& s, int64_t b, V3 F, V3 M, int apply_kick);
+__device__ __forceinline__ void finish_body(const Scene& s, int64_t b, V3 F, V3 M, int apply_kick,
+                                            float* kin = nullptr);
 __device__ __forceinline__ void gather_body(const Scene& s, int64_t b, int apply_kick) {
   if (s.is_heavy[b] == 2) {
     // a driven body whose resultant feeds no state (no force / moment
@@ -161,8 +162,10 @@ __device__ __forceinline__ void gather_body(const Scene& s, int64_t b, int apply
   finish_body(s, b, F, M, apply_kick);
 }
 
-// Newton-Euler and the second half-kick of body b from its resultant.
-__device__ __forceinline__ void finish_body(const Scene& s, int64_t b, V3 F, V3 M, int apply_kick) {
+// Newton-Euler and the second half-kick of body b from its resultant; kin
+// (may be null): a free body's velocity, acceleration, angular velocity and
+// angular acceleration after the step, as floats, for the skin's guard.
+__device__ __forceinline__ void finish_body(const Scene& s, int64_t b, V3 F, V3 M, int apply_kick, float* kin) {
   const bool driven = b < s.n_driven;
   const double fm = 1.0 - s.num_damp, fp = 1.0 + s.num_damp;
   const V3 vel = ld3(s.vel, b), vrot = ld3(s.vrot, b);
@@ -240,9 +243,21 @@ __device__ __forceinline__ void finish_body(const Scene& s, int64_t b, V3 F, V3 
     V3 arot = qrot(q, euler_domega(inertia, om, Mb));
     st3(s.acc, b, acc);
     st3(s.arot, b, arot);
+    V3 v = vel, wr = vrot;
     if (apply_kick) {
-      st3(s.vel, b, vel + s.dt_2 * acc);
-      st3(s.vrot, b, vrot + s.dt_2 * arot);
+      v = vel + s.dt_2 * acc;
+      wr = vrot + s.dt_2 * arot;
+      st3(s.vel, b, v);
+      st3(s.vrot, b, wr);
+    }
+    if (kin) {
+      const V3 k[4] = {v, acc, wr, arot};
+#pragma unroll
+      for (int d = 0; d < 4; d++) {
+        kin[3 * d] = d2f(k[d].x);
+        kin[3 * d + 1] = d2f(k[d].y);
+        kin[3 * d + 2] = d2f(k[d].z);
+      }
     }
   }
   st3(s.force, b, F);
@@ -335,52 +350,67 @@ __global__ void k_gather_accel(Scene s, int apply_kick) {
 }
 
 // The same on the near set: a body's few near entries (glist, in the serial
-// order) instead of its whole list.  The first nbig blocks take a big body
-// each (walls under force control: thousands of entries): the block loads the
-// contributions of 128 positions at a time, packs the active ones in shared
-// memory, and six lanes add the six components in the serial order while the
-// next positions are on their way -- a chain of one addition per contact, with
-// its operands at hand, instead of one that also broadcasts them by shuffles.
+// order) instead of its whole list.
+//   Sums: 8 lanes per body load 8 positions at a time (the next 8 while these
+//   are added), and lanes 0-5 add one component each in the serial order: one
+//   FP64 instruction per contact instead of six, and one round of loads per 8
+//   contacts.  (A warp-wide FP64 instruction holds its scheduler for 64 cycles
+//   on GB300 however many lanes it has and however independent it is.)
+//   Update: then one thread per body.
+// That is kBodies = 16 per block, for scenes that 8 such blocks per SM hold.
+// Larger scenes (kBodies = 128) have warps enough for one thread per body
+// throughout, whose updates fill their warps (50 000 grains: 34 us, against
+// 43 us in blocks of 32 bodies).
+// The first nbig blocks take a big body each (walls under force control:
+// thousands of entries): the whole block loads 128 positions at a time and
+// packs the active ones in shared memory, and six lanes add them in the
+// serial order while the next positions are on their way.
 // Bodies whose resultant the step does not use (driven, no force or moment
 // control) have no state to update.
-// kGatherNear threads per block.
-template <int kGatherNear>
+// 3000 grains 42 us (GEOM list, thread per body) before; the box of 200 000
+// grains 1.19 ms on whole lists with shuffles instead of shared memory.
+constexpr int kGatherNear = 128;
+template <int kBodies>
 __global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
   if (step_halted(s)) return;
   __shared__ double sh[2][kGatherNear][6];
+  __shared__ double res[kBodies == kGatherNear ? 1 : kBodies][6];
   __shared__ int wcnt[2][kGatherNear / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int64_t guard = s.n;
+  float kin[12] = {};  // the guard's velocities and accelerations of a free body
+  bool have = false;
+  double sum[6] = {0, 0, 0, 0, 0, 0};  // the resultant of body `guard`
+  double c[6];
+  bool on = false;
+  auto fetch = [&](const int* list, int p, int L) {
+    on = false;
+    if (p >= L) return;
+    const int x = list[p];
+    const int64_t e = x & kGlistEntry;
+    on = s.act[e] != 0;
+    if (!on) return;
+    const bool jside = x < 0;
+    const V3 f = ld3(s.cf, e), m = ld3(jside ? s.cmj : s.cmi, e);
+    c[0] = jside ? -f.x : f.x; c[1] = jside ? -f.y : f.y; c[2] = jside ? -f.z : f.z;
+    c[3] = m.x; c[4] = m.y; c[5] = m.z;
+  };
+  auto component = [&](V3 F, V3 M, int d) {
+    return d == 0 ? F.x : d == 1 ? F.y : d == 2 ? F.z : d == 3 ? M.x : d == 4 ? M.y : M.z;
+  };
   if ((int)blockIdx.x < s.nbig) {
     const int64_t b = s.big[blockIdx.x];
     const int* list = s.glist + s.iofs[b] + s.jofs[b];
-    const int L = s.gcnt[b], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int L = s.gcnt[b];
     V3 F, M;
     init_resultant(s, b, F, M);
-    const double start[6] = {F.x, F.y, F.z, M.x, M.y, M.z};
-    double acc = 0.0;
-#pragma unroll
-    for (int d = 0; d < 6; d++)
-      if (lane == d) acc = start[d];
-    double c[6];
-    bool on = false;
-    auto fetch = [&](int p) {
-      on = false;
-      if (p >= L) return;
-      const int x = list[p];
-      const int64_t e = x & kGlistEntry;
-      on = s.act[e] != 0;
-      if (!on) return;
-      const bool jside = x < 0;
-      const V3 f = ld3(s.cf, e), m = jside ? ld3(s.cmj, e) : ld3(s.cmi, e);
-      c[0] = jside ? -f.x : f.x; c[1] = jside ? -f.y : f.y; c[2] = jside ? -f.z : f.z;
-      c[3] = m.x; c[4] = m.y; c[5] = m.z;
-    };
-    fetch(threadIdx.x);
+    double acc = component(F, M, lane);
+    fetch(list, threadIdx.x, L);
     int buf = 0;
     for (int p0 = 0; p0 < L; p0 += kGatherNear, buf ^= 1) {
       const unsigned bal = __ballot_sync(0xffffffffu, on);
       if (lane == 0) wcnt[buf][warp] = __popc(bal);
-      __syncthreads();  // (also: the sums of the buffer before this one are done)
+      __syncthreads();
       int at = __popc(bal & ((1u << lane) - 1u)), all = 0;
       for (int w = 0; w < kGatherNear / 32; w++) {
         if (w < warp) at += wcnt[buf][w];
@@ -390,7 +420,7 @@ __global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
 #pragma unroll
         for (int d = 0; d < 6; d++) sh[buf][at][d] = c[d];
       __syncthreads();
-      fetch(p0 + kGatherNear + threadIdx.x);
+      fetch(list, p0 + kGatherNear + threadIdx.x, L);
       if (warp == 0 && lane < 6) {
         int k = 0;
         for (; k + 8 <= all; k += 8) {
@@ -403,53 +433,105 @@ __global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
         for (; k < all; k++) acc = acc + sh[buf][k][lane];
       }
     }
-    if (warp == 0) {
-      const double r0 = __shfl_sync(0xffffffffu, acc, 0), r1 = __shfl_sync(0xffffffffu, acc, 1);
-      const double r2 = __shfl_sync(0xffffffffu, acc, 2), r3 = __shfl_sync(0xffffffffu, acc, 3);
-      const double r4 = __shfl_sync(0xffffffffu, acc, 4), r5 = __shfl_sync(0xffffffffu, acc, 5);
-      if (lane == 0) {
-        finish_body(s, b, v3(r0, r1, r2), v3(r3, r4, r5), 1);
-        guard = b;
-      }
+    if (warp == 0 && lane < 6) res[0][lane] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      guard = b;
+#pragma unroll
+      for (int d = 0; d < 6; d++) sum[d] = res[0][d];
     }
   } else {
-    const int64_t b = ((int64_t)blockIdx.x - s.nbig) * kGatherNear + threadIdx.x;
-    if (b < s.n) {
-      const int64_t base = s.iofs[b] + s.jofs[b];
-      const bool used = s.needres[b] != 0;
-      const bool big = used && s.iofs[b + 1] + s.jofs[b + 1] - base > kNearBig;
-      if (!big) guard = b;
-      if (used && !big) {
-        const int L = s.gcnt[b];
-        const int* list = s.glist + base;
-        V3 F, M;
-        init_resultant(s, b, F, M);
-        for (int p0 = 0; p0 < L; p0 += 4) {  // four positions loaded together, added in order
-          int x[4];
-          bool a[4];
-          V3 f[4], m[4];
+    const int64_t b0 = ((int64_t)blockIdx.x - s.nbig) * kBodies;
+    if constexpr (kBodies == kGatherNear) {
+      const int64_t b = b0 + threadIdx.x;
+      if (b < s.n) {
+        const int64_t base = s.iofs[b] + s.jofs[b];
+        const bool used = s.needres[b] != 0;
+        if (!(used && s.iofs[b + 1] + s.jofs[b + 1] - base > kNearBig)) guard = b;
+        if (used && guard == b) {
+          const int L = s.gcnt[b];
+          const int* list = s.glist + base;
+          V3 F, M;
+          init_resultant(s, b, F, M);
+          for (int p0 = 0; p0 < L; p0 += 4) {  // four positions loaded together, added in order
+            int x[4];
+            bool a[4];
+            V3 f[4], m[4];
 #pragma unroll
-          for (int u = 0; u < 4; u++) x[u] = p0 + u < L ? list[p0 + u] : 0;
+            for (int u = 0; u < 4; u++) x[u] = p0 + u < L ? list[p0 + u] : 0;
 #pragma unroll
-          for (int u = 0; u < 4; u++) a[u] = p0 + u < L && s.act[x[u] & kGlistEntry];
+            for (int u = 0; u < 4; u++) a[u] = p0 + u < L && s.act[x[u] & kGlistEntry];
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const int64_t e = x[u] & kGlistEntry;
-            f[u] = a[u] ? ld3(s.cf, e) : v3(0, 0, 0);
-            m[u] = a[u] ? ld3(x[u] < 0 ? s.cmj : s.cmi, e) : v3(0, 0, 0);
+            for (int u = 0; u < 4; u++) {
+              const int64_t e = x[u] & kGlistEntry;
+              f[u] = a[u] ? ld3(s.cf, e) : v3(0, 0, 0);
+              m[u] = a[u] ? ld3(x[u] < 0 ? s.cmj : s.cmi, e) : v3(0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              if (!a[u]) continue;
+              F = x[u] < 0 ? F - f[u] : F + f[u];
+              M = M + m[u];
+            }
           }
+          const double r[6] = {F.x, F.y, F.z, M.x, M.y, M.z};
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
-            if (!a[u]) continue;
-            F = x[u] < 0 ? F - f[u] : F + f[u];
-            M = M + m[u];
+          for (int d = 0; d < 6; d++) sum[d] = r[d];
+        }
+      }
+    } else {
+      const int g = threadIdx.x >> 3, l = threadIdx.x & 7, shift = lane & 24;
+      double(*stage)[6] = &sh[0][8 * g];  // this group's 8 contributions
+      for (int r = 0; r < kBodies; r += kGatherNear / 8) {
+        const int64_t b = b0 + r + g;
+        const int* list = nullptr;
+        int L = 0;
+        double acc = 0.0;
+        if (b < s.n && s.needres[b]) {
+          const int64_t base = s.iofs[b] + s.jofs[b];
+          if (s.iofs[b + 1] + s.jofs[b + 1] - base <= kNearBig) {
+            L = s.gcnt[b];
+            list = s.glist + base;
+            if (b < s.n_driven || s.bf_kind != RK_BF_NONE) {
+              V3 F, M;
+              init_resultant(s, b, F, M);
+              acc = component(F, M, l);
+            }
           }
         }
-        finish_body(s, b, F, M, 1);
+        int Lw = L;  // rounds of the warp's longest list
+        Lw = max(Lw, __shfl_xor_sync(0xffffffffu, Lw, 8));
+        Lw = max(Lw, __shfl_xor_sync(0xffffffffu, Lw, 16));
+        fetch(list, l, L);
+        for (int p0 = 0; p0 < Lw; p0 += 8) {
+          const unsigned bal = (__ballot_sync(0xffffffffu, on) >> shift) & 0xffu;
+          if (on)
+#pragma unroll
+            for (int d = 0; d < 6; d++) stage[l][d] = c[d];
+          __syncwarp();
+          fetch(list, p0 + 8 + l, L);
+          for (unsigned m = bal; m; m &= m - 1u)
+            if (l < 6) acc = acc + stage[__ffs(m) - 1][l];
+          __syncwarp();
+        }
+        if (l < 6) res[r + g][l] = acc;
+      }
+      __syncthreads();
+      if (threadIdx.x < kBodies) {
+        const int64_t b = b0 + threadIdx.x;
+        if (b < s.n && !(s.needres[b] && s.iofs[b + 1] + s.jofs[b + 1] - s.iofs[b] - s.jofs[b] > kNearBig)) {
+          guard = b;
+#pragma unroll
+          for (int d = 0; d < 6; d++) sum[d] = res[threadIdx.x][d];
+        }
       }
     }
   }
-  if (s.sk_out) skin_guard_body(s, guard);
+  if (guard < s.n && s.needres[guard]) {
+    finish_body(s, guard, v3(sum[0], sum[1], sum[2]), v3(sum[3], sum[4], sum[5]), 1, kin);
+    have = guard >= s.n_driven;
+  }
+  if (s.sk_out) skin_guard_body_t<CvtBits>(s, guard, have, kin);
   if (s.sk_ctl) skin_batch_step_end(s);
 }
 

@@ -24,11 +24,8 @@ __device__ __forceinline__ double rot_bound(const double* q, const double* q0) {
   return 2.0 * c * (1.0 + c);
 }
 
-// FP64 -> float conversion of the guard: the hardware one (FP64 form) or
-// the integer-pipe one (mixed form); the margins below cover either.
-struct CvtHw {
-  __device__ static float f(double x) { return (float)x; }
-};
+// FP64 -> float conversion of the guard on the integer pipe; the margins
+// below cover its rounding.
 struct CvtBits {
   __device__ static float f(double x) { return d2f(x); }
 };
@@ -58,42 +55,60 @@ __device__ __forceinline__ void skin_guard_body_t(const Scene& s, int64_t b, boo
   unsigned int* out = s.sk_out;
   float dmax = 0.f, vmax = 0.f, gmax = 0.f, pdmax = 0.f, pgmax = 0.f;
   unsigned nflag = 0;
+  // (a batch reads no prediction: its steps are decided on the device)
+  const bool predict = s.sk_ctl == nullptr;
   if (b < s.n) {
+    const bool free_body = b >= s.n_driven;
+    // every load before the first store: one round trip instead of one per store
+    double x[3], x0[3], q[4], q0[4];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      x[d] = s.pos[3 * b + d];
+      x0[d] = ref_pos[3 * b + d];
+    }
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+      q[d] = s.Q[4 * b + d];
+      q0[d] = ref_q[4 * b + d];
+    }
+    const float sw = rsw[b], md0 = maxd[b], pth = free_body ? path[b] : INFINITY;
+    float k[12] = {};
+    if (have_kin) {
+#pragma unroll
+      for (int d = 0; d < 12; d++) k[d] = kin[d];
+    } else if (free_body) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        k[d] = C::f(s.vel[3 * b + d]);
+        k[3 + d] = C::f(s.acc[3 * b + d]);
+        k[6 + d] = C::f(s.vrot[3 * b + d]);
+        k[9 + d] = C::f(s.arot[3 * b + d]);
+      }
+    }
     // differences in FP64, the rest in float rounded up (relative 1e-5 covers
     // the float rounding of the norms, 1e-12 m the conversions)
-    const float dx = C::f(s.pos[3 * b] - ref_pos[3 * b]), dy = C::f(s.pos[3 * b + 1] - ref_pos[3 * b + 1]),
-                dz = C::f(s.pos[3 * b + 2] - ref_pos[3 * b + 2]);
+    const float dx = C::f(x[0] - x0[0]), dy = C::f(x[1] - x0[1]), dz = C::f(x[2] - x0[2]);
     float m2 = 0.f, p2 = 0.f;
+#pragma unroll
     for (int d = 0; d < 4; d++) {
-      const float m = C::f(s.Q[4 * b + d] - ref_q[4 * b + d]), p = C::f(s.Q[4 * b + d] + ref_q[4 * b + d]);
+      const float m = C::f(q[d] - q0[d]), p = C::f(q[d] + q0[d]);
       m2 += m * m;
       p2 += p * p;
     }
     const float chord = sqrtf(fminf(m2, p2)) * (1.f + 1e-5f);
-    dmax = (sqrtf(dx * dx + dy * dy + dz * dz) + 2.f * chord * (1.f + chord) * rsw[b]) * (1.f + 1e-5f) + 1e-12f;
-    const float md = fmaxf(maxd[b], dmax);
+    dmax = (sqrtf(dx * dx + dy * dy + dz * dz) + 2.f * chord * (1.f + chord) * sw) * (1.f + 1e-5f) + 1e-12f;
+    const float md = fmaxf(md0, dmax);
     maxd[b] = md;
     // driven bodies are moved by their controls, not by the drift: no path
-    const float pth = b >= s.n_driven ? path[b] : INFINITY;
     gmax = fminf(pth, 2.f * md);
     const bool f = gmax >= flag_at;
     flag[b] = f ? 1 : 0;
     nflag = f ? 1u : 0u;
-    if (b >= s.n_driven) {
-      float k[12];
-      if (have_kin) {
-#pragma unroll
-        for (int d = 0; d < 12; d++) k[d] = kin[d];
-      } else {
-        for (int d = 0; d < 3; d++) {
-          k[d] = C::f(s.vel[3 * b + d]);
-          k[3 + d] = C::f(s.acc[3 * b + d]);
-          k[6 + d] = C::f(s.vrot[3 * b + d]);
-          k[9 + d] = C::f(s.arot[3 * b + d]);
-        }
-      }
+    if (free_body) {
       const float vx = k[0], vy = k[1], vz = k[2];
       vmax = sqrtf(vx * vx + vy * vy + vz * vz);
+    }
+    if (predict && free_body) {
       // bound of the next drift: |dt v + dt^2/2 a| and a rotation of at most
       // |w| dt + |alpha| dt^2/2 (the normalised quaternion update, 1 % margin
       // for its second-order terms); a step of angle t moves the chord c by at
@@ -105,9 +120,9 @@ __device__ __forceinline__ void skin_guard_body_t(const Scene& s, int64_t b, boo
       const float dt = (float)s.dt, dt2 = (float)s.dt2_2;
       const float dxb = dt * vmax + dt2 * sqrtf(ax * ax + ay * ay + az * az);
       const float thb = dt * sqrtf(wx * wx + wy * wy + wz * wz) + dt2 * sqrtf(lx * lx + ly * ly + lz * lz);
-      const float inc = 1.01f * (dxb + thb * rsw[b] * (1.f + 2.f * chord + thb)) + 1e-12f;
+      const float inc = 1.01f * (dxb + thb * sw * (1.f + 2.f * chord + thb)) + 1e-12f;
       pdmax = dmax + inc;
-      pgmax = fminf(path[b] + inc, 2.f * fmaxf(md, pdmax));
+      pgmax = fminf(pth + inc, 2.f * fmaxf(md, pdmax));
     } else {
       pdmax = dmax;
       pgmax = gmax;
@@ -148,8 +163,10 @@ __device__ __forceinline__ void skin_guard_body_t(const Scene& s, int64_t b, boo
     atomicMax(&out[1], __float_as_uint(vmax));
     atomicMax(&out[2], __float_as_uint(gmax));
     if (nflag) atomicAdd(&out[3], nflag);
-    atomicMax(&out[6], __float_as_uint(pdmax));
-    atomicMax(&out[7], __float_as_uint(pgmax));
+    if (predict) {
+      atomicMax(&out[6], __float_as_uint(pdmax));
+      atomicMax(&out[7], __float_as_uint(pgmax));
+    }
   }
 }
 
@@ -166,31 +183,37 @@ __device__ __forceinline__ void skin_batch_step_end(const Scene& s) {
     last = atomicAdd(&s.sk_ctl[7], 1u) == gridDim.x - 1 ? 1 : 0;
   }
   __syncthreads();
-  if (!last || threadIdx.x != 0) return;
+  if (!last || threadIdx.x >= 32) return;
   __threadfence();
+  // a lane per word of the control block and of the guard: one round trip
+  // instead of one per word
   volatile unsigned int* ctl = s.sk_ctl;
   volatile unsigned int* out = s.sk_out;
-  const unsigned ex = ctl[1] + 1u, since = ctl[2] + 1u;
-  ctl[1] = ex;
-  ctl[2] = since;
-  ctl[7] = 0u;
-  unsigned int g[8];
-  for (int d = 0; d < 8; d++) {
-    g[d] = out[d];
-    ctl[8 + d] = g[d];
-  }
-  const float crit = __uint_as_float(ctl[6] ? g[2] : g[0]);
-  if (crit >= __uint_as_float(ctl[5]) || since >= ctl[4] || ex >= ctl[3]) {
-    ctl[0] = 1u;
-  } else {
-    for (int d = 0; d < 8; d++) out[d] = 0u;
+  const int l = threadIdx.x;
+  const unsigned full = 0xffffffffu;
+  const unsigned v = l < 8 ? ctl[l] : l < 16 ? out[l - 8] : 0u;
+  const unsigned ex = __shfl_sync(full, v, 1) + 1u, since = __shfl_sync(full, v, 2) + 1u;
+  const unsigned budget = __shfl_sync(full, v, 3), interval = __shfl_sync(full, v, 4);
+  const float trig = __uint_as_float(__shfl_sync(full, v, 5));
+  const unsigned path = __shfl_sync(full, v, 6);
+  const unsigned g0 = __shfl_sync(full, v, 8), g2 = __shfl_sync(full, v, 10);
+  const float crit = __uint_as_float(path ? g2 : g0);
+  const bool halt = crit >= trig || since >= interval || ex >= budget;
+  if (l == 0 && halt) ctl[0] = 1u;
+  else if (l == 1) ctl[1] = ex;
+  else if (l == 2) ctl[2] = since;
+  else if (l == 7) ctl[7] = 0u;
+  else if (l >= 8 && l < 16) {
+    ctl[l] = v;
+    if (!halt) out[l - 8] = 0u;
+  } else if (l == 16 && !halt) {
     s.flags[FLAG_NACTIVE] = 0ull;
   }
 }
 
 __device__ __forceinline__ void skin_guard_body(const Scene& s, int64_t b) {
   const float none[12] = {};
-  skin_guard_body_t<CvtHw>(s, b, false, none);
+  skin_guard_body_t<CvtBits>(s, b, false, none);
 }
 
 }  // namespace rk

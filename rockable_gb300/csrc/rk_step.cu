@@ -666,11 +666,11 @@ int launch_narrow_near(const Scene& s, cudaStream_t st) {
   return 1;
 }
 int launch_gather_near(const Scene& s, cudaStream_t st) {
-  const bool small = s.n < kSmallLaunch * 32;
-  const int t = small ? 32 : 128;
+  const int t = s.n < kSmallLaunch * 32 ? 32 : 128;
   if (s.fast_body) return launch_fused_gather_near(s, nblk(s.n, t), t, st);
-  if (small) exact::k_gather_near<32><<<(unsigned)s.nbig + nblk(s.n, 32), 32, 0, st>>>(s);
-  else exact::k_gather_near<128><<<(unsigned)s.nbig + nblk(s.n, 128), 128, 0, st>>>(s);
+  // 16 bodies a block until they fill the GPU (8 resident blocks per SM)
+  if (s.n < 16 * 8 * 152) exact::k_gather_near<16><<<(unsigned)s.nbig + nblk(s.n, 16), exact::kGatherNear, 0, st>>>(s);
+  else exact::k_gather_near<128><<<(unsigned)s.nbig + nblk(s.n, 128), exact::kGatherNear, 0, st>>>(s);
   return 1;
 }
 int launch_gather_accel(const Scene& s, int apply_kick, cudaStream_t st) {
