@@ -290,40 +290,39 @@ __device__ __forceinline__ bool obb_pair_intersect(const Scene& s, int64_t i, in
 }
 
 // All-pairs broad phase: float AABB filter (tiled through shared memory),
-// then eligibility and the FP64 SAT of the enlarged OBBs.
+// then eligibility and the FP64 SAT of the enlarged OBBs.  One block per
+// pair of tiles (upper triangle; blockIdx.x, blockIdx.y the tiles): a block
+// per tile that walked all others left a few long blocks on the GPU (1.15 ms
+// at 1700 bodies).
 constexpr int kPairTile = 128;
-__global__ void k_pairs(Scene s, const uint8_t* only, uint64_t* pairs, int64_t cap, unsigned long long* counter) {
+__global__ void __launch_bounds__(kPairTile) k_pairs(Scene s, const uint8_t* only, uint64_t* pairs, int64_t cap,
+                                                     unsigned long long* counter) {
+  if (blockIdx.y < blockIdx.x) return;
   __shared__ float sb[kPairTile][6];
   const int64_t i = blockIdx.x * (int64_t)kPairTile + threadIdx.x;
-  const bool vi = i < s.n;
+  const int64_t j0 = blockIdx.y * (int64_t)kPairTile, jl = j0 + threadIdx.x;
   float a[6];
-  for (int k = 0; k < 6; k++) a[k] = vi ? s.baabb[6 * i + k] : 0.f;
-  const int64_t jstart = blockIdx.x * (int64_t)kPairTile;
-  for (int64_t j0 = jstart; j0 < s.n; j0 += kPairTile) {
-    __syncthreads();
-    int64_t jl = j0 + threadIdx.x;
-    if (jl < s.n)
-      for (int k = 0; k < 6; k++) sb[threadIdx.x][k] = s.baabb[6 * jl + k];
-    __syncthreads();
-    if (!vi) continue;
-    int jn = (int)min((int64_t)kPairTile, s.n - j0);
-    for (int t = 0; t < jn; t++) {
-      int64_t j = j0 + t;
-      if (j <= i) continue;
-      if (a[0] > sb[t][3] || sb[t][0] > a[3] || a[1] > sb[t][4] || sb[t][1] > a[4] || a[2] > sb[t][5] ||
-          sb[t][2] > a[5])
-        continue;
-      if (i < s.n_driven && j < s.n_driven) continue;
-      if (only && !only[i] && !only[j]) continue;
-      if (s.scene_of && s.scene_of[i] != s.scene_of[j]) continue;
-      if (has_iface(s, (int)i, (int)j)) continue;
-      if (!obb_pair_intersect(s, i, j)) continue;
-      unsigned long long k = atomicAdd(counter, 1ull);
-      if ((int64_t)k < cap) pairs[k] = ((uint64_t)i << 21) | (uint64_t)j;
-    }
+  for (int k = 0; k < 6; k++) a[k] = i < s.n ? s.baabb[6 * i + k] : 0.f;
+  if (jl < s.n)
+    for (int k = 0; k < 6; k++) sb[threadIdx.x][k] = s.baabb[6 * jl + k];
+  __syncthreads();
+  if (i >= s.n) return;
+  const int jn = (int)min((int64_t)kPairTile, s.n - j0);
+  for (int t = 0; t < jn; t++) {
+    const int64_t j = j0 + t;
+    if (j <= i) continue;
+    if (a[0] > sb[t][3] || sb[t][0] > a[3] || a[1] > sb[t][4] || sb[t][1] > a[4] || a[2] > sb[t][5] ||
+        sb[t][2] > a[5])
+      continue;
+    if (i < s.n_driven && j < s.n_driven) continue;
+    if (only && !only[i] && !only[j]) continue;
+    if (s.scene_of && s.scene_of[i] != s.scene_of[j]) continue;
+    if (has_iface(s, (int)i, (int)j)) continue;
+    if (!obb_pair_intersect(s, i, j)) continue;
+    unsigned long long k = atomicAdd(counter, 1ull);
+    if ((int64_t)k < cap) pairs[k] = ((uint64_t)i << 21) | (uint64_t)j;
   }
 }
-
 
 // ------------------------------------------------------------- grid ----
 // Uniform grid broad phase (the role of Rockable's linkCells,
@@ -1577,9 +1576,9 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
     RKCHK(cudaStreamSynchronize(st));
     nover = (int64_t)no_;
     if ((rc = ensure_tmp(c, (int64_t)sort_temp_bytes(N)))) return rc;
-    radix_sort_u64(w.gkeys, w.gtmp, N, 21, 21 + fmt.total, w.tmp, st);
+    c.kernels += radix_sort_u64(w.gkeys, w.gtmp, N, 21, 21 + fmt.total, w.tmp, st, s.flags + FLAG_ERROR);
     if (nover > 0) k_mark_over<<<nblk(nover, 256), 256, 0, st>>>(w.gover, (int)nover, w.gis_over);
-    c.kernels += 16;
+    c.kernels += 2;
     for (int attempt = 0; attempt < 4; attempt++) {
       RKCHK(cudaMemsetAsync(w.counter, 0, 8, st));
       k_grid_pairs<<<nblk(9 * kGridLanes * (N - nover), 128), 128, 0, st>>>(s, fmt, only, w.gkeys, N - nover,
@@ -1602,7 +1601,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
   } else {
     for (int attempt = 0; attempt < 4; attempt++) {
       RKCHK(cudaMemsetAsync(w.counter, 0, 8, st));
-      k_pairs<<<nblk(N, kPairTile), kPairTile, 0, st>>>(s, only, w.pairs, w.pair_cap, w.counter);
+      k_pairs<<<dim3(nblk(N, kPairTile), nblk(N, kPairTile)), kPairTile, 0, st>>>(s, only, w.pairs, w.pair_cap, w.counter);
       c.kernels++;
       unsigned long long cnt = 0;
       RKCHK(cudaMemcpyAsync(&cnt, w.counter, 8, cudaMemcpyDeviceToHost, st));
@@ -1652,8 +1651,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
   if (np > 0) {
     k_half_pairs<<<nblk(np, 256), 256, 0, st>>>(w.pairs, np, w.hp);
     c.kernels++;
-    radix_sort_u64(w.hp, w.hp_tmp, nhp, 0, 21 + body_bits(N), w.tmp, st);  // (owner << 21) | partner
-    c.kernels += 13;
+    c.kernels += radix_sort_u64(w.hp, w.hp_tmp, nhp, 0, 21 + body_bits(N), w.tmp, st, s.flags + FLAG_ERROR);  // (owner << 21) | partner
   }
   // ---- candidates: appended by one warp per half-pair, then sorted by key
   int64_t ncand = 0, nunsure = 0;
@@ -1706,8 +1704,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
       // (vertex-vertex, vertex-edge, vertex-face, edge-edge, each by
       // ascending sub-element indices, i.e. by ascending key), chunk after
       // chunk with increasing atomically reserved offsets.
-      radix_sort_u64(w.cand, w.cand_tmp, ncand, 22, 43 + body_bits(N), w.tmp, st);
-      c.kernels += 25;
+      c.kernels += radix_sort_u64(w.cand, w.cand_tmp, ncand, 22, 43 + body_bits(N), w.tmp, st, s.flags + FLAG_ERROR);
     }
   }
   // ---- old entries kept untouched
@@ -1762,9 +1759,9 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
   c.kernels++;
   if (nf > 0) {
     k_jkeys<<<nblk(nf, 256), 256, 0, st>>>(s.ej, nf, w.jkeys);
-    radix_sort_u64(w.jkeys, w.jtmp, nf, 27, 51, w.tmp, st);
+    c.kernels += radix_sort_u64(w.jkeys, w.jtmp, nf, 27, 27 + body_bits(N), w.tmp, st, s.flags + FLAG_ERROR);
     k_jlist<<<nblk(nf, 256), 256, 0, st>>>(w.jkeys, nf, s.jlist);
-    c.kernels += 11;
+    c.kernels += 2;
   }
   k_jofs<<<nblk(N + 1, 256), 256, 0, st>>>(w.jkeys, nf, N, s.jofs);
   c.kernels++;
@@ -1800,9 +1797,9 @@ static int entry_order(Ctx& c) {
     return RK_ERR_STATE;
   }
   k_type_keys<<<nblk(ne, 256), 256, 0, c.stream>>>(s.etsub, ne, w.jkeys);
-  radix_sort_u64(w.jkeys, w.jtmp, ne, 40, 42, w.tmp, c.stream);
+  c.kernels += radix_sort_u64(w.jkeys, w.jtmp, ne, 40, 42, w.tmp, c.stream, s.flags + FLAG_ERROR);
   k_type_perm<<<nblk(ne, 256), 256, 0, c.stream>>>(w.jkeys, ne, s.nperm, s.flags + FLAG_TOFS);
-  c.kernels += 5;
+  c.kernels += 2;
   return 0;
 }
 

@@ -19,8 +19,8 @@
 // whole array, so calls that overlap on the GPU (two streams, or two host
 // threads on one device) overwrite each other's data: the caller must order
 // them.  Calls in sequence share the array, which keeps what the last call
-// left; no part of it has to start at zero, because each radix pass writes
-// its histogram, offsets and output keys before reading them.
+// left; no part of it has to start at zero, because a sort clears its counters
+// and status words and each pass writes its output keys before they are read.
 //
 // The first call on each device does a one-time set-up: it looks up the
 // device address of the array (cudaGetSymbolAddress) with that device current.
