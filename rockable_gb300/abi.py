@@ -453,13 +453,19 @@ class GpuScene:
         """(Particles lines, Interactions lines, number of the latter) of a
         conf file, formatted on the device (rk_format_conf)."""
         lp, li, na = C.c_int64(), C.c_int64(), C.c_int64()
-        self._chk(self.L.rk_format_conf(self.h, precision, None, 0, C.byref(lp), C.byref(li), C.byref(na)),
-                  "rk_format_conf")
-        buf = C.create_string_buffer(lp.value + li.value + 1)
-        self._chk(self.L.rk_format_conf(self.h, precision, buf, lp.value + li.value, C.byref(lp), C.byref(li),
-                                        C.byref(na)), "rk_format_conf")
-        raw = buf.raw[:lp.value + li.value].decode()
-        return raw[:lp.value], raw[lp.value:], na.value
+        # room for the bodies and six contacts each (pages that are not
+        # written cost nothing); more contacts: a second call with the lengths
+        width = precision + 9
+        cap = self.n * (20 * width + 64) + 6 * self.n * (18 * width + 40)
+        while True:
+            buf = np.empty(max(cap, 1), np.uint8)
+            rc = self.L.rk_format_conf(self.h, precision, buf.ctypes.data_as(C.c_char_p), cap, C.byref(lp), C.byref(li), C.byref(na))
+            if ERRORS.get(rc) != "RK_ERR_CAPACITY" or lp.value + li.value <= cap:
+                break
+            cap = lp.value + li.value
+        self._chk(rc, "rk_format_conf")
+        raw = memoryview(buf)
+        return str(raw[:lp.value], "utf-8"), str(raw[lp.value:lp.value + li.value], "utf-8"), na.value
 
     def contributions(self):
         """Per-entry force on i and moments on i and j of the last force

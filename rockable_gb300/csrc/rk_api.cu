@@ -873,6 +873,7 @@ void rk_destroy(rk_ctx* x) {
   dfree(w.tmp); dfree(w.counter); dfree(w.gkeys); dfree(w.gtmp); dfree(w.gover); dfree(w.gis_over); dfree(w.gmark);
   if (w.gstat) cudaFree(w.gstat);
   if (w.split) cudaEventDestroy(w.split);
+  dfree(c.conf.lens); dfree(c.conf.ofs); dfree(c.conf.flag); dfree(c.conf.tmp); dfree(c.conf.slots); dfree(c.conf.out);
   dfree(c.kin_stage);
   dfree(c.ext_part);
   dfree(c.ext_u);
@@ -1773,34 +1774,34 @@ int rk_format_conf(rk_ctx* x, int32_t prec, char* buf, int64_t cap, int64_t* par
   cudaStream_t st = c.stream;
   const int64_t nb = s.n, ne = s.ne;
   // bodies: one slot each, then the active entries: flags, their positions
-  char* slots = nullptr;
-  int64_t *lens = nullptr, *ofs = nullptr, *flag = nullptr;
-  void* tmp = nullptr;
-  char* out = nullptr;
+  // (the context keeps the buffers for the next file)
+  Ctx::ConfWork& w = c.conf;
   int rc = RK_OK;
   int64_t lp = 0, li = 0, na = 0;
-  auto cleanup = [&]() {
-    dfree(slots); dfree(lens); dfree(ofs); dfree(flag); dfree(out);
-    if (tmp) cudaFree(tmp);
-  };
   const int64_t nmax = std::max<int64_t>(nb, ne) + 1;
-  if ((rc = dalloc(c, lens, nmax)) || (rc = dalloc(c, ofs, nmax)) || (rc = dalloc(c, flag, ne + 1))) {
-    cleanup();
-    return rc;
+  if (w.lines < nmax) {
+    const int64_t cap = nmax + nmax / 4;
+    w.lines = 0;
+    if ((rc = dalloc(c, w.lens, cap)) || (rc = dalloc(c, w.ofs, cap)) || (rc = dalloc(c, w.flag, cap)) ||
+        (rc = dalloc(c, w.tmp, (int64_t)scan_temp_bytes(cap))))
+      return rc;
+    w.lines = cap;
   }
-  if (cudaMalloc(&tmp, scan_temp_bytes(nmax)) != cudaSuccess) {
-    cleanup();
-    return fail(c, RK_ERR_CUDA, "no device memory for the conf text");
-  }
+  int64_t *const lens = w.lens, *const ofs = w.ofs, *const flag = w.flag;
+  char* const tmp = w.tmp;
+  auto grow = [&](char*& p, int64_t& have, int64_t want) {
+    if (have >= want) return (int)RK_OK;
+    have = 0;
+    const int r = dalloc(c, p, want + want / 4);
+    if (!r) have = want + want / 4;
+    return r;
+  };
   if (ne > 0) {
     k_conf_active<<<nblk(ne, 256), 256, 0, st>>>(s, flag);
     cudaMemsetAsync(flag + ne, 0, sizeof(int64_t), st);
     exclusive_scan_i64(flag, flag, ne + 1, tmp, st);
     cudaMemcpyAsync(&na, flag + ne, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
-      cleanup();
-      return fail(c, RK_ERR_CUDA, "conf text: active entries");
-    }
+    if (cudaStreamSynchronize(st) != cudaSuccess) return fail(c, RK_ERR_CUDA, "conf text: active entries");
   }
   // the two sections, one after the other
   for (int part = 0; part < 2; part++) {
@@ -1808,9 +1809,9 @@ int rk_format_conf(rk_ctx* x, int32_t prec, char* buf, int64_t cap, int64_t* par
     const int slot = part == 0 ? kConfBodySlot : kConfEntrySlot;
     int64_t& len = part == 0 ? lp : li;
     if (nl == 0) continue;
-    dfree(slots);
-    if ((rc = dalloc(c, slots, nl * (int64_t)slot))) break;
-    if (part == 0) k_conf_bodies<<<nblk(nb, 128), 128, 0, st>>>(s, c.name_chars, c.name_ofs, prec, slots, lens);
+    if ((rc = grow(w.slots, w.slot_bytes, nl * (int64_t)slot))) break;
+    char* const slots = w.slots;
+    if (part == 0) k_conf_bodies<<<nblk(32 * nb, 128), 128, 0, st>>>(s, c.name_chars, c.name_ofs, prec, slots, lens);
     else k_conf_entries<<<nblk(ne, 128), 128, 0, st>>>(s, flag, prec, slots, lens);
     cudaMemsetAsync(lens + nl, 0, sizeof(int64_t), st);
     exclusive_scan_i64(lens, ofs, nl + 1, tmp, st);
@@ -1818,17 +1819,15 @@ int rk_format_conf(rk_ctx* x, int32_t prec, char* buf, int64_t cap, int64_t* par
     if (cudaStreamSynchronize(st) != cudaSuccess) { rc = fail(c, RK_ERR_CUDA, "conf text: formatting"); break; }
     const int64_t at = part == 0 ? 0 : lp;
     if (buf && at + len <= cap) {
-      dfree(out);
-      if ((rc = dalloc(c, out, std::max<int64_t>(len, 1)))) break;
-      k_conf_pack<<<nblk(nl * 32, 256), 256, 0, st>>>(slots, slot, ofs, lens, nl, out);
-      if (cudaMemcpyAsync(buf + at, out, (size_t)len, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      if ((rc = grow(w.out, w.out_bytes, std::max<int64_t>(len, 1)))) break;
+      k_conf_pack<<<nblk(nl * 32, 256), 256, 0, st>>>(slots, slot, ofs, lens, nl, w.out);
+      if (cudaMemcpyAsync(buf + at, w.out, (size_t)len, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
           cudaStreamSynchronize(st) != cudaSuccess) {
         rc = fail(c, RK_ERR_CUDA, "conf text: copy");
         break;
       }
     }
   }
-  cleanup();
   if (rc) return rc;
   if (particles_len) *particles_len = lp;
   if (interactions_len) *interactions_len = li;

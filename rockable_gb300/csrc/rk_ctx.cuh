@@ -162,6 +162,12 @@ struct Ctx {
   int64_t kin_stage_n = 0;
   std::vector<uint8_t> needres_host;
   int64_t bf_n = 0;  // body count the body force was set for
+  // buffers of the device-formatted conf text, grown on demand
+  struct ConfWork {
+    int64_t lines = 0, slot_bytes = 0, out_bytes = 0;
+    int64_t *lens = nullptr, *ofs = nullptr, *flag = nullptr;
+    char *tmp = nullptr, *slots = nullptr, *out = nullptr;
+  } conf;
   // shape names for the device-formatted conf text (rk_set_shape_names)
   char* name_chars = nullptr;
   int* name_ofs = nullptr;
