@@ -369,9 +369,12 @@ __global__ void k_gather_accel(Scene s, int apply_kick) {
 // control) have no state to update.
 // 3000 grains 42 us (GEOM list, thread per body) before; the box of 200 000
 // grains 1.19 ms on whole lists with shuffles instead of shared memory.
+// WHOLE: the same on the whole list, for small scenes (kBodies = 16): every
+// body that is not deferred (is_heavy 2), its positions found through the
+// serial order.
 constexpr int kGatherNear = 128;
-template <int kBodies>
-__global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
+template <int kBodies, bool WHOLE>
+__global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s, int apply_kick) {
   if (step_halted(s)) return;
   __shared__ double sh[2][kGatherNear][6];
   __shared__ double res[kBodies == kGatherNear ? 1 : kBodies][6];
@@ -383,10 +386,16 @@ __global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
   double sum[6] = {0, 0, 0, 0, 0, 0};  // the resultant of body `guard`
   double c[6];
   bool on = false;
+  // position p of a list (WHOLE: of the body whose offsets are in `own`)
+  int64_t own[5] = {0, 0, 0, 0, 0};  // j-side positions before the own block, end of the block, iofs, jofs, jsplit
   auto fetch = [&](const int* list, int p, int L) {
     on = false;
     if (p >= L) return;
-    const int x = list[p];
+    int x;
+    if (!WHOLE) x = list[p];
+    else if (p < own[0]) x = s.jlist[own[3] + p] | (int)0x80000000;
+    else if (p < own[1]) x = (int)(own[2] + (p - own[0]));
+    else x = s.jlist[own[4] + (p - own[1])] | (int)0x80000000;
     const int64_t e = x & kGlistEntry;
     on = s.act[e] != 0;
     if (!on) return;
@@ -395,13 +404,28 @@ __global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
     c[0] = jside ? -f.x : f.x; c[1] = jside ? -f.y : f.y; c[2] = jside ? -f.z : f.z;
     c[3] = m.x; c[4] = m.y; c[5] = m.z;
   };
+  // whether the step uses body b's resultant, and the length of its list
+  auto used = [&](int64_t b) { return WHOLE ? s.is_heavy[b] != 2 : s.needres[b] != 0; };
+  auto list_of = [&](int64_t b, int& L) -> const int* {
+    if (!WHOLE) {
+      L = s.gcnt[b];
+      return s.glist + s.iofs[b] + s.jofs[b];
+    }
+    own[2] = s.iofs[b];
+    own[3] = s.jofs[b];
+    own[4] = s.jsplit[b];
+    own[0] = own[4] - own[3];
+    own[1] = own[0] + (s.iofs[b + 1] - own[2]);
+    L = (int)(own[1] + (s.jofs[b + 1] - own[4]));
+    return nullptr;
+  };
   auto component = [&](V3 F, V3 M, int d) {
     return d == 0 ? F.x : d == 1 ? F.y : d == 2 ? F.z : d == 3 ? M.x : d == 4 ? M.y : M.z;
   };
   if ((int)blockIdx.x < s.nbig) {
     const int64_t b = s.big[blockIdx.x];
-    const int* list = s.glist + s.iofs[b] + s.jofs[b];
-    const int L = s.gcnt[b];
+    int L;
+    const int* list = list_of(b, L);
     V3 F, M;
     init_resultant(s, b, F, M);
     double acc = component(F, M, lane);
@@ -442,13 +466,13 @@ __global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
     }
   } else {
     const int64_t b0 = ((int64_t)blockIdx.x - s.nbig) * kBodies;
-    if constexpr (kBodies == kGatherNear) {
+    if constexpr (kBodies == kGatherNear) {  // (near set only)
       const int64_t b = b0 + threadIdx.x;
       if (b < s.n) {
         const int64_t base = s.iofs[b] + s.jofs[b];
-        const bool used = s.needres[b] != 0;
-        if (!(used && s.iofs[b + 1] + s.jofs[b + 1] - base > kNearBig)) guard = b;
-        if (used && guard == b) {
+        const bool take = s.needres[b] != 0;
+        if (!(take && s.iofs[b + 1] + s.jofs[b + 1] - base > kNearBig)) guard = b;
+        if (take && guard == b) {
           const int L = s.gcnt[b];
           const int* list = s.glist + base;
           V3 F, M;
@@ -487,11 +511,9 @@ __global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
         const int* list = nullptr;
         int L = 0;
         double acc = 0.0;
-        if (b < s.n && s.needres[b]) {
-          const int64_t base = s.iofs[b] + s.jofs[b];
-          if (s.iofs[b + 1] + s.jofs[b + 1] - base <= kNearBig) {
-            L = s.gcnt[b];
-            list = s.glist + base;
+        if (b < s.n && used(b)) {
+          if (!(s.needres[b] && s.iofs[b + 1] + s.jofs[b + 1] - s.iofs[b] - s.jofs[b] > kNearBig)) {
+            list = list_of(b, L);
             if (b < s.n_driven || s.bf_kind != RK_BF_NONE) {
               V3 F, M;
               init_resultant(s, b, F, M);
@@ -527,11 +549,15 @@ __global__ void __launch_bounds__(kGatherNear) k_gather_near(Scene s) {
       }
     }
   }
-  if (guard < s.n && s.needres[guard]) {
-    finish_body(s, guard, v3(sum[0], sum[1], sum[2]), v3(sum[3], sum[4], sum[5]), 1, kin);
+  if (guard < s.n && used(guard)) {
+    finish_body(s, guard, v3(sum[0], sum[1], sum[2]), v3(sum[3], sum[4], sum[5]), apply_kick, kin);
     have = guard >= s.n_driven;
+  } else if (WHOLE && guard < s.n) {
+    // a driven body whose resultant feeds no state: summed on demand
+    st3(s.acc, guard, v3(0, 0, 0));
+    st3(s.arot, guard, v3(0, 0, 0));
   }
-  if (s.sk_out) skin_guard_body_t<CvtBits>(s, guard, have, kin);
+  if (s.sk_out && apply_kick) skin_guard_body_t<CvtBits>(s, guard, have, kin);
   if (s.sk_ctl) skin_batch_step_end(s);
 }
 

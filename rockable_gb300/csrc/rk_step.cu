@@ -436,54 +436,61 @@ __global__ void __launch_bounds__(kNarrowNear) k_narrow_near(Scene s) {
 // ----------------------------------------------------------------- K3 ----
 // Bodies with many entries: one warp per body.  The lanes load 32 positions
 // of the serial order at a time (the j-side entries before the body's own
-// block, its block, the rest of the j-side: jsplit), and lanes 0-5 each add
-// one of the six components (F.x, F.y, F.z, M.x, M.y, M.z) of those 32
-// contributions, broadcast by shuffles, in that order: the same sums as the
-// one-thread loop (F - f added as F + (-f), which IEEE arithmetic makes the
-// same number), six short chains instead of one long one.
+// block, its block, the rest of the j-side: jsplit) and pack the active ones
+// in shared memory, and lanes 0-5 each add one of the six components (F.x,
+// F.y, F.z, M.x, M.y, M.z) in that order while the next 32 positions are on
+// their way: the same sums as the one-thread loop (F - f added as F + (-f),
+// which IEEE arithmetic makes the same number), one addition per contact
+// (64 cycles on GB300; broadcasting by shuffles took about 160).
 constexpr int kHeavyWarps = 4;  // warps per block
 __global__ void __launch_bounds__(32 * kHeavyWarps) k_gather_heavy(Scene s, const int* list, int count) {
   if (step_halted(s)) return;
+  __shared__ double stage[kHeavyWarps][32][6];
   const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= count) return;
+  double(*sh)[6] = stage[threadIdx.x >> 5];
   const int b = list[w];
   const int64_t i0 = s.iofs[b], i1 = s.iofs[b + 1];
   const int64_t j0 = s.jofs[b], j1 = s.jofs[b + 1], js = s.jsplit[b];
   const int64_t nA = js - j0, nB = i1 - i0, L = nA + nB + (j1 - js);
   V3 F, M;
   init_resultant(s, b, F, M);
-  const double start[6] = {F.x, F.y, F.z, M.x, M.y, M.z};
-  double acc = lane < 6 ? start[lane] : 0.0;
+  double acc = lane == 0 ? F.x : lane == 1 ? F.y : lane == 2 ? F.z : lane == 3 ? M.x : lane == 4 ? M.y : M.z;
+  double c[6];
+  bool on = false;
+  auto fetch = [&](int64_t p) {
+    on = false;
+    if (p >= L) return;
+    int64_t e;
+    bool jside = true;
+    if (p < nA) e = s.jlist[j0 + p];
+    else if (p < nA + nB) {
+      e = i0 + (p - nA);
+      jside = false;
+    } else e = s.jlist[js + (p - nA - nB)];
+    on = s.act[e] != 0;
+    if (!on) return;
+    const V3 f = ld3(s.cf, e), m = jside ? ld3(s.cmj, e) : ld3(s.cmi, e);
+    c[0] = jside ? -f.x : f.x;
+    c[1] = jside ? -f.y : f.y;
+    c[2] = jside ? -f.z : f.z;
+    c[3] = m.x; c[4] = m.y; c[5] = m.z;
+  };
+  fetch(lane);
   for (int64_t c0 = 0; c0 < L; c0 += 32) {
-    const int64_t p = c0 + lane;
-    int valid = 0;
-    double c[6] = {0, 0, 0, 0, 0, 0};
-    if (p < L) {
-      int64_t e;
-      bool jside;
-      if (p < nA) { e = s.jlist[j0 + p]; jside = true; }
-      else if (p < nA + nB) { e = i0 + (p - nA); jside = false; }
-      else { e = s.jlist[js + (p - nA - nB)]; jside = true; }
-      if (s.act[e]) {
-        valid = 1;
-        const V3 f = ld3(s.cf, e), m = jside ? ld3(s.cmj, e) : ld3(s.cmi, e);
-        c[0] = jside ? -f.x : f.x;
-        c[1] = jside ? -f.y : f.y;
-        c[2] = jside ? -f.z : f.z;
-        c[3] = m.x; c[4] = m.y; c[5] = m.z;
-      }
+    const unsigned any = __ballot_sync(0xffffffffu, on);
+    if (on) {
+      const int at = __popc(any & ((1u << lane) - 1u));
+#pragma unroll
+      for (int d = 0; d < 6; d++) sh[at][d] = c[d];
     }
-    const unsigned any = __ballot_sync(0xffffffffu, valid);
-    const int nk = (int)min((int64_t)32, L - c0);
-    for (int k = 0; k < nk; k++) {
-      if (!((any >> k) & 1u)) continue;
-      const double v0 = __shfl_sync(0xffffffffu, c[0], k), v1 = __shfl_sync(0xffffffffu, c[1], k);
-      const double v2 = __shfl_sync(0xffffffffu, c[2], k), v3_ = __shfl_sync(0xffffffffu, c[3], k);
-      const double v4 = __shfl_sync(0xffffffffu, c[4], k), v5 = __shfl_sync(0xffffffffu, c[5], k);
-      const double v = lane == 0 ? v0 : lane == 1 ? v1 : lane == 2 ? v2 : lane == 3 ? v3_ : lane == 4 ? v4 : v5;
-      if (lane < 6) acc = acc + v;
-    }
+    __syncwarp();
+    fetch(c0 + 32 + lane);
+    const int nk = __popc(any);
+    if (lane < 6)
+      for (int k = 0; k < nk; k++) acc = acc + sh[k][lane];
+    __syncwarp();
   }
   if (lane < 3) s.force[3 * (int64_t)b + lane] = acc;
   else if (lane < 6) s.moment[3 * (int64_t)b + lane - 3] = acc;
@@ -665,18 +672,24 @@ int launch_narrow_near(const Scene& s, cudaStream_t st) {
   k_narrow_near<<<(unsigned)std::max<int64_t>(blocks, 1), t, 0, st>>>(s);
   return 1;
 }
+// 16 bodies a block until they fill the GPU (8 resident blocks per SM)
+static inline bool gather_small(const Scene& s) { return s.n < 16 * 8 * 152; }
 int launch_gather_near(const Scene& s, cudaStream_t st) {
   const int t = s.n < kSmallLaunch * 32 ? 32 : 128;
   if (s.fast_body) return launch_fused_gather_near(s, nblk(s.n, t), t, st);
-  // 16 bodies a block until they fill the GPU (8 resident blocks per SM)
-  if (s.n < 16 * 8 * 152) exact::k_gather_near<16><<<(unsigned)s.nbig + nblk(s.n, 16), exact::kGatherNear, 0, st>>>(s);
-  else exact::k_gather_near<128><<<(unsigned)s.nbig + nblk(s.n, 128), exact::kGatherNear, 0, st>>>(s);
+  const unsigned big = (unsigned)s.nbig;
+  if (gather_small(s)) exact::k_gather_near<16, false><<<big + nblk(s.n, 16), exact::kGatherNear, 0, st>>>(s, 1);
+  else exact::k_gather_near<128, false><<<big + nblk(s.n, 128), exact::kGatherNear, 0, st>>>(s, 1);
   return 1;
 }
 int launch_gather_accel(const Scene& s, int apply_kick, cudaStream_t st) {
   if (s.n <= 0) return 0;
   const int t = tpb_or(s, 1, 128, s.n);
   if (s.fast_body) return launch_fused_gather(s, nblk(s.n, t), t, apply_kick, st);  // one body per thread
+  if (gather_small(s)) {  // (the bodies of many entries included: 32 us -> 13 us at 512 bodies)
+    exact::k_gather_near<16, true><<<(unsigned)s.nbig + nblk(s.n, 16), exact::kGatherNear, 0, st>>>(s, apply_kick);
+    return 1;
+  }
   exact::k_gather_accel<<<nblk(s.n, t), t, 0, st>>>(s, apply_kick);
   return 1;
 }
@@ -695,6 +708,7 @@ int max_tpb(int which, int form_mixed) {
 int launch_gather_heavy(const Scene& s, cudaStream_t st) {
   if (s.nheavy <= 0) return 0;
   if (s.fast_body) return launch_fused_heavy(s, s.heavy, (int)s.nheavy, st);
+  if (gather_small(s)) return 0;  // (summed by the resultant kernel itself)
   k_gather_heavy<<<(unsigned)((s.nheavy + kHeavyWarps - 1) / kHeavyWarps), 32 * kHeavyWarps, 0, st>>>(
       s, s.heavy, (int)s.nheavy);
   return 1;

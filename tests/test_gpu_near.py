@@ -90,3 +90,28 @@ def test_near_set_steps_equal_whole_list_steps(gpu_lib, form, kind, speed):
     assert seen > 20
     a.close()
     b.close()
+
+
+def test_big_body_resultant_is_the_serial_sum(gpu_lib):
+    """The block that sums a body of more than 1024 entries (whole list and
+    near set) adds the contributions in the serial order, bit for bit: the
+    components that start from zero of the servo walls' resultants."""
+    sc = _scene("wall", 0.3)
+    g = _engine(sc, 0, False)
+    for steps in (1, 6):
+        g.step(steps)
+        e, f = g.entries(), g.contributions()
+        b = g.bodies()
+        for w, axis in ((1, 0), (3, 1)):
+            idx = np.nonzero(((e["i"] == w) | (e["j"] == w)))[0]
+            assert len(idx) > 1024
+            F, M = np.zeros(3), np.zeros(3)
+            for k in idx[e["active"][idx]]:
+                own = e["i"][k] == w
+                F = F + f[0][k] if own else F - f[0][k]
+                M = M + (f[1][k] if own else f[2][k])
+            for d in range(3):
+                if d != axis:
+                    assert bitwise_equal(F[d:d + 1], b["force"][w, d:d + 1]), (steps, w, d)
+            assert bitwise_equal(M, b["moment"][w]), (steps, w)
+    g.close()
