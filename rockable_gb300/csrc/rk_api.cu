@@ -868,7 +868,7 @@ void rk_destroy(rk_ctx* x) {
   free_entrybuf(c.eb[0]);
   free_entrybuf(c.eb[1]);
   NLWork& w = c.w;
-  dfree(w.pairs); dfree(w.hp); dfree(w.hp_tmp); dfree(w.hp_mask); dfree(w.cand); dfree(w.cand_tmp); dfree(w.cand_unsure);
+  dfree(w.pairs); dfree(w.pair_tmp); dfree(w.cand); dfree(w.cand_tmp); dfree(w.cand_unsure);
   dfree(w.flag); dfree(w.stale); dfree(w.stale_src); dfree(w.fkey); dfree(w.fsrc); dfree(w.jkeys); dfree(w.jtmp);
   dfree(w.tmp); dfree(w.counter); dfree(w.gkeys); dfree(w.gtmp); dfree(w.gover); dfree(w.gis_over); dfree(w.gmark);
   if (w.gstat) cudaFree(w.gstat);

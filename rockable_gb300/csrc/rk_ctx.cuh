@@ -25,11 +25,9 @@ struct EntryBuf {
 struct NLWork {
   cudaEvent_t split = nullptr;   // recorded after the pairs (when timing_split)
   bool timing_split = false;
-  int64_t pair_cap = 0, hp_cap = 0, cand_cap = 0, old_cap = 0, fin_cap = 0, tmp_bytes = 0;
+  int64_t pair_cap = 0, pair_tmp_cap = 0, cand_cap = 0, old_cap = 0, fin_cap = 0, tmp_bytes = 0;
   uint64_t* pairs = nullptr;     // pair_cap
-  uint64_t* hp = nullptr;        // hp_cap (half-pair keys owner<<21 | partner)
-  uint64_t* hp_tmp = nullptr;    // hp_cap
-  uint32_t* hp_mask = nullptr;   // kMaskWords * hp_cap
+  uint64_t* pair_tmp = nullptr;  // pair_tmp_cap (sort)
   uint64_t* cand = nullptr;      // cand_cap new entry keys
   uint64_t* cand_tmp = nullptr;  // cand_cap (sort)
   uint32_t* cand_unsure = nullptr;  // cand_cap: positions of the keys the float classification left undecided

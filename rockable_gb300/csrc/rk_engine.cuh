@@ -29,7 +29,6 @@ constexpr int kGatherLanes = 8;
 
 constexpr int kMaxSub = 1024;       // sub-element index limit of the sort key
 constexpr int kMaxBody = 1 << 21;   // body index limit of the sort key
-constexpr int kMaskWords = 2;       // vertex cull mask words per half-pair (<= 64 vertices)
 constexpr int kHeavy = 64;          // entries above which a body's resultant is summed by a block
 constexpr int kHeavyWarp = 1024;    // mixed form: up to this many, by its warp inside the resultant kernel
 constexpr int kGlistLane = 28, kGlistEntry = (1 << 27) - 1;  // fields of a glist word (entry indices have 27 bits)
@@ -266,6 +265,11 @@ void launch_mlp_grad(const void* w, const float* X, const float* T, int nb, floa
 void launch_mlp_adam(float* master, void* w, float* m, float* v, const float* grad, float lr, int step,
                      cudaStream_t st);
 void launch_mlp_to_half(const float* master, void* w, cudaStream_t st);
+
+// candidates of the list build (rk_cand.cu; the distance-only ones in rk_nl.cu)
+void launch_candidates_float(const Scene& s, unsigned grid, size_t smem, const uint64_t* pairs, int64_t np, int mv, int me,
+                             int mf, uint64_t* out, uint32_t* unc, int64_t cap, unsigned long long* counter,
+                             cudaStream_t st);
 
 // primitives (rk_prims.cu)
 size_t scan_temp_bytes(int64_t n);

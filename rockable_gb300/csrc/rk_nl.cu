@@ -15,15 +15,15 @@
 //
 // Pipeline (all on the context stream, a few host reads of counts):
 //   body_obb -> pairs (all-pairs AABB filter or uniform grid, then the FP64
-//   SAT) -> half-pairs (both directions, radix-sorted) -> cull mask ->
-//   candidates (one warp per half-pair: NEAR keys appended) -> FP64 predicate
-//   of the undecided ones -> key sort -> old-entry classification and order-preserving compaction -> merge by key ->
+//   SAT; radix-sorted) -> candidates (one warp per pair: NEAR keys of both
+//   directions appended) -> FP64 cull and predicate of the undecided ones ->
+//   key sort -> old-entry classification and order-preserving compaction -> merge by key ->
 //   history carry -> i-side offsets and j-side list.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
 
-#include "rk_bits.cuh"
+#include "rk_cand.cuh"
 #include "rk_ctx.cuh"
 
 namespace rk {
@@ -522,15 +522,6 @@ __global__ void k_mark_pair_bodies(const uint64_t* pairs, int64_t np, uint8_t* m
   mark[p & ((1u << 21) - 1)] = 1;
 }
 
-__global__ void k_half_pairs(const uint64_t* pairs, int64_t np, uint64_t* hp) {
-  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k >= np) return;
-  uint64_t p = pairs[k];
-  uint64_t i = p >> 21, j = p & ((1u << 21) - 1);
-  hp[2 * k] = (i << 21) | j;
-  hp[2 * k + 1] = (j << 21) | i;
-}
-
 // ------------------------------------------------- NEAR predicates ----
 // Particle.cpp:88-209, with vertex positions from the per-step table.
 struct PairView {
@@ -610,235 +601,6 @@ __device__ __forceinline__ bool near_ee(const Scene& s, const PairView& P, int e
   return false;
 }
 
-// ------------------------------------------ geometric NEAR (skin mode) ----
-// Distance-only tests on float coordinates (the vertex spheres' centres are
-// the vertices): vertex-vertex, vertex-segment, vertex-polygon and
-// segment-segment distances against R_b + R_p + dVerlet plus a rounding
-// margin.  Rockable's NEAR predicates also require the projection of a
-// vertex inside the face, or the closest points inside both edges, so a
-// sub-contact can start to touch after an arbitrarily small sliding motion;
-// with distances only, every sub-contact that touches now was within
-// dVerlet of touching at its last test whenever the motion since is below
-// dVerlet -- what makes the learned-skin guard exact.  Used only with the
-// learned skin; the plain and mixed forms keep the reference predicates.
-struct G3 {
-  float x, y, z;
-};
-__device__ __forceinline__ G3 gsub(G3 a, G3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ G3 gmad(G3 a, float t, G3 d) { return {a.x + t * d.x, a.y + t * d.y, a.z + t * d.z}; }
-__device__ __forceinline__ float gdot(G3 a, G3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ G3 gcross(G3 a, G3 b) {
-  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
-}
-__device__ __forceinline__ G3 gpt(float4 a) { return {a.x, a.y, a.z}; }
-__device__ __forceinline__ float clamp01(float t) { return fminf(fmaxf(t, 0.f), 1.f); }
-
-__device__ __forceinline__ float pt_seg_d2(G3 p, G3 a, G3 b) {
-  const G3 ab = gsub(b, a), ap = gsub(p, a);
-  const float l2 = gdot(ab, ab);
-  const float t = l2 > 0.f ? clamp01(gdot(ap, ab) / l2) : 0.f;
-  const G3 d = gmad(ap, -t, ab);
-  return gdot(d, d);
-}
-
-// squared distance of a point to the line through a and b
-__device__ __forceinline__ float pt_line_d2(G3 p, G3 a, G3 b) {
-  const G3 ab = gsub(b, a), ap = gsub(p, a);
-  const float l2 = gdot(ab, ab);
-  const float t = l2 > 0.f ? gdot(ap, ab) / l2 : 0.f;
-  const G3 d = gmad(ap, -t, ab);
-  return gdot(d, d);
-}
-
-// true when the lines through two segments are farther apart than sqrt(lim2)
-// (the line distance bounds the segment distance from below); never for
-// nearly parallel lines, where that distance is ill-conditioned
-__device__ __forceinline__ bool lines_far(G3 p1, G3 q1, G3 p2, G3 q2, float lim2) {
-  const G3 d1 = gsub(q1, p1), d2 = gsub(q2, p2), r = gsub(p1, p2);
-  const G3 n = gcross(d1, d2);
-  const float nn = gdot(n, n);
-  if (!(nn > 1e-6f * gdot(d1, d1) * gdot(d2, d2))) return false;
-  const float rn = gdot(r, n);
-  return rn * rn > lim2 * nn;
-}
-
-// Float classification in front of the FP64 NEAR predicates (Rockable's,
-// above): from the float world coordinates of the sub-elements (the vertex
-// spheres' centres, rounded to nearest from the FP64 world vertices: errors
-// of a few 1e-8 of the coordinates' magnitude `mag`), each returns 1 only
-// when the FP64 predicate is true for sure -- its distance within `alim` (the
-// NEAR distance shrunk by the rejection's rounding margin) and its projection
-// parameters or point inside their ranges by more than their rounding error
-// -- and -1 only when it is false for sure: a projection parameter or point
-// outside its range by more than that error.  On 0 the FP64 predicate
-// decides.  (The distance rejections sit at the call sites.)
-__device__ __forceinline__ bool accept_vv(G3 a, G3 b, float alim) {
-  const G3 d = gsub(a, b);
-  return alim > 0.f && gdot(d, d) <= alim * alim;
-}
-__device__ __forceinline__ int classify_ve(G3 p, G3 a, G3 b, float alim, float dmax, float mag) {
-  const G3 E = gsub(b, a), w = gsub(p, a);
-  const float E2 = gdot(E, E);
-  if (!(E2 > 0.f)) return 0;
-  const float r = gdot(w, E) / E2;
-  const float tol = 1e-5f + 4e-6f * mag * rsqrtf(E2) * (1.f + fabsf(r));
-  if (r < -dmax - tol || r > 1.f + dmax + tol) return -1;  // the FP64 projection test fails too
-  if (!(alim > 0.f) || !(r >= -dmax + tol && r <= 1.f + dmax - tol)) return 0;
-  const G3 d = gmad(w, -r, E);
-  return gdot(d, d) <= alim * alim ? 1 : 0;
-}
-__device__ __forceinline__ int classify_vf_tri(G3 p, G3 A, G3 B, G3 C, float alim, float mag) {
-  const G3 bA = gsub(B, A), cA = gsub(C, A), w = gsub(p, A);
-  G3 n = gcross(bA, cA);
-  const float nn = gdot(n, n);
-  // a well-shaped triangle (the sine of its angle at A above 1e-3), so that
-  // the float normal and in-plane distances carry only rounding errors
-  if (!(nn > 1e-6f * gdot(bA, bA) * gdot(cA, cA))) return 0;
-  const float inv = rsqrtf(nn);
-  n = {n.x * inv, n.y * inv, n.z * inv};
-  const float dist = gdot(w, n);
-  const G3 P = gmad(w, -dist, n);
-  const float tol = 1e-9f + 2e-6f * mag;
-  const G3 ed[3] = {bA, gsub(cA, bA), {-cA.x, -cA.y, -cA.z}};
-  const G3 st[3] = {{0.f, 0.f, 0.f}, bA, cA};
-  bool inside = true;
-  for (int q = 0; q < 3; q++) {  // counter-clockwise about n: inside is to the left of every edge
-    const float side = gdot(gcross(ed[q], gsub(P, st[q])), n) * rsqrtf(gdot(ed[q], ed[q]));
-    if (side < -tol) return -1;  // projection outside the triangle: even crossing number in FP64 too
-    inside = inside && side > tol;
-  }
-  return inside && alim > 0.f && fabsf(dist) <= alim ? 1 : 0;
-}
-__device__ __forceinline__ int classify_ee(G3 pi0, G3 pi1, G3 pj0, G3 pj1, float alim, float mag) {
-  const G3 Ei = gsub(pi1, pi0), Ej = gsub(pj1, pj0), w = gsub(pi0, pj0);
-  const float c = gdot(Ei, Ei), d = gdot(Ej, Ej), e = gdot(Ei, Ej);
-  const float f = c * d - e * e;
-  // well away from the FP64 test's parallel threshold (1e-12) and from
-  // parallel edges (the sine of their angle above 0.1)
-  if (!(f > 2e-12f + 0.01f * c * d)) return 0;
-  const float a = gdot(Ei, w), b = gdot(Ej, w);
-  const float fi = 1.f / f;
-  const float ss = (e * b - a * d) * fi, tt = (c * b - e * a) * fi;
-  const float tol = 1e-5f + 4e-5f * mag * rsqrtf(fminf(c, d)) * (1.f + fabsf(ss) + fabsf(tt));
-  if (ss < -tol || ss > 1.f + tol || tt < -tol || tt > 1.f + tol) return -1;  // closest points off an edge
-  if (!(alim > 0.f) || !(ss >= tol && ss <= 1.f - tol && tt >= tol && tt <= 1.f - tol)) return 0;
-  const G3 n = gsub(gmad(pi0, ss, Ei), gmad(pj0, tt, Ej));
-  return gdot(n, n) <= alim * alim ? 1 : 0;
-}
-
-// squared distance of two segments: the closest-point parameters minimise
-// |p1 + s d1 - p2 - t d2| over [0,1]^2 (interior stationary point, else the
-// best clamped edge of the square)
-__device__ __forceinline__ float seg_seg_d2(G3 p1, G3 q1, G3 p2, G3 q2) {
-  const G3 d1 = gsub(q1, p1), d2 = gsub(q2, p2), r = gsub(p1, p2);
-  const float a = gdot(d1, d1), e = gdot(d2, d2), f = gdot(d2, r), c = gdot(d1, r), b = gdot(d1, d2);
-  float s = 0.f, t = 0.f;
-  if (a <= 1e-30f && e <= 1e-30f) {
-    s = t = 0.f;
-  } else if (a <= 1e-30f) {
-    t = clamp01(f / e);
-  } else if (e <= 1e-30f) {
-    s = clamp01(-c / a);
-  } else {
-    const float den = a * e - b * b;
-    s = den > 0.f ? clamp01((b * f - c * e) / den) : 0.f;
-    t = (b * s + f) / e;
-    if (t < 0.f) {
-      t = 0.f;
-      s = clamp01(-c / a);
-    } else if (t > 1.f) {
-      t = 1.f;
-      s = clamp01((b - c) / a);
-    }
-  }
-  const G3 w = gsub(gmad(p1, s, d1), gmad(p2, t, d2));
-  return gdot(w, w);
-}
-
-// squared distance of a point to a planar polygon (vertices in order)
-__device__ __forceinline__ float pt_poly_d2(const Scene& s, const float4* sp, int sh, int f, G3 p) {
-  const int fo = s.face_ofs[sh] + f;
-  const int v0 = s.face_vofs[fo], nbv = s.face_vofs[fo + 1] - v0;
-  const int* fv = s.face_verts + v0;
-  const G3 A = gpt(sp[fv[0]]), B = gpt(sp[fv[1]]), C = gpt(sp[fv[nbv - 1]]);
-  G3 n = gcross(gsub(B, A), gsub(C, A));
-  const float nn = gdot(n, n);
-  float best = 3.0e38f;
-  if (nn > 0.f) {
-    const float inv = rsqrtf(nn);
-    n = {n.x * inv, n.y * inv, n.z * inv};
-    const float dist = gdot(gsub(p, A), n);
-    // crossing number of the projection, in the plane
-    const G3 u = gsub(B, A);
-    const float iu = rsqrtf(fmaxf(gdot(u, u), 1e-30f));
-    const G3 e1 = {u.x * iu, u.y * iu, u.z * iu};
-    const G3 e2 = gcross(n, e1);
-    const G3 q = gsub(p, A);
-    const float o1 = gdot(q, e1), o2 = gdot(q, e2);
-    int odd = 0;
-    for (int k = 0; k < nbv; k++) {
-      const G3 pa = gsub(gpt(sp[fv[k]]), A), pb = gsub(gpt(sp[fv[k + 1 == nbv ? 0 : k + 1]]), A);
-      const float a1 = gdot(pa, e1), b1 = gdot(pb, e1), a2 = gdot(pa, e2), b2 = gdot(pb, e2);
-      if ((a2 < o2 && b2 >= o2) || (b2 < o2 && a2 >= o2))
-        if (a1 + (o2 - a2) / (b2 - a2) * (b1 - a1) < o1) odd = 1 - odd;
-    }
-    if (odd) best = dist * dist;
-  }
-  for (int k = 0; k < nbv; k++)
-    best = fminf(best, pt_seg_d2(p, gpt(sp[fv[k]]), gpt(sp[fv[k + 1 == nbv ? 0 : k + 1]])));
-  return best;
-}
-
-// classify_vf_tri on a face of the partner's shape (triangles only: other
-// polygons go to the FP64 predicate)
-__device__ __forceinline__ int classify_vf(const Scene& s, const float4* sp, int sh, int f, G3 p, float alim,
-                                           float mag) {
-  const int fo = s.face_ofs[sh] + f;
-  const int v0 = s.face_vofs[fo], nbv = s.face_vofs[fo + 1] - v0;
-  if (nbv != 3) return 0;
-  const int* fv = s.face_verts + v0;
-  return classify_vf_tri(p, gpt(sp[fv[0]]), gpt(sp[fv[1]]), gpt(sp[fv[2]]), alim, mag);
-}
-
-// Candidate sub-contacts of the half-pairs: one warp per half-pair (owner b
-// -> partner p).  The lanes first narrow both bodies down to the
-// sub-elements that can be near the other one (a separating slab between the
-// two cores, the other body's box and bounding sphere; index lists in shared
-// memory; k_cull_mask gave the owner vertices that pass Rockable's OBB cull),
-// then sweep the products of the lists 32 candidates at a time: float sphere
-// prefilter, then the float classification of the NEAR predicate, and what
-// it accepts or leaves undecided is appended with one atomic per warp and
-// ballot; k_near_exact runs the FP64 predicate on the undecided ones.
-// Appending leaves the half-pairs unordered; the keys are sorted afterwards.
-// The float tests only skip candidates that cannot be NEAR, so the NEAR set
-// is exactly the one of testing every candidate.
-// Measured on the packed column of 50 000 grains (1.6 M entries): 7.92 ms
-// with the vertex cull and the FP64 predicates inlined and no slab, 6.8 ms
-// with the slab, 3.14 ms split (plus 0.60 ms k_cull_mask, 0.065 ms
-// k_near_exact); bound by the instruction stream (1.8 G warp instructions).
-constexpr int kCandWarps = 4;  // warps per block
-// counters of a candidate pass, after the number of keys: undecided candidates, those the FP64 predicate rejected
-constexpr int kCandUnsure = 2, kCandRejected = 3;
-
-// Root-versus-leaf test of the two-level pruning: true when a sub-element
-// sphere (centre, radius in .w) lies farther than `reach` from the other
-// body's vertex box bx (float: centre, 3 axes, half extents).  The box holds
-// that body's core, so such an element is farther than `reach` from every
-// sub-element of it; the margin covers the float rounding of the box, the
-// centre and the projections.
-__device__ __forceinline__ bool box_far(const float* bx, float4 c, float reach, float slack) {
-  const float dx = c.x - bx[0], dy = c.y - bx[1], dz = c.z - bx[2];
-  float d2 = 0.f;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const float t = fabsf(dx * bx[3 + 3 * k] + dy * bx[4 + 3 * k] + dz * bx[5 + 3 * k]) - bx[12 + k];
-    if (t > 0.f) d2 += t * t;
-  }
-  float lim = c.w + reach;
-  lim = lim + 1e-4f * lim + slack + 1e-6f * (fabsf(dx) + fabsf(dy) + fabsf(dz) + bx[12] + bx[13] + bx[14]);
-  return d2 > lim * lim;
-}
-
 // The owner-vertex cull's FP64 test (Rockable.cpp:1385-1391): the cube of
 // half-size r around vertex v against the partner's OBB enlarged by dmax.
 // Not inlined: inlined, the compiler evaluated it for every vertex and
@@ -856,427 +618,57 @@ __device__ __noinline__ bool cull_fp64(const double* obb, double dmax, const dou
   return obb_intersect(op, sub);
 }
 
-// One warp's lists in dynamic shared memory, sized by the shapes' largest
-// vertex, edge and face counts (fixed 1024-entry lists held the kernel to 4
-// blocks per SM): the vertices' coordinates along the pair's separating
-// direction, owner / partner vertices, owner edges, partner edges and faces.
-struct CandLists {
-  float *bproj, *pproj;
-  uint16_t *bv, *pv, *be, *pe, *pf;
-};
-__host__ __device__ inline size_t cand_list_bytes(int mv, int me, int mf) {
-  return (size_t)((2 * mv * 4 + 2 * (2 * mv + 2 * me + mf) + 15) / 16 * 16);
-}
-__device__ __forceinline__ CandLists cand_lists(char* p, int mv, int me) {
-  CandLists L;
-  L.bproj = reinterpret_cast<float*>(p);
-  L.pproj = L.bproj + mv;
-  L.bv = reinterpret_cast<uint16_t*>(L.pproj + mv);
-  L.pv = L.bv + mv;
-  L.be = L.pv + mv;
-  L.pe = L.be + me;
-  L.pf = L.pe + me;
-  return L;
-}
-
-// Slab between two bodies' cores along one direction: the owner's vertices
-// all lie below bmax, the partner's above pmin (coordinates along the unit
-// direction, relative to the partner's centre; also left per vertex in L).
-struct Slab {
-  float bmax, pmin;
-};
-
-__device__ __forceinline__ unsigned int slab_ord(float f) {
-  const unsigned int u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-// A direction that separates the vertices of b and p about as far as their
-// hulls are apart, by Gilbert's algorithm on the hulls' difference, the whole
-// warp on one pair: each step takes the two hulls' extreme vertices along the
-// current difference v (a lane per vertex, warp-wide integer min / max
-// reductions of ordered float bits) and moves v to the point of the segment
-// towards their difference that is nearest the origin.  Any direction gives
-// a valid slab; a few steps make it tight enough for the pruning, and the
-// search stops once the gap exceeds `enough` (no sub-element can be near).
-__device__ __forceinline__ Slab pair_slab(const float4* sb, int nvb, const float4* sp, int nvp, G3 cb, G3 cp,
-                                          float enough, float tol, int lane, const CandLists& L) {
-  const unsigned full = 0xffffffffu;
-  const int b0 = min(lane, nvb - 1), b1 = min(lane + 32, nvb - 1), p0 = min(lane, nvp - 1), p1 = min(lane + 32, nvp - 1);
-  const G3 xb0 = gsub(gpt(sb[b0]), cp), xp0 = gsub(gpt(sp[p0]), cp);
-  G3 xb1 = xb0, xp1 = xp0;
-  if (nvb > 32) xb1 = gsub(gpt(sb[b1]), cp);
-  if (nvp > 32) xp1 = gsub(gpt(sp[p1]), cp);
-  G3 v = gsub(cp, cb), dir = {0.f, 0.f, 0.f};
-  float best = -3.0e38f;
-  Slab S = {3.0e38f, -3.0e38f};
-  for (int it = 0; it < 12; it++) {
-    const float v2 = gdot(v, v);
-    if (!(v2 > 1e-20f)) break;
-    const float inv = rsqrtf(v2);
-    const G3 d = {v.x * inv, v.y * inv, v.z * inv};
-    const float tb0 = gdot(xb0, d), tb1 = gdot(xb1, d), tp0 = gdot(xp0, d), tp1 = gdot(xp1, d);
-    const bool ub = tb1 > tb0, up = tp1 < tp0;
-    const unsigned ob = slab_ord(ub ? tb1 : tb0), op = slab_ord(up ? tp1 : tp0);
-    const unsigned mb = __reduce_max_sync(full, ob), mp = __reduce_min_sync(full, op);
-    const int lb = __ffs(__ballot_sync(full, ob == mb)) - 1, lp = __ffs(__ballot_sync(full, op == mp)) - 1;
-    const float bmax = __shfl_sync(full, ub ? tb1 : tb0, lb), pmin = __shfl_sync(full, up ? tp1 : tp0, lp);
-    if (pmin - bmax > best) {
-      best = pmin - bmax;
-      S.bmax = bmax;
-      S.pmin = pmin;
-      dir = d;
-    }
-    const float len = v2 * inv;
-    if (best > enough || len - best < tol) break;
-    const G3 eb = ub ? xb1 : xb0, ep = up ? xp1 : xp0;
-    const G3 w = {__shfl_sync(full, ep.x, lp) - __shfl_sync(full, eb.x, lb),
-                  __shfl_sync(full, ep.y, lp) - __shfl_sync(full, eb.y, lb),
-                  __shfl_sync(full, ep.z, lp) - __shfl_sync(full, eb.z, lb)};
-    const G3 vw = gsub(v, w);
-    const float l2 = gdot(vw, vw);
-    if (!(l2 > 1e-20f)) break;
-    v = gmad(v, -clamp01(gdot(v, vw) / l2), vw);
-  }
-  if (lane < nvb) L.bproj[lane] = gdot(xb0, dir);
-  if (lane + 32 < nvb) L.bproj[lane + 32] = gdot(xb1, dir);
-  if (lane < nvp) L.pproj[lane] = gdot(xp0, dir);
-  if (lane + 32 < nvp) L.pproj[lane + 32] = gdot(xp1, dir);
-  __syncwarp();
-  return S;
-}
-
-// Indices k < n with pred(k), in increasing order, written by the warp.
-template <class Pred>
-__device__ __forceinline__ int warp_list(uint16_t* list, int n, int lane, Pred pred) {
-  int cnt = 0;
-  for (int base = 0; base < n; base += 32) {
-    const int k = base + lane;
-    const bool ok = k < n && pred(k);
-    const unsigned bal = __ballot_sync(0xffffffffu, ok);
-    if (ok) list[cnt + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)k;
-    cnt += __popc(bal);
-  }
-  __syncwarp();
-  return cnt;
-}
-
-// Which owner vertices of a half-pair (b -> p) pass Rockable's OBB cull
-// (Rockable.cpp:1385-1391: the vertex cube against the partner's OBB enlarged
-// by dVerlet); the mask also tells the old-entry pass which candidates were
-// tested.  16 lanes per half-pair, a lane per vertex.
-// Float pre-test of the fifteen axes of the separating-axis test (the
-// partner box's axes, the cube's -- the world axes -- and their cross
-// products): separated along one by more than the rounding margin -> the
-// FP64 test is false as well; the vertex inside the box shrunk by the margin,
-// or an overlap by more than the margin along all fifteen -> the FP64 test is
-// true as well; only the cases in between run the FP64 test, so the mask is
-// the FP64 test's.  With the distance-only tests (GEOM) a conservative float
-// test does (a vertex out of reach of the partner's bounding sphere), since
-// an untested candidate only keeps its old entry.
-template <bool GEOM>
-__global__ void __launch_bounds__(128) k_cull_mask(Scene s, const uint64_t* hp, int64_t nhp, uint32_t* mask) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t h = t >> 4;
-  const int l = (int)(t & 15), shift = threadIdx.x & 16;
-  const bool live = h < nhp;
-  const uint64_t key = live ? hp[h] : 0ull;
-  const int b = (int)(key >> 21), p = (int)(key & ((1u << 21) - 1));
-  const int sh = s.shape[b];
-  const int nvb = live ? s.vert_ofs[sh + 1] - s.vert_ofs[sh] : 0;
-  const float4* sbv = s.sph + s.sph_ofs[b];
-  const float dmax = d2f(s.dVerlet), fr = d2f(s.rad[b] + s.dVerlet);
+// Whether owner vertex v of b passes Rockable's OBB cull against p: the FP64
+// test's answer.  A float pre-test of the fifteen axes of the separating-axis
+// test (the partner box's axes, the cube's -- the world axes -- and their
+// cross products) decides most cases: separated along one by more than the
+// rounding margin -> the FP64 test is false as well; the vertex inside the box
+// shrunk by the margin, or an overlap by more than the margin along all
+// fifteen -> it is true as well.
+__device__ __forceinline__ bool cull_hit(const Scene& s, int b, int v, int p) {
   const float* of = s.bobbf + 15 * (int64_t)p;
-  const float4 cpp = make_float4(d2f(s.pos[3 * (int64_t)p]), d2f(s.pos[3 * (int64_t)p + 1]),
-                                 d2f(s.pos[3 * (int64_t)p + 2]), s.bnd[p]);
-  const float reach = d2f(s.rad[b] + s.rad[p] + s.dVerlet);
+  const float dmax = (float)s.dVerlet, fr = (float)(s.rad[b] + s.dVerlet);
   const float fe[3][3] = {{of[3], of[4], of[5]}, {of[6], of[7], of[8]}, {of[9], of[10], of[11]}};
   const float fext[3] = {of[12] + dmax, of[13] + dmax, of[14] + dmax};
   const float mag = fmaxf(fmaxf(fabsf(of[0]), fabsf(of[1])), fabsf(of[2])) + fext[0] + fext[1] + fext[2] + fr;
-  uint32_t m[2] = {0u, 0u};
-  int rounds = (nvb + 15) >> 4;
-  rounds = max(rounds, __shfl_xor_sync(0xffffffffu, rounds, 16));
-  for (int it = 0; it < rounds; it++) {
-    const int v = 16 * it + l;
-    bool hit = false;
-    if (v < nvb) {
-      const float4 pv = sbv[v];
-      if (GEOM) {
-        const float dx = pv.x - cpp.x, dy = pv.y - cpp.y, dz = pv.z - cpp.z;
-        const float mg = fmaxf(fmaxf(fmaxf(fabsf(cpp.x), fabsf(cpp.y)), fabsf(cpp.z)) + cpp.w,
-                               fmaxf(fmaxf(fabsf(pv.x), fabsf(pv.y)), fabsf(pv.z)));
-        float lim = reach + cpp.w;
-        lim = lim + 1e-4f * lim + 1e-6f * mg + 2e-6f;
-        hit = dx * dx + dy * dy + dz * dz <= lim * lim;
-      } else {
-        const float dw[3] = {pv.x - of[0], pv.y - of[1], pv.z - of[2]};
-        bool out = false, in = true, clear = true;
-        float tb[3];
+  const float4 pv = s.sph[s.sph_ofs[b] + v];
+  const float dw[3] = {pv.x - of[0], pv.y - of[1], pv.z - of[2]};
+  bool in = true, clear = true;
+  float tb[3];
 #pragma unroll
-        for (int i = 0; i < 3; i++) {  // the box's axes
-          tb[i] = dw[0] * fe[i][0] + dw[1] * fe[i][1] + dw[2] * fe[i][2];
-          const float tt = fabsf(tb[i]);
-          const float lim = fext[i] + fr * (fabsf(fe[i][0]) + fabsf(fe[i][1]) + fabsf(fe[i][2]));
-          const float mm = 1e-6f * (mag + tt) + 1e-9f;
-          out = out || tt > lim + mm;
-          in = in && tt < fext[i] - mm;
-          clear = clear && tt < lim - mm;
-        }
-        if (!out && !in) {
-          const float mm = 1e-6f * mag + 1e-9f, mc = 4e-6f * mag + 1e-9f;
-#pragma unroll
-          for (int j = 0; j < 3; j++) {  // the world axes
-            const float tt = fabsf(dw[j]);
-            const float lim = fext[0] * fabsf(fe[0][j]) + fext[1] * fabsf(fe[1][j]) + fext[2] * fabsf(fe[2][j]) + fr;
-            out = out || tt > lim + mm;
-            clear = clear && tt < lim - mm;
-          }
-#pragma unroll
-          for (int i = 0; i < 3; i++) {  // box axis i x world axis j
-            const int i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-              const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
-              const float tt = fabsf(tb[i2] * fe[i1][j] - tb[i1] * fe[i2][j]);
-              const float lim = fext[i1] * fabsf(fe[i2][j]) + fext[i2] * fabsf(fe[i1][j]) +
-                                fr * (fabsf(fe[i][j2]) + fabsf(fe[i][j1]));
-              out = out || tt > lim + mc;
-              clear = clear && tt < lim - mc;
-            }
-          }
-        }
-        if (out) hit = false;
-        else if (in || clear) hit = true;
-        else hit = cull_fp64(s.bobb + 15 * (int64_t)p, s.dVerlet, s.gv + 3 * s.gv_ofs[b], v, s.rad[b] + s.dVerlet);
-      }
-    }
-    const uint32_t bits = (__ballot_sync(0xffffffffu, hit) >> shift) & 0xffffu;
-    if (it < 2) m[0] |= bits << (16 * (it & 1));
-    else m[1] |= bits << (16 * (it & 1));
+  for (int i = 0; i < 3; i++) {  // the box's axes
+    tb[i] = dw[0] * fe[i][0] + dw[1] * fe[i][1] + dw[2] * fe[i][2];
+    const float tt = fabsf(tb[i]);
+    const float lim = fext[i] + fr * (fabsf(fe[i][0]) + fabsf(fe[i][1]) + fabsf(fe[i][2]));
+    const float mm = 1e-6f * (mag + tt) + 1e-9f;
+    if (tt > lim + mm) return false;
+    in = in && tt < fext[i] - mm;
+    clear = clear && tt < lim - mm;
   }
-  if (live && l == 0) {
-    mask[kMaskWords * h] = m[0];
-    mask[kMaskWords * h + 1] = m[1];
+  if (in) return true;
+  const float mm = 1e-6f * mag + 1e-9f, mc = 4e-6f * mag + 1e-9f;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {  // the world axes
+    const float tt = fabsf(dw[j]);
+    const float lim = fext[0] * fabsf(fe[0][j]) + fext[1] * fabsf(fe[1][j]) + fext[2] * fabsf(fe[2][j]) + fr;
+    if (tt > lim + mm) return false;
+    clear = clear && tt < lim - mm;
   }
-}
-
-// Appends the keys of the lanes with ok; those the float classification left
-// undecided (unsure) are also listed by their position, for k_near_exact.
-__device__ __forceinline__ void warp_emit(bool ok, bool unsure, uint64_t key, int lane, uint64_t* out, uint32_t* unc,
-                                          int64_t cap, unsigned long long* counter) {
-  const unsigned bal = __ballot_sync(0xffffffffu, ok);
-  if (!bal) return;
-  unsigned long long base = 0;
-  if (lane == 0) base = atomicAdd(counter, (unsigned long long)__popc(bal));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  const unsigned lt = (1u << lane) - 1u;
-  const unsigned long long at = base + __popc(bal & lt);
-  if (ok && (int64_t)at < cap) out[at] = key;
-  const unsigned un = __ballot_sync(0xffffffffu, ok && unsure);
-  if (!un) return;
-  if (lane == 0) base = atomicAdd(counter + kCandUnsure, (unsigned long long)__popc(un));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (ok && unsure) {
-    const unsigned long long u = base + __popc(un & lt);
-    if ((int64_t)u < cap) unc[u] = (uint32_t)at;
-  }
-}
-
-// Float only: the FP64 predicates of the undecided candidates run in
-// k_near_exact.  Inlined here they made the kernel's code too large for the
-// instruction caches (more than half of its stall cycles were instruction
-// fetches) and held it to 128 registers.
-template <bool GEOM>
-__global__ void __launch_bounds__(32 * kCandWarps)
-k_candidates(Scene s, const uint64_t* hp, int64_t nhp, const uint32_t* mask, int mv, int me, int mf, uint64_t* out,
-             uint32_t* unc, int64_t cap, unsigned long long* counter) {
-  extern __shared__ __align__(16) char list_mem[];
-  const int lane = threadIdx.x & 31;
-  const CandLists L = cand_lists(list_mem + (threadIdx.x >> 5) * cand_list_bytes(mv, me, mf), mv, me);
-  const int64_t stride = (int64_t)gridDim.x * kCandWarps;
-  for (int64_t h = (int64_t)blockIdx.x * kCandWarps + (threadIdx.x >> 5); h < nhp; h += stride) {
-    __syncwarp();  // the previous half-pair's lists have been read
-    const uint64_t key = hp[h];
-    const int b = (int)(key >> 21), p = (int)(key & ((1u << 21) - 1));
-    const int shb = s.shape[b], shp = s.shape[p];
-    const double Rb = s.rad[b], Rp = s.rad[p], dmax = s.dVerlet;
-    const int nvb = s.vert_ofs[shb + 1] - s.vert_ofs[shb];
-    const int nvp = s.vert_ofs[shp + 1] - s.vert_ofs[shp];
-    const int ob0 = s.edge_ofs[shb], op0 = s.edge_ofs[shp];
-    const int neb = s.edge_ofs[shb + 1] - ob0;
-    const int nep = s.edge_ofs[shp + 1] - op0;
-    const int nfp = s.face_ofs[shp + 1] - s.face_ofs[shp];
-    const uint32_t m0 = mask[kMaskWords * h], m1 = mask[kMaskWords * h + 1];
-    // conservative float filter: a candidate whose bounding spheres are
-    // farther apart than the NEAR distance allows cannot be NEAR
-    const float4* sb = s.sph + s.sph_ofs[b];
-    const float4* sp = s.sph + s.sph_ofs[p];
-    const float sum = d2f(Rb + Rp + dmax);
-    const float4 cb = make_float4(d2f(s.pos[3 * b]), d2f(s.pos[3 * b + 1]), d2f(s.pos[3 * b + 2]), s.bnd[b]);
-    const float4 cp = make_float4(d2f(s.pos[3 * p]), d2f(s.pos[3 * p + 1]), d2f(s.pos[3 * p + 2]), s.bnd[p]);
-    // margin for the float rounding of coordinates of magnitude up to `mag`
-    // (about 16 ulps of it) on top of a relative 1e-4
-    const float mag = fmaxf(fmaxf(fmaxf(fabsf(cb.x), fabsf(cb.y)), fabsf(cb.z)) + cb.w,
-                            fmaxf(fmaxf(fabsf(cp.x), fabsf(cp.y)), fabsf(cp.z)) + cp.w);
-    const float slack = 1e-6f * mag + 2e-6f;
-    auto far = [&](float4 a, float4 c, float extent) {
-      float dx = a.x - c.x, dy = a.y - c.y, dz = a.z - c.z;
-      float lim = sum + extent;
-      lim = lim + 1e-4f * lim + slack;
-      return dx * dx + dy * dy + dz * dz > lim * lim;
-    };
-    const float ve_ext = d2f(1.0 + 2.0 * dmax);
-    const float glim = sum + 1e-4f * sum + slack;
-    const float glim2 = glim * glim;
-    const float alim = sum - (1e-4f * sum + slack);  // float acceptance: the NEAR distance shrunk by the margin
-    const float dmaxf = d2f(dmax);
-    const bool lower = b < p;  // vertex-vertex and edge-edge pairs are tested in the i < j direction only
-    // Two-level pruning (the role of Rockable's per-shape OBB trees,
-    // Rockable.cpp:1440-1541, Shape.cpp:628-670): a sub-element stays in
-    // its list only when its sphere reaches the other body's bounding
-    // sphere and its vertex box (root against leaf); the products of the
-    // lists then test sphere against sphere (leaf against leaf) before the
-    // NEAR predicate.  Only elements that cannot be NEAR are dropped.
-    const float* bxb = s.bbox + 15 * b;
-    const float* bxp = s.bbox + 15 * p;
-    // an owner vertex meets the partner's edges up to dmax x their length
-    // beyond their ends (the vertex-edge projection test), so its reach
-    // grows by that much (an edge is at most the partner's diameter long)
-    const float vreach = sum + 2.f * dmaxf * cp.w;
-    // First the slab between the two cores along a separating direction: an
-    // element beyond the NEAR distance from the other core's side of it is
-    // farther than that from all of the other body's elements.  Two hulls in
-    // touch keep the few elements within dVerlet of the plane between them
-    // (the boxes and spheres, kept as second tests, leave most of the facing
-    // half), and a pair whose gap exceeds the NEAR distance keeps none.
-    const float slim = vreach + 1e-4f * vreach + slack;
-    const Slab S = pair_slab(sb, nvb, sp, nvp, gpt(cb), gpt(cp), slim, 0.05f * sum, lane, L);
-    if (S.pmin - S.bmax > slim) continue;
-    const float blow = S.pmin - slim, phigh = S.bmax + slim;
-    const int nbv = warp_list(L.bv, nvb, lane, [&](int v) {
-      return (((v < 32 ? m0 : m1) >> (v & 31)) & 1u) != 0u && L.bproj[v] >= blow && !box_far(bxp, sb[v], vreach, slack);
-    });
-    const int npv = lower ? warp_list(L.pv, nvp, lane, [&](int w) {
-      return L.pproj[w] <= phigh && !far(sp[w], cb, cb.w) && !box_far(bxb, sp[w], sum, slack);
-    }) : 0;
-    const int npe = warp_list(L.pe, nep, lane, [&](int e) {
-      const int* ev = s.edges + 2 * (op0 + e);
-      if (fminf(L.pproj[ev[0]], L.pproj[ev[1]]) > phigh) return false;
-      const float4 se = sp[nvp + e];
-      const float4 sx = make_float4(se.x, se.y, se.z, ve_ext * se.w);  // the vertex-edge test's extended edge
-      return !far(se, cb, cb.w + sx.w) && !box_far(bxb, sx, sum, slack);
-    });
-    const int npf = warp_list(L.pf, nfp, lane, [&](int f) {
-      const int fo = s.face_ofs[shp] + f;
-      float low = 3.0e38f;
-      for (int q = s.face_vofs[fo]; q < s.face_vofs[fo + 1]; q++) low = fminf(low, L.pproj[s.face_verts[q]]);
-      if (low > phigh) return false;
-      const float4 sf = sp[nvp + nep + f];
-      return !far(sf, cb, cb.w + sf.w) && !box_far(bxb, sf, sum, slack);
-    });
-    const int nbe = lower ? warp_list(L.be, neb, lane, [&](int e) {
-      const int* ev = s.edges + 2 * (ob0 + e);
-      if (fmaxf(L.bproj[ev[0]], L.bproj[ev[1]]) < blow) return false;
-      const float4 se = sb[nvb + e];
-      return !far(se, cp, cp.w + se.w) && !box_far(bxp, se, sum, slack);
-    }) : 0;
-    // vertex-vertex
-    for (int base = 0, tot = nbv * npv; base < tot; base += 32) {
-      const int c = base + lane;
-      bool ok = false, unsure = false;
-      int v = 0, w = 0;
-      if (c < tot) {
-        v = L.bv[c / npv];
-        w = L.pv[c % npv];
-        if (GEOM) {
-          const G3 d = gsub(gpt(sb[v]), gpt(sp[w]));
-          ok = gdot(d, d) <= glim2;
-        } else {
-          ok = !far(sb[v], sp[w], 0.f);
-          unsure = !accept_vv(gpt(sb[v]), gpt(sp[w]), alim);
-        }
-      }
-      warp_emit(ok, unsure, entry_key((uint32_t)b, (uint32_t)p, 0u, (uint32_t)v, (uint32_t)w), lane, out, unc, cap, counter);
-    }
-    // vertex-edge
-    for (int base = 0, tot = nbv * npe; base < tot; base += 32) {
-      const int c = base + lane;
-      bool ok = false, unsure = false;
-      int v = 0, e = 0;
-      if (c < tot) {
-        v = L.bv[c / npe];
-        e = L.pe[c % npe];
-        const float4 se = sp[nvp + e];
-        if (GEOM) {
-          const int eo = s.edge_ofs[shp] + e;
-          ok = !far(sb[v], se, se.w) &&
-               pt_seg_d2(gpt(sb[v]), gpt(sp[s.edges[2 * eo]]), gpt(sp[s.edges[2 * eo + 1]])) <= glim2;
-        } else {
-          // exact rejection first: Rockable's vertex-edge test accepts a
-          // projection slightly off the edge, never a line distance above it
-          const int eo = s.edge_ofs[shp] + e;
-          const G3 pv = gpt(sb[v]), e0 = gpt(sp[s.edges[2 * eo]]), e1 = gpt(sp[s.edges[2 * eo + 1]]);
-          if (!far(sb[v], se, ve_ext * se.w) && pt_line_d2(pv, e0, e1) <= glim2) {
-            const int c_ = classify_ve(pv, e0, e1, alim, dmaxf, mag);
-            ok = c_ >= 0;
-            unsure = c_ == 0;
-          }
-        }
-      }
-      warp_emit(ok, unsure, entry_key((uint32_t)b, (uint32_t)p, 1u, (uint32_t)v, (uint32_t)e), lane, out, unc, cap, counter);
-    }
-    // vertex-face
-    for (int base = 0, tot = nbv * npf; base < tot; base += 32) {
-      const int c = base + lane;
-      bool ok = false, unsure = false;
-      int v = 0, f = 0;
-      if (c < tot) {
-        v = L.bv[c / npf];
-        f = L.pf[c % npf];
-        const float4 sf = sp[nvp + nep + f];
-        if (GEOM) ok = !far(sb[v], sf, sf.w) && pt_poly_d2(s, sp, shp, f, gpt(sb[v])) <= glim2;
-        else if (!far(sb[v], sf, sf.w) && pt_poly_d2(s, sp, shp, f, gpt(sb[v])) <= glim2) {
-          // (exact rejection first: NEAR needs the polygon within reach)
-          const int c_ = classify_vf(s, sp, shp, f, gpt(sb[v]), alim, mag);
-          ok = c_ >= 0;
-          unsure = c_ == 0;
-        }
-      }
-      warp_emit(ok, unsure, entry_key((uint32_t)b, (uint32_t)p, 2u, (uint32_t)v, (uint32_t)f), lane, out, unc, cap, counter);
-    }
-    // edge-edge
-    for (int base = 0, tot = nbe * npe; base < tot; base += 32) {
-      const int c = base + lane;
-      bool ok = false, unsure = false;
-      int e1 = 0, e2 = 0;
-      if (c < tot) {
-        e1 = L.be[c / npe];
-        e2 = L.pe[c % npe];
-        const float4 s1 = sb[nvb + e1], s2 = sp[nvp + e2];
-        if (GEOM) {
-          // nearly parallel edges (ill-conditioned closest points) within
-          // sphere reach are kept: an extra entry is harmless, a missing one not
-          const int ob = s.edge_ofs[shb] + e1, op = s.edge_ofs[shp] + e2;
-          const G3 a0 = gpt(sb[s.edges[2 * ob]]), a1 = gpt(sb[s.edges[2 * ob + 1]]);
-          const G3 b0 = gpt(sp[s.edges[2 * op]]), b1 = gpt(sp[s.edges[2 * op + 1]]);
-          const G3 d1 = gsub(a1, a0), d2 = gsub(b1, b0), nx = gcross(d1, d2);
-          const bool parallel = !(gdot(nx, nx) > 1e-6f * gdot(d1, d1) * gdot(d2, d2));
-          ok = !far(s1, s2, s1.w + s2.w) && (parallel || seg_seg_d2(a0, a1, b0, b1) <= glim2);
-        } else {
-          // exact rejection first: NEAR needs the edges' lines within reach
-          const int ob = s.edge_ofs[shb] + e1, op = s.edge_ofs[shp] + e2;
-          const G3 a0 = gpt(sb[s.edges[2 * ob]]), a1 = gpt(sb[s.edges[2 * ob + 1]]);
-          const G3 b0 = gpt(sp[s.edges[2 * op]]), b1 = gpt(sp[s.edges[2 * op + 1]]);
-          if (!far(s1, s2, s1.w + s2.w) && !lines_far(a0, a1, b0, b1, glim2)) {
-            const int c_ = classify_ee(a0, a1, b0, b1, alim, mag);
-            ok = c_ >= 0;
-            unsure = c_ == 0;
-          }
-        }
-      }
-      warp_emit(ok, unsure, entry_key((uint32_t)b, (uint32_t)p, 3u, (uint32_t)e1, (uint32_t)e2), lane, out, unc, cap, counter);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {  // box axis i x world axis j
+    const int i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
+      const float tt = fabsf(tb[i2] * fe[i1][j] - tb[i1] * fe[i2][j]);
+      const float lim = fext[i1] * fabsf(fe[i2][j]) + fext[i2] * fabsf(fe[i1][j]) +
+                        fr * (fabsf(fe[i][j2]) + fabsf(fe[i][j1]));
+      if (tt > lim + mc) return false;
+      clear = clear && tt < lim - mc;
     }
   }
+  if (clear) return true;
+  return cull_fp64(s.bobb + 15 * (int64_t)p, s.dVerlet, s.gv + 3 * s.gv_ofs[b], v, s.rad[b] + s.dVerlet);
 }
 
 // The undecided candidates' FP64 NEAR predicate (Particle.cpp:88-209), one
@@ -1298,8 +690,10 @@ __global__ void k_near_exact(Scene s, const uint32_t* unc, int64_t n, uint64_t* 
     P.Rb = s.rad[b];
     P.Rp = s.rad[p];
     P.dmax = s.dVerlet;
-    bool near;
-    if (t == 0) near = near_vv(P, is, js);
+    // (undecided may be the cull of the owner vertex, the predicate or both)
+    bool near = t == 3 || cull_hit(s, b, is, p);
+    if (!near) {
+    } else if (t == 0) near = near_vv(P, is, js);
     else if (t == 1) near = near_ve(s, P, is, js);
     else if (t == 2) near = near_vf(s, P, is, js);
     else near = near_ee(s, P, is, js);
@@ -1311,21 +705,32 @@ __global__ void k_near_exact(Scene s, const uint32_t* unc, int64_t n, uint64_t* 
 }
 
 
-// Old entries that were not tested this time are kept as they are.
-__global__ void k_stale_flag(const uint64_t* okey, int64_t no, const uint64_t* hp, int64_t nhp, const uint32_t* mask,
+// Old entries that were not tested this time are kept as they are: those of
+// pairs that were not visited (pairs: sorted), and vertex-owned ones whose
+// vertex fails the cull.
+template <bool GEOM>
+__global__ void k_stale_flag(Scene s, const uint64_t* okey, int64_t no, const uint64_t* pairs, int64_t np,
                              int64_t* flag) {
   int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= no) return;
   const uint64_t k = okey[e];
   const uint64_t i = k >> 43, j = (k >> 22) & ((1u << 21) - 1);
   const int t = (int)((k >> 20) & 3u), isub = (int)((k >> 10) & 1023u);
-  const uint64_t hk = (i << 21) | j;
-  int64_t h = lower_bound_u64(hp, nhp, hk);
+  const uint64_t pk = i < j ? (i << 21) | j : (j << 21) | i;
   bool tested = false;
-  if (h < nhp && hp[h] == hk) {
-    // vertex-vertex and edge-edge candidates exist only in the i < j direction
-    if ((t == 0 || t == 3) && i > j) tested = false;
-    else tested = (t == 3) || ((mask[kMaskWords * h + (isub >> 5)] >> (isub & 31)) & 1u);
+  // (vertex-vertex and edge-edge candidates exist only in the i < j direction)
+  if (!((t == 0 || t == 3) && i > j)) {
+    const int64_t h = lower_bound_u64(pairs, np, pk);
+    tested = h < np && pairs[h] == pk;
+    if (tested && t != 3) {
+      if (GEOM) {
+        const float4 cp = make_float4(d2f(s.pos[3 * j]), d2f(s.pos[3 * j + 1]), d2f(s.pos[3 * j + 2]), s.bnd[j]);
+        tested = cull_class<true>(s, s.sph[s.sph_ofs[i] + isub], (int)j, 0.f,
+                                  d2f(s.rad[i] + s.rad[j] + s.dVerlet), cp) != 0;
+      } else {
+        tested = cull_hit(s, (int)i, isub, (int)j);
+      }
+    }
   }
   flag[e] = tested ? 0 : 1;
 }
@@ -1636,27 +1041,19 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
     c.grid_n = N;
   }
   if (w.timing_split && w.split) RKCHK(cudaEventRecord(w.split, st));
-  const int64_t nhp = 2 * np;
-  if (w.hp_cap < nhp + 1) {
-    int64_t nc = nhp + nhp / 2 + 1024;
-    if ((rc = grow(c, w.hp, w.hp_cap, nc))) return rc;
-    if ((rc = grow(c, w.hp_tmp, w.hp_cap, nc))) return rc;
-    if ((rc = grow(c, w.hp_mask, w.hp_cap, kMaskWords * nc))) return rc;
-    w.hp_cap = nc;
+  if (w.pair_tmp_cap < w.pair_cap) {
+    if ((rc = grow(c, w.pair_tmp, w.pair_tmp_cap, w.pair_cap))) return rc;
+    w.pair_tmp_cap = w.pair_cap;
   }
   const EntryBuf& ob = c.eb[c.cur];
   const int64_t no = s.ne;
-  int64_t need_tmp = (int64_t)std::max(sort_temp_bytes(nhp), scan_temp_bytes(no + 1));
+  int64_t need_tmp = (int64_t)std::max(sort_temp_bytes(np), scan_temp_bytes(no + 1));
   if ((rc = ensure_tmp(c, need_tmp))) return rc;
-  if (np > 0) {
-    k_half_pairs<<<nblk(np, 256), 256, 0, st>>>(w.pairs, np, w.hp);
-    c.kernels++;
-    c.kernels += radix_sort_u64(w.hp, w.hp_tmp, nhp, 0, 21 + body_bits(N), w.tmp, st, s.flags + FLAG_ERROR);  // (owner << 21) | partner
-  }
-  // ---- candidates: appended by one warp per half-pair, then sorted by key
+  c.kernels += radix_sort_u64(w.pairs, w.pair_tmp, np, 0, 21 + body_bits(N), w.tmp, st, s.flags + FLAG_ERROR);
+  // ---- candidates: appended by one warp per pair, then sorted by key
   int64_t ncand = 0, nunsure = 0;
-  if (nhp > 0) {
-    const int64_t want = std::max<int64_t>(w.cand_hint, 4 * nhp) + 1024;
+  if (np > 0) {
+    const int64_t want = std::max<int64_t>(w.cand_hint, 8 * np) + 1024;
     if (w.cand_cap < want) {
       int64_t nc = want + want / 4;
       if ((rc = grow(c, w.cand, w.cand_cap, nc)) || (rc = grow(c, w.cand_tmp, w.cand_cap, nc)) ||
@@ -1664,19 +1061,16 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
         return rc;
       w.cand_cap = nc;
     }
-    if (s.near_geometric) k_cull_mask<true><<<nblk(16 * nhp, 128), 128, 0, st>>>(s, w.hp, nhp, w.hp_mask);
-    else k_cull_mask<false><<<nblk(16 * nhp, 128), 128, 0, st>>>(s, w.hp, nhp, w.hp_mask);
-    c.kernels++;
     const size_t smem = kCandWarps * cand_list_bytes(c.max_nv, c.max_ne, c.max_nf);
-    const unsigned grid = (unsigned)std::min<int64_t>((nhp + kCandWarps - 1) / kCandWarps, 152 * 16);
+    const unsigned grid = (unsigned)std::min<int64_t>((np + kCandWarps - 1) / kCandWarps, 152 * 16);
     for (int attempt = 0; attempt < 4; attempt++) {
       RKCHK(cudaMemsetAsync(w.counter + 3, 0, 32, st));
       if (s.near_geometric)
-        k_candidates<true><<<grid, 32 * kCandWarps, smem, st>>>(s, w.hp, nhp, w.hp_mask, c.max_nv, c.max_ne, c.max_nf,
-                                                                w.cand, w.cand_unsure, w.cand_cap, w.counter + 3);
+        k_candidates<true><<<grid, 32 * kCandWarps, smem, st>>>(s, w.pairs, np, c.max_nv, c.max_ne, c.max_nf, w.cand,
+                                                                w.cand_unsure, w.cand_cap, w.counter + 3);
       else
-        k_candidates<false><<<grid, 32 * kCandWarps, smem, st>>>(s, w.hp, nhp, w.hp_mask, c.max_nv, c.max_ne, c.max_nf,
-                                                                 w.cand, w.cand_unsure, w.cand_cap, w.counter + 3);
+        launch_candidates_float(s, grid, smem, w.pairs, np, c.max_nv, c.max_ne, c.max_nf, w.cand, w.cand_unsure,
+                                w.cand_cap, w.counter + 3, st);
       c.kernels++;
       unsigned long long cnt[kCandUnsure + 1] = {};
       RKCHK(cudaMemcpyAsync(cnt, w.counter + 3, sizeof cnt, cudaMemcpyDeviceToHost, st));
@@ -1700,7 +1094,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
     if (ncand > 1) {
       if ((rc = ensure_tmp(c, (int64_t)sort_temp_bytes(ncand)))) return rc;
       // A stable sort by (owner, partner) alone orders the keys completely:
-      // one warp appends a half-pair's candidates, in its sweeps' order
+      // one warp appends a pair's candidates, each half-pair's in its sweeps' order
       // (vertex-vertex, vertex-edge, vertex-face, edge-edge, each by
       // ascending sub-element indices, i.e. by ascending key), chunk after
       // chunk with increasing atomically reserved offsets.
@@ -1717,7 +1111,8 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
   }
   int64_t nstale = 0;
   if (no > 0) {
-    k_stale_flag<<<nblk(no, 256), 256, 0, st>>>(ob.ekey, no, w.hp, nhp, w.hp_mask, w.flag);
+    if (s.near_geometric) k_stale_flag<true><<<nblk(no, 128), 128, 0, st>>>(s, ob.ekey, no, w.pairs, np, w.flag);
+    else k_stale_flag<false><<<nblk(no, 128), 128, 0, st>>>(s, ob.ekey, no, w.pairs, np, w.flag);
     RKCHK(cudaMemsetAsync(w.flag + no, 0, sizeof(int64_t), st));
     // positions in place of the flags, keeping a copy of the flags in stale_src
     RKCHK(cudaMemcpyAsync(w.stale_src, w.flag, (size_t)no * sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
