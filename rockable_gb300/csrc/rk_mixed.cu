@@ -570,29 +570,21 @@ __global__ void k_narrow_mixed_quick(Scene s) {
 constexpr int kSlowThreads = 128;
 __global__ void __launch_bounds__(kSlowThreads, 5) k_narrow_mixed_full(Scene s) {
   if (step_halted(s)) return;
-  int64_t cnt[4], total = 0;
+  int64_t cnt[4];
 #pragma unroll
-  for (int t = 0; t < 4; t++) {  // (a list never exceeds its type run)
+  for (int t = 0; t < 4; t++)  // (a list never exceeds its type run)
     cnt[t] = min((int64_t)s.flags[FLAG_NSLOW + t], (int64_t)(s.flags[FLAG_TOFS + t + 1] - s.flags[FLAG_TOFS + t]));
-    total += cnt[t];
-  }
+  const int64_t total = padded_total(cnt);
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t base = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; base < total;
        base += nwarps * 32) {
-    const int64_t q = base + lane;
+    int t;
+    int64_t r;
+    padded_place(cnt, base, lane, &t, &r);
     bool active = false;
-    if (q < total) {
-      int t = 0;
-      int64_t r = q;
-#pragma unroll
-      for (int u = 0; u < 3; u++)  // the list of q (constant indices: cnt stays in registers)
-        if (t == u && r >= cnt[u]) {
-          r -= cnt[u];
-          t = u + 1;
-        }
-      active = narrow_mixed_full(s, s.slow[(int64_t)s.flags[FLAG_TOFS + t] + r]);
-    }
+    const int64_t len = t == 0 ? cnt[0] : t == 1 ? cnt[1] : t == 2 ? cnt[2] : cnt[3];
+    if (r < len) active = narrow_mixed_full(s, s.slow[(int64_t)s.flags[FLAG_TOFS + t] + r]);
     const unsigned m = __ballot_sync(0xffffffffu, active);
     if (lane == 0 && m) atomicAdd(&s.flags[FLAG_NACTIVE], (unsigned long long)__popc(m));
   }

@@ -72,24 +72,18 @@ __global__ void __launch_bounds__(128) k_near_entries(Scene s) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane;
   if (!stale) {
-    int64_t cnt[4], total = 0;
+    int64_t cnt[4];
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      cnt[t] = (int64_t)s.flags[FLAG_NNEAR + t];
-      total += cnt[t];
-    }
+    for (int t = 0; t < 4; t++) cnt[t] = (int64_t)s.flags[FLAG_NNEAR + t];
+    const int64_t total = padded_total(cnt);
     for (int64_t k0 = first; k0 < total; k0 += stride) {
-      int64_t r = k0 + lane;
+      int type;
+      int64_t r;
+      padded_place(cnt, k0, lane, &type, &r);
       bool need = false;
-      int type = 0;
       int4 R = make_int4(0, 0, 0, 0), G = R;
-      if (r < total) {
-#pragma unroll
-        for (int u = 0; u < 3; u++)
-          if (type == u && r >= cnt[u]) {
-            r -= cnt[u];
-            type = u + 1;
-          }
+      const int64_t len = type == 0 ? cnt[0] : type == 1 ? cnt[1] : type == 2 ? cnt[2] : cnt[3];
+      if (r < len) {
         const int64_t at = (int64_t)s.flags[FLAG_TOFS + type] + r;
         R = s.nrec[2 * at];
         G = s.nrec[2 * at + 1];
@@ -229,9 +223,11 @@ __global__ void __launch_bounds__(kNearThreads) k_near_bodies(Scene s) {
 }
 
 int launch_near_update(const Scene& s, cudaStream_t st) {
-  const int64_t cb = std::min<int64_t>((s.ne + 127) / 128, 152 * 12);
+  // (an update of a small scene's set is a warp per SM: blocks of one warp)
+  const int ct = s.ne < kSmallLaunch * 32 * 32 ? 32 : 128;
+  const int64_t cb = std::min<int64_t>((s.ne + ct - 1) / ct, 152 * 1536 / ct);
   const int64_t bb = std::min<int64_t>((s.n + 7) / 8, 152 * 6);
-  k_near_entries<<<(unsigned)std::max<int64_t>(cb, 1), 128, 0, st>>>(s);
+  k_near_entries<<<(unsigned)std::max<int64_t>(cb, 1), ct, 0, st>>>(s);
   k_near_bodies<<<(unsigned)std::max<int64_t>(bb, 1), kNearThreads, 0, st>>>(s);
   return 2;
 }

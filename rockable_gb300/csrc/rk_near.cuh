@@ -192,9 +192,10 @@ __device__ __forceinline__ float near_distance(const Scene& s, int i, int j, uin
     } else {
       if (inside) *inside = false;
       // nearly parallel (sine of the angle below 0.032): the smallest
-      // distance lies at an end up to that sine times the shorter edge
+      // distance lies at an end up to that sine (its square rounded up)
+      // times the shorter edge
       const float m = fminf(fminf(seg_d2(p1, p2, q2), seg_d2(q1, p2, q2)), fminf(seg_d2(p2, p1, q1), seg_d2(q2, p1, q1)));
-      D = sqrtf(m) - 0.032f * sqrtf(fminf(a, e));
+      D = sqrtf(m) - sqrtf((fmaxf(den, 0.f) / fmaxf(a * e, 1e-37f) + 1e-6f) * fminf(a, e));
     }
   }
   // float errors: a few units of the coordinates' last place, and of D's
@@ -224,30 +225,51 @@ __device__ __forceinline__ void append_record(const Scene& s, bool ok, int type,
   }
 }
 
+// Lane-wise position in four type lists laid one after the other, each padded
+// to whole warps: warp w of the launch gets the list *t and the place *r in it
+// (r >= cnt[t]: none), so that no warp mixes types -- a warp issues every
+// type's FP64 instructions one after the other, and in a small scene its time
+// is the step's.
+__device__ __forceinline__ int64_t padded_total(const int64_t* cnt) {
+  int64_t n = 0;
+#pragma unroll
+  for (int t = 0; t < 4; t++) n += (cnt[t] + 31) & ~(int64_t)31;
+  return n;
+}
+__device__ __forceinline__ void padded_place(const int64_t* cnt, int64_t base, int lane, int* t, int64_t* r) {
+  int64_t b = base;
+  int u = 0;
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    if (u == q) {
+      const int64_t len = (cnt[q] + 31) & ~(int64_t)31;
+      if (b >= len) {
+        b -= len;
+        u = q + 1;
+      }
+    }
+  *t = u;
+  *r = b + lane;
+}
+
 // The records of the entries that the step's narrow phase has to compute
 // (k_near_entries lists them by type): its threads call full on dense warps,
 // and the last block to finish empties the lists for the next step.
 template <class Full>
 __device__ __forceinline__ void near_narrow(const Scene& s, Full full) {
-  int64_t cnt[4], total = 0;
+  int64_t cnt[4];
 #pragma unroll
-  for (int t = 0; t < 4; t++) {
-    cnt[t] = (int64_t)s.flags[FLAG_NSLOW + t];
-    total += cnt[t];
-  }
+  for (int t = 0; t < 4; t++) cnt[t] = (int64_t)s.flags[FLAG_NSLOW + t];
+  const int64_t total = padded_total(cnt);
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; base < total; base += stride) {
-    int64_t r = base + lane;
+    int t;
+    int64_t r;
+    padded_place(cnt, base, lane, &t, &r);
     bool active = false;
-    if (r < total) {
-      int t = 0;
-#pragma unroll
-      for (int u = 0; u < 3; u++)  // the list of r (constant indices: cnt stays in registers)
-        if (t == u && r >= cnt[u]) {
-          r -= cnt[u];
-          t = u + 1;
-        }
+    const int64_t len = t == 0 ? cnt[0] : t == 1 ? cnt[1] : t == 2 ? cnt[2] : cnt[3];
+    if (r < len) {
       const int64_t at = (int64_t)s.flags[FLAG_TOFS + t] + r;
       active = full(s.srec[2 * at], s.srec[2 * at + 1]);
     }

@@ -415,12 +415,22 @@ __device__ __forceinline__ bool narrow_entry(const Scene& s, int64_t e, int i, i
 
 __global__ void k_narrow_force(Scene s) {
   if (step_halted(s)) return;
-  // threads follow the entries grouped by sub-contact type (fewer divergent
-  // branches per warp); every entry is computed on its own
-  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  // threads follow the entries grouped by sub-contact type, a warp's all of
+  // one type; every entry is computed on its own
+  int64_t ofs[5], cnt[4];
+#pragma unroll
+  for (int t = 0; t < 5; t++) ofs[t] = (int64_t)s.flags[FLAG_TOFS + t];
+#pragma unroll
+  for (int t = 0; t < 4; t++) cnt[t] = ofs[t + 1] - ofs[t];
+  const int lane = threadIdx.x & 31;
+  int t;
+  int64_t k;
+  padded_place(cnt, blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane, lane, &t, &k);
   bool active = false;
-  if (k < s.ne) {
-    const int64_t e = s.nperm[k];
+  const int64_t len = t == 0 ? cnt[0] : t == 1 ? cnt[1] : t == 2 ? cnt[2] : cnt[3];
+  const int64_t first = t == 0 ? ofs[0] : t == 1 ? ofs[1] : t == 2 ? ofs[2] : ofs[3];
+  if (k < len) {
+    const int64_t e = s.nperm[first + k];
     active = narrow_entry<false>(s, e, s.ei[e], s.ej[e], s.etsub[e], make_int4(0, 0, 0, 0));
   }
   unsigned m = __ballot_sync(0xffffffffu, active);
@@ -662,7 +672,7 @@ int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all, const uint8_
 int launch_narrow_force(const Scene& s, cudaStream_t st) {
   if (s.ne <= 0) return 0;
   const int t = tpb_or(s, 0, 128, s.ne);
-  k_narrow_force<<<nblk(s.ne, t), t, 0, st>>>(s);
+  k_narrow_force<<<nblk(s.ne + 4 * 31, t), t, 0, st>>>(s);  // (each type's run padded to warps)
   return 1;
 }
 int launch_narrow_near(const Scene& s, cudaStream_t st) {
