@@ -84,12 +84,13 @@ __device__ __forceinline__ f3v euler_f(f3v I, f3v iI, f3v w, f3v M) {
 
 // First half of the velocity-Verlet step for the free bodies (the FP64 form:
 // Rockable.cpp:2056-2083 through rk_body.cuh's k_drift).
-__device__ __forceinline__ void drift_body(const Scene& s, int64_t i) {
+__device__ __forceinline__ BodyState drift_body(const Scene& s, int64_t i) {
   const float dt = d2f(s.dt), dt_2 = d2f(s.dt_2), dt2_2 = d2f(s.dt2_2);
   const V3 p = ld3(s.pos, i), v = ld3(s.vel, i), w = ld3(s.vrot, i);
   const Q4 q = ldq(s.Q, i);
   const f3v vf = cvt3(v), af = ld3f(s.acc, i), wf = cvt3(w), lf = ld3f(s.arot, i);
   const q4f qf = cvt4(q);
+  float path = s.sk_path ? s.sk_path[i] : 0.f;
   const f3v dx = dt * vf + dt2_2 * af;
   // quaternion: the same two terms as the FP64 form (the second from the
   // quaternion after the first) as an FP32 increment dq; qd = q + dq in FP64,
@@ -120,12 +121,16 @@ __device__ __forceinline__ void drift_body(const Scene& s, int64_t i) {
     // times the swing radius, rounded up
     const float ch = sqrtf(dq.s * dq.s + dq.x * dq.x + dq.y * dq.y + dq.z * dq.z) + fabsf(cf) * 1.001f;
     const float d = sqrtf(dotf(dx, dx)) + 2.f * ch * (1.f + ch) * s.sk_rsw[i];
-    s.sk_path[i] += d * (1.f + 1e-5f) + 1e-12f;
+    path += d * (1.f + 1e-5f) + 1e-12f;
+    s.sk_path[i] = path;
   }
-  st3(s.pos, i, addinc(p, dx));
-  st3(s.vel, i, addinc(v, dt_2 * af));
-  st3(s.vrot, i, addinc(w, dt_2 * lf));
-  stq(s.Q, i, q4(fma(c, qd.s, qd.s), fma(c, qd.v.x, qd.v.x), fma(c, qd.v.y, qd.v.y), fma(c, qd.v.z, qd.v.z)));
+  const V3 pn = addinc(p, dx), vn = addinc(v, dt_2 * af), wn = addinc(w, dt_2 * lf);
+  const Q4 qn = q4(fma(c, qd.s, qd.s), fma(c, qd.v.x, qd.v.x), fma(c, qd.v.y, qd.v.y), fma(c, qd.v.z, qd.v.z));
+  st3(s.pos, i, pn);
+  st3(s.vel, i, vn);
+  st3(s.vrot, i, wn);
+  stq(s.Q, i, qn);
+  return {{pn.x, pn.y, pn.z}, {vn.x, vn.y, vn.z}, {qn.s, qn.v.x, qn.v.y, qn.v.z}, {wn.x, wn.y, wn.z}, path};
 }
 
 // Resultants, Newton-Euler and the second half-kick (Rockable.cpp:3837-3866,
@@ -181,6 +186,7 @@ __global__ void k_gather_sums(Scene s) {
     for (int d = 0; d < 6; d++) s.gsum[6 * b + d] = a[d];
 }
 
+constexpr int kOnNearSet = 2;  // apply_kick of a step on the near set
 __global__ void k_gather_accel(Scene s, int apply_kick) {
   if (step_halted(s)) return;
   float kin[12] = {};
@@ -235,22 +241,25 @@ __global__ void k_gather_accel(Scene s, int apply_kick) {
     }
   }
   // the learned skin's guard on the state this step leaves (every thread)
-  if (s.sk_out && apply_kick) skin_guard_body_t<CvtBits>(s, b < s.n ? b : s.n, have, kin);
-  if (s.sk_ctl) skin_batch_step_end(s);
+  if (s.sk_out && apply_kick && !s.sk_ctl) skin_guard_body(s, b < s.n ? b : s.n, have, kin);
+  if (s.sk_ctl && apply_kick != kOnNearSet) skin_batch_step_end(s);
 }
 
 // k_gather_sums on the near set: the same lanes add the same contributions in
 // the same order (an entry left out of the set is inactive), found through
 // the body's short list (glist, the own block first), whose words name the
 // lane, so that a step gives the same bits on the near set and on the whole
-// list.  The 8 lanes load and convert 8 positions at a time, each its own, and
-// every lane picks the ones it adds from shared memory; with each lane loading
-// what it adds, the lanes of a warp took turns (6.5 of 32 active, 32 us at
-// 50 000 grains).
-constexpr int kSumThreads = 128;
+// list.  The 8 lanes look at 32 positions together, queue the active ones in
+// order, load and convert 8 of them at a time, each its own, and every lane
+// picks the ones it adds from shared memory: one chain of loads for most
+// bodies (1.7 % of the step of 50 000 grains faster than a chain per 8 positions).  With each
+// lane loading what it adds, the lanes of a warp took turns (6.5 of 32 active,
+// 32 us).
+constexpr int kSumThreads = 128, kSumAhead = 4;
 __global__ void __launch_bounds__(kSumThreads) k_gather_sums_near(Scene s) {
   if (step_halted(s)) return;
   __shared__ float stage[kSumThreads][7];
+  __shared__ int queue[kSumThreads * kSumAhead];
   const int64_t t = blockIdx.x * (int64_t)kSumThreads + threadIdx.x;
   const int64_t b = t / kGatherLanes;
   const int l = (int)(t % kGatherLanes), g0 = (int)threadIdx.x - l;
@@ -265,29 +274,47 @@ __global__ void __launch_bounds__(kSumThreads) k_gather_sums_near(Scene s) {
   Lw = max(Lw, __shfl_xor_sync(0xffffffffu, Lw, 8));
   Lw = max(Lw, __shfl_xor_sync(0xffffffffu, Lw, 16));
   float a[6] = {0, 0, 0, 0, 0, 0};
-  for (int p0 = 0; p0 < Lw; p0 += kGatherLanes) {
-    int to = -1;  // the lane that adds this position
-    if (p0 + l < L) {
-      const int x = list[p0 + l];
-      const int e = x & kGlistEntry;
-      if (s.act[e]) {
-        to = (x >> kGlistLane) & (kGatherLanes - 1);
-        const V3 f = ld3(s.cf, e), m = ld3(x < 0 ? s.cmj : s.cmi, e);
-        const float sg = x < 0 ? -1.f : 1.f;
-        float* c = stage[threadIdx.x];
-        c[0] = sg * d2f(f.x); c[1] = sg * d2f(f.y); c[2] = sg * d2f(f.z);
-        c[3] = d2f(m.x); c[4] = d2f(m.y); c[5] = d2f(m.z);
-      }
+  for (int p0 = 0; p0 < Lw; p0 += kGatherLanes * kSumAhead) {
+    int x[kSumAhead];
+    bool on[kSumAhead];
+#pragma unroll
+    for (int u = 0; u < kSumAhead; u++) x[u] = p0 + kGatherLanes * u + l < L ? list[p0 + kGatherLanes * u + l] : 0;
+#pragma unroll
+    for (int u = 0; u < kSumAhead; u++)
+      on[u] = p0 + kGatherLanes * u + l < L && s.act[x[u] & kGlistEntry];
+    int cnt = 0;
+#pragma unroll
+    for (int u = 0; u < kSumAhead; u++) {
+      const unsigned bal = (__ballot_sync(0xffffffffu, on[u]) >> (threadIdx.x & 24)) & 0xffu;
+      if (on[u]) queue[g0 * kSumAhead + cnt + __popc(bal & ((1u << l) - 1u))] = x[u];
+      cnt += __popc(bal);
     }
     __syncwarp();
-#pragma unroll
-    for (int k = 0; k < kGatherLanes; k++)
-      if (__shfl_sync(0xffffffffu, to, (threadIdx.x & 24) + k) == l) {
-        const float* c = stage[g0 + k];
-#pragma unroll
-        for (int d = 0; d < 6; d++) a[d] += c[d];
+    int most = cnt;
+    most = max(most, __shfl_xor_sync(0xffffffffu, most, 8));
+    most = max(most, __shfl_xor_sync(0xffffffffu, most, 16));
+    for (int m = 0; m < most; m += kGatherLanes) {
+      int to = -1;  // the lane that adds this contribution
+      if (m + l < cnt) {
+        const int y = queue[g0 * kSumAhead + m + l];
+        const int e = y & kGlistEntry;
+        to = (y >> kGlistLane) & (kGatherLanes - 1);
+        const V3 f = ld3(s.cf, e), mo = ld3(y < 0 ? s.cmj : s.cmi, e);
+        const float sg = y < 0 ? -1.f : 1.f;
+        float* c = stage[threadIdx.x];
+        c[0] = sg * d2f(f.x); c[1] = sg * d2f(f.y); c[2] = sg * d2f(f.z);
+        c[3] = d2f(mo.x); c[4] = d2f(mo.y); c[5] = d2f(mo.z);
       }
-    __syncwarp();
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < kGatherLanes; k++)
+        if (__shfl_sync(0xffffffffu, to, (threadIdx.x & 24) + k) == l) {
+          const float* c = stage[g0 + k];
+#pragma unroll
+          for (int d = 0; d < 6; d++) a[d] += c[d];
+        }
+      __syncwarp();
+    }
   }
 #pragma unroll
   for (int d = 0; d < 6; d++)
@@ -318,15 +345,22 @@ __device__ __forceinline__ void frame64(const Scene& s, int64_t b, double* R) {
 // computes the rotation matrix of the quaternion (the matrix of qrot,
 // Particle.cpp:55-65 places the vertices with it), from which the narrow
 // phase's FP64 path places the few vertices it needs; and every body's part
-// of the near set's check.
+// of the near set's check and of a batched skin step's guard (GUARD).
+template <bool GUARD>
 __global__ void k_drift_frames(Scene s) {
-  if (step_halted(s)) return;
+  if (GUARD && batch_halted(s)) return;
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (b >= s.n) return;
-  if (b >= s.n_driven) drift_body(s, b);
-  double R[9];
-  frame64(s, b, R);
-  near_track(s, b);
+  BodyState k = {};
+  SkinRef ref = {};
+  if (b < s.n) {
+    const NearRef near = near_ref(s, b);
+    if (GUARD) ref = skin_ref(s, b);
+    k = b >= s.n_driven ? drift_body(s, b) : body_state(s, b);
+    double R[9];
+    frame64(s, b, R);
+    near_track(s, b, k, near);
+  }
+  if (GUARD) skin_guard_drift(s, b < s.n ? b : s.n, k, ref);
 }
 
 // What a step on the whole list and a list update need besides: the FP32
@@ -430,13 +464,14 @@ int launch_fused_gather(const Scene& s, unsigned blocks, int threads, int apply_
   return 2;
 }
 int launch_drift_frames(const Scene& s, unsigned blocks, int threads, cudaStream_t st) {
-  mx::k_drift_frames<<<blocks, threads, 0, st>>>(s);
+  if (s.sk_ctl) mx::k_drift_frames<true><<<blocks, threads, 0, st>>>(s);
+  else mx::k_drift_frames<false><<<blocks, threads, 0, st>>>(s);
   return 1;
 }
 int launch_fused_gather_near(const Scene& s, unsigned blocks, int threads, cudaStream_t st) {
   int k = launch_gather_heavy(s, st);
   mx::k_gather_sums_near<<<(unsigned)((s.n * kGatherLanes + mx::kSumThreads - 1) / mx::kSumThreads), mx::kSumThreads, 0, st>>>(s);
-  mx::k_gather_accel<<<blocks, threads, 0, st>>>(s, 1);
+  mx::k_gather_accel<<<blocks, threads, 0, st>>>(s, mx::kOnNearSet);
   return k + 2;
 }
 int launch_fused_heavy(const Scene& s, const int* list, int count, cudaStream_t st) {
@@ -446,7 +481,7 @@ int launch_fused_heavy(const Scene& s, const int* list, int count, cudaStream_t 
 cudaError_t fused_attributes(int which, cudaFuncAttributes* a) {
   if (which == 1) return cudaFuncGetAttributes(a, mx::k_gather_accel);
   if (which == 2) return cudaFuncGetAttributes(a, mx::k_body_frames<true>);
-  return cudaFuncGetAttributes(a, mx::k_drift_frames);
+  return cudaFuncGetAttributes(a, mx::k_drift_frames<true>);
 }
 
 }  // namespace rk

@@ -1,9 +1,10 @@
 // rk_guard.cuh -- per-body evaluation of the learned skin's exact guard
-// (see rk_skin.cu for the bounds), shared by the resultant kernel, which
-// runs it at the end of every step of the skin mode.
+// (see rk_skin.cu for the bounds), shared by the kernels that run it once per
+// step of the skin mode.
 #pragma once
 #include "rk_bits.cuh"
 #include "rk_engine.cuh"
+#include "rk_near.cuh"
 
 namespace rk {
 
@@ -24,85 +25,65 @@ __device__ __forceinline__ double rot_bound(const double* q, const double* q0) {
   return 2.0 * c * (1.0 + c);
 }
 
-// FP64 -> float conversion of the guard on the integer pipe; the margins
-// below cover its rounding.
-struct CvtBits {
-  __device__ static float f(double x) { return d2f(x); }
+// The snapshot body b's guard compares with, its swing radius and its largest
+// delta so far.
+struct SkinRef {
+  double x[3], q[4];
+  float sw, maxd;
 };
+__device__ __forceinline__ SkinRef skin_ref(const Scene& s, int64_t b) {
+  SkinRef r;
+#pragma unroll
+  for (int d = 0; d < 3; d++) r.x[d] = s.sk_ref_pos[3 * b + d];
+#pragma unroll
+  for (int d = 0; d < 4; d++) r.q[d] = s.sk_ref_q[4 * b + d];
+  r.sw = s.sk_rsw[b];
+  r.maxd = s.sk_maxd[b];
+  return r;
+}
+// Largest value of the warp's lanes; values that are not numbers count as zero
+// (the others are not negative, so that their bits compare as they do).
+__device__ __forceinline__ float warp_max(float x) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(x, 0.f))));
+}
 
-// Guard of body b after a step, evaluated by the thread that finished the
-// body's update (the resultant kernel); every thread of the block must call
-// it (block reduction, blocks of at most 512 threads).  sk_out (zeroed before the step): [0] max delta,
-// [1] max |v| of the free bodies, [2] max g (float bits, atomicMax),
+// Guard of body b (position x, orientation q) for the state a step leaves;
+// every thread of the block must call it (block reduction, blocks of at most
+// 512 threads; b == n: no body).  sk_out (zeroed before the step): [0] max
+// delta, [1] max |v| of the free bodies, [2] max g (float bits, atomicMax),
 // [3] number of flagged bodies (g >= flag_at), [4..5] unused,
 // [6] max delta and [7] max g bounded for the state after the NEXT step:
 // the next drift's motion is bounded from the velocities and accelerations
 // this step leaves (free bodies); driven bodies do not move between steps
 // when no control drives them, which is the only case the host uses the
 // bound for.
-// With have_kin, kin holds the body's velocity, acceleration, angular
-// velocity and angular acceleration after the step as floats (12 values,
-// the caller's registers); otherwise they are read back and converted.
-template <class C>
-__device__ __forceinline__ void skin_guard_body_t(const Scene& s, int64_t b, bool have_kin, const float* kin) {
-  const double* ref_pos = s.sk_ref_pos;
-  const double* ref_q = s.sk_ref_q;
-  const float* rsw = s.sk_rsw;
-  float* maxd = s.sk_maxd;
-  const float* path = s.sk_path;
-  const float flag_at = s.sk_flag_at;
-  uint8_t* flag = s.sk_flag;
+// r: the body's snapshot; path: its path bound (driven bodies: none, infinity).
+// k: the body's velocity, acceleration, angular velocity and angular
+// acceleration as floats; only the velocity without `predict`.
+__device__ __forceinline__ void skin_guard_core(const Scene& s, int64_t b, const double* x, const double* q,
+                                                const SkinRef& r, float path, const float* k, bool predict) {
   unsigned int* out = s.sk_out;
   float dmax = 0.f, vmax = 0.f, gmax = 0.f, pdmax = 0.f, pgmax = 0.f;
   unsigned nflag = 0;
-  // (a batch reads no prediction: its steps are decided on the device)
-  const bool predict = s.sk_ctl == nullptr;
   if (b < s.n) {
     const bool free_body = b >= s.n_driven;
-    // every load before the first store: one round trip instead of one per store
-    double x[3], x0[3], q[4], q0[4];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      x[d] = s.pos[3 * b + d];
-      x0[d] = ref_pos[3 * b + d];
-    }
-#pragma unroll
-    for (int d = 0; d < 4; d++) {
-      q[d] = s.Q[4 * b + d];
-      q0[d] = ref_q[4 * b + d];
-    }
-    const float sw = rsw[b], md0 = maxd[b], pth = free_body ? path[b] : INFINITY;
-    float k[12] = {};
-    if (have_kin) {
-#pragma unroll
-      for (int d = 0; d < 12; d++) k[d] = kin[d];
-    } else if (free_body) {
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        k[d] = C::f(s.vel[3 * b + d]);
-        k[3 + d] = C::f(s.acc[3 * b + d]);
-        k[6 + d] = C::f(s.vrot[3 * b + d]);
-        k[9 + d] = C::f(s.arot[3 * b + d]);
-      }
-    }
     // differences in FP64, the rest in float rounded up (relative 1e-5 covers
     // the float rounding of the norms, 1e-12 m the conversions)
-    const float dx = C::f(x[0] - x0[0]), dy = C::f(x[1] - x0[1]), dz = C::f(x[2] - x0[2]);
+    const float dx = d2f(x[0] - r.x[0]), dy = d2f(x[1] - r.x[1]), dz = d2f(x[2] - r.x[2]);
     float m2 = 0.f, p2 = 0.f;
 #pragma unroll
     for (int d = 0; d < 4; d++) {
-      const float m = C::f(q[d] - q0[d]), p = C::f(q[d] + q0[d]);
+      const float m = d2f(q[d] - r.q[d]), p = d2f(q[d] + r.q[d]);
       m2 += m * m;
       p2 += p * p;
     }
     const float chord = sqrtf(fminf(m2, p2)) * (1.f + 1e-5f);
-    dmax = (sqrtf(dx * dx + dy * dy + dz * dz) + 2.f * chord * (1.f + chord) * sw) * (1.f + 1e-5f) + 1e-12f;
-    const float md = fmaxf(md0, dmax);
-    maxd[b] = md;
-    // driven bodies are moved by their controls, not by the drift: no path
-    gmax = fminf(pth, 2.f * md);
-    const bool f = gmax >= flag_at;
-    flag[b] = f ? 1 : 0;
+    dmax = (sqrtf(dx * dx + dy * dy + dz * dz) + 2.f * chord * (1.f + chord) * r.sw) * (1.f + 1e-5f) + 1e-12f;
+    const float md = fmaxf(r.maxd, dmax);
+    s.sk_maxd[b] = md;
+    gmax = fminf(path, 2.f * md);
+    const bool f = gmax >= s.sk_flag_at;
+    s.sk_flag[b] = f ? 1 : 0;
     nflag = f ? 1u : 0u;
     if (free_body) {
       const float vx = k[0], vy = k[1], vz = k[2];
@@ -120,9 +101,9 @@ __device__ __forceinline__ void skin_guard_body_t(const Scene& s, int64_t b, boo
       const float dt = (float)s.dt, dt2 = (float)s.dt2_2;
       const float dxb = dt * vmax + dt2 * sqrtf(ax * ax + ay * ay + az * az);
       const float thb = dt * sqrtf(wx * wx + wy * wy + wz * wz) + dt2 * sqrtf(lx * lx + ly * ly + lz * lz);
-      const float inc = 1.01f * (dxb + thb * sw * (1.f + 2.f * chord + thb)) + 1e-12f;
+      const float inc = 1.01f * (dxb + thb * r.sw * (1.f + 2.f * chord + thb)) + 1e-12f;
       pdmax = dmax + inc;
-      pgmax = fminf(pth + inc, 2.f * fmaxf(md, pdmax));
+      pgmax = fminf(path + inc, 2.f * fmaxf(md, pdmax));
     } else {
       pdmax = dmax;
       pgmax = gmax;
@@ -130,14 +111,14 @@ __device__ __forceinline__ void skin_guard_body_t(const Scene& s, int64_t b, boo
   }
   // warp, then block reduction through shared memory: one atomic per block
   // and quantity (the block size is at most 512 threads)
-  for (int o = 16; o > 0; o >>= 1) {
-    dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-    vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-    gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
-    pdmax = fmaxf(pdmax, __shfl_xor_sync(0xffffffffu, pdmax, o));
-    pgmax = fmaxf(pgmax, __shfl_xor_sync(0xffffffffu, pgmax, o));
-    nflag += __shfl_xor_sync(0xffffffffu, nflag, o);
+  dmax = warp_max(dmax);
+  vmax = warp_max(vmax);
+  gmax = warp_max(gmax);
+  if (predict) {
+    pdmax = warp_max(pdmax);
+    pgmax = warp_max(pgmax);
   }
+  nflag = __reduce_add_sync(0xffffffffu, nflag);
   __shared__ float red[16][5];
   __shared__ unsigned redn[16];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -170,23 +151,61 @@ __device__ __forceinline__ void skin_guard_body_t(const Scene& s, int64_t b, boo
   }
 }
 
-// End of a batched skin step (control block sk_ctl, see rk_skin.cu): every
-// block of the resultant kernel calls it after its guard atomics (all its
-// threads); the last block to arrive reads the step's guard words, counts the
-// step and halts the batch when the host has to act -- a refresh is due or
-// the batch's step budget is spent -- and otherwise zeroes the counters for
-// the next step (the guard words and the active-contact count).
-__device__ __forceinline__ void skin_batch_step_end(const Scene& s) {
-  __shared__ int last;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(&s.sk_ctl[7], 1u) == gridDim.x - 1 ? 1 : 0;
+// In a batch the guard is evaluated by the kernel that makes the drift (the
+// positions it leaves are the step's), so that its reduction is complete when
+// the next kernel starts.
+__device__ __forceinline__ void skin_guard_drift(const Scene& s, int64_t b, const BodyState& k, const SkinRef& r) {
+  const float v[3] = {d2f(k.v[0]), d2f(k.v[1]), d2f(k.v[2])};
+  skin_guard_core(s, b, k.x, k.q, r, k.path, v, false);
+}
+
+// Without a batch, by the resultant kernel, with the prediction; have: kin
+// holds the 12 values, otherwise they are read back.
+__device__ __forceinline__ void skin_guard_body(const Scene& s, int64_t b, bool have = false, const float* kin = nullptr) {
+  double x[3] = {}, q[4] = {};
+  float k[12] = {}, path = INFINITY;
+  SkinRef r = {};
+  if (b < s.n) {
+    r = skin_ref(s, b);
+    if (b >= s.n_driven) path = s.sk_path[b];
+#pragma unroll
+    for (int d = 0; d < 3; d++) x[d] = s.pos[3 * b + d];
+#pragma unroll
+    for (int d = 0; d < 4; d++) q[d] = s.Q[4 * b + d];
+    if (have) {
+#pragma unroll
+      for (int d = 0; d < 12; d++) k[d] = kin[d];
+    } else if (b >= s.n_driven) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        k[d] = d2f(s.vel[3 * b + d]);
+        k[3 + d] = d2f(s.acc[3 * b + d]);
+        k[6 + d] = d2f(s.vrot[3 * b + d]);
+        k[9 + d] = d2f(s.arot[3 * b + d]);
+      }
+    }
   }
-  __syncthreads();
-  if (!last || threadIdx.x >= 32) return;
-  __threadfence();
-  // a lane per word of the control block and of the guard: one round trip
-  // instead of one per word
+  skin_guard_core(s, b, x, q, r, path, k, true);
+}
+
+// First kernel of a batched skin step (the drift): whether the step before it
+// asked the batch to halt; the kernels behind it then return at once
+// (step_halted).
+__device__ __forceinline__ bool batch_halted(const Scene& s) {
+  if (s.sk_ctl == nullptr) return false;
+  if ((s.sk_ctl[0] | s.sk_ctl[16]) == 0u) return false;
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.sk_ctl[0] = 1u;
+  return true;
+}
+
+// End of a batched skin step (control block sk_ctl, see rk_skin.cu), called by
+// a kernel behind the drift (on the near set by k_near_bodies, most of whose
+// launches have nothing else to do): one warp reads the step's guard words, a lane
+// per word, counts the step and asks for a halt when the host has to act -- a
+// refresh is due or the batch's step budget is spent -- and otherwise zeroes
+// the guard words for the next step.
+__device__ __forceinline__ void skin_batch_step_end(const Scene& s) {
+  if (blockIdx.x != gridDim.x - 1 || threadIdx.x >= 32) return;
   volatile unsigned int* ctl = s.sk_ctl;
   volatile unsigned int* out = s.sk_out;
   const int l = threadIdx.x;
@@ -199,21 +218,14 @@ __device__ __forceinline__ void skin_batch_step_end(const Scene& s) {
   const unsigned g0 = __shfl_sync(full, v, 8), g2 = __shfl_sync(full, v, 10);
   const float crit = __uint_as_float(path ? g2 : g0);
   const bool halt = crit >= trig || since >= interval || ex >= budget;
-  if (l == 0 && halt) ctl[0] = 1u;
-  else if (l == 1) ctl[1] = ex;
+  if (l == 1) ctl[1] = ex;
   else if (l == 2) ctl[2] = since;
-  else if (l == 7) ctl[7] = 0u;
   else if (l >= 8 && l < 16) {
     ctl[l] = v;
     if (!halt) out[l - 8] = 0u;
-  } else if (l == 16 && !halt) {
-    s.flags[FLAG_NACTIVE] = 0ull;
+  } else if (l == 16 && halt) {
+    ctl[16] = 1u;
   }
-}
-
-__device__ __forceinline__ void skin_guard_body(const Scene& s, int64_t b) {
-  const float none[12] = {};
-  skin_guard_body_t<CvtBits>(s, b, false, none);
 }
 
 }  // namespace rk

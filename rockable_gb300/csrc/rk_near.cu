@@ -28,6 +28,7 @@
 // sqrt(0.15 dVerlet rate dt), at least dVerlet / 128.
 #include <algorithm>
 
+#include "rk_guard.cuh"
 #include "rk_near.cuh"
 
 namespace rk {
@@ -65,8 +66,8 @@ __device__ __forceinline__ bool compute_needed(const Scene& s, int64_t e, bool a
 // FP64 path is issued for dense warps of the entries that need it: about half
 // of the near set of a flowing pile.
 __global__ void __launch_bounds__(128) k_near_entries(Scene s) {
-  if (step_halted(s)) return;
   const bool stale = s.flags[FLAG_NEAR_STALE] != 0ull;
+  if (step_halted(s)) return;
   int* slow = s.fast_body ? s.slow : nullptr;  // (the mixed form's kernel takes entries)
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -141,9 +142,11 @@ __device__ __forceinline__ int serial_entry(const Scene& s, int64_t p, int64_t n
 // resultant the step does not use have none), and the snapshot the set is
 // checked against.  The last block puts the set into use.
 constexpr int kNearThreads = 256;
-__global__ void __launch_bounds__(kNearThreads) k_near_bodies(Scene s) {
+__global__ void __launch_bounds__(kNearThreads, 6) k_near_bodies(Scene s) {
+  const bool stale = s.flags[FLAG_NEAR_STALE] != 0ull;
   if (step_halted(s)) return;
-  if (!s.flags[FLAG_NEAR_STALE]) return;
+  if (s.sk_ctl) skin_batch_step_end(s);
+  if (!stale) return;
   __shared__ int wsum[kNearThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;

@@ -7,13 +7,50 @@
 
 namespace rk {
 
-// Body b at the step's positions: its speed bound and FP32 orientation for
+// A body's state after the step's drift, in the registers of its thread
+// (path: the skin's path-length bound, when that is kept).
+struct BodyState {
+  double x[3], v[3], q[4], w[3];
+  float path;
+};
+__device__ __forceinline__ BodyState body_state(const Scene& s, int64_t b) {
+  BodyState k;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    k.x[d] = s.pos[3 * b + d];
+    k.v[d] = s.vel[3 * b + d];
+    k.w[d] = s.vrot[3 * b + d];
+  }
+#pragma unroll
+  for (int d = 0; d < 4; d++) k.q[d] = s.Q[4 * b + d];
+  k.path = INFINITY;  // driven bodies are moved by their controls, not by the drift: no path
+  return k;
+}
+// What near_track compares with.  Loaded before the drift's first store it
+// shares the round of loads that the drift waits for anyway.
+struct NearRef {
+  double x[3], q[4];
+  float sw, allow;
+  bool stale;
+};
+__device__ __forceinline__ NearRef near_ref(const Scene& s, int64_t b) {
+  NearRef r;
+#pragma unroll
+  for (int d = 0; d < 3; d++) r.x[d] = s.npos[3 * b + d];
+#pragma unroll
+  for (int d = 0; d < 4; d++) r.q[d] = s.nq[4 * b + d];
+  r.sw = s.swing[b];
+  r.allow = s.nallow[b];
+  r.stale = s.flags[FLAG_NEAR_STALE] != 0ull;
+  return r;
+}
+// Body b at the step's positions (k): its speed bound and FP32 orientation for
 // the next near set, and the check of the present one: the largest motion of
 // a point of the body since the set was made, |x - x0| plus the swing radius
 // times the rotation bound 2 c (1 + c) of the quaternion chord c (differences
 // in FP64, the rest in float rounded up, as in the skin's guard), against the
 // body's allowance.  A motion that is not a number fails the check.
-__device__ __forceinline__ void near_track(const Scene& s, int64_t b) {
+__device__ __forceinline__ void near_track(const Scene& s, int64_t b, const BodyState& k, const NearRef& r) {
   if (b == 0) {  // the step's counters
     s.flags[FLAG_NACTIVE] = 0ull;
     if (s.sk_out && !s.sk_ctl)
@@ -22,33 +59,31 @@ __device__ __forceinline__ void near_track(const Scene& s, int64_t b) {
   float v2 = 0.f, w2 = 0.f;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    const float v = d2f(s.vel[3 * b + d]), w = d2f(s.vrot[3 * b + d]);
+    const float v = d2f(k.v[d]), w = d2f(k.w[d]);
     v2 += v * v;
     w2 += w * w;
   }
-  double q[4];
-#pragma unroll
-  for (int d = 0; d < 4; d++) q[d] = s.Q[4 * b + d];
-  const float sw = s.swing[b];
+  const double* q = k.q;
+  const float sw = r.sw;
   s.rate[b] = sqrtf(v2) + sqrtf(w2) * sw;
   s.qf[b] = make_float4(d2f(q[0]), d2f(q[1]), d2f(q[2]), d2f(q[3]));
-  if (s.flags[FLAG_NEAR_STALE]) return;
+  if (r.stale) return;
   float d2 = 0.f, m2 = 0.f, p2 = 0.f;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    const float x = d2f(s.pos[3 * b + d] - s.npos[3 * b + d]);
+    const float x = d2f(k.x[d] - r.x[d]);
     d2 += x * x;
   }
 #pragma unroll
   for (int d = 0; d < 4; d++) {
-    const double q0 = s.nq[4 * b + d];
+    const double q0 = r.q[d];
     const float m = d2f(q[d] - q0), p = d2f(q[d] + q0);
     m2 += m * m;
     p2 += p * p;
   }
   const float c = sqrtf(fminf(m2, p2)) * (1.f + 1e-5f);
   const float moved = (sqrtf(d2) + 2.f * c * (1.f + c) * sw) * (1.f + 1e-5f) + 1e-12f;
-  if (!(moved < s.nallow[b])) s.flags[FLAG_NEAR_STALE] = 1ull;
+  if (!(moved < r.allow)) s.flags[FLAG_NEAR_STALE] = 1ull;
 }
 
 struct N3 {

@@ -82,23 +82,21 @@ int launch_skin_reset(const Scene& s, const uint8_t* only, double* rp, double* r
 
 // ------------------------------------------------------ batched steps ----
 // A batch of steps runs as one graph without a host round trip per step:
-// k_skin_begin opens the batch, and the last block of each step's resultant
-// kernel reads the exact guard the kernel just reduced (skin_batch_step_end,
-// rk_guard.cuh) and halts the rest of the batch when the host has to act (a
-// refresh is due, or the batch's step budget is spent); a halted step's
-// kernels return at once.  Control block sk_ctl (words, set by the host
-// before the batch):
-//   [0] halt  [1] steps executed  [2] steps since the last refresh
+// k_skin_begin opens the batch; each step's drift kernel evaluates the exact
+// guard, and a kernel behind it reads it and asks for a halt when the host
+// has to act (skin_batch_step_end, rk_guard.cuh: a refresh is due, or the
+// batch's step budget is spent), which the next step's drift kernel puts into
+// effect; a halted step's kernels return at once.  Control block sk_ctl
+// (words; the first eight set by the host before the batch):
+//   [0] halted  [1] steps executed  [2] steps since the last refresh
 //   [3] step budget  [4] refresh interval (steps)  [5] trigger (float bits,
 //   the smallest float >= skin/2)  [6] 1: the trigger compares the path bound
-//   g, 0: the displacement bound delta  [7] arrival ticket of the resultant
-//   kernel's blocks  [8..15] guard words of the last executed step (the
-//   layout of sk_out).
+//   g, 0: the displacement bound delta  [7] unused  [8..15] guard words of the
+//   last executed step (the layout of sk_out)  [16] halt requested
 __global__ void k_skin_begin(Scene s) {
-  if (step_halted(s)) return;
   const int t = threadIdx.x;
-  if (t == 0) s.flags[FLAG_NACTIVE] = 0ull;
   if (t < 8) s.sk_out[t] = 0u;
+  else if (t == 16) s.sk_ctl[16] = 0u;
 }
 
 int launch_skin_begin(const Scene& s, cudaStream_t st) {

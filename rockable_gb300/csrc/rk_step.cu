@@ -648,11 +648,15 @@ int launch_body_verts(const Scene& s, cudaStream_t st) {
   return 1;
 }
 
+// 16 bodies a block until they fill the GPU (8 resident blocks per SM)
+static inline bool few_bodies(const Scene& s) { return s.n < 16 * 8 * 152; }
 int launch_drift(const Scene& s, cudaStream_t st) {
   if (s.n <= 0) return 0;
   const int t = tpb_or(s, 3, 128, s.n);
   if (s.fast_body) return launch_drift_frames(s, nblk(s.n, t), t, st);
-  exact::k_drift<<<nblk(s.n, t), t, 0, st>>>(s);
+  if (s.sk_ctl) exact::k_drift<true, true><<<nblk(s.n, t), t, 0, st>>>(s);
+  else if (few_bodies(s)) exact::k_drift<false, true><<<nblk(s.n, t), t, 0, st>>>(s);
+  else exact::k_drift<false, false><<<nblk(s.n, t), t, 0, st>>>(s);
   return 1;
 }
 int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all, const uint8_t* mark) {
@@ -682,13 +686,11 @@ int launch_narrow_near(const Scene& s, cudaStream_t st) {
   k_narrow_near<<<(unsigned)std::max<int64_t>(blocks, 1), t, 0, st>>>(s);
   return 1;
 }
-// 16 bodies a block until they fill the GPU (8 resident blocks per SM)
-static inline bool gather_small(const Scene& s) { return s.n < 16 * 8 * 152; }
 int launch_gather_near(const Scene& s, cudaStream_t st) {
   const int t = s.n < kSmallLaunch * 32 ? 32 : 128;
   if (s.fast_body) return launch_fused_gather_near(s, nblk(s.n, t), t, st);
   const unsigned big = (unsigned)s.nbig;
-  if (gather_small(s)) exact::k_gather_near<16, false><<<big + nblk(s.n, 16), exact::kGatherNear, 0, st>>>(s, 1);
+  if (few_bodies(s)) exact::k_gather_near<16, false><<<big + nblk(s.n, 16), exact::kGatherNear, 0, st>>>(s, 1);
   else exact::k_gather_near<128, false><<<big + nblk(s.n, 128), exact::kGatherNear, 0, st>>>(s, 1);
   return 1;
 }
@@ -696,7 +698,7 @@ int launch_gather_accel(const Scene& s, int apply_kick, cudaStream_t st) {
   if (s.n <= 0) return 0;
   const int t = tpb_or(s, 1, 128, s.n);
   if (s.fast_body) return launch_fused_gather(s, nblk(s.n, t), t, apply_kick, st);  // one body per thread
-  if (gather_small(s)) {  // (the bodies of many entries included: 32 us -> 13 us at 512 bodies)
+  if (few_bodies(s)) {  // (the bodies of many entries included: 32 us -> 13 us at 512 bodies)
     exact::k_gather_near<16, true><<<(unsigned)s.nbig + nblk(s.n, 16), exact::kGatherNear, 0, st>>>(s, apply_kick);
     return 1;
   }
@@ -712,13 +714,13 @@ int max_tpb(int which, int form_mixed) {
   else if (form_mixed) e = fused_attributes(which, &a);
   else if (which == 1) e = cudaFuncGetAttributes(&a, exact::k_gather_accel);
   else if (which == 2) e = cudaFuncGetAttributes(&a, exact::k_glob_vertices);
-  else e = cudaFuncGetAttributes(&a, exact::k_drift);
+  else e = cudaFuncGetAttributes(&a, exact::k_drift<true, true>);
   return e == cudaSuccess ? a.maxThreadsPerBlock : 128;
 }
 int launch_gather_heavy(const Scene& s, cudaStream_t st) {
   if (s.nheavy <= 0) return 0;
   if (s.fast_body) return launch_fused_heavy(s, s.heavy, (int)s.nheavy, st);
-  if (gather_small(s)) return 0;  // (summed by the resultant kernel itself)
+  if (few_bodies(s)) return 0;  // (summed by the resultant kernel itself)
   k_gather_heavy<<<(unsigned)((s.nheavy + kHeavyWarps - 1) / kHeavyWarps), 32 * kHeavyWarps, 0, st>>>(
       s, s.heavy, (int)s.nheavy);
   return 1;

@@ -115,3 +115,33 @@ def test_big_body_resultant_is_the_serial_sum(gpu_lib):
                     assert bitwise_equal(F[d:d + 1], b["force"][w, d:d + 1]), (steps, w, d)
             assert bitwise_equal(M, b["moment"][w]), (steps, w)
     g.close()
+
+
+@pytest.mark.parametrize("scale,longest", [(1.0, 0), (3.0, 64), (8.0, 128)])
+def test_resultants_of_lists_of_several_rounds(gpu_lib, scale, longest):
+    """Small scenes, whose lanes look at 64 positions of a whole list (32 of a
+    near list) together: lists within one round and over several give every
+    free body the serial sum of its contributions, bit for bit (the moment,
+    which starts from zero), on the near set as on the whole list."""
+    sc = _scene("avalanche", 0.5)
+    sc["dVerlet"] *= scale
+    sc["DVerlet"] *= scale
+    a, b = _engine(sc, 0, False), _engine(sc, 0, False)
+    shift = np.zeros((a.n, 3))
+    shift[sc["n_driven"]::2, 2] = 2e-5
+    for g in (a, b):
+        g.upload_kinematics(pos=np.ascontiguousarray(g.bodies()["pos"] + shift))
+    for _ in range(12):
+        a.step(1)
+    b.step(12)
+    e = _same(a, b, 0)
+    f, bodies = b.contributions(), b.bodies()
+    lengths = np.bincount(np.concatenate([e["i"], e["j"]]), minlength=a.n)[sc["n_driven"]:]
+    assert lengths.max() > longest and e["active"].sum() > 20
+    M = np.zeros((a.n, 3))
+    for k in np.nonzero(e["active"])[0]:
+        M[e["i"][k]] = M[e["i"][k]] + f[1][k]
+        M[e["j"][k]] = M[e["j"][k]] + f[2][k]
+    assert bitwise_equal(M[sc["n_driven"]:], bodies["moment"][sc["n_driven"]:])
+    a.close()
+    b.close()
