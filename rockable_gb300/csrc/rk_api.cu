@@ -472,6 +472,7 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
   c.kernels += launch_skin_reset(s, nullptr, k.ref_pos, k.ref_q, k.maxd, k.path, c.stream);
   CK(cudaMemsetAsync(s.flags + FLAG_NEED_UPDATE, 0, sizeof(unsigned long long), c.stream));
   k.since = 0;
+  k.crit = 0.0;
   k.partial_since_global = 0;
   k.partial_in_window = 0;
   CK(cudaEventRecord(k.ea, c.stream));
@@ -600,12 +601,16 @@ static int step_graph(Ctx& c, bool near) {
   return RK_OK;
 }
 
-// Largest batch of the device-decided skin mode (skin_batch): long enough to
-// take the host round trip out of almost every step, short enough that the
-// steps skipped after a trigger (each a handful of launches that return at
-// once) stay cheap.  A call for fewer steps runs the largest power-of-two
-// batch that fits, so that no step is skipped for want of work.
-constexpr int kSkinBatch = 16;
+// Largest batches of the device-decided skin mode (skin_batch), as a graph
+// and launched one kernel after the other.  A batch costs a host round trip
+// (about 30 us in which the GPU idles) and, when a trigger ends it early, the
+// launches behind the halting step (about 8 us a step, each returns at once).
+// A graph's batch is a power of two, captured once per list; a launched one
+// has any length, so it ends with the refresh interval or where the last
+// guard's growth puts the trigger, and can be longer without being cut short.
+// Measured at 3000 bodies, FP64, 8000 steps: 578 ms (587 in batches of 16).
+constexpr int kSkinBatchLg = 4;
+constexpr int64_t kSkinBatch = 64, kSkinBatchFirst = 16, kSkinBatchLeast = 4;
 
 // Whether a step runs on the near set (rk_near.cu): another step of the call
 // follows, and the contact geometry is not being recorded for every entry.
@@ -613,8 +618,8 @@ static bool near_step(const Ctx& c, bool more_follow) {
   return more_follow && c.s.ne > 0 && c.s.egv_ok && !c.s.record_geom;
 }
 
-// The graph of a batch of 2^lg steps, opened by k_skin_begin; each step's
-// resultant kernel closes it (skin_batch_step_end).  Captured with s.sk_ctl set,
+// The graph of a batch of 2^lg steps, opened by k_skin_begin; each step
+// ends with skin_batch_step_end.  Captured with s.sk_ctl set,
 // like the launches it holds.
 // `near` (the batches that another step follows) is part of the key: a batch
 // of one step exists in both variants, at 0 and at 5.
@@ -661,8 +666,15 @@ static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   // the call's last step is a batch of its own: it computes the whole list
   const bool near = near_step(c, left > 1);
   int lg = 0;
-  while (near && lg < 4 && (int64_t)2 << lg <= left - 1) lg++;
-  const int64_t want = (int64_t)1 << lg;
+  while (near && lg < kSkinBatchLg && (int64_t)2 << lg <= left - 1) lg++;
+  int64_t want = (int64_t)1 << lg;
+  if (near && !c.use_graphs) {
+    want = kSkinBatchFirst;
+    if (k.crit > 0.0 && k.partial_since_global == 0)
+      want = (int64_t)std::min((0.5 * k.skin / k.crit - 1.0) * (double)k.since + 1.0, (double)kSkinBatch);
+    want = std::max(want, kSkinBatchLeast);
+    want = std::max<int64_t>(std::min(want, std::min(k.interval - k.since, left - 1)), 1);
+  }
   unsigned int* in = k.h_ctl;
   unsigned int* out = k.h_ctl + 16;
   float trig = (float)(0.5 * k.skin);
@@ -709,6 +721,7 @@ static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   const double dmax = to_f(hg[0]), vmax = to_f(hg[1]), gmax = to_f(hg[2]);
   const int64_t nflag = (int64_t)hg[3];
   const double crit = k.partial_since_global > 0 ? gmax : dmax;
+  k.crit = crit;
   if (k.since >= k.interval) return skin_rebuild(c, dmax, vmax, false);
   if (crit >= 0.5 * k.skin) {
     if (k.cfg.partial_fraction > 0.0 && nflag > 0 && (double)nflag <= k.cfg.partial_fraction * (double)s.n)
@@ -1425,6 +1438,7 @@ int rk_set_skin(rk_ctx* x, const rk_skin_config* cfg) {
   k.skin = std::min(cfg->skin_max, std::max(cfg->skin_min, s.dVerlet));
   k.interval = cfg->interval_min;
   k.since = 0;
+  k.crit = 0.0;
   k.rebuilds = k.forced = k.scheduled = 0;
   k.partial = k.partial_bodies = k.partial_since_global = 0;
   k.rebuild_bp_ms = k.rebuild_var_ms = 0.0;
@@ -1590,6 +1604,7 @@ int rk_update_nl(rk_ctx* x) {
     Skin& k = c.skin;
     c.kernels += launch_skin_reset(c.s, nullptr, k.ref_pos, k.ref_q, k.maxd, k.path, c.stream);
     k.since = 0;
+    k.crit = 0.0;
     k.partial_since_global = 0;
     k.have_pred = false;
   }

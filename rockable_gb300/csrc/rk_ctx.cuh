@@ -70,6 +70,7 @@ struct Skin {
   unsigned int* d_ctl = nullptr;
   unsigned int* h_ctl = nullptr;
   cudaEvent_t bev = nullptr;
+  double crit = 0.0;  // the guard's value after the last batch (0: none since the refresh)
   int64_t partial = 0, partial_bodies = 0, partial_since_global = 0, since_global = 0;
   // partial refreshes of the current window, and their measured cost
   double partial_ms = 0.0;
