@@ -246,6 +246,9 @@ static const int kMinWindows = 2;
 // Time of the candidates-to-index part of a rebuild on a list small enough
 // that its launches and read-backs are all of it.
 static const double kRebuildFixedMs = 0.6;
+// Time per list entry of making a near set, and of a step on the whole list
+// (FP64, mixed): measured on a list of 2.5 M entries, 0.22, 0.72 and 0.2 ms.
+static const double kMakeMs = 9e-8, kWholeMs[2] = {2.9e-7, 8e-8};
 // Longest window the cost model proposes: its displacement rate is a
 // prediction for the next window, and the network learns once per window.
 static const int64_t kMaxWindow = 320;
@@ -392,12 +395,17 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
   // faster than the skin (more sub-element pairs come within reach): the
   // non-active entries are scaled by (skin ratio)^alpha, alpha learnt from
   // the rebuilds that changed the skin (1.6, the power measured on hull-grain
-  // piles, to start).  A step itself does not depend on the list's size (it
-  // runs on the near set); the last full rebuild is timed in two parts, the
-  // broad phase (70 % fixed) and the candidates-to-index part, proportional
-  // to the list beyond the latency of its launches and read-backs
-  // (kRebuildFixedMs); the partial refreshes of the window are counted and
-  // timed.  The interval is the number of steps the predicted displacement
+  // piles, to start).  A step on the near set does not depend on the list's
+  // size, but the making of a set does, and so does a step on the whole list
+  // (the last one of a call): both are counted in the window and priced per
+  // entry (kMakeMs, kWholeMs); a larger allowance goes with a larger skin, so
+  // the sets made fall with its square root.  (256 scenes with grains that use
+  // up their allowance in a step or two: a list of 19 M entries; without these
+  // terms 160 M, and steps of 16 instead of 3 ms.)  The last full rebuild is
+  // timed in two parts, the broad phase (70 % fixed) and the
+  // candidates-to-index part, proportional to the list beyond the latency of
+  // its launches and read-backs (kRebuildFixedMs); the partial refreshes of
+  // the window are counted and timed.  The interval is the number of steps the predicted displacement
   // rate takes to use half the skin (with a margin), which is also when the
   // guard would force it.
   const double margin = 1.3, alpha = k.alpha;
@@ -410,6 +418,12 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
   const double Rbp = k.rebuild_bp_ms > 0 ? k.rebuild_bp_ms : 2.0;
   const double Rvar = k.rebuild_var_ms > 0 ? k.rebuild_var_ms : 2.0;
   const double Rfix = std::min(Rvar, kRebuildFixedMs);
+  const double window = (double)std::max<int64_t>(1, k.since);
+  const unsigned long long made_now = c.h_flags[FLAG_NEAR_MADE];
+  const double made = made_now > k.made_before ? (double)(made_now - k.made_before) / window : 0.0;
+  const double whole = (double)k.whole_in_window / window;
+  k.made_before = made_now;
+  k.whole_in_window = 0;
   double best = 1e300, best_s = k.skin;
   int64_t best_k = k.interval;
   for (int m = -4; m <= 4; m++) {
@@ -418,6 +432,7 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
     int64_t ki = (int64_t)std::max<double>(k.cfg.interval_min, std::min<double>((double)std::min<int64_t>(k.cfg.interval_max, std::max<int64_t>(kMaxWindow, k.cfg.interval_min)), kk));
     double ratio = (A + (C - A) * std::pow(sk / std::max(k.skin, 1e-30), alpha)) / C;
     double J = (Rbp * (0.7 + 0.3 * ratio) + Rfix + (Rvar - Rfix) * ratio) / (double)ki + P * (k.skin / sk) * Rp;
+    J += (made * std::sqrt(k.skin / sk) * kMakeMs + whole * kWholeMs[c.form == RK_FORM_MIXED]) * C * ratio;
     if (J < best) { best = J; best_s = sk; best_k = ki; }
   }
   k.skin = best_s;
@@ -615,7 +630,7 @@ constexpr int64_t kSkinBatch = 64, kSkinBatchFirst = 16, kSkinBatchLeast = 4;
 // Whether a step runs on the near set (rk_near.cu): another step of the call
 // follows, and the contact geometry is not being recorded for every entry.
 static bool near_step(const Ctx& c, bool more_follow) {
-  return more_follow && c.s.ne > 0 && c.s.egv_ok && !c.s.record_geom;
+  return more_follow && c.s.ne > 0 && c.s.ne <= kGlistMost && c.s.egv_ok && !c.s.record_geom;
 }
 
 // The graph of a batch of 2^lg steps, opened by k_skin_begin; each step
@@ -665,6 +680,7 @@ static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   Scene& s = c.s;
   // the call's last step is a batch of its own: it computes the whole list
   const bool near = near_step(c, left > 1);
+  if (!near) k.whole_in_window++;
   int lg = 0;
   while (near && lg < kSkinBatchLg && (int64_t)2 << lg <= left - 1) lg++;
   int64_t want = (int64_t)1 << lg;
@@ -768,6 +784,7 @@ static bool guard_pipelined(const Ctx& c) {
 int skin_after_step(Ctx& c) {
   Skin& k = c.skin;
   Scene& s = c.s;
+  if (!near_step(c, c.more_steps_follow)) k.whole_in_window++;
   // the step's resultant kernel evaluated the guard into d_guard
   const int slot = k.gslot;
   unsigned int* hg = k.h_guard + 8 * slot;

@@ -70,6 +70,8 @@ struct Skin {
   unsigned int* d_ctl = nullptr;
   unsigned int* h_ctl = nullptr;
   cudaEvent_t bev = nullptr;
+  unsigned long long made_before = 0;  // near sets made up to the last full rebuild
+  int64_t whole_in_window = 0;         // steps of the current window on the whole list
   double crit = 0.0;  // the guard's value after the last batch (0: none since the refresh)
   int64_t partial = 0, partial_bodies = 0, partial_since_global = 0, since_global = 0;
   // partial refreshes of the current window, and their measured cost

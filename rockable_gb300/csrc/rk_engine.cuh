@@ -31,7 +31,9 @@ constexpr int kMaxSub = 1024;       // sub-element index limit of the sort key
 constexpr int kMaxBody = 1 << 21;   // body index limit of the sort key
 constexpr int kHeavy = 64;          // entries above which a body's resultant is summed by a block
 constexpr int kHeavyWarp = 1024;    // mixed form: up to this many, by its warp inside the resultant kernel
-constexpr int kGlistLane = 28, kGlistEntry = (1 << 27) - 1;  // fields of a glist word (entry indices have 27 bits)
+constexpr int kGlistLane = 28, kGlistEntry = (1 << 28) - 1;  // fields of a glist word
+constexpr int64_t kGlistMost = kGlistEntry + (int64_t)1;     // longer lists have no near set
+static_assert(kGlistEntry < (1 << kGlistLane) && kGlistLane + 3 == 31, "a glist word: entry, lane (8), sign");
 // Per-entry and per-body kernels over fewer items than this (one warp per SM) run in blocks of one
 // warp by default: a warp-wide FP64 instruction holds an SM's FP64 pipe for about 20 cycles, so a
 // small launch is faster spread over all SMs than packed into blocks of four warps.
@@ -211,7 +213,7 @@ struct Scene {
 
 enum { FLAG_NEED_UPDATE = 0, FLAG_NACTIVE = 1, FLAG_NBROKEN = 2, FLAG_GPOS = 3, FLAG_GROT = 4, FLAG_GRESET = 5,
        FLAG_ERROR = 6, FLAG_NONFINITE = 7, FLAG_NSLOW = 8, FLAG_SLOW_TICKET = 12, FLAG_TOFS = 13, FLAG_NEAR_STALE = 18, FLAG_NNEAR = 19, FLAG_NNEW = 23,
-       FLAG_NEAR_TICKET = 27, FLAG_COUNT = 28 };
+       FLAG_NEAR_TICKET = 27, FLAG_NEAR_MADE = 28, FLAG_COUNT = 29 };  // (NEAR_MADE: near sets made, never reset)
 
 // step kernels (rk_step.cu)
 int launch_controls_pre(const Scene& s, cudaStream_t st);

@@ -564,9 +564,10 @@ __global__ void k_narrow_mixed_quick(Scene s) {
 
 // Pass 2: the full path over the four lists (also the narrow phase of a step
 // on the near set: k_near_entries fills the same lists then, and both give
-// the same bits), one after the other, by whole warps (grid-stride); the last block to finish empties the lists for the
-// next step.  At least 5 blocks per SM: 96 registers, no spills, 20 warps
-// per SM instead of 16 (latency-bound otherwise).
+// the same bits), one after the other, by whole warps (grid-stride); the last
+// block to finish empties the lists for the next step.  At least 5 blocks per
+// SM: 96 registers, no spills, 20 warps per SM instead of 16 (latency-bound
+// otherwise).
 constexpr int kSlowThreads = 128;
 __global__ void __launch_bounds__(kSlowThreads, 5) k_narrow_mixed_full(Scene s) {
   if (step_halted(s)) return;

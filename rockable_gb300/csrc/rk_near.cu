@@ -138,9 +138,11 @@ __device__ __forceinline__ int serial_entry(const Scene& s, int64_t p, int64_t n
 }
 
 // Second kernel: each body's near entries in the serial order of its
-// resultant (mixed form: its own block, then the j side; one warp per body, a block for the big ones; bodies whose
-// resultant the step does not use have none), and the snapshot the set is
-// checked against.  The last block puts the set into use.
+// resultant (mixed form: its own block, then the j side), one warp per body, a
+// block for the big ones (bodies whose resultant the step does not use have
+// none), and the snapshot the set is checked against.  The last block puts the
+// set into use.  At least 6 blocks per SM, the launch's resident wave: with the
+// 48 registers it takes otherwise 50 000 bodies lost 0.4 % of the step.
 constexpr int kNearThreads = 256;
 __global__ void __launch_bounds__(kNearThreads, 6) k_near_bodies(Scene s) {
   const bool stale = s.flags[FLAG_NEAR_STALE] != 0ull;
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(kNearThreads, 6) k_near_bodies(Scene s) {
         s.flags[FLAG_NNEW + t] = 0ull;
       }
       s.flags[FLAG_NEAR_TICKET] = 0ull;
+      s.flags[FLAG_NEAR_MADE]++;
       s.flags[FLAG_NEAR_STALE] = 0ull;
     }
   }

@@ -649,7 +649,7 @@ int launch_body_verts(const Scene& s, cudaStream_t st) {
 }
 
 // 16 bodies a block until they fill the GPU (8 resident blocks per SM)
-static inline bool few_bodies(const Scene& s) { return s.n < 16 * 8 * 152; }
+static inline bool few_bodies(const Scene& s) { return s.n < 16 * 8 * 152 && s.ne <= kGlistMost; }
 int launch_drift(const Scene& s, cudaStream_t st) {
   if (s.n <= 0) return 0;
   const int t = tpb_or(s, 3, 128, s.n);
