@@ -1007,7 +1007,8 @@ int rk_upload_shapes(rk_ctx* x, const rk_shapes* sh) {
     }
     c.kernels += launch_body_verts(c.s, c.stream);
     CK(cudaGetLastError());
-    CK(near_set_stale(c));
+    // the entries' vertex indices (egv) name other edges and faces now; the near set follows them
+    if (c.s.ne > 0 && (rc = heavy_list(c))) return rc;
   }
   return RK_OK;
 }
