@@ -116,7 +116,9 @@ __device__ __forceinline__ float seg_d2(N3 p, N3 a, N3 b) {
 
 // A lower bound of the distance between the two sub-elements of entry e (not
 // counting the rounding radii), from its FP32 vertices in coordinates relative
-// to body j's centre.  With inside, also whether the projection or the closest
+// to body j's centre.  A vertex of body i is the sum of its offset and the
+// centres' difference, which cancel where the bodies touch: mag, which the
+// margins scale with, covers that difference besides the vertices.  With inside, also whether the projection or the closest
 // points lie inside their ranges by more than the rounding errors, so that
 // the narrow phase finds the same.
 __device__ __forceinline__ float near_distance(const Scene& s, int i, int j, uint32_t ts, int4 G, bool* inside) {
@@ -133,15 +135,15 @@ __device__ __forceinline__ float near_distance(const Scene& s, int i, int j, uin
     const float4 u = s.uvf[k];
     return nrot(qj, n3(u.x, u.y, u.z));
   };
-  float D, mag;
+  float D, mag = namax(dx);
   if (type == 0) {
     const N3 a = I(G.x), b = J(G.y), d = a - b;
-    mag = fmaxf(namax(a), namax(b));
+    mag = fmaxf(mag, fmaxf(namax(a), namax(b)));
     D = sqrtf(ndot(d, d));
     if (inside) *inside = true;
   } else if (type == 1) {
     const N3 a = I(G.x), p = J(G.y), q = J(G.z);
-    mag = fmaxf(namax(a), fmaxf(namax(p), namax(q)));
+    mag = fmaxf(mag, fmaxf(namax(a), fmaxf(namax(p), namax(q))));
     D = sqrtf(seg_d2(a, p, q));
     if (inside) {
       const N3 E = q - p;
@@ -167,7 +169,7 @@ __device__ __forceinline__ float near_distance(const Scene& s, int i, int j, uin
     const N3 bA = B - A, cA = C - A, w = a - A;
     N3 n = ncross(bA, cA);
     const float nn = ndot(n, n);
-    mag = fmaxf(namax(a), fmaxf(namax(A), fmaxf(namax(B), namax(C))));
+    mag = fmaxf(fmaxf(mag, namax(a)), fmaxf(namax(A), fmaxf(namax(B), namax(C))));
     float best = 3.0e38f, off = 0.f;
     // (a needle's float normal is not usable: its entries stay in the set)
     if (!(nn > 1e-5f * fmaxf(ndot(bA, bA), ndot(cA, cA)) * fminf(ndot(bA, bA), ndot(cA, cA)))) {
@@ -205,7 +207,7 @@ __device__ __forceinline__ float near_distance(const Scene& s, int i, int j, uin
     }
   } else {
     const N3 p1 = I(G.x), q1 = I(G.y), p2 = J(G.z), q2 = J(G.w);
-    mag = fmaxf(fmaxf(namax(p1), namax(q1)), fmaxf(namax(p2), namax(q2)));
+    mag = fmaxf(mag, fmaxf(fmaxf(namax(p1), namax(q1)), fmaxf(namax(p2), namax(q2))));
     const N3 d1 = q1 - p1, d2 = q2 - p2, r = p1 - p2;
     const float a = ndot(d1, d1), e = ndot(d2, d2), b = ndot(d1, d2), c = ndot(d1, r), f = ndot(d2, r);
     const float den = a * e - b * b;

@@ -33,3 +33,42 @@ def test_new_shape_tables_reach_the_near_set(gpu_lib, form):
     assert _same(a, b, form)["active"].sum() > 20
     a.close()
     b.close()
+
+
+def _tips(count, length, rng):
+    """Long rods (driven, all centred at the origin) with a sphere at the tip of each."""
+    from rockable_gb300 import scenes
+    r, rho = 0.005, 2700.0
+    rod = {"name": "ROD", "radius": r, "vertices": np.array([[0.0, 0.0, 0.0], [length, 0.0, 0.0]]),
+           "edges": np.array([[0, 1]]), "faces": [], "obb_center": np.array([0.5 * length, 0.0, 0.0]),
+           "obb_extent": np.array([0.5 * length + r, r, r])}
+    ball = {"name": "BALL", "radius": r, "vertices": np.zeros((1, 3)), "edges": np.zeros((0, 2), int), "faces": [],
+            "obb_center": np.zeros(3), "obb_extent": np.full(3, r)}
+    Q = scenes.random_quaternions(rng, count)
+    w, x, y, z = Q.T
+    axis = np.stack([1.0 - 2.0 * (y * y + z * z), 2.0 * (x * y + w * z), 2.0 * (x * z - w * y)], 1)
+    overlap = rng.uniform(2e-8, 4e-6, count)
+    zero = np.zeros((2 * count, 3))
+    bodies = {"pos": np.concatenate([np.zeros((count, 3)), axis * (length + 2.0 * r - overlap)[:, None]]),
+              "vel": zero, "acc": zero, "vrot": zero, "arot": zero, "Q": np.concatenate([Q, Q]),
+              "homothety": np.ones(2 * count), "mass": np.full(2 * count, 4.0 / 3.0 * np.pi * r ** 3 * rho),
+              "inertia": np.full((2 * count, 3), 0.4 * 4.0 / 3.0 * np.pi * r ** 5 * rho),
+              "shape": np.repeat([0, 1], count), "group": np.repeat([1, 0], count), "cluster": np.zeros(2 * count)}
+    return {"shape_tables": scenes.flatten_shapes([rod, ball]), "bodies": bodies, "n_driven": count, "law": "Default",
+            "ngroup": 2, "table": scenes.law_table(1e6, 1e6, 0.25, 0.4), "dt": 1e-6, "gravity": (0.0, 0.0, 0.0),
+            "DVerlet": 2e-3, "dVerlet": 1e-3, "interVerlet": 1.0}
+
+
+@pytest.mark.parametrize("form", [0, 1])
+@pytest.mark.parametrize("length", [0.5, 30.0, 200.0])
+def test_contacts_far_from_their_bodys_centre(gpu_lib, form, length):
+    """Overlaps that are small against the rounding of a float vertex offset
+    of a large body: the near set's float distance must not pass them by."""
+    sc = _tips(64, length, np.random.default_rng(3))
+    a, b = _engine(sc, form, False), _engine(sc, form, False)
+    for _ in range(12):
+        a.step(1)
+    b.step(12)
+    assert _same(a, b, form)["active"].sum() == 64
+    a.close()
+    b.close()
