@@ -1107,6 +1107,7 @@ int rk_upload_bodies(rk_ctx* x, const rk_bodies* b) {
   c.body_shape.assign(b->shape, b->shape + n);
   c.body_hom.assign(b->homothety, b->homothety + n);
   s.ne = 0;
+  s.bonds = 0;
   s.nif = 0;
   c.have_bodies = true;
   return RK_OK;
@@ -1171,6 +1172,7 @@ int rk_upload_entries(rk_ctx* x, const rk_entries* e) {
   bind_entries(c);
   Scene& s = c.s;
   s.ne = n;
+  s.bonds = e->bond && std::any_of(e->bond, e->bond + n, [](int32_t k) { return k >= 0; }) ? 1 : 0;
   if (n > 0) {
     int* d_t = nullptr;
     int* d_is = nullptr;

@@ -146,6 +146,7 @@ struct Scene {
   // vertex-vertex (a, b), vertex-edge (a, p1, p2), vertex-triangle (a, A, B, C; w = -1 for
   // faces of more than 3 vertices), edge-edge (pi1, pi2, pj1, pj2)
   int4* egv;
+  int bonds;      // 1: entries were uploaded with bonds (whether their interfaces were or not)
   int egv_ok;     // egv holds the current list (global vertex indices fit in an int)
   // near set (rk_near.cu): the entries that can be active before some body has moved more than its
   // allowance; all others are skipped by the steps that another step of the same call follows

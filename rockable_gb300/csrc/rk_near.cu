@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(128) k_near_entries(Scene s) {
         const int64_t at = (int64_t)s.flags[FLAG_TOFS + type] + r;
         R = s.nrec[2 * at];
         G = s.nrec[2 * at + 1];
-        need = s.nif > 0 && s.bond[R.x] >= 0;
+        need = s.bonds && s.bond[R.x] >= 0;
         if (!need) {
           bool inside;
           const float D = near_distance(s, R.y, R.z, (uint32_t)R.w, G, &inside);

@@ -72,3 +72,37 @@ def test_contacts_far_from_their_bodys_centre(gpu_lib, form, length):
     assert _same(a, b, form)["active"].sum() == 64
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("form", [0, 1])
+def test_bonds_without_interfaces(gpu_lib, form):
+    """Entries uploaded with a bond in a scene without interfaces count as
+    active while apart, which restarts their history from zero: balls that
+    bounce on a rod's tip, dragged sideways, in flights of 20 steps."""
+    from rockable_gb300 import scenes
+    n = 4
+    sc = _tips(n, 0.6, np.random.default_rng(5))
+    sc["dVerlet"], sc["DVerlet"] = 0.3, 0.6  # (near sets that last for several bounces)
+    sc["table"] = scenes.law_table(1e6, 1e6, 1.0, 10.0)
+    d = sc["bodies"]["pos"][n:] / np.linalg.norm(sc["bodies"]["pos"][n:], axis=1)[:, None]
+    side = np.cross(d, np.eye(3)[np.argmin(np.abs(d), axis=1)])
+    sc["bodies"]["pos"][n:] = d * (0.61 - 1e-9)
+    vel = np.zeros((2 * n, 3))
+    vel[n:] = 10.0 * d + side
+    sc["bodies"]["vel"] = vel
+    a, b = _engine(sc, form, False), _engine(sc, form, False)
+    e = a.entries()
+    tips = e["type"] == 0
+    assert tips.sum() == n
+    e["bond"][tips] = 0
+    for g in (a, b):
+        g.upload_entries(e)
+        g.set_body_force("AttractingPoint", (0.0, 0.0, 0.0, 1e6))
+    for k in (100, 600, 800):
+        for _ in range(k):
+            ra = a.step(1)
+        rb = b.step(k)
+        assert ra["n_active"] == rb["n_active"] == n
+        _same(a, b, form)
+    a.close()
+    b.close()
