@@ -195,7 +195,7 @@ int build_index(Ctx& c) {
   k_iofs2<<<nblk(N + 1, 256), 256, 0, c.stream>>>(s.ekey, ne, N, s.iofs);
   if (ne > 0) {
     k_jkeys2<<<nblk(ne, 256), 256, 0, c.stream>>>(s.ej, ne, w.jkeys);
-    radix_sort_u64(w.jkeys, w.jtmp, ne, 27, 51, w.tmp, c.stream, s.flags + FLAG_ERROR);
+    radix_sort_u64(w.jkeys, w.jtmp, ne, 27, 51, w.tmp, c.stream);
     k_jlist2<<<nblk(ne, 256), 256, 0, c.stream>>>(w.jkeys, ne, s.jlist);
   }
   k_jofs2<<<nblk(N + 1, 256), 256, 0, c.stream>>>(w.jkeys, ne, N, s.jofs);
@@ -208,9 +208,7 @@ int read_flags(Ctx& c) {
                      c.stream));
   CK(cudaStreamSynchronize(c.stream));
   if (c.h_flags[FLAG_ERROR]) {
-    c.err = c.h_flags[FLAG_ERROR] == 2ull
-                ? "neighbour-list sort: a block gave up waiting for the blocks before it"
-                : "mixed narrow phase: an entry's type run disagrees with the entry order (entries skipped)";
+    c.err = "mixed narrow phase: an entry's type run disagrees with the entry order (entries skipped)";
     return RK_ERR_STATE;
   }
   return 0;
@@ -2154,20 +2152,15 @@ int rk_sort_keys(uint64_t* keys, int64_t n, int lo_bit, int hi_bit, void* stream
   uint64_t* tmp = nullptr;
   void* temp = nullptr;
   if (cudaMalloc(&tmp, (size_t)n * sizeof(uint64_t)) != cudaSuccess) return RK_ERR_CUDA;
-  if (cudaMalloc(&temp, sort_temp_bytes(n) + 8) != cudaSuccess) {
+  if (cudaMalloc(&temp, sort_temp_bytes(n)) != cudaSuccess) {
     cudaFree(tmp);
     return RK_ERR_CUDA;
   }
-  // (the word behind the sort's scratch: set when a block gave up waiting)
-  unsigned long long* err = (unsigned long long*)((char*)temp + sort_temp_bytes(n));
-  unsigned long long bad = 0;
-  cudaMemsetAsync(err, 0, sizeof bad, st);
-  radix_sort_u64(keys, tmp, n, lo_bit, hi_bit, temp, st, err);
-  cudaMemcpyAsync(&bad, err, sizeof bad, cudaMemcpyDeviceToHost, st);
+  radix_sort_u64(keys, tmp, n, lo_bit, hi_bit, temp, st);
   cudaError_t e = cudaStreamSynchronize(st);
   cudaFree(tmp);
   cudaFree(temp);
-  return e != cudaSuccess ? RK_ERR_CUDA : bad ? RK_ERR_TIMEOUT : RK_OK;
+  return e == cudaSuccess ? RK_OK : RK_ERR_CUDA;
 }
 
 int rk_set_profiling(rk_ctx* x, int on) {

@@ -278,7 +278,6 @@ void launch_candidates_float(const Scene& s, unsigned grid, size_t smem, const u
 size_t scan_temp_bytes(int64_t n);
 void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, void* temp, cudaStream_t st);
 size_t sort_temp_bytes(int64_t n);
-int radix_sort_u64(uint64_t* keys, uint64_t* tmp, int64_t n, int lo_bit, int hi_bit, void* temp, cudaStream_t st,
-                   unsigned long long* err = nullptr);
+int radix_sort_u64(uint64_t* keys, uint64_t* tmp, int64_t n, int lo_bit, int hi_bit, void* temp, cudaStream_t st);
 
 }  // namespace rk

@@ -981,7 +981,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
     RKCHK(cudaStreamSynchronize(st));
     nover = (int64_t)no_;
     if ((rc = ensure_tmp(c, (int64_t)sort_temp_bytes(N)))) return rc;
-    c.kernels += radix_sort_u64(w.gkeys, w.gtmp, N, 21, 21 + fmt.total, w.tmp, st, s.flags + FLAG_ERROR);
+    c.kernels += radix_sort_u64(w.gkeys, w.gtmp, N, 21, 21 + fmt.total, w.tmp, st);
     if (nover > 0) k_mark_over<<<nblk(nover, 256), 256, 0, st>>>(w.gover, (int)nover, w.gis_over);
     c.kernels += 2;
     for (int attempt = 0; attempt < 4; attempt++) {
@@ -1049,7 +1049,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
   const int64_t no = s.ne;
   int64_t need_tmp = (int64_t)std::max(sort_temp_bytes(np), scan_temp_bytes(no + 1));
   if ((rc = ensure_tmp(c, need_tmp))) return rc;
-  c.kernels += radix_sort_u64(w.pairs, w.pair_tmp, np, 0, 21 + body_bits(N), w.tmp, st, s.flags + FLAG_ERROR);
+  c.kernels += radix_sort_u64(w.pairs, w.pair_tmp, np, 0, 21 + body_bits(N), w.tmp, st);
   // ---- candidates: appended by one warp per pair, then sorted by key
   int64_t ncand = 0, nunsure = 0;
   if (np > 0) {
@@ -1098,7 +1098,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
       // (vertex-vertex, vertex-edge, vertex-face, edge-edge, each by
       // ascending sub-element indices, i.e. by ascending key), chunk after
       // chunk with increasing atomically reserved offsets.
-      c.kernels += radix_sort_u64(w.cand, w.cand_tmp, ncand, 22, 43 + body_bits(N), w.tmp, st, s.flags + FLAG_ERROR);
+      c.kernels += radix_sort_u64(w.cand, w.cand_tmp, ncand, 22, 43 + body_bits(N), w.tmp, st);
     }
   }
   // ---- old entries kept untouched
@@ -1154,7 +1154,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
   c.kernels++;
   if (nf > 0) {
     k_jkeys<<<nblk(nf, 256), 256, 0, st>>>(s.ej, nf, w.jkeys);
-    c.kernels += radix_sort_u64(w.jkeys, w.jtmp, nf, 27, 27 + body_bits(N), w.tmp, st, s.flags + FLAG_ERROR);
+    c.kernels += radix_sort_u64(w.jkeys, w.jtmp, nf, 27, 27 + body_bits(N), w.tmp, st);
     k_jlist<<<nblk(nf, 256), 256, 0, st>>>(w.jkeys, nf, s.jlist);
     c.kernels += 2;
   }
@@ -1192,7 +1192,7 @@ static int entry_order(Ctx& c) {
     return RK_ERR_STATE;
   }
   k_type_keys<<<nblk(ne, 256), 256, 0, c.stream>>>(s.etsub, ne, w.jkeys);
-  c.kernels += radix_sort_u64(w.jkeys, w.jtmp, ne, 40, 42, w.tmp, c.stream, s.flags + FLAG_ERROR);
+  c.kernels += radix_sort_u64(w.jkeys, w.jtmp, ne, 40, 42, w.tmp, c.stream);
   k_type_perm<<<nblk(ne, 256), 256, 0, c.stream>>>(w.jkeys, ne, s.nperm, s.flags + FLAG_TOFS);
   c.kernels += 2;
   return 0;

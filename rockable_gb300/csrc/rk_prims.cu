@@ -104,7 +104,8 @@ void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, void* temp, 
 // pass: the digit counts of all passes come from one sweep over the keys (a
 // pass only permutes them), and a pass's blocks learn where their keys go
 // from the running totals that the blocks before them publish (a block waits
-// only for blocks that took their tickets earlier, hence are running).  A
+// only for blocks that took their tickets earlier, hence are running, and
+// counts their keys itself when the wait lasts too long).  A
 // histogram, a scan of blocks x 256 counts and a scatter per pass took 39 us
 // at 165 000 keys and 41 us at 1.6 M, most of it launches and the scatter's
 // 64 barriers per block.
@@ -114,10 +115,10 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr int64_t kSortTile = (int64_t)kSortThreads * kSortItems;
 constexpr int kMaxPasses = 8;
 
-// Scratch: digit counts of every pass, a ticket counter per pass, an error
-// word, then one status word per block and digit: pass << 56 | state << 54 |
-// count, state 1 the block's own count, 2 the total including all blocks
-// before it (the pass tag makes the words of earlier passes stale).
+// Scratch: digit counts of every pass, a ticket counter per pass, then one
+// status word per block and digit: pass << 56 | state << 54 | count, state 1
+// the block's own count, 2 the total including all blocks before it (the pass
+// tag makes the words of earlier passes stale).
 struct SortTemp {
   unsigned int* hist;           // kMaxPasses * 256
   unsigned int* ticket;         // kMaxPasses
@@ -176,24 +177,28 @@ __device__ __forceinline__ unsigned block_excl_scan(unsigned v, unsigned* ws) {
 
 // One pass.  Each warp ranks 16 x 32 consecutive keys with warp matches, the
 // block's keys are put in digit order in shared memory and written out as
-// runs.  The wait for the blocks before gives up after kSortSpins reads
-// (which no running predecessor needs): the error word is set and the block
-// writes nothing.
-constexpr int kSortSpins = 1 << 24;
+// runs.  A thread waits for the blocks before through at most RK_SORT_SPINS
+// reads (far more than a running predecessor needs); then the block counts the
+// digits of all keys in front of its tile itself, from the pass's input, which
+// is complete: the sort ends, and its result is right, whatever the blocks
+// before do.
+#ifndef RK_SORT_SPINS
+#define RK_SORT_SPINS (1 << 24)
+#endif
+constexpr int kSortSpins = RK_SORT_SPINS;
 __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const uint64_t* __restrict__ in, uint64_t* __restrict__ out,
-                                                             int64_t n, int sh, unsigned mask, int pass, void* temp,
-                                                             unsigned long long* err) {
+                                                             int64_t n, int sh, unsigned mask, int pass, void* temp) {
   __shared__ uint64_t skey[kSortTile];
   __shared__ unsigned whist[kSortWarps][256];
   __shared__ unsigned lbase[256], ws[kSortWarps];
   __shared__ long long gofs[256];
   __shared__ unsigned s_block;
-  __shared__ int s_bad;
+  __shared__ int s_late;
   const SortTemp T = sort_temp(temp);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   if (t == 0) {
     s_block = atomicAdd(&T.ticket[pass], 1u);
-    s_bad = 0;
+    s_late = 0;
   }
 #pragma unroll
   for (int w = 0; w < kSortWarps; w++) whist[w][t] = 0;
@@ -237,12 +242,13 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const uint64_t* 
   const unsigned gb = block_excl_scan(T.hist[pass * 256 + t], ws);  // first position of digit t
   unsigned long long before = 0;
   int spins = 0;
+  bool late = false;
   for (int64_t p = blk - 1; p >= 0;) {
     const unsigned long long v = st[p * 256 + t];
     if ((v >> 56) != (tag >> 56)) {
-      if (++spins > kSortSpins) {
-        s_bad = 1;
-        if (err) *err = 2ull;
+      if (spins++ >= kSortSpins) {
+        late = true;
+        s_late = 1;
         break;
       }
       continue;
@@ -251,13 +257,23 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const uint64_t* 
     if (((v >> 54) & 3ull) == 2ull) break;
     p--;
   }
-  if (blk > 0) {
+  auto publish = [&]() {
     __threadfence();
     st[blk * 256 + t] = tag | (2ull << 54) | (before + tot);
+  };
+  if (blk > 0 && !late) publish();
+  __syncthreads();
+  if (s_late) {  // (skey is not in use yet)
+    unsigned* front = reinterpret_cast<unsigned*>(skey);
+    front[t] = 0;
+    __syncthreads();
+    for (int64_t k = t; k < tile; k += kSortThreads) atomicAdd(&front[(unsigned)(in[k] >> sh) & mask], 1u);
+    __syncthreads();
+    before = front[t];
+    if (late) publish();
   }
   gofs[t] = (long long)gb + (long long)before - (long long)lb;
   __syncthreads();
-  if (s_bad) return;
 #pragma unroll
   for (int u = 0; u < kSortItems; u++)
     if (first + 32 * u < count) {
@@ -274,10 +290,9 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const uint64_t* 
 size_t sort_temp_bytes(int64_t n) { return kSortHead + (size_t)cdiv(n > 0 ? n : 1, kSortTile) * 256 * sizeof(uint64_t); }
 
 // Stable sort of keys on bits [lo_bit, hi_bit); tmp has n slots.  The
-// result ends in keys.  err (may be null) gets 2 if a block gave up waiting.
-// Returns the number of kernels launched.
+// result ends in keys.  Returns the number of kernels launched.
 int radix_sort_u64(uint64_t* keys, uint64_t* tmp, int64_t n, int lo_bit, int hi_bit, void* temp,
-                   cudaStream_t st, unsigned long long* err) {
+                   cudaStream_t st) {
   if (n <= 1) return 0;
   const int64_t nb = cdiv(n, kSortTile);
   cudaMemsetAsync(temp, 0, sort_temp_bytes(n), st);
@@ -288,7 +303,7 @@ int radix_sort_u64(uint64_t* keys, uint64_t* tmp, int64_t n, int lo_bit, int hi_
   int pass = 0;
   for (int sh = lo_bit; sh < hi_bit; sh += 8, pass++) {
     const unsigned mask = hi_bit - sh < 8 ? (1u << (hi_bit - sh)) - 1u : 255u;
-    k_radix_pass<<<(unsigned)nb, kSortThreads, 0, st>>>(src, dst, n, sh, mask, pass, temp, err);
+    k_radix_pass<<<(unsigned)nb, kSortThreads, 0, st>>>(src, dst, n, sh, mask, pass, temp);
     uint64_t* x = src;
     src = dst;
     dst = x;
