@@ -12,6 +12,7 @@
 #include "rk_conf.cuh"
 #include "rk_extract.cuh"
 #include "rk_ctx.cuh"
+#include "rk_jkey.cuh"
 
 using namespace rk;
 
@@ -86,6 +87,10 @@ static void free_entrybuf(EntryBuf& b) {
 int ensure_entry_capacity(Ctx& c, int which, int64_t n) {
   EntryBuf& b = c.eb[which];
   int rc;
+  if (n > kMaxEntries) {
+    c.err = "more than 2^31 - 1 neighbour-list entries";
+    return RK_ERR_CAPACITY;
+  }
   if (b.cap < n || b.cap == 0) {
     int64_t cap = std::max<int64_t>(n + n / 2, 1024);
     free_entrybuf(b);
@@ -148,18 +153,18 @@ __global__ void k_iofs2(const uint64_t* key, int64_t ne, int64_t nb, int64_t* io
 __global__ void k_jkeys2(const int* ej, int64_t ne, uint64_t* jk) {
   int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= ne) return;
-  jk[e] = ((uint64_t)ej[e] << 27) | (uint64_t)e;
+  jk[e] = jkey(ej[e], e);
 }
 __global__ void k_jlist2(const uint64_t* jk, int64_t ne, int* jlist) {
   int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= ne) return;
-  jlist[e] = (int)(jk[e] & ((1ull << 27) - 1));
+  jlist[e] = jkey_entry(jk[e]);
 }
 __global__ void k_jofs2(const uint64_t* jk, int64_t ne, int64_t nb, int64_t* jofs) {
   int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b > nb) return;
   int64_t lo = 0, hi = ne;
-  uint64_t x = (uint64_t)b << 27;
+  uint64_t x = jkey((int)b, 0);
   while (lo < hi) {
     int64_t m = (lo + hi) >> 1;
     if (jk[m] < x) lo = m + 1;
@@ -195,7 +200,7 @@ int build_index(Ctx& c) {
   k_iofs2<<<nblk(N + 1, 256), 256, 0, c.stream>>>(s.ekey, ne, N, s.iofs);
   if (ne > 0) {
     k_jkeys2<<<nblk(ne, 256), 256, 0, c.stream>>>(s.ej, ne, w.jkeys);
-    radix_sort_u64(w.jkeys, w.jtmp, ne, 27, 51, w.tmp, c.stream);
+    radix_sort_u64(w.jkeys, w.jtmp, ne, kJkeyBody, kJkeyBody + 21, w.tmp, c.stream);
     k_jlist2<<<nblk(ne, 256), 256, 0, c.stream>>>(w.jkeys, ne, s.jlist);
   }
   k_jofs2<<<nblk(N + 1, 256), 256, 0, c.stream>>>(w.jkeys, ne, N, s.jofs);

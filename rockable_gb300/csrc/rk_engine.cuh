@@ -32,7 +32,7 @@ constexpr int kMaxBody = 1 << 21;   // body index limit of the sort key
 constexpr int kHeavy = 64;          // entries above which a body's resultant is summed by a block
 constexpr int kHeavyWarp = 1024;    // mixed form: up to this many, by its warp inside the resultant kernel
 constexpr int kGlistLane = 28, kGlistEntry = (1 << 28) - 1;  // fields of a glist word
-constexpr int64_t kGlistMost = kGlistEntry + (int64_t)1;     // longer lists have no near set
+constexpr int64_t kGlistMost = kGlistEntry + (int64_t)1;     // longer lists have no near set (rk_jkey.cuh: up to 2^31 - 1 entries)
 static_assert(kGlistEntry < (1 << kGlistLane) && kGlistLane + 3 == 31, "a glist word: entry, lane (8), sign");
 // Per-entry and per-body kernels over fewer items than this (one warp per SM) run in blocks of one
 // warp by default: a warp-wide FP64 instruction holds an SM's FP64 pipe for about 20 cycles, so a

@@ -25,6 +25,7 @@
 
 #include "rk_cand.cuh"
 #include "rk_ctx.cuh"
+#include "rk_jkey.cuh"
 
 namespace rk {
 
@@ -815,19 +816,19 @@ __global__ void k_iofs(const uint64_t* key, int64_t ne, int64_t nb, int64_t* iof
 __global__ void k_jkeys(const int* ej, int64_t ne, uint64_t* jk) {
   int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= ne) return;
-  jk[e] = ((uint64_t)ej[e] << 27) | (uint64_t)e;
+  jk[e] = jkey(ej[e], e);
 }
 
 __global__ void k_jlist(const uint64_t* jk, int64_t ne, int* jlist) {
   int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= ne) return;
-  jlist[e] = (int)(jk[e] & ((1ull << 27) - 1));
+  jlist[e] = jkey_entry(jk[e]);
 }
 
 __global__ void k_jofs(const uint64_t* jk, int64_t ne, int64_t nb, int64_t* jofs) {
   int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b > nb) return;
-  jofs[b] = lower_bound_u64(jk, ne, (uint64_t)b << 27);
+  jofs[b] = lower_bound_u64(jk, ne, jkey((int)b, 0));
 }
 
 // ----------------------------------------------------------------- host ----
@@ -1154,7 +1155,7 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
   c.kernels++;
   if (nf > 0) {
     k_jkeys<<<nblk(nf, 256), 256, 0, st>>>(s.ej, nf, w.jkeys);
-    c.kernels += radix_sort_u64(w.jkeys, w.jtmp, nf, 27, 27 + body_bits(N), w.tmp, st);
+    c.kernels += radix_sort_u64(w.jkeys, w.jtmp, nf, kJkeyBody, kJkeyBody + body_bits(N), w.tmp, st);
     k_jlist<<<nblk(nf, 256), 256, 0, st>>>(w.jkeys, nf, s.jlist);
     c.kernels += 2;
   }
