@@ -639,12 +639,11 @@ static bool near_step(const Ctx& c, bool more_follow) {
 // The graph of a batch of 2^lg steps, opened by k_skin_begin; each step
 // ends with skin_batch_step_end.  Captured with s.sk_ctl set,
 // like the launches it holds.
-// `near` (the batches that another step follows) is part of the key: a batch
-// of one step exists in both variants, at 0 and at 5.
+// `near` is part of the key: the batches on the whole list follow the others.
 static int batch_graph(Ctx& c, int lg, bool near) {
   Scene& s = c.s;
   const int steps = 1 << lg;
-  if (!near) lg = 5;
+  if (!near) lg += kSkinBatchLg + 1;
   const bool stale =
       !c.bexec[lg] || c.bform[lg] != c.form || std::memcmp(&c.bscene[lg], &s, sizeof(Scene)) != 0;
   if (stale) {
@@ -681,18 +680,20 @@ static int skin_partial(Ctx& c, int64_t nflag);
 static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   Skin& k = c.skin;
   Scene& s = c.s;
-  // the call's last step is a batch of its own: it computes the whole list
+  // behind steps on the near set, the call's last step is a batch of its own:
+  // it computes the whole list, like all steps of a call that has no near set
+  // (an empty list, recorded geometry)
   const bool near = near_step(c, left > 1);
-  if (!near) k.whole_in_window++;
+  const int64_t most = near ? left - 1 : left;
   int lg = 0;
-  while (near && lg < kSkinBatchLg && (int64_t)2 << lg <= left - 1) lg++;
+  while (lg < kSkinBatchLg && (int64_t)2 << lg <= most) lg++;
   int64_t want = (int64_t)1 << lg;
-  if (near && !c.use_graphs) {
+  if (!c.use_graphs) {
     want = kSkinBatchFirst;
     if (k.crit > 0.0 && k.partial_since_global == 0)
       want = (int64_t)std::min((0.5 * k.skin / k.crit - 1.0) * (double)k.since + 1.0, (double)kSkinBatch);
     want = std::max(want, kSkinBatchLeast);
-    want = std::max<int64_t>(std::min(want, std::min(k.interval - k.since, left - 1)), 1);
+    want = std::max<int64_t>(std::min(want, std::min(k.interval - k.since, most)), 1);
   }
   unsigned int* in = k.h_ctl;
   unsigned int* out = k.h_ctl + 16;
@@ -731,6 +732,7 @@ static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
     c.interVerletC += s.dt;
   }
   c.steps += ex;
+  if (!near) k.whole_in_window += ex;
   *done = ex;
   c.more_steps_follow = ex < left;
   c.forces_stale = s.nheavy_lazy > 0;

@@ -185,12 +185,12 @@ struct Ctx {
   int gform[2] = {-1, -1};
   int glaunched[2] = {0, 0};     // kernels per replay
   int64_t graph_captures = 0, graph_replays = 0;
-  // the graphs of batches of 1, 2, 4, 8, 16 skin steps on the near set, and of
-  // one step on the whole list (same rules as the step graph)
-  cudaGraphExec_t bexec[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  Scene bscene[6]{};
-  int bform[6] = {-1, -1, -1, -1, -1, -1};
-  int blaunched[6] = {0, 0, 0, 0, 0, 0};
+  // the graphs of batches of 1, 2, 4, 8, 16 skin steps on the near set, then
+  // of as many on the whole list (same rules as the step graph)
+  cudaGraphExec_t bexec[10] = {};
+  Scene bscene[10]{};
+  int bform[10] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
+  int blaunched[10] = {};
 };
 
 // Neighbour-list update; with `only` (device flags per body), only the pairs

@@ -1,0 +1,84 @@
+"""Learned skin (GPU): the decisions of its batches of steps, their cost in
+host round trips, and the windows of its policy."""
+import numpy as np
+import pytest
+
+from test_gpu_near import _scene
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(src, form=0):
+    from rockable_gb300 import scenes
+    from rockable_gb300.abi import GpuScene
+    g = GpuScene(form=form)
+    g.upload_shapes(src["shape_tables"])
+    g.upload_bodies(src["bodies"], src["n_driven"])
+    scenes.set_scene_params(g, src)
+    if src.get("entries") is not None:
+        g.upload_entries(src["entries"])
+    return g
+
+
+@pytest.mark.parametrize("form", [0, 1])
+def test_batches_match_the_host_decided_path(gpu_lib, form):
+    """With the skin and the interval pinned the refreshes depend on the state
+    alone: batches decided on the device (as a graph, and launched one by one)
+    and the path that decides on the host after every step, which profiled
+    steps take, make the same refreshes and leave the same bits."""
+    from rockable_gb300 import scenes
+    scene = scenes.column_collapse(n=2000, nshapes=64, semi=(0.0025, 0.0075))
+    gs = scenes.settle(scene, steps=1500)
+    src = scenes.scene_from_gpu(scene, gs)
+    gs.close()
+    skin = 0.1 * scene["dVerlet"]
+    out = {}
+    for arm in ("host", "launched", "graph"):
+        g = _engine(src, form)
+        g.set_skin(use_mlp=False, skin_min=skin, skin_max=skin, interval_min=45, interval_max=45)
+        g.set_graphs(arm == "graph")
+        g.set_profiling(arm == "host")
+        for n in (7, 100, 33, 160):
+            g.step(n)
+        out[arm] = (g.bodies(), g.skin_stats(), g.entries())
+        g.close()
+    b0, s0, e0 = out.pop("host")
+    assert s0["rebuilds"] >= 3 and s0["partial"] + s0["forced"] >= 1
+    for arm, (b, s, e) in out.items():
+        for k in ("rebuilds", "forced", "scheduled", "partial", "partial_bodies"):
+            assert s0[k] == s[k], (arm, k, s0[k], s[k])
+        for k in b0:
+            assert np.array_equal(b0[k], b[k]), (arm, k)
+        for k in ("i", "j", "type", "isub", "jsub", "fn", "ft"):
+            assert np.array_equal(e0[k], e[k]), (arm, k)
+
+
+@pytest.mark.parametrize("kind", ["free flight", "recorded"])
+def test_steps_without_a_near_set_run_in_batches(gpu_lib, kind):
+    """An empty list (grains in free flight) and recorded contact geometry
+    have no near set: their steps share host round trips all the same."""
+    from rockable_gb300 import scenes
+    if kind == "free flight":
+        src = scenes.drop_bodies(scenes.sphero_cube_box(4), range(6))
+        src["bodies"]["pos"] *= 2.0
+    else:
+        src = _scene("avalanche", 0.0)
+    src["gravity"] = (0.0, 0.0, 0.0)
+    a, b = _engine(src), _engine(src)
+    for g, graphs in ((a, True), (b, False)):
+        g.set_skin(use_mlp=False, skin_min=src["dVerlet"], skin_max=src["dVerlet"], interval_min=4000,
+                   interval_max=4000)
+        g.set_record_geometry(kind == "recorded")
+        g.set_graphs(graphs)
+    assert (a.n_entries == 0) == (kind == "free flight")
+    r0 = a.graph_stats()["replays"]
+    for k in (128, 3, 1, 40):
+        a.step(k)
+        for _ in range(k):
+            b.step(1)
+    assert a.graph_stats()["replays"] - r0 <= 20
+    x, y = a.bodies(), b.bodies()
+    for k in x:
+        assert np.array_equal(x[k], y[k]), k
+    a.close()
+    b.close()
