@@ -312,6 +312,22 @@ static void skin_bind(Ctx& c, bool on) {
   s.sk_flag_at = on ? (float)(0.25 * k.skin) : 0.f;
 }
 
+// A list update that the policy did not make (rk_set_skin, rk_update_nl) opens
+// a window: what was counted before it is not the window's.
+static int skin_restart(Ctx& c) {
+  Skin& k = c.skin;
+  unsigned long long made = 0;
+  CK(cudaMemcpyAsync(&made, c.s.flags + FLAG_NEAR_MADE, sizeof made, cudaMemcpyDeviceToHost, c.stream));
+  CK(cudaStreamSynchronize(c.stream));
+  k.made_before = made;
+  k.whole_in_window = 0;
+  k.since = 0;
+  k.crit = 0.0;
+  k.partial_since_global = 0;
+  k.have_pred = false;
+  return 0;
+}
+
 static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
   {  // the flags are not read every step when the guard is pipelined
     const int rf = read_flags(c);
@@ -1462,10 +1478,8 @@ int rk_set_skin(rk_ctx* x, const rk_skin_config* cfg) {
   k.have_prev = false;
   k.skin = std::min(cfg->skin_max, std::max(cfg->skin_min, s.dVerlet));
   k.interval = cfg->interval_min;
-  k.since = 0;
-  k.crit = 0.0;
   k.rebuilds = k.forced = k.scheduled = 0;
-  k.partial = k.partial_bodies = k.partial_since_global = 0;
+  k.partial = k.partial_bodies = 0;
   k.rebuild_bp_ms = k.rebuild_var_ms = 0.0;
   k.alpha = 1.6;
   k.step_ms = k.rebuild_ms = 0.0;
@@ -1475,7 +1489,6 @@ int rk_set_skin(rk_ctx* x, const rk_skin_config* cfg) {
   for (cudaEvent_t* e : {&k.pa, &k.pb, &k.gev[0], &k.gev[1]})
     if (!*e) CK(cudaEventCreate(e));
   k.gslot = 0;
-  k.have_pred = false;
   k.partial_ms = 0.0;
   k.partial_in_window = 0;
   k.on = true;
@@ -1486,8 +1499,7 @@ int rk_set_skin(rk_ctx* x, const rk_skin_config* cfg) {
   if ((rc = rebuild_nl(c))) return rc;
   launch_skin_reset(s, nullptr, k.ref_pos, k.ref_q, k.maxd, k.path, c.stream);
   CK(cudaEventRecord(k.ea, c.stream));
-  CK(cudaStreamSynchronize(c.stream));
-  return RK_OK;
+  return skin_restart(c);
 }
 
 int rk_get_skin_stats(rk_ctx* x, rk_skin_stats* o) {
@@ -1628,10 +1640,7 @@ int rk_update_nl(rk_ctx* x) {
     // the skin's guard restarts from it, as after a full skin rebuild
     Skin& k = c.skin;
     c.kernels += launch_skin_reset(c.s, nullptr, k.ref_pos, k.ref_q, k.maxd, k.path, c.stream);
-    k.since = 0;
-    k.crit = 0.0;
-    k.partial_since_global = 0;
-    k.have_pred = false;
+    if ((rc = skin_restart(c))) return rc;
   }
   CK(cudaStreamSynchronize(c.stream));
   return RK_OK;

@@ -82,3 +82,28 @@ def test_steps_without_a_near_set_run_in_batches(gpu_lib, kind):
         assert np.array_equal(x[k], y[k]), k
     a.close()
     b.close()
+
+
+def test_a_new_skin_does_not_pay_for_earlier_steps(gpu_lib):
+    """Near sets that a context made before rk_set_skin are not charged to the
+    policy's first window: the same state in a new context gets the same skin."""
+    from rockable_gb300 import scenes
+    sc = scenes.column_collapse(n=3000, nshapes=24, tries=2, law="Default")
+    nd, n = sc["n_driven"], len(sc["bodies"]["mass"])
+    sc["bodies"]["vel"][nd:] = np.random.default_rng(1).normal(0.0, 3.0, (n - nd, 3))
+    sc["gravity"] = (0.0, 0.0, 0.0)
+    sc["interVerlet"] = 40 * sc["dt"]
+    a = _engine(sc)
+    a.update_nl()
+    a.step(1500)
+    src = scenes.scene_from_gpu(sc, a)
+    b = _engine(src)
+    d = sc["dVerlet"]
+    skins = []
+    for g in (a, b):
+        g.set_skin(use_mlp=False, skin_min=0.25 * d, skin_max=d, interval_min=20, interval_max=1000)
+        while g.skin_stats()["rebuilds"] == 0:
+            g.step(20)
+        skins.append(g.skin_stats()["skin"] / d)
+        g.close()
+    assert skins[0] == skins[1], skins
