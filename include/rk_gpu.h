@@ -359,13 +359,16 @@ int rk_sort_keys_noalloc(uint64_t* keys, int64_t n, int lo_bit, int hi_bit, void
  * forced rebuilds, a 16-64-64-2 MLP (FP16, trained online on the run's own
  * displacement and churn history) predicts the next window's displacement
  * rate, from which the skin (dVerlet, DVerlet = ratio * dVerlet) and the
- * rebuild interval are chosen by minimising the measured step + rebuild cost. */
+ * rebuild interval are chosen by minimising the cost per step: the measured
+ * times of full and partial refreshes, and a price per list entry of the near
+ * sets made and of the steps on the whole list in the window. */
 typedef struct rk_skin_config {
   int32_t enabled;
   int32_t use_mlp;        /* 0: predict the next window from the last one only */
   double skin_min, skin_max;
   double dverlet_ratio;   /* DVerlet / dVerlet */
-  int32_t interval_min, interval_max;
+  int32_t interval_min, interval_max;  /* steps; with use_mlp at most 320 (or interval_min) until the network
+                                          has 24 windows to learn from */
   double learning_rate;
   int32_t train_steps;    /* optimiser steps per rebuild */
   uint64_t seed;

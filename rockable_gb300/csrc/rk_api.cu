@@ -252,9 +252,13 @@ static const double kRebuildFixedMs = 0.6;
 // Time per list entry of making a near set, and of a step on the whole list
 // (FP64, mixed): measured on a list of 2.5 M entries, 0.22, 0.72 and 0.2 ms.
 static const double kMakeMs = 9e-8, kWholeMs[2] = {2.9e-7, 8e-8};
-// Longest window the cost model proposes: its displacement rate is a
-// prediction for the next window, and the network learns once per window.
+// Longest window that the cost model proposes while the network has fewer than
+// kLearnWindows windows to learn from (it learns once per window); then, and
+// without the network, interval_max alone bounds it.  (A collapsing column of
+// 3000 grains, 8000 steps: 579 ms in windows of at most 320, 573 ms in windows
+// of up to 1000, of which a run of that length has 8.)
 static const int64_t kMaxWindow = 320;
+static const size_t kLearnWindows = 24;
 
 static double to_f(unsigned int bits) {
   float f;
@@ -445,10 +449,13 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
   k.whole_in_window = 0;
   double best = 1e300, best_s = k.skin;
   int64_t best_k = k.interval;
+  int64_t longest = k.cfg.interval_max;
+  if (k.cfg.use_mlp && k.rx.size() < kLearnWindows)
+    longest = std::min<int64_t>(longest, std::max<int64_t>(kMaxWindow, k.cfg.interval_min));
   for (int m = -4; m <= 4; m++) {
     double sk = std::min(k.cfg.skin_max, std::max(k.cfg.skin_min, k.skin * std::pow(2.0, 0.25 * m)));
     double kk = std::floor(0.5 * sk / std::max(u * margin * (1.0 + churn), 1e-30));
-    int64_t ki = (int64_t)std::max<double>(k.cfg.interval_min, std::min<double>((double)std::min<int64_t>(k.cfg.interval_max, std::max<int64_t>(kMaxWindow, k.cfg.interval_min)), kk));
+    int64_t ki = (int64_t)std::max<double>(k.cfg.interval_min, std::min<double>((double)longest, kk));
     double ratio = (A + (C - A) * std::pow(sk / std::max(k.skin, 1e-30), alpha)) / C;
     double J = (Rbp * (0.7 + 0.3 * ratio) + Rfix + (Rvar - Rfix) * ratio) / (double)ki + P * (k.skin / sk) * Rp;
     J += (made * std::sqrt(k.skin / sk) * kMakeMs + whole * kWholeMs[c.form == RK_FORM_MIXED]) * C * ratio;

@@ -107,3 +107,19 @@ def test_a_new_skin_does_not_pay_for_earlier_steps(gpu_lib):
         skins.append(g.skin_stats()["skin"] / d)
         g.close()
     assert skins[0] == skins[1], skins
+
+
+@pytest.mark.parametrize("use_mlp,steps", [(False, 6000), (True, 14000)])
+def test_windows_reach_interval_max(gpu_lib, use_mlp, steps):
+    """Grains at rest: nothing uses up the skin, so the refreshes become as
+    rare as the caller allows (with the network, once it has learnt)."""
+    src = _scene("default", 0.0)
+    src["bodies"]["pos"][src["n_driven"]:, 2] += 0.002  # (off the floor)
+    src["gravity"] = (0.0, 0.0, 0.0)
+    g = _engine(src)
+    d = src["dVerlet"]
+    g.set_skin(use_mlp=use_mlp, skin_min=0.1 * d, skin_max=d, interval_min=2, interval_max=2000)
+    g.step(steps)
+    st = g.skin_stats()
+    assert st["interval"] == 2000, st
+    g.close()
