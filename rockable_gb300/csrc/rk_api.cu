@@ -531,7 +531,7 @@ static int step_launches(Ctx& c, bool near) {
   Scene& s = c.s;
   int n = 0;
   n += launch_controls_pre(s, c.stream);
-  n += launch_drift(s, c.stream);
+  n += launch_drift(s, near, c.stream);
   if (near) n += launch_near_update(s, c.stream);
   else n += launch_glob_vertices(s, c.stream);
   if (near) n += launch_narrow_near(s, c.stream);
@@ -559,7 +559,7 @@ static int tune_step(Ctx& c) {
   cudaStream_t st = c.stream;
   int n = launch_controls_pre(s, st);
   CK(cudaEventRecord(c.tev[0], st));
-  n += launch_drift(s, st);
+  n += launch_drift(s, false, st);
   CK(cudaEventRecord(c.tev[1], st));
   n += launch_glob_vertices(s, st);
   CK(cudaEventRecord(c.tev[2], st));
@@ -585,6 +585,7 @@ static int tune_step(Ctx& c) {
         if (c.tune_ms[k][q] < c.tune_ms[k][best]) best = q;
       s.tpb[k] = std::min(kTuneCand[best], max_tpb(k, c.form == RK_FORM_MIXED));
     }
+    if (c.form == RK_FORM_MIXED) s.tpb[3] = 0;  // (no drift kernel in these steps: the vertices' makes it)
   }
   return RK_OK;
 }
@@ -1704,7 +1705,7 @@ int rk_step(rk_ctx* x, int64_t nsteps, rk_step_report* rep) {
       if ((rc = tune_step(c))) return rc;
     } else if (!graphed) {
       mark(0, false); phase(0, launch_controls_pre(s, c.stream));
-      mark(1, false); phase(1, launch_drift(s, c.stream));
+      mark(1, false); phase(1, launch_drift(s, near, c.stream));
       mark(2, false); phase(2, near ? launch_near_update(s, c.stream) : launch_glob_vertices(s, c.stream));
       mark(3, false);
       phase(3, near ? launch_narrow_near(s, c.stream)

@@ -218,7 +218,9 @@ enum { FLAG_NEED_UPDATE = 0, FLAG_NACTIVE = 1, FLAG_NBROKEN = 2, FLAG_GPOS = 3, 
 
 // step kernels (rk_step.cu)
 int launch_controls_pre(const Scene& s, cudaStream_t st);
-int launch_drift(const Scene& s, cudaStream_t st);
+// near: a step on the near set (in the mixed form's steps on the whole list,
+// launch_glob_vertices makes the drift)
+int launch_drift(const Scene& s, bool near, cudaStream_t st);
 // all = false: only bodies with neighbour-list entries (the step's use)
 // all: every body's vertices (a list update), or with `mark` those of the marked bodies
 int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all = false, const uint8_t* mark = nullptr);
@@ -243,7 +245,7 @@ __device__ __forceinline__ bool step_halted(const Scene& s) { return s.sk_ctl !=
 
 int launch_fused_glob(const Scene& s, unsigned blocks, int threads, int only_listed, const uint8_t* mark,
                       cudaStream_t st);
-// in_step: the matrices are the step's (launch_drift_frames)
+// in_step: with the step's drift
 int launch_body_frames(const Scene& s, unsigned blocks, int threads, int in_step, cudaStream_t st);
 int launch_drift_frames(const Scene& s, unsigned blocks, int threads, cudaStream_t st);
 int launch_body_verts(const Scene& s, cudaStream_t st);

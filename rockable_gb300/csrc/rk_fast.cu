@@ -341,11 +341,31 @@ __device__ __forceinline__ void frame64(const Scene& s, int64_t b, double* R) {
 }
 
 // The step's drift (the first half of the velocity-Verlet step, above) and
-// FP64 frames: one thread per body makes the drift of a free body and
-// computes the rotation matrix of the quaternion (the matrix of qrot,
-// Particle.cpp:55-65 places the vertices with it), from which the narrow
-// phase's FP64 path places the few vertices it needs; and every body's part
-// of the near set's check and of a batched skin step's guard (GUARD).
+// FP64 frame of body b: the drift of a free body and the rotation matrix of
+// the quaternion (the matrix of qrot, Particle.cpp:55-65 places the vertices
+// with it), from which the narrow phase's FP64 path places the few vertices it
+// needs; and the body's part of the near set's check.  A step on the whole
+// list (NEAR false) makes no set: it needs no speed bounds, and loads what the
+// check compares with only when there is a set.
+template <bool NEAR>
+__device__ __forceinline__ BodyState drift_frame(const Scene& s, int64_t b, double* R) {
+  NearRef near = {};
+  bool stale = true;
+  if (NEAR) near = near_ref(s, b);
+  else stale = s.flags[FLAG_NEAR_STALE] != 0ull;
+  const BodyState k = b >= s.n_driven ? drift_body(s, b) : body_state(s, b);
+  frame64(s, b, R);
+  if (NEAR) {
+    near_track(s, b, k, near);
+  } else {
+    step_counters(s, b);
+    if (!stale) near_check(s, k, near_ref(s, b));
+  }
+  return k;
+}
+
+// Steps on the near set: one thread per body, with its part of a batched skin
+// step's guard (GUARD).
 template <bool GUARD>
 __global__ void k_drift_frames(Scene s) {
   if (GUARD && batch_halted(s)) return;
@@ -353,12 +373,9 @@ __global__ void k_drift_frames(Scene s) {
   BodyState k = {};
   SkinRef ref = {};
   if (b < s.n) {
-    const NearRef near = near_ref(s, b);
     if (GUARD) ref = skin_ref(s, b);
-    k = b >= s.n_driven ? drift_body(s, b) : body_state(s, b);
     double R[9];
-    frame64(s, b, R);
-    near_track(s, b, k, near);
+    k = drift_frame<true>(s, b, R);
   }
   if (GUARD) skin_guard_drift(s, b < s.n ? b : s.n, k, ref);
 }
@@ -366,40 +383,44 @@ __global__ void k_drift_frames(Scene s) {
 // What a step on the whole list and a list update need besides: the FP32
 // vertex offsets (world vertex - centre, the FP32 test's coordinates) of every
 // body, written coalesced by the block from FP32 copies of its bodies'
-// rotation matrices, and the centres rounded to FP32.  STEP: the matrices are
-// those of the step (rotm); otherwise they are computed here.
-template <bool STEP>
+// rotation matrices, and the centres rounded to FP32.  DRIFT: the step's
+// launch, which makes the drift as well, in one pass over the bodies: 25 us at
+// 50 000 grains in blocks of 128 (27 us in blocks of 256), 32 us in two passes.
+template <bool DRIFT, bool GUARD>
 __global__ void k_body_frames(Scene s) {
-  if (step_halted(s)) return;
+  if (GUARD ? batch_halted(s) : step_halted(s)) return;
   extern __shared__ float fr[];  // [blockDim.x][10]: the FP32 matrix (and a pad)
   const int64_t b0 = blockIdx.x * (int64_t)blockDim.x;
   const int64_t b = b0 + threadIdx.x;
+  BodyState k = {};
+  SkinRef ref = {};
   if (b < s.n) {
-    float* f = fr + 10 * threadIdx.x;
     double R[9];
-    if (STEP) {
-#pragma unroll
-      for (int d = 0; d < 9; d++) R[d] = s.rotm[9 * b + d];
+    if (GUARD) ref = skin_ref(s, b);
+    if (DRIFT) {
+      k = drift_frame<false>(s, b, R);
     } else {
+      k = body_state(s, b);
       frame64(s, b, R);
     }
+    float* f = fr + 10 * threadIdx.x;
 #pragma unroll
     for (int d = 0; d < 9; d++) f[d] = d2f(R[d]);
     f[9] = 0.f;
-    const V3 p = ld3(s.pos, b);
-    s.posf[b] = make_float4(d2f(p.x), d2f(p.y), d2f(p.z), d2f(s.rad[b]));
+    s.posf[b] = make_float4(d2f(k.x[0]), d2f(k.x[1]), d2f(k.x[2]), d2f(s.rad[b]));
   }
+  if (GUARD) skin_guard_drift(s, b < s.n ? b : s.n, k, ref);
   __syncthreads();
   const int64_t bend = min(b0 + (int64_t)blockDim.x, s.n);
   if (b0 >= bend) return;
   const int64_t k1 = s.gv_ofs[bend];
-  for (int64_t k = s.gv_ofs[b0] + threadIdx.x; k < k1; k += blockDim.x) {
-    const float* f = fr + 10 * (s.gv_body[k] - b0);
-    const float4 u = s.uvf[k];  // h v, FP32
+  for (int64_t v = s.gv_ofs[b0] + threadIdx.x; v < k1; v += blockDim.x) {
+    const float* f = fr + 10 * (s.gv_body[v] - b0);
+    const float4 u = s.uvf[v];  // h v, FP32
     const float ux = u.x, uy = u.y, uz = u.z;
-    s.gvr[3 * k] = f[0] * ux + f[1] * uy + f[2] * uz;
-    s.gvr[3 * k + 1] = f[3] * ux + f[4] * uy + f[5] * uz;
-    s.gvr[3 * k + 2] = f[6] * ux + f[7] * uy + f[8] * uz;
+    s.gvr[3 * v] = f[0] * ux + f[1] * uy + f[2] * uz;
+    s.gvr[3 * v + 1] = f[3] * ux + f[4] * uy + f[5] * uz;
+    s.gvr[3 * v + 2] = f[6] * ux + f[7] * uy + f[8] * uz;
   }
 }
 
@@ -449,8 +470,10 @@ __global__ void __launch_bounds__(kHeavyThreads) k_gather_heavy(Scene s, const i
 }  // namespace mx
 
 int launch_body_frames(const Scene& s, unsigned blocks, int threads, int in_step, cudaStream_t st) {
-  if (in_step) mx::k_body_frames<true><<<blocks, threads, 10 * sizeof(float) * threads, st>>>(s);
-  else mx::k_body_frames<false><<<blocks, threads, 10 * sizeof(float) * threads, st>>>(s);
+  const size_t smem = 10 * sizeof(float) * threads;
+  if (!in_step) mx::k_body_frames<false, false><<<blocks, threads, smem, st>>>(s);
+  else if (s.sk_ctl) mx::k_body_frames<true, true><<<blocks, threads, smem, st>>>(s);
+  else mx::k_body_frames<true, false><<<blocks, threads, smem, st>>>(s);
   return 1;
 }
 int launch_fused_glob(const Scene& s, unsigned blocks, int threads, int only_listed, const uint8_t* mark,
@@ -480,7 +503,7 @@ int launch_fused_heavy(const Scene& s, const int* list, int count, cudaStream_t 
 }
 cudaError_t fused_attributes(int which, cudaFuncAttributes* a) {
   if (which == 1) return cudaFuncGetAttributes(a, mx::k_gather_accel);
-  if (which == 2) return cudaFuncGetAttributes(a, mx::k_body_frames<true>);
+  if (which == 2) return cudaFuncGetAttributes(a, mx::k_body_frames<true, true>);
   return cudaFuncGetAttributes(a, mx::k_drift_frames<true>);
 }
 

@@ -44,30 +44,21 @@ __device__ __forceinline__ NearRef near_ref(const Scene& s, int64_t b) {
   r.stale = s.flags[FLAG_NEAR_STALE] != 0ull;
   return r;
 }
-// Body b at the step's positions (k): its speed bound and FP32 orientation for
-// the next near set, and the check of the present one: the largest motion of
-// a point of the body since the set was made, |x - x0| plus the swing radius
-// times the rotation bound 2 c (1 + c) of the quaternion chord c (differences
-// in FP64, the rest in float rounded up, as in the skin's guard), against the
-// body's allowance.  A motion that is not a number fails the check.
-__device__ __forceinline__ void near_track(const Scene& s, int64_t b, const BodyState& k, const NearRef& r) {
-  if (b == 0) {  // the step's counters
-    s.flags[FLAG_NACTIVE] = 0ull;
-    if (s.sk_out && !s.sk_ctl)
-      for (int d = 0; d < 8; d++) s.sk_out[d] = 0u;
-  }
-  float v2 = 0.f, w2 = 0.f;
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    const float v = d2f(k.v[d]), w = d2f(k.w[d]);
-    v2 += v * v;
-    w2 += w * w;
-  }
+// The step's counters, emptied by the thread of body 0.
+__device__ __forceinline__ void step_counters(const Scene& s, int64_t b) {
+  if (b != 0) return;
+  s.flags[FLAG_NACTIVE] = 0ull;
+  if (s.sk_out && !s.sk_ctl)
+    for (int d = 0; d < 8; d++) s.sk_out[d] = 0u;
+}
+// Check of the present near set for body b at the step's positions (k): the
+// largest motion of a point of the body since the set was made, |x - x0| plus
+// the swing radius times the rotation bound 2 c (1 + c) of the quaternion
+// chord c (differences in FP64, the rest in float rounded up, as in the skin's
+// guard), against the body's allowance.  A motion that is not a number fails
+// the check.
+__device__ __forceinline__ void near_check(const Scene& s, const BodyState& k, const NearRef& r) {
   const double* q = k.q;
-  const float sw = r.sw;
-  s.rate[b] = sqrtf(v2) + sqrtf(w2) * sw;
-  s.qf[b] = make_float4(d2f(q[0]), d2f(q[1]), d2f(q[2]), d2f(q[3]));
-  if (r.stale) return;
   float d2 = 0.f, m2 = 0.f, p2 = 0.f;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
@@ -82,8 +73,22 @@ __device__ __forceinline__ void near_track(const Scene& s, int64_t b, const Body
     p2 += p * p;
   }
   const float c = sqrtf(fminf(m2, p2)) * (1.f + 1e-5f);
-  const float moved = (sqrtf(d2) + 2.f * c * (1.f + c) * sw) * (1.f + 1e-5f) + 1e-12f;
+  const float moved = (sqrtf(d2) + 2.f * c * (1.f + c) * r.sw) * (1.f + 1e-5f) + 1e-12f;
   if (!(moved < r.allow)) s.flags[FLAG_NEAR_STALE] = 1ull;
+}
+// Both, and the body's speed bound and FP32 orientation for the next near set.
+__device__ __forceinline__ void near_track(const Scene& s, int64_t b, const BodyState& k, const NearRef& r) {
+  step_counters(s, b);
+  float v2 = 0.f, w2 = 0.f;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const float v = d2f(k.v[d]), w = d2f(k.w[d]);
+    v2 += v * v;
+    w2 += w * w;
+  }
+  s.rate[b] = sqrtf(v2) + sqrtf(w2) * r.sw;
+  s.qf[b] = make_float4(d2f(k.q[0]), d2f(k.q[1]), d2f(k.q[2]), d2f(k.q[3]));
+  if (!r.stale) near_check(s, k, r);
 }
 
 struct N3 {

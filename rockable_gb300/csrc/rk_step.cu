@@ -650,8 +650,8 @@ int launch_body_verts(const Scene& s, cudaStream_t st) {
 
 // 16 bodies a block until they fill the GPU (8 resident blocks per SM)
 static inline bool few_bodies(const Scene& s) { return s.n < 16 * 8 * 152 && s.ne <= kGlistMost; }
-int launch_drift(const Scene& s, cudaStream_t st) {
-  if (s.n <= 0) return 0;
+int launch_drift(const Scene& s, bool near, cudaStream_t st) {
+  if (s.n <= 0 || (s.fast_body && !near)) return 0;
   const int t = tpb_or(s, 3, 128, s.n);
   if (s.fast_body) return launch_drift_frames(s, nblk(s.n, t), t, st);
   if (s.sk_ctl) exact::k_drift<true, true><<<nblk(s.n, t), t, 0, st>>>(s);
@@ -662,10 +662,10 @@ int launch_drift(const Scene& s, cudaStream_t st) {
 int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all, const uint8_t* mark) {
   const int64_t nv = all || s.fast_body ? s.nvert : s.nlv;
   if (nv <= 0) return 0;
-  const int t = tpb_or(s, 2, 256, nv);
+  const int t = s.fast_body && !all ? tpb_or(s, 2, 128, s.n) : tpb_or(s, 2, 256, nv);
   if (s.fast_body) {
-    // the mixed form's step needs only the FP32 offsets (and the drift's frames);
-    // a list update needs the FP64 world vertices as well
+    // the mixed form's step needs only the FP32 offsets (and makes its drift with
+    // them); a list update needs the FP64 world vertices as well
     int k = launch_body_frames(s, nblk(s.n, t), t, all ? 0 : 1, st);
     if (all) k += launch_fused_glob(s, nblk(nv, t), t, 0, mark, st);
     return k;

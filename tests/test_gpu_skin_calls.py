@@ -53,8 +53,9 @@ def test_batches_match_the_host_decided_path(gpu_lib, form):
             assert np.array_equal(e0[k], e[k]), (arm, k)
 
 
+@pytest.mark.parametrize("form", [0, 1])
 @pytest.mark.parametrize("kind", ["free flight", "recorded"])
-def test_steps_without_a_near_set_run_in_batches(gpu_lib, kind):
+def test_steps_without_a_near_set_run_in_batches(gpu_lib, kind, form):
     """An empty list (grains in free flight) and recorded contact geometry
     have no near set: their steps share host round trips all the same."""
     from rockable_gb300 import scenes
@@ -64,7 +65,7 @@ def test_steps_without_a_near_set_run_in_batches(gpu_lib, kind):
     else:
         src = _scene("avalanche", 0.0)
     src["gravity"] = (0.0, 0.0, 0.0)
-    a, b = _engine(src), _engine(src)
+    a, b = _engine(src, form), _engine(src, form)
     for g, graphs in ((a, True), (b, False)):
         g.set_skin(use_mlp=False, skin_min=src["dVerlet"], skin_max=src["dVerlet"], interval_min=4000,
                    interval_max=4000)
