@@ -240,12 +240,18 @@ int rk_set_graphs(rk_ctx* ctx, int on);
 /* Number of step-graph captures and replays since the context was created. */
 int rk_get_graph_stats(const rk_ctx* ctx, int64_t* captures, int64_t* replays);
 /* Block-size autotuner: the next 5 * rounds steps run the narrow phase, the
- * resultants, the global vertices and the drift with block sizes 32, 64,
- * 128, 256 and 512 in turn, timed with events; each kernel then keeps its
- * fastest size.  These kernels give the same results at any block size, so the
- * tuning steps are ordinary steps.  No reference counterpart. */
+ * resultants, the global vertices and the drift of a step on the whole list
+ * with block sizes 32, 64, 128, 256 and 512 in turn, timed with events; each
+ * kernel then keeps its fastest size.  These kernels give the same results at
+ * any block size, so the tuning steps are ordinary steps.  Two sizes are not
+ * tuned: the resultants' of an FP64 scene below 19 456 bodies (8 lanes per
+ * body, blocks of 128) and the drift's of the mixed form (part of the vertex
+ * kernel on the whole list).  Steps that another step of the same call follows
+ * run other kernels, of fixed sizes, behind the same drift; so the tuned sizes
+ * are those of calls of one step and of each call's last.
+ * No reference counterpart. */
 int rk_set_autotune(rk_ctx* ctx, int rounds);
-/* Current block sizes of those four kernels, in that order. */
+/* Block sizes, in that order, that steps launch those four kernels with. */
 int rk_get_block_sizes(const rk_ctx* ctx, int32_t* tpb);
 /* When on, every step also stores each entry's contact normal, point and
  * relative velocity (needed to write a conf file); off by default. */

@@ -1566,10 +1566,7 @@ int rk_set_autotune(rk_ctx* x, int rounds) {
 
 int rk_get_block_sizes(const rk_ctx* x, int32_t* tpb) {
   if (!x || !tpb) return RK_ERR_ARG;
-  const Scene& s = x->c.s;
-  const int def[4] = {128, 128, 256, 128};
-  const int64_t items[4] = {s.ne, s.n, s.nvert, s.n};
-  for (int k = 0; k < 4; k++) tpb[k] = s.tpb[k] > 0 ? s.tpb[k] : items[k] < kSmallLaunch * 32 ? 32 : def[k];
+  for (int k = 0; k < 4; k++) tpb[k] = step_block_size(x->c.s, k);
   return RK_OK;
 }
 

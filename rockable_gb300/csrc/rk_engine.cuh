@@ -239,6 +239,9 @@ int launch_guard(const Scene& s, cudaStream_t st);
 int launch_kinetic_energy(const Scene& s, double* d_out2, cudaStream_t st);
 int launch_kin_pack(const Scene& s, double* stage, int dir, cudaStream_t st);
 int max_tpb(int which, int form_mixed);
+// threads per block of a step's narrow phase (the mixed form's first pass), resultants, vertices and
+// drift: tuned, or by default (steps on the near set: the drift's alone)
+int step_block_size(const Scene& s, int which);
 // per-body kernels compiled with fused multiply-adds (rk_fast.cu, mixed form)
 // a batched skin step after the guard asked for a refresh: the kernel does nothing
 __device__ __forceinline__ bool step_halted(const Scene& s) { return s.sk_ctl != nullptr && s.sk_ctl[0] != 0u; }

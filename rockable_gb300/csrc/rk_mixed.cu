@@ -611,7 +611,7 @@ int launch_narrow_near_mixed(const Scene& s, cudaStream_t st) {
 
 int launch_narrow_force_mixed(const Scene& s, cudaStream_t st) {
   if (s.ne <= 0) return 0;
-  const int t = s.tpb[0] > 0 ? s.tpb[0] : 128;
+  const int t = step_block_size(s, 0);
   k_narrow_mixed_quick<<<(unsigned)((s.ne + t - 1) / t), t, 0, st>>>(s);
   return 1 + launch_narrow_near_mixed(s, st);
 }

@@ -620,8 +620,18 @@ int launch_controls_pre(const Scene& s, cudaStream_t st) {
   k_controls_pre<<<1, 32, 0, st>>>(s);
   return 1;
 }
+// 16 bodies a block until they fill the GPU (8 resident blocks per SM)
+static inline bool few_bodies(const Scene& s) { return s.n < 16 * 8 * 152 && s.ne <= kGlistMost; }
 static inline int tpb_or(const Scene& s, int k, int d, int64_t items) {
   return s.tpb[k] > 0 ? s.tpb[k] : items < kSmallLaunch * 32 ? 32 : d;
+}
+int step_block_size(const Scene& s, int which) {
+  switch (which) {
+    case 0: return s.fast_body ? (s.tpb[0] > 0 ? s.tpb[0] : 128) : tpb_or(s, 0, 128, s.ne);
+    case 1: return !s.fast_body && few_bodies(s) ? exact::kGatherNear : tpb_or(s, 1, 128, s.n);
+    case 2: return s.fast_body ? tpb_or(s, 2, 128, s.n) : tpb_or(s, 2, 256, s.nlv);
+    default: return tpb_or(s, 3, 128, s.n);
+  }
 }
 
 // The per-body kernels come in two builds (rk_body.cuh): exact (this file,
@@ -648,11 +658,9 @@ int launch_body_verts(const Scene& s, cudaStream_t st) {
   return 1;
 }
 
-// 16 bodies a block until they fill the GPU (8 resident blocks per SM)
-static inline bool few_bodies(const Scene& s) { return s.n < 16 * 8 * 152 && s.ne <= kGlistMost; }
 int launch_drift(const Scene& s, bool near, cudaStream_t st) {
   if (s.n <= 0 || (s.fast_body && !near)) return 0;
-  const int t = tpb_or(s, 3, 128, s.n);
+  const int t = step_block_size(s, 3);
   if (s.fast_body) return launch_drift_frames(s, nblk(s.n, t), t, st);
   if (s.sk_ctl) exact::k_drift<true, true><<<nblk(s.n, t), t, 0, st>>>(s);
   else if (few_bodies(s)) exact::k_drift<false, true><<<nblk(s.n, t), t, 0, st>>>(s);
@@ -662,7 +670,7 @@ int launch_drift(const Scene& s, bool near, cudaStream_t st) {
 int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all, const uint8_t* mark) {
   const int64_t nv = all || s.fast_body ? s.nvert : s.nlv;
   if (nv <= 0) return 0;
-  const int t = s.fast_body && !all ? tpb_or(s, 2, 128, s.n) : tpb_or(s, 2, 256, nv);
+  const int t = all ? tpb_or(s, 2, 256, nv) : step_block_size(s, 2);
   if (s.fast_body) {
     // the mixed form's step needs only the FP32 offsets (and makes its drift with
     // them); a list update needs the FP64 world vertices as well
@@ -675,7 +683,7 @@ int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all, const uint8_
 }
 int launch_narrow_force(const Scene& s, cudaStream_t st) {
   if (s.ne <= 0) return 0;
-  const int t = tpb_or(s, 0, 128, s.ne);
+  const int t = step_block_size(s, 0);
   k_narrow_force<<<nblk(s.ne + 4 * 31, t), t, 0, st>>>(s);  // (each type's run padded to warps)
   return 1;
 }
@@ -696,7 +704,7 @@ int launch_gather_near(const Scene& s, cudaStream_t st) {
 }
 int launch_gather_accel(const Scene& s, int apply_kick, cudaStream_t st) {
   if (s.n <= 0) return 0;
-  const int t = tpb_or(s, 1, 128, s.n);
+  const int t = step_block_size(s, 1);
   if (s.fast_body) return launch_fused_gather(s, nblk(s.n, t), t, apply_kick, st);  // one body per thread
   if (few_bodies(s)) {  // (the bodies of many entries included: 32 us -> 13 us at 512 bodies)
     exact::k_gather_near<16, true><<<(unsigned)s.nbig + nblk(s.n, 16), exact::kGatherNear, 0, st>>>(s, apply_kick);
