@@ -106,3 +106,32 @@ def test_bonds_without_interfaces(gpu_lib, form):
         _same(a, b, form)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("form", [0, 1])
+def test_near_set_steps_of_a_large_scene(gpu_lib, form):
+    """More than 19 456 bodies (one thread per body in the resultants and in
+    the drift), not a multiple of a block, with walls of more than 1024
+    entries whose resultants a block sums."""
+    from rockable_gb300 import scenes
+    sc = scenes.iso_compression(n=20011, nshapes=24, tries=1)
+    sc["dVerlet"] *= 3.0
+    sc["DVerlet"] *= 3.0
+    nd, n = sc["n_driven"], len(sc["bodies"]["mass"])
+    rng = np.random.default_rng(11)
+    sc["bodies"]["vel"][nd:] = rng.normal(0, 0.3, (n - nd, 3))
+    sc["bodies"]["vrot"][nd:] = rng.normal(0, 30.0, (n - nd, 3))
+    sc["interVerlet"] = 20 * sc["dt"]
+    a, b = _engine(sc, form, False), _engine(sc, form, True)
+    e = a.entries()
+    assert max(np.sum((e["i"] == w) | (e["j"] == w)) for w in (1, 3, 5)) > 1024
+    shift = np.zeros((n, 3))
+    shift[nd::2, 2] = 2e-5  # half of the grains into their neighbours
+    for g in (a, b):
+        g.upload_kinematics(pos=np.ascontiguousarray(g.bodies()["pos"] + shift))
+    for _ in range(33):
+        a.step(1)
+    b.step(33)
+    assert _same(a, b, form)["active"].sum() > 1000
+    a.close()
+    b.close()
