@@ -303,21 +303,20 @@ __device__ __forceinline__ BodyState drift_body(const Scene& s, int64_t i) {
   return {{p.x, p.y, p.z}, {v.x, v.y, v.z}, {q.s, q.v.x, q.v.y, q.v.z}, {w.x, w.y, w.z}, path};
 }
 // the free bodies' drift; every body's part of the near set's check and of a
-// batched skin step's guard (GUARD).  AHEAD: what these compare with is loaded
-// before the drift's stores, for scenes that leave load latencies uncovered
-// (3000 bodies 10.2 -> 9.2 us); 50 000 bodies are 2 % faster without it.
-template <bool GUARD, bool AHEAD>
+// batched skin step's guard (GUARD).  What these compare with is loaded before
+// the drift's stores, so that it shares the drift's round of loads (loaded
+// after them, scenes of 3000 to 200 000 bodies take the same time within 1 %,
+// 22 000 to 30 000 up to 1 % more).
+template <bool GUARD>
 __global__ void k_drift(Scene s) {
   if (GUARD && batch_halted(s)) return;
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   BodyState k = {};
   SkinRef ref = {};
   if (i < s.n) {
-    NearRef near;
-    if (AHEAD) near = near_ref(s, i);
+    const NearRef near = near_ref(s, i);
     if (GUARD) ref = skin_ref(s, i);
     k = i >= s.n_driven ? drift_body(s, i) : body_state(s, i);
-    if (!AHEAD) near = near_ref(s, i);
     near_track(s, i, k, near);
   }
   if (GUARD) skin_guard_drift(s, i < s.n ? i : s.n, k, ref);

@@ -663,9 +663,8 @@ int launch_drift(const Scene& s, bool near, cudaStream_t st) {
   if (s.n <= 0 || (s.fast_body && !near)) return 0;
   const int t = step_block_size(s, 3);
   if (s.fast_body) return launch_drift_frames(s, nblk(s.n, t), t, st);
-  if (s.sk_ctl) exact::k_drift<true, true><<<nblk(s.n, t), t, 0, st>>>(s);
-  else if (few_bodies(s)) exact::k_drift<false, true><<<nblk(s.n, t), t, 0, st>>>(s);
-  else exact::k_drift<false, false><<<nblk(s.n, t), t, 0, st>>>(s);
+  if (s.sk_ctl) exact::k_drift<true><<<nblk(s.n, t), t, 0, st>>>(s);
+  else exact::k_drift<false><<<nblk(s.n, t), t, 0, st>>>(s);
   return 1;
 }
 int launch_glob_vertices(const Scene& s, cudaStream_t st, bool all, const uint8_t* mark) {
@@ -723,7 +722,7 @@ int max_tpb(int which, int form_mixed) {
   else if (form_mixed) e = fused_attributes(which, &a);
   else if (which == 1) e = cudaFuncGetAttributes(&a, exact::k_gather_accel);
   else if (which == 2) e = cudaFuncGetAttributes(&a, exact::k_glob_vertices);
-  else e = cudaFuncGetAttributes(&a, exact::k_drift<true, true>);
+  else e = cudaFuncGetAttributes(&a, exact::k_drift<true>);
   return e == cudaSuccess ? a.maxThreadsPerBlock : 128;
 }
 int launch_gather_heavy(const Scene& s, cudaStream_t st) {
