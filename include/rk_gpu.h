@@ -354,8 +354,10 @@ int rk_sort_keys(uint64_t* keys, int64_t n, int lo_bit, int hi_bit, void* stream
 int rk_sort_keys_noalloc(uint64_t* keys, int64_t n, int lo_bit, int hi_bit, void* stream);
 /* Per-phase device time: when on, rk_step brackets each phase with CUDA
  * events on the context stream (adds one event pair per phase and step).
- * Phases: 0 controls, 1 drift, 2 global vertices, 3 narrow phase + law,
- * 4 resultants + accelerations, 5 breakage, 6 NL rebuild, 7 guard. */
+ * Phases: 0 controls, 1 drift, 2 global vertices (steps that another step of
+ * the call follows: the update of the near set; the mixed form's steps on the
+ * whole list: the drift too), 3 narrow phase + law, 4 resultants +
+ * accelerations, 5 breakage, 6 NL rebuild, 7 guard. */
 #define RK_NPHASE 8
 
 /* Learned Verlet skin (no reference counterpart; replaces the fixed

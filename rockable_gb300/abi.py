@@ -396,6 +396,7 @@ class GpuScene:
         self._chk(self.L.rk_mlp_gradient(self.h, _p(X), _p(T), len(X), _p(g), _p(loss)), "rk_mlp_gradient")
         return g, float(loss[0])
 
+    # (glob_vertices: in steps on the near set, its update)
     PHASES = ["controls", "drift", "glob_vertices", "narrow_force", "gather_accel", "breakage", "nl_rebuild", "guard"]
 
     def profile(self):

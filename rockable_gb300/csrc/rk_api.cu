@@ -520,8 +520,8 @@ static int skin_rebuild(Ctx& c, double dmax, double vmax, bool forced) {
   return 0;
 }
 
-// The launches of one step body (flag reset, controls, drift, global
-// vertices, narrow phase + law, resultants + accelerations, breakage) as one
+// The launches of one step body (controls, drift, near set or global vertices,
+// narrow phase + law, resultants + accelerations, breakage), and the same as a
 // CUDA graph: captured on the context stream the first time and whenever the
 // scene description the kernels receive by value has changed since (a
 // rebuild swaps the entry buffers, a parameter call changes scalars), then

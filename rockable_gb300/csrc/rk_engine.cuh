@@ -184,7 +184,7 @@ struct Scene {
   const double* sk_ref_q;
   float* sk_maxd;
   uint8_t* sk_flag;
-  unsigned int* sk_out;  // 8 words, zeroed by the resultant kernel's launcher (by k_skin_begin in a batch)
+  unsigned int* sk_out;  // 8 words, zeroed by the drift's thread of body 0 (in a batch by k_skin_begin and each step's end)
   float sk_flag_at;
   // batched skin steps (rk_skin.cu, skin_batch_step_end): when set, every step kernel
   // returns at once while sk_ctl[0] (halt) is set
