@@ -76,6 +76,23 @@ cudaError_t near_set_stale(Ctx& c) {
   return cudaMemsetAsync(c.s.flags + FLAG_NEAR_STALE, 1, 1, c.stream);
 }
 
+// Looked at when a list update or the end of a call reads the count of sets
+// made: in the mixed form, a step that makes its set costs about half as much
+// more than a step on the whole list as a step on a set that lasts costs less
+// (50 000 grains: 195, 165 and 100 us; 24 000: 110, 85 and 60 us), so when more
+// than half of the steps made theirs -- grains that use up their allowance in
+// a step or two, positions set by the host before every short call -- the next
+// kNearRest steps run on the whole list before sets are tried again (24 000
+// fast grains, calls of 10 steps: 109 -> 81 us a step, 4300: 59 -> 55 us).  The
+// FP64 form's whole list costs four times a set (950 and 230 us).
+constexpr int64_t kNearLook = 8, kNearRest = 200;
+void near_review(Ctx& c, unsigned long long made) {
+  if (c.near_steps < kNearLook) return;
+  if (c.form == RK_FORM_MIXED && 2 * (int64_t)(made - c.near_made) > c.near_steps) c.near_rest = kNearRest;
+  c.near_made = made;
+  c.near_steps = 0;
+}
+
 static void free_entrybuf(EntryBuf& b) {
   dfree(b.ei); dfree(b.ej); dfree(b.etsub); dfree(b.ekey); dfree(b.dn); dfree(b.fn); dfree(b.ft); dfree(b.mom);
   dfree(b.damp); dfree(b.bond); dfree(b.gn); dfree(b.gpos); dfree(b.gvel);
@@ -655,9 +672,10 @@ constexpr int kSkinBatchLg = 4;
 constexpr int64_t kSkinBatch = 64, kSkinBatchFirst = 16, kSkinBatchLeast = 4;
 
 // Whether a step runs on the near set (rk_near.cu): another step of the call
-// follows, and the contact geometry is not being recorded for every entry.
+// follows, the contact geometry is not being recorded for every entry, and
+// sets last (near_review).
 static bool near_step(const Ctx& c, bool more_follow) {
-  return more_follow && c.s.ne > 0 && c.s.ne <= kGlistMost && c.s.egv_ok && !c.s.record_geom;
+  return more_follow && c.near_rest <= 0 && c.s.ne > 0 && c.s.ne <= kGlistMost && c.s.egv_ok && !c.s.record_geom;
 }
 
 // The graph of a batch of 2^lg steps, opened by k_skin_begin; each step
@@ -757,6 +775,8 @@ static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   }
   c.steps += ex;
   if (!near) k.whole_in_window += ex;
+  if (near) c.near_steps += ex;
+  else c.near_rest = std::max<int64_t>(c.near_rest - ex, 0);
   *done = ex;
   c.more_steps_follow = ex < left;
   c.forces_stale = s.nheavy_lazy > 0;
@@ -810,10 +830,10 @@ static bool guard_pipelined(const Ctx& c) {
   return s.ncontrols == 0 && s.servo_kind == 0 && s.nif == 0 && s.dynamic_nl == 0;
 }
 
-int skin_after_step(Ctx& c) {
+int skin_after_step(Ctx& c, bool near) {
   Skin& k = c.skin;
   Scene& s = c.s;
-  if (!near_step(c, c.more_steps_follow)) k.whole_in_window++;
+  if (!near) k.whole_in_window++;
   // the step's resultant kernel evaluated the guard into d_guard
   const int slot = k.gslot;
   unsigned int* hg = k.h_guard + 8 * slot;
@@ -1679,6 +1699,8 @@ int rk_step(rk_ctx* x, int64_t nsteps, rk_step_report* rep) {
     c.interVerletC += s.dt;
     c.more_steps_follow = it + 1 < nsteps;
     const bool near = !tuning && near_step(c, c.more_steps_follow);
+    if (near) c.near_steps++;
+    else if (c.near_rest > 0) c.near_rest--;
     if (graphed) {
       if ((rc = step_graph(c, near))) return rc;
     }
@@ -1714,7 +1736,7 @@ int rk_step(rk_ctx* x, int64_t nsteps, rk_step_report* rep) {
     }
     c.forces_stale = s.nheavy_lazy > 0;
     if (c.skin.on) {
-      if ((rc = skin_after_step(c))) return rc;
+      if ((rc = skin_after_step(c, near))) return rc;
       c.steps++;
       continue;
     }
@@ -1748,6 +1770,7 @@ int rk_step(rk_ctx* x, int64_t nsteps, rk_step_report* rep) {
   c.last_kernels = c.kernels - k0;
   if (rep) {
     if ((rc = read_flags(c))) return rc;
+    near_review(c, c.h_flags[FLAG_NEAR_MADE]);
     rep->steps_done = nsteps;
     rep->nl_updates = c.nl_updates - nl0;
     rep->n_entries = s.ne;

@@ -158,6 +158,10 @@ struct Ctx {
   int64_t grid_n = -1;  // bodies of that build (-1: none yet)
   bool forces_stale = false;
   bool more_steps_follow = false;  // inside rk_step, before its last step
+  // whether near sets last (near_review): steps on the near set since the last
+  // look, sets made up to it, and the steps that stay on the whole list
+  int64_t near_steps = 0, near_rest = 0;
+  unsigned long long near_made = 0;
   int64_t nsph = 0;                // sub-element spheres of all bodies
   double* kin_stage = nullptr;     // packed kinematics transfers (19 doubles per body)
   int64_t kin_stage_n = 0;
@@ -200,5 +204,6 @@ int heavy_list(Ctx& c);
 int ensure_entry_capacity(Ctx& c, int which, int64_t n);
 void bind_entries(Ctx& c);
 cudaError_t near_set_stale(Ctx& c);
+void near_review(Ctx& c, unsigned long long made);
 
 }  // namespace rk

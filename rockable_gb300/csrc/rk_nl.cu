@@ -906,9 +906,11 @@ int rebuild_nl(Ctx& c, const uint8_t* only) {
   k_body_obb<<<nblk(N, 128), 128, 0, st>>>(s);
   c.kernels++;
   {  // a body whose state is no longer finite: stop here, loudly
-    unsigned long long bad = 0;
-    RKCHK(cudaMemcpyAsync(&bad, s.flags + FLAG_NONFINITE, sizeof bad, cudaMemcpyDeviceToHost, st));
+    unsigned long long f[FLAG_NEAR_MADE - FLAG_NONFINITE + 1] = {};
+    RKCHK(cudaMemcpyAsync(f, s.flags + FLAG_NONFINITE, sizeof f, cudaMemcpyDeviceToHost, st));
     RKCHK(cudaStreamSynchronize(st));
+    near_review(c, f[FLAG_NEAR_MADE - FLAG_NONFINITE]);
+    const unsigned long long bad = f[0];
     if (bad) {
       c.err = "non-finite position or orientation of body " + std::to_string(bad - 1) +
               " (unstable time step or exploding contact?)";
