@@ -1113,7 +1113,7 @@ int rk_upload_bodies(rk_ctx* x, const rk_bodies* b) {
       (rc = dupload(c, s.bobb, (const double*)nullptr, 15 * n)) ||
       (rc = dupload(c, s.bobbf, (const float*)nullptr, 15 * n)) ||
       (rc = dupload(c, s.bbox, (const float*)nullptr, 15 * n)) ||
-      (rc = dalloc(c, s.posf, n)) || (rc = dalloc(c, s.rotm, 9 * n)) || (rc = dalloc(c, s.gsum, 6 * n)) ||
+      (rc = dalloc(c, s.posf, 2 * n)) || (rc = dalloc(c, s.rotm, 9 * n)) || (rc = dalloc(c, s.gsum, 6 * n)) ||
       (rc = dalloc(c, s.uv64, 3 * std::max<int64_t>(nv, 1))) || (rc = dalloc(c, s.uvf, std::max<int64_t>(nv, 1))) ||
       (rc = dupload(c, s.baabb, (const float*)nullptr, 6 * n)) ||
       (rc = dupload(c, s.dpos, (const double*)nullptr, 3 * n)) || (rc = dupload(c, s.dq, (const double*)nullptr, 4 * n)) ||

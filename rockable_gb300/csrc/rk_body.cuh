@@ -336,7 +336,6 @@ __global__ void k_glob_vertices(Scene s, int only_listed, const uint8_t* mark) {
   if (only_listed) k = s.lv[k];
   int b = s.gv_body[k];
   if (mark && !mark[b]) return;
-  const int local = (int)(k - s.gv_ofs[b]);
   const V3 u = v3(s.uv64[3 * k], s.uv64[3 * k + 1], s.uv64[3 * k + 2]);  // h v, computed at upload
   V3 r = qrot(ldq(s.Q, b), u);
   V3 g = ld3(s.pos, b) + r;
@@ -345,10 +344,6 @@ __global__ void k_glob_vertices(Scene s, int only_listed, const uint8_t* mark) {
     s.gvr[3 * k] = (float)r.x;
     s.gvr[3 * k + 1] = (float)r.y;
     s.gvr[3 * k + 2] = (float)r.z;
-    if (local == 0) {
-      const V3 p = ld3(s.pos, b);
-      s.posf[b] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)s.rad[b]);
-    }
   }
 }
 

@@ -90,8 +90,8 @@ struct Scene {
   double* gv;        // 3*nvert
   float* gvr;        // 3*nvert: the same vertices relative to their body's centre, in FP32 (the
                      // mixed form's test of clearly separated entries)
-  float4* posf;      // n: body centre rounded to FP32 and its Minkowski radius, written with the
-                     // world vertices (the same test)
+  float4* posf;      // 2 per body: its centre as the sum of two floats, the first with the Minkowski
+                     // radius behind it, written with gvr (the same test)
   double* uv64;      // 3*nvert: each body vertex scaled by the body's homothety, h v, in the shape
                      // frame (written at upload: what every placement of a vertex starts from)
   float4* uvf;       // nvert: the same rounded to FP32

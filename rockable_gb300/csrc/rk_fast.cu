@@ -383,7 +383,7 @@ __global__ void k_drift_frames(Scene s) {
 // What a step on the whole list and a list update need besides: the FP32
 // vertex offsets (world vertex - centre, the FP32 test's coordinates) of every
 // body, written coalesced by the block from FP32 copies of its bodies'
-// rotation matrices, and the centres rounded to FP32.  DRIFT: the step's
+// rotation matrices, and the centres as sums of two floats.  DRIFT: the step's
 // launch, which makes the drift as well, in one pass over the bodies: 25 us at
 // 50 000 grains in blocks of 128 (27 us in blocks of 256), 32 us in two passes.
 template <bool DRIFT, bool GUARD>
@@ -407,7 +407,9 @@ __global__ void k_body_frames(Scene s) {
 #pragma unroll
     for (int d = 0; d < 9; d++) f[d] = d2f(R[d]);
     f[9] = 0.f;
-    s.posf[b] = make_float4(d2f(k.x[0]), d2f(k.x[1]), d2f(k.x[2]), d2f(s.rad[b]));
+    const float4 hi = make_float4(d2f(k.x[0]), d2f(k.x[1]), d2f(k.x[2]), d2f(s.rad[b]));
+    s.posf[2 * b] = hi;
+    s.posf[2 * b + 1] = make_float4(d2f(k.x[0] - f2d(hi.x)), d2f(k.x[1] - f2d(hi.y)), d2f(k.x[2] - f2d(hi.z)), 0.f);
   }
   if (GUARD) skin_guard_drift(s, b < s.n ? b : s.n, k, ref);
   __syncthreads();

@@ -79,13 +79,13 @@ __device__ __forceinline__ float amax(F3 a) { return fmaxf(fabsf(a.x), fmaxf(fab
 
 // What FP32 geometry alone proves about an entry: its sub-elements'
 // vertices relative to body j's centre (the FP32 offsets gvr, plus the
-// difference of the two centres rounded to FP32, posf), the same projection
-// parameters as the FP64 path, and the separation's length.
+// difference dxij of the two centres, from posf), the same projection
+// parameters as the FP64 path, and the separation's length.  All of them err
+// by a few ulps of `mag`, the largest of the relative coordinates and of dxij
+// (which a large body's offsets cancel).
 //   kApart    the projection or the closest points lie inside their ranges by
-//             more than their rounding error, and the overlap estimate dnf errs by a few ulps of the coordinates
-//             (relative ones, and the centres' absolute ones: `cmag`), so an
-//             estimate above a margin of 2e-6 m plus 2e-6 of the relative
-//             coordinates' magnitude plus 4e-7 of the centres' proves dn > 0:
+//             more than their rounding error, and the overlap estimate dnf is
+//             above a margin of 2e-6 m plus 2e-6 of mag, which proves dn > 0:
 //             the FP64 length, the contact point and everything after are
 //             skipped, and dnf is kept as the entry's dn (a separated entry's
 //             dn only matters through its sign);
@@ -103,16 +103,16 @@ __device__ __forceinline__ bool lost_before(double dn) {
   return __double_as_longlong(dn) == (long long)0x8000000000000000ull;
 }
 __device__ __forceinline__ int apart_f32(const Scene& s, int type, int i, int j, int isub, int jsub, bool pre,
-                                         int4 G, F3 dxij, float rsum, float cmag, float* dnf) {
+                                         int4 G, F3 dxij, float rsum, float* dnf) {
   const float* g = s.gvr;
   auto gi = [&](int local) { return (int64_t)s.gv_ofs[i] + local; };
   auto gj = [&](int local) { return (int64_t)s.gv_ofs[j] + local; };
   F3 d;
-  float mag;
+  float mag = amax(dxij);
   if (type == 0) {
     const F3 a = ldgvr(g, pre ? G.x : gi(isub)) + dxij, b = ldgvr(g, pre ? G.y : gj(jsub));
     d = a - b;
-    mag = fmaxf(amax(a), amax(b));
+    mag = fmaxf(mag, fmaxf(amax(a), amax(b)));
   } else if (type == 1) {
     int64_t k1, k2;
     if (pre) { k1 = G.y; k2 = G.z; }
@@ -125,9 +125,9 @@ __device__ __forceinline__ int apart_f32(const Scene& s, int type, int i, int j,
     const F3 E = p2 - p1, w = a - p1;
     const float E2 = dotf(E, E);
     const float r = dotf(w, E) / E2;
-    mag = fmaxf(amax(a), fmaxf(amax(p1), amax(p2)));
+    mag = fmaxf(mag, fmaxf(amax(a), fmaxf(amax(p1), amax(p2))));
     // r's error: that of w and E (a few ulps of the coordinates) over |E|
-    const float tol = 1e-5f + 4e-7f * (mag + cmag) * rsqrtf(E2) * (1.f + fabsf(r));
+    const float tol = 1e-5f + 4e-6f * mag * rsqrtf(E2) * (1.f + fabsf(r));
     if (!(r > tol && r < 1.f - tol)) return (r < -tol || r > 1.f + tol) ? kOutside : 0;
     d = w - r * E;
   } else if (type == 2) {
@@ -153,13 +153,13 @@ __device__ __forceinline__ int apart_f32(const Scene& s, int type, int i, int j,
     edge(z, bA);
     edge(bA, cA);
     edge(cA, z);
-    mag = fmaxf(amax(a), fmaxf(amax(A), fmaxf(amax(B), amax(C))));
+    mag = fmaxf(fmaxf(mag, amax(a)), fmaxf(amax(A), fmaxf(amax(B), amax(C))));
     {
       // the projection clearly outside the triangle: farther than the
       // rounding of the coordinates beyond one of its edges (in the plane,
       // on the side away from the third vertex); clearly inside: farther than
       // that from all three
-      const float tol = 1e-9f + 1e-6f * (mag + cmag);
+      const float tol = 1e-9f + 4e-6f * mag;
       const F3 Pv = P, cA2 = cA;
       const float o = dotf(crossf(bA, cA2), nn);  // the triangle's winding about nn
       if (!(fabsf(o) > 0.f)) return 0;
@@ -176,7 +176,7 @@ __device__ __forceinline__ int apart_f32(const Scene& s, int type, int i, int j,
       if (!in) return 0;
     }
     *dnf = dist - rsum;
-    return *dnf > 2e-6f + 2e-6f * mag + 4e-7f * cmag ? kApart : 0;
+    return *dnf > 2e-6f + 2e-6f * mag ? kApart : 0;
   } else {
     int64_t a1, a2, b1, b2;
     if (pre) { a1 = G.x; a2 = G.y; b1 = G.z; b2 = G.w; }
@@ -193,18 +193,18 @@ __device__ __forceinline__ int apart_f32(const Scene& s, int type, int i, int j,
     f = 1.0f / f;
     const float a = dotf(Ei, w), b = dotf(Ej, w);
     const float ss = (ee * b - a * dd) * f, tt = (c * b - ee * a) * f;
-    mag = fmaxf(fmaxf(amax(pi1), amax(pi2)), fmaxf(amax(pj1), amax(pj2)));
+    mag = fmaxf(mag, fmaxf(fmaxf(amax(pi1), amax(pi2)), fmaxf(amax(pj1), amax(pj2))));
     // well-conditioned pairs only (the sine of the edges' angle above
     // 0.1): the parameters' error is then a few ulps of the coordinates
     // over the shorter edge, amplified by at most 100 by the solve
     if (!(f * c * dd < 100.f)) return 0;
-    const float tol = 1e-5f + 4e-5f * (mag + cmag) * rsqrtf(fminf(c, dd)) * (1.f + fabsf(ss) + fabsf(tt));
+    const float tol = 1e-5f + 4e-5f * mag * rsqrtf(fminf(c, dd)) * (1.f + fabsf(ss) + fabsf(tt));
     if (!(ss > tol && ss < 1.f - tol && tt > tol && tt < 1.f - tol))
       return (ss < -tol || ss > 1.f + tol || tt < -tol || tt > 1.f + tol) ? kOutside : 0;
     d = (w + ss * Ei) - tt * Ej;
   }
   *dnf = sqrtf(dotf(d, d)) - rsum;
-  return *dnf > 2e-6f + 2e-6f * mag + 4e-7f * cmag ? kApart : 0;
+  return *dnf > 2e-6f + 2e-6f * mag ? kApart : 0;
 }
 
 // The full path of entry e (everything the FP32 proof did not settle);
@@ -523,12 +523,9 @@ __global__ void k_narrow_mixed_quick(Scene s) {
     if (bond < 0 && !s.record_geom && s.gvr) {
       const int i = s.ei[e], j = s.ej[e];
       const int4 G = s.egv_ok ? s.egv[e] : make_int4(-1, -1, -1, -1);
-      const float4 pi = s.posf[i], pj = s.posf[j];
-      const F3 dxij = f3(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z);
-      const float cmag = fmaxf(fmaxf(fabsf(pi.x), fabsf(pi.y)), fmaxf(fabsf(pi.z), fmaxf(fabsf(pj.x),
-                         fmaxf(fabsf(pj.y), fabsf(pj.z)))));
-      quick = apart_f32(s, type, i, j, tsub_isub(ts), tsub_jsub(ts), s.egv_ok != 0, G, dxij, pi.w + pj.w, cmag,
-                        &dnf);
+      const float4 pi = s.posf[2 * i], pj = s.posf[2 * j], li = s.posf[2 * i + 1], lj = s.posf[2 * j + 1];
+      const F3 dxij = f3((pi.x - pj.x) + (li.x - lj.x), (pi.y - pj.y) + (li.y - lj.y), (pi.z - pj.z) + (li.z - lj.z));
+      quick = apart_f32(s, type, i, j, tsub_isub(ts), tsub_jsub(ts), s.egv_ok != 0, G, dxij, pi.w + pj.w, &dnf);
     }
     if (quick == kApart) {  // dn > 0 proven: separated, history untouched
       const double dn_old = s.dn[e];
