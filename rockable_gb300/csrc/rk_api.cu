@@ -77,18 +77,22 @@ cudaError_t near_set_stale(Ctx& c) {
 }
 
 // Looked at when a list update or the end of a call reads the count of sets
-// made: in the mixed form, a step that makes its set costs about half as much
-// more than a step on the whole list as a step on a set that lasts costs less
-// (50 000 grains: 195, 165 and 100 us; 24 000: 110, 85 and 60 us), so when more
-// than half of the steps made theirs -- grains that use up their allowance in
-// a step or two, positions set by the host before every short call -- the next
-// kNearRest steps run on the whole list before sets are tried again (24 000
-// fast grains, calls of 10 steps: 109 -> 81 us a step, 4300: 59 -> 55 us).  The
-// FP64 form's whole list costs four times a set (950 and 230 us).
+// made: in the mixed form, a step that makes its set costs more than a step on
+// the whole list, about twice as much more as a step on a set that lasts costs
+// less (50 000 grains: 292, 161 and 103 us; 20 000: 140, 86 and 64 us; 8000: 78,
+// 63 and 49 us), so when more than a third of the steps made theirs -- grains
+// that use up their allowance in a step or two, positions set by the host
+// before every short call -- the next kNearRest steps run on the whole list
+// before sets are tried again (24 000 fast grains, calls of 10 steps: 109 ->
+// 81 us a step, 4300: 59 -> 55 us).  Not in the FP64 form, whose whole list
+// costs four times a set (950 and 230 us), nor with the learned skin, whose
+// policy prices sets and whole-list steps itself (24 000 fast grains: 215 us a
+// step, 227 to 248 with this rule on top).
 constexpr int64_t kNearLook = 8, kNearRest = 200;
 void near_review(Ctx& c, unsigned long long made) {
   if (c.near_steps < kNearLook) return;
-  if (c.form == RK_FORM_MIXED && 2 * (int64_t)(made - c.near_made) > c.near_steps) c.near_rest = kNearRest;
+  if (c.form == RK_FORM_MIXED && !c.skin.on && 3 * (int64_t)(made - c.near_made) > c.near_steps)
+    c.near_rest = kNearRest;
   c.near_made = made;
   c.near_steps = 0;
 }
@@ -776,7 +780,6 @@ static int skin_batch(Ctx& c, int64_t left, int64_t* done) {
   c.steps += ex;
   if (!near) k.whole_in_window += ex;
   if (near) c.near_steps += ex;
-  else c.near_rest = std::max<int64_t>(c.near_rest - ex, 0);
   *done = ex;
   c.more_steps_follow = ex < left;
   c.forces_stale = s.nheavy_lazy > 0;
@@ -1520,6 +1523,7 @@ int rk_set_skin(rk_ctx* x, const rk_skin_config* cfg) {
   k.partial_ms = 0.0;
   k.partial_in_window = 0;
   k.on = true;
+  c.near_rest = 0;
   skin_bind(c, true);
   s.near_geometric = cfg->exact_contacts ? 1 : 0;
   // start from a fresh list built with the initial skin
