@@ -29,10 +29,11 @@ Legs of one run (rank 0 prints one JSON line):
   e2e         : the same metric through the C ABI with host-owned state:
                 every bench step uploads the bodies' kinematics from pinned
                 host memory, runs rk_step(segment) and downloads the result;
-  roofline    : the headline form's dominant kernel (narrow phase or
-                resultants), algorithmic bytes over its event-timed launch
-                duration against the measured HBM copy bandwidth, with the
-                ncu DRAM traffic and FP64 rate from profiles/;
+  roofline    : the larger of the headline form's force phases (narrow phase
+                or resultants), algorithmic bytes of the active sub-contacts
+                or bodies over its event-timed duration against the measured
+                HBM copy bandwidth, with the ncu DRAM traffic and FP64 rate
+                from profiles/;
   cpu_baseline: the oracle (CPU restatement of the reference path, OpenMP on
                 the host's cores) on a bounded sample of the same segment;
   iso         : the 200k-grain isotropic compression (six servo walls at
@@ -145,7 +146,7 @@ def peaks():
 def profile_constants():
     """Per-unit figures of the headline kernels from the committed ncu
     summary: lines `bench: <key> = <value>` (DRAM bytes and FP64 operations
-    per entry / per body, with the capture they come from)."""
+    per active sub-contact / per body, with the capture they come from)."""
     out = {}
     try:
         for line in open(PROFILE):
@@ -430,24 +431,24 @@ def time_form(scene, label, a, dev, dist, ws, steps, warmup):
 
 
 def roofline(rec, scene, consts, fp64):
-    """The dominant kernel of a form (narrow phase or resultants, by device
-    time per DEM step): algorithmic bytes per launch (140 B per entry: 12 B key
-    + the history read and written; 352 B per body: 200 B of state read and
-    152 B written) over its event-timed launch duration, against the measured
-    HBM copy bandwidth; DRAM traffic and FP64 operations per unit from the
-    committed ncu summary."""
+    """The larger of a form's two force phases (narrow phase, resultants) in
+    the steps on the near set, which a call's steps are but for its last:
+    algorithmic bytes per launch (140 B per active sub-contact: 12 B key + the
+    history read and written; 352 B per body: 200 B of state read and 152 B
+    written) over the event-timed phase, against the measured HBM copy
+    bandwidth; DRAM traffic and FP64 operations per unit from the committed ncu
+    summary.  What a step spends on finding those sub-contacts (the near set's
+    update) is in phase_ms_per_dem_step beside it."""
     ph = rec["phases_ms_per_dem_step"]
     la = rec["phases_launches"]
     hbm, src = peaks()
     nb = len(scene["bodies"]["mass"])
     dom = "narrow_force" if ph["narrow_force"] >= ph["gather_accel"] else "gather_accel"
     if dom == "narrow_force":
-        unit_bytes, units, unit_name, key = 140.0, rec["entries"], "entries", "narrow"
+        unit_bytes, units, unit_name, key = 140.0, rec["active"], "active sub-contacts", "narrow"
     else:
         unit_bytes, units, unit_name, key = 352.0, nb, "bodies", "gather"
-    # the phase's kernels per DEM step (one launch of k_narrow_force; the
-    # resultant kernel plus, when a body has many entries, its block sums),
-    # event-timed in the profiled segment
+    # the phase's kernels per DEM step, event-timed in the profiled segment
     per_step_ms = ph[dom]
     launches_per_step = la[dom] / max(1, rec["profiled_steps"])
     achieved = unit_bytes * units / (per_step_ms / 1e3) / 1e9 if per_step_ms > 0 else None
@@ -456,11 +457,13 @@ def roofline(rec, scene, consts, fp64):
            "frac": (achieved / hbm) if achieved else None, "peak_source": src,
            "algorithmic_bytes_per_unit": unit_bytes, "units": int(units), "unit_name": unit_name,
            "ms_per_dem_step": per_step_ms, "launches_per_dem_step": launches_per_step,
-           "ms_per_launch": per_launch_ms, "phase_ms_per_dem_step": {k: ph[k] for k in ("narrow_force", "gather_accel")}}
+           "ms_per_launch": per_launch_ms,
+           "phase_ms_per_dem_step": {"near_set": ph["glob_vertices"], "narrow_force": ph["narrow_force"],
+                                     "gather_accel": ph["gather_accel"]}}
     tb = consts.get(key + "_dram_bytes_per_unit")
     out["traffic"] = tb * units if tb is not None else None
-    out["traffic_note"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum per %s of this kernel (%s) x this "
-                           "form's %s" % (unit_name[:-1], os.path.relpath(PROFILE, ROOT), unit_name)
+    out["traffic_note"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum per unit of this phase's kernels (%s) x "
+                           "this form's %s" % (os.path.relpath(PROFILE, ROOT), unit_name)
                            if tb is not None else "no ncu capture of this kernel on this workload")
     fl = consts.get(key + "_fp64_ops_per_unit")
     if fl is not None and per_step_ms > 0:

@@ -384,8 +384,8 @@ __global__ void k_drift_frames(Scene s) {
 // vertex offsets (world vertex - centre, the FP32 test's coordinates) of every
 // body, written coalesced by the block from FP32 copies of its bodies'
 // rotation matrices, and the centres as sums of two floats.  DRIFT: the step's
-// launch, which makes the drift as well, in one pass over the bodies: 25 us at
-// 50 000 grains in blocks of 128 (27 us in blocks of 256), 32 us in two passes.
+// launch, which makes the drift as well, in one pass over the bodies: 26 us at
+// 50 000 grains in blocks of 128 (2 us more in blocks of 256), 32 us in two passes.
 template <bool DRIFT, bool GUARD>
 __global__ void k_body_frames(Scene s) {
   if (GUARD ? batch_halted(s) : step_halted(s)) return;
