@@ -833,6 +833,7 @@ static bool guard_pipelined(const Ctx& c) {
   return s.ncontrols == 0 && s.servo_kind == 0 && s.nif == 0 && s.dynamic_nl == 0;
 }
 
+// near: the step does not count as one on the whole list in the policy's window.
 int skin_after_step(Ctx& c, bool near) {
   Skin& k = c.skin;
   Scene& s = c.s;
@@ -1740,7 +1741,7 @@ int rk_step(rk_ctx* x, int64_t nsteps, rk_step_report* rep) {
     }
     c.forces_stale = s.nheavy_lazy > 0;
     if (c.skin.on) {
-      if ((rc = skin_after_step(c, near))) return rc;
+      if ((rc = skin_after_step(c, near || tuning))) return rc;  // (tuning: whole lists that the next window will not have)
       c.steps++;
       continue;
     }
