@@ -123,8 +123,9 @@ __device__ __forceinline__ float seg_d2(N3 p, N3 a, N3 b) {
 // counting the rounding radii), from its FP32 vertices in coordinates relative
 // to body j's centre.  A vertex of body i is the sum of its offset and the
 // centres' difference, which cancel where the bodies touch: mag, which the
-// margins scale with, covers that difference besides the vertices.  With inside, also whether the projection or the closest
-// points lie inside their ranges by more than the rounding errors, so that
+// margins scale with, covers half that difference besides the vertices (the
+// sum errs by up to 6e-7 of it; the margins are 2e-6 of it and more).  With
+// inside, also whether the projection or the closest points lie inside their ranges by more than the rounding errors, so that
 // the narrow phase finds the same.
 __device__ __forceinline__ float near_distance(const Scene& s, int i, int j, uint32_t ts, int4 G, bool* inside) {
   const int type = tsub_type(ts);
@@ -140,7 +141,7 @@ __device__ __forceinline__ float near_distance(const Scene& s, int i, int j, uin
     const float4 u = s.uvf[k];
     return nrot(qj, n3(u.x, u.y, u.z));
   };
-  float D, mag = namax(dx);
+  float D, mag = 0.5f * namax(dx);
   if (type == 0) {
     const N3 a = I(G.x), b = J(G.y), d = a - b;
     mag = fmaxf(mag, fmaxf(namax(a), namax(b)));
